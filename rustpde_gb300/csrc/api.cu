@@ -487,8 +487,8 @@ void build_case(RbcCase* c, bool with_graph = true, char* state_region = nullptr
     h.ht_x = upload_fdma(A, {adi_factor(c->sp_t.hb0, ct[0])});
     std::vector<double> fwd, bwd;
     h.pois_y = upload_fdma(A, hholtz_rows(c->sp_p1.hb0, c->sp_p1.hb1, cp[0], cp[1], 0.0, true, nullptr, &fwd, &bwd, &err));
-    h.pois_fwd = A.upload(fwd);
-    h.pois_bwd = A.upload(bwd);
+    h.pois_fwd = A.upload(transposed(fwd, nx - 2));
+    h.pois_bwd = A.upload(transposed(bwd, nx - 2));
     if (p.precision == RBC_PREC_MIXED) {
       const int mxc = nx - 2;
       // the eigenbasis depends on the basis and the size only

@@ -433,18 +433,31 @@ static double cospi_frac(long jk, int N) {
 static std::vector<double> cheb_dense_forward_impl(int n);
 static std::vector<double> cheb_dense_backward_impl(int n);
 
-// The dense transform matrices depend on n only: computed once per size.
-static std::vector<double> cheb_dense_cached(int n, bool fwd) {
+// The split transform tables depend on n only: computed once per size (map
+// entries stay where they are, so the reference is valid for good).
+const ChebDense& cheb_dense(int n) {
   static std::mutex mu;
-  static std::map<std::pair<int, bool>, std::vector<double>> cache;
+  static std::map<int, ChebDense> cache;
   std::lock_guard<std::mutex> lk(mu);
-  auto key = std::make_pair(n, fwd);
-  auto it = cache.find(key);
-  if (it == cache.end()) it = cache.emplace(key, fwd ? cheb_dense_forward_impl(n) : cheb_dense_backward_impl(n)).first;
-  return it->second;
+  auto it = cache.find(n);
+  if (it != cache.end()) return it->second;
+  const std::vector<double> F = cheb_dense_forward_impl(n), B = cheb_dense_backward_impl(n);
+  const int half = n / 2, H = n - half, ne = H, no = half;
+  ChebDense t;
+  t.fwd.resize((size_t)H * ne + (size_t)no * no);
+  t.bwd.resize((size_t)n * H);
+  for (int j = 0; j < H; j++) {
+    for (int m = 0; m < ne; m++) {
+      t.fwd[(size_t)j * ne + m] = F[(size_t)(2 * m) * n + j];
+      t.bwd[(size_t)m * H + j] = B[(size_t)j * n + 2 * m];
+    }
+    for (int m = 0; m < no; m++) {
+      if (j < no) t.fwd[(size_t)H * ne + (size_t)j * no + m] = F[(size_t)(2 * m + 1) * n + j];
+      t.bwd[(size_t)ne * H + (size_t)m * H + j] = j < half ? B[(size_t)j * n + 2 * m + 1] : 0.0;
+    }
+  }
+  return cache.emplace(n, std::move(t)).first->second;
 }
-std::vector<double> cheb_dense_forward(int n) { return cheb_dense_cached(n, true); }
-std::vector<double> cheb_dense_backward(int n) { return cheb_dense_cached(n, false); }
 
 static std::vector<double> cheb_dense_forward_impl(int n) {
   int N = n - 1;

@@ -66,9 +66,12 @@ std::vector<double> matmul(int n, int k, int m, const std::vector<double>& A, co
 // Tables
 std::vector<double> twiddles(int L);  // interleaved (re, im) of exp(-2 pi i t / L), t < L
 // Dense Chebyshev transform matrices including the correction factors of
-// ortho.rs:235-312.  fwd: ortho = M phys; bwd: phys = M ortho.  Row-major n x n.
-std::vector<double> cheb_dense_forward(int n);
-std::vector<double> cheb_dense_backward(int n);
+// ortho.rs:235-312 (fwd: ortho = M phys; bwd: phys = M ortho), split by parity
+// in the layout of ChebXformDev.
+struct ChebDense {
+  std::vector<double> fwd, bwd;
+};
+const ChebDense& cheb_dense(int n);
 
 inline bool is_pow2(int v) { return v > 0 && (v & (v - 1)) == 0; }
 

@@ -129,8 +129,9 @@ ChebXformDev upload_cheb(Arena& a, int n, bool allow_fft) {
     d.tw = reinterpret_cast<const double2*>(a.upload(twiddles(d.L)));
   } else {
     d.L = 0;
-    d.fwd = a.upload(cheb_dense_forward(n));
-    d.bwd = a.upload(cheb_dense_backward(n));
+    const ChebDense& t = cheb_dense(n);
+    d.fwd = a.upload(t.fwd);
+    d.bwd = a.upload(t.bwd);
   }
   return d;
 }
@@ -342,6 +343,13 @@ std::vector<Band4> hholtz_rows(const HostBasis& bx, const HostBasis& by, double 
   return rows;
 }
 
+std::vector<double> transposed(const std::vector<double>& a, int n) {
+  std::vector<double> t((size_t)n * n);
+  for (int i = 0; i < n; i++)
+    for (int j = 0; j < n; j++) t[(size_t)j * n + i] = a[(size_t)i * n + j];
+  return t;
+}
+
 bool build_solver(Arena& a, const SpaceDev& s, int kind, const double c[2], SolverDev& out, std::string* err) {
   try {
     out = SolverDev();
@@ -365,8 +373,8 @@ bool build_solver(Arena& a, const SpaceDev& s, int kind, const double c[2], Solv
     out.rows = upload_fdma(a, rows);
     out.dense = !s.hb0.fourier();
     if (out.dense) {
-      out.fwd = a.upload(fwd);
-      out.bwd = a.upload(bwd);
+      out.fwd = a.upload(transposed(fwd, out.m0));
+      out.bwd = a.upload(transposed(bwd, out.m0));
     }
     return true;
   } catch (std::exception& e) {
@@ -406,109 +414,140 @@ struct PassDesc {
 };
 
 namespace dev {
+// One lane per CTA, or a pair of real lanes.  T and PAIR:
+//   double2, 0  complex lanes (either side may be real: imaginary part 0 / dropped)
+//   double,  0  real lanes
+//   double2, 1  two real lanes as the parts of one complex lane: every operation
+//               here but the Fourier ones is linear with real coefficients
+// FP64 issue bounds the pass, so a real lane run as a complex one with a zero
+// imaginary part cost twice its products.
+template <class T> __device__ __forceinline__ double first_part(T v);
+template <> __device__ __forceinline__ double first_part<double>(double v) { return v; }
+template <> __device__ __forceinline__ double first_part<double2>(double2 v) { return v.x; }
+
+template <class T, int PAIR>
+__device__ __forceinline__ T pass_load(const void* p, int cplx, long long off, long long off2, bool two) {
+  if constexpr (sizeof(T) == 8) return static_cast<const double*>(p)[off];
+  else if constexpr (PAIR) return c2(static_cast<const double*>(p)[off], two ? static_cast<const double*>(p)[off2] : 0.0);
+  else return cplx ? static_cast<const double2*>(p)[off] : c2(static_cast<const double*>(p)[off], 0.0);
+}
+
+template <class T, int PAIR>
 __global__ void __launch_bounds__(128) k_pass(const __grid_constant__ PassDesc d) {
-  const int lane = blockIdx.x;
+  const int lane = PAIR ? 2 * blockIdx.x : blockIdx.x;
+  const bool two = PAIR && lane + 1 < d.lanes;
   const int tid = threadIdx.x, nth = blockDim.x;
   extern __shared__ double2 sm[];
-  double2* A = sm;
-  double2* B = A + d.lmax;
-  double2* T = B + d.lmax;
-  double2* WA = T + d.lmax;
+  double2* WA = sm;
   double2* WB = WA + d.wl;
-  double* R = reinterpret_cast<double*>(WB + d.wl);
+  T* A = reinterpret_cast<T*>(WB + d.wl);
+  T* B = A + d.lmax;
+  T* Q = B + d.lmax;
   int len = d.in_len;
   for (int k = tid; k < len; k += nth) {
-    long long off = lane * d.in_ls + k * d.in_es;
-    A[k] = d.in_cplx ? static_cast<const double2*>(d.in)[off] : c2(static_cast<const double*>(d.in)[off], 0.0);
+    const long long off = lane * d.in_ls + k * d.in_es;
+    A[k] = pass_load<T, PAIR>(d.in, d.in_cplx, off, off + d.in_ls, two);
   }
   __syncthreads();
   for (int o = 0; o < d.nops; o++) {
     const PassOp op = d.ops[o];
     switch (op.code) {
       case P_TO_ORTHO:
-        to_ortho<double2>(d.basis, A, 0, B, 0, 1, tid, nth);
+        to_ortho<T>(d.basis, A, 0, B, 0, 1, tid, nth);
         len = d.basis.kind == 5 ? d.basis.m : d.basis.n;
-        { double2* t = A; A = B; B = t; }
+        { T* t = A; A = B; B = t; }
         break;
       case P_FROM_ORTHO:
-        from_ortho<double2>(d.basis, A, 0, B, 0, 1, tid, nth);
+        from_ortho<T>(d.basis, A, 0, B, 0, 1, tid, nth);
         len = d.basis.m;
-        { double2* t = A; A = B; B = t; }
+        { T* t = A; A = B; B = t; }
         break;
       case P_DIFF:
         if (op.arg > 0) {
-          cheb_diff<double2>(A, 0, B, 0, len, 1, op.arg, T, 0, tid, nth);
-          double2* t = A; A = B; B = t;
+          cheb_diff<T>(A, 0, B, 0, len, 1, op.arg, Q, 0, tid, nth);
+          T* t = A; A = B; B = t;
         }
-        break;
-      case P_FDIFF:
-        for (int k = tid; k < len; k += nth) {
-          double2 v = A[k];
-          for (int t = 0; t < op.arg; t++) v = mul_ik(v, (double)k);
-          A[k] = v;
-        }
-        __syncthreads();
         break;
       case P_DCT_FWD:
       case P_DCT_BWD: {
-        bool fwd = op.code == P_DCT_FWD;
-        if (d.cx.use_fft) dct1_fft_c(d.cx, fwd, A, 0, B, 0, 1, WA, WB, d.wl, tid, nth);
-        else dct1_dense<double2>(d.cx, fwd, A, 0, B, 0, 1, tid, nth);
-        double2* t = A; A = B; B = t;
+        const bool fwd = op.code == P_DCT_FWD;
+        if (!d.cx.use_fft) dct1_dense<T>(d.cx, fwd, A, 0, B, 0, 1, tid, nth);
+        else if constexpr (sizeof(T) == 16) dct1_fft_c(d.cx, fwd, A, 0, B, 0, 1, WA, WB, d.wl, tid, nth);
+        else dct1_fft_r(d.cx, fwd, A, 0, B, 0, 1, WA, WB, d.wl, tid, nth);
+        T* t = A; A = B; B = t;
         break;
       }
+      case P_FDIFF:
       case P_R2C:
-        for (int k = tid; k < len; k += nth) R[k] = A[k].x;
-        __syncthreads();
-        r2c(d.fx, R, 0, B, 0, 1, d.fx.n / 2 + 1, 1, WA, WB, d.wl, tid, nth);
-        len = d.fx.n / 2 + 1;
-        { double2* t = A; A = B; B = t; }
-        break;
       case P_C2R:
-        c2r(d.fx, A, 0, 1, R, 0, 1, WA, WB, d.wl, tid, nth);
-        len = d.fx.n;
-        for (int k = tid; k < len; k += nth) B[k] = c2(R[k], 0.0);
-        __syncthreads();
-        { double2* t = A; A = B; B = t; }
+        if constexpr (sizeof(T) == 16 && !PAIR) {  // Fourier axis: complex lanes only
+          if (op.code == P_FDIFF) {
+            for (int k = tid; k < len; k += nth) {
+              double2 v = A[k];
+              for (int t = 0; t < op.arg; t++) v = mul_ik(v, (double)k);
+              A[k] = v;
+            }
+            __syncthreads();
+            break;
+          }
+          double* R = reinterpret_cast<double*>(Q);
+          if (op.code == P_R2C) {
+            for (int k = tid; k < len; k += nth) R[k] = A[k].x;
+            __syncthreads();
+            r2c(d.fx, R, 0, B, 0, 1, d.fx.n / 2 + 1, 1, WA, WB, d.wl, tid, nth);
+            len = d.fx.n / 2 + 1;
+          } else {
+            c2r(d.fx, A, 0, 1, R, 0, 1, WA, WB, d.wl, tid, nth);
+            len = d.fx.n;
+            for (int k = tid; k < len; k += nth) B[k] = c2(R[k], 0.0);
+            __syncthreads();
+          }
+          T* t = A; A = B; B = t;
+        }
         break;
       case P_SCALE:
-        for (int k = tid; k < len; k += nth) A[k] = A[k] * d.scale;
+        for (int k = tid; k < len; k += nth) A[k] = scal(A[k], d.scale);
         __syncthreads();
         break;
       case P_MATVEC:
-        matvec_pinv<double2>(d.pinv, A, 0, B, 0, 1, tid, nth);
+        matvec_pinv<T>(d.pinv, A, 0, B, 0, 1, tid, nth);
         len = d.pinv.n - 2;
-        { double2* t = A; A = B; B = t; }
+        { T* t = A; A = B; B = t; }
         break;
       case P_FDMA:
-        fdma_solve<double2>(d.fdma, A, 0, 1, lane, 0, tid, nth);
+        fdma_solve<T>(d.fdma, A, 0, 1, lane, 0, tid, nth);
         break;
       case P_ADD:
         for (int k = tid; k < len; k += nth) {
-          long long off = lane * d.add_ls + k;
-          A[k] = A[k] + (d.in_cplx ? static_cast<const double2*>(d.add)[off] : c2(static_cast<const double*>(d.add)[off], 0.0));
+          const long long off = lane * d.add_ls + k;
+          A[k] = A[k] + pass_load<T, PAIR>(d.add, d.in_cplx, off, off + d.add_ls, two);
         }
         __syncthreads();
         break;
       case P_DENSE:
-        for (int r = tid; r < d.dense_rows; r += nth) {
-          const double* row = d.dense + (size_t)r * d.dense_cols;
-          double2 acc = c2(0.0, 0.0);
-          for (int k = 0; k < d.dense_cols; k++) acc = fmas(acc, A[k], __ldg(row + k));
-          B[r] = acc;
-        }
+        for (int r = tid; r < d.dense_rows; r += nth) B[r] = table_dot<T>(d.dense + r, d.dense_rows, d.dense_cols, A, 1);
         __syncthreads();
         len = d.dense_rows;
-        { double2* t = A; A = B; B = t; }
+        { T* t = A; A = B; B = t; }
         break;
       default:
         break;
     }
   }
   for (int k = tid; k < len; k += nth) {
-    long long off = lane * d.out_ls + k * d.out_es;
-    if (d.out_cplx) static_cast<double2*>(d.out)[off] = A[k];
-    else static_cast<double*>(d.out)[off] = A[k].x;
+    const long long off = lane * d.out_ls + k * d.out_es;
+    if constexpr (PAIR) {
+      static_cast<double*>(d.out)[off] = A[k].x;
+      if (two) static_cast<double*>(d.out)[off + d.out_ls] = A[k].y;
+    } else {
+      if constexpr (sizeof(T) == 16) {
+        if (d.out_cplx) {
+          static_cast<double2*>(d.out)[off] = A[k];
+          continue;
+        }
+      }
+      static_cast<double*>(d.out)[off] = first_part<T>(A[k]);
+    }
   }
 }
 
@@ -579,13 +618,29 @@ __global__ void k_sumsq(const double* v, size_t n, double* out) {
 }
 }  // namespace dev
 
+// shared memory of a pass: what sizes are checked against, and the part that
+// lanes of 8- or 16-byte elements use
 static size_t pass_smem(const PassDesc& d) {
   return (size_t)(3 * d.lmax + 2 * d.wl) * 16 + (size_t)d.lmax * 2 * 8 + 64;
 }
+static size_t pass_smem_used(const PassDesc& d, size_t elem) {
+  return (size_t)2 * d.wl * 16 + (size_t)3 * d.lmax * elem + 64;
+}
 
+// Real lanes run as pairs where the pairs still give every SM two CTAs and no
+// operation has factors per lane (a pair shares them), else one by one.
 static void run_pass(PassDesc& d, cudaStream_t st) {
-  size_t sm = pass_smem(d);
-  dev::k_pass<<<d.lanes, 128, sm, st>>>(d);
+  bool real = !d.in_cplx && !d.out_cplx, per_lane = false;
+  for (int k = 0; k < d.nops; k++) {
+    const int code = d.ops[k].code;
+    if (code == P_FDIFF || code == P_R2C || code == P_C2R) real = false;
+    if (code == P_FDMA && d.fdma.rows > 1) per_lane = true;
+  }
+  constexpr int kPairLanes = 2 * 2 * 152;
+  if (!real) dev::k_pass<double2, 0><<<d.lanes, 128, pass_smem_used(d, 16), st>>>(d);
+  else if (!per_lane && d.lanes >= kPairLanes)
+    dev::k_pass<double2, 1><<<(d.lanes + 1) / 2, 128, pass_smem_used(d, 16), st>>>(d);
+  else dev::k_pass<double, 0><<<d.lanes, 128, pass_smem_used(d, 8), st>>>(d);
   cuda_check(cudaGetLastError(), "pass kernel launch");
 }
 
@@ -994,7 +1049,10 @@ size_t smem_limit() {
 cudaError_t configure_prim_kernels() {
   static PerDeviceFlag done;
   if (done.test()) return cudaSuccess;
-  cudaError_t e = cudaFuncSetAttribute(dev::k_pass, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_limit());
+  const int big = (int)smem_limit();
+  cudaError_t e = cudaFuncSetAttribute(dev::k_pass<double2, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(dev::k_pass<double2, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(dev::k_pass<double, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
   if (e == cudaSuccess) done.set();
   return e;
 }

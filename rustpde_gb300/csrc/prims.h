@@ -99,6 +99,8 @@ std::vector<Band4> hholtz_rows(const HostBasis& bx, const HostBasis& by, double 
                                bool poisson, std::vector<double>* lam_out, std::vector<double>* fwd,
                                std::vector<double>* bwd, std::string* err);
 Band4 adi_factor(const HostBasis& b, double c);
+// n x n matrix, row-major -> column-major
+std::vector<double> transposed(const std::vector<double>& a, int n);
 
 // 2-D operations (enqueued on `st`; `tmp` must hold max(phys0,spec0,ortho0) x
 // max(phys1,spec1,ortho1) complex values).

@@ -59,8 +59,10 @@ struct ChebXformDev {
   int log2L;
   const double2* tw;  // exp(-2 pi i t / L), t < L
   double inv_nm1;     // 1 / (n - 1)
-  const double* fwd;  // dense n x n forward matrix (row = output)
-  const double* bwd;  // dense n x n backward matrix
+  // dense form, split by parity (H = ceil(n/2); ne = H even and no = n - H odd
+  // coefficients), neighbouring outputs adjacent in memory:
+  const double* fwd;  // [H][ne] F_{2m,j}, then [no][no] F_{2m+1,j} (j < H, j < no)
+  const double* bwd;  // [ne][H] B_{j,2m}, then [no][H] B_{j,2m+1}
 };
 
 // Fourier r2c/c2r along x of physical length n (any n >= 4).  Even n runs
@@ -105,8 +107,8 @@ struct CaseDev {
   FdmaDev hu_y, hu_x;    // box ADI velocity (y, x); periodic: hu_y per row
   FdmaDev ht_y, ht_x;    // box ADI temperature; periodic: per row
   FdmaDev pois_y;        // per-row factors of the pressure Poisson solve
-  const double* pois_fwd;  // box: (mxc x mxc) eigenbasis forward, row-major
-  const double* pois_bwd;  // box: eigenbasis backward
+  const double* pois_fwd;  // box: (mxc x mxc) eigenbasis forward, column-major (outputs adjacent)
+  const double* pois_bwd;  // box: eigenbasis backward, column-major
 
   // state (spectral): real (box) or double2 (periodic) elements
   void* ux;   // mxc x myc

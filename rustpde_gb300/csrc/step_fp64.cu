@@ -819,10 +819,7 @@ __global__ void __launch_bounds__(256) k_box_x3(const CaseDev* __restrict__ case
   // dense eigenbasis forward along x
   double* zf = static_cast<double*>(c.s[6]);
   for (int r = tid; r < mxc; r += nth) {
-    const double* row = c.pois_fwd + (size_t)r * mxc;
-    double acc = 0.0;
-    for (int k = 0; k < mxc; k++) acc = fma(__ldg(row + k), Z[k], acc);
-    zf[(size_t)r * ny + j] = acc;
+    zf[(size_t)r * ny + j] = table_dot<double>(c.pois_fwd + r, mxc, mxc, Z, 1);
   }
 }
 
@@ -893,9 +890,7 @@ __global__ void __launch_bounds__(256) k_box_x4(const CaseDev* __restrict__ case
     for (int k = tid; k < mxc; k += nth) W[k] = wv[(size_t)k * myc + j];
     __syncthreads();
     for (int r = tid; r < mxc; r += nth) {
-      const double* row = c.pois_bwd + (size_t)r * mxc;
-      double acc = 0.0;
-      for (int k = 0; k < mxc; k++) acc = fma(__ldg(row + k), W[k], acc);
+      double acc = table_dot<double>(c.pois_bwd + r, mxc, mxc, W, 1);
       if (j == 0 && r == 0) acc = 0.0;
       PV[r] = acc;
       p1[(size_t)r * myc + j] = acc;
