@@ -9,6 +9,7 @@
 #include <mutex>
 #include <stdexcept>
 #include <string>
+#include <tuple>
 #include <vector>
 
 #include "case_access.h"
@@ -20,6 +21,7 @@
 #include "solid_masks.h"
 #include "spectral_rbc.h"
 #include "step_fp64.h"
+#include "step_split.h"
 
 namespace rbc {
 
@@ -69,6 +71,7 @@ struct DevPlan {
   std::vector<GemmJobDev*> jobs;
   std::vector<int4*> tiles;
   std::vector<int> ntiles, max_nt;
+  std::vector<SplitJobDev*> sjobs;
   std::shared_ptr<Arena> own;
 };
 
@@ -79,7 +82,14 @@ static void upload_plan(Arena& A, const StepPlan& plan, DevPlan& dp) {
     GemmJobDev* j = nullptr;
     int4* t = nullptr;
     int nt = 0, mnt = 0;
-    if (L.kernel == K_GEMM) {
+    SplitJobDev* sj = nullptr;
+    if (L.kernel == K_SPLIT_GEMM) {
+      std::vector<int4> tiles;
+      split_tiles(L.sjobs, tiles);
+      sj = A.upload(L.sjobs);
+      t = A.upload(tiles);
+      nt = (int)tiles.size();
+    } else if (L.kernel == K_GEMM) {
       std::vector<int4> tiles;
       gemm_tiles(L.jobs, tiles);
       j = A.upload(L.jobs);
@@ -94,6 +104,7 @@ static void upload_plan(Arena& A, const StepPlan& plan, DevPlan& dp) {
     dp.tiles.push_back(t);
     dp.ntiles.push_back(nt);
     dp.max_nt.push_back(mnt);
+    dp.sjobs.push_back(sj);
   }
 }
 
@@ -111,6 +122,7 @@ static void upload_plan_owned(const StepPlan& plan, DevPlan& dp) {
 
 static cudaError_t launch_entry(const StepLaunch& L, const DevPlan& dp, size_t k, cudaStream_t st,
                                 const CaseDev* cases) {
+  if (L.kernel == K_SPLIT_GEMM) return launch_split_gemm(dp.sjobs[k], dp.tiles[k], dp.ntiles[k], st);
   if (L.kernel == K_GEMM)
     return launch_lane_gemm(dp.jobs[k], dp.tiles[k], dp.ntiles[k], dp.max_nt[k], st, L.gemm_ws != 0);
   return launch_step_kernel(L.kernel, (int)L.items.size(), L.smem, st, cases, dp.work[k]);
@@ -128,6 +140,7 @@ static StepPlan merge_plans(const std::vector<const StepPlan*>& plans, const std
     StepLaunch& L = P.launches[li];
     L.items.clear();
     L.jobs.clear();
+    L.sjobs.clear();
     for (size_t m = 0; m < plans.size(); m++) {
       const StepLaunch& S = plans[m]->launches.at(li);
       if (S.kernel != L.kernel) throw std::runtime_error("merge_plans: plans of different structure");
@@ -137,12 +150,17 @@ static StepPlan merge_plans(const std::vector<const StepPlan*>& plans, const std
         if (!gates.empty()) j.active = gates[m];
         L.jobs.push_back(j);
       }
+      for (SplitJobDev j : S.sjobs) {
+        if (!gates.empty()) j.active = gates[m];
+        L.sjobs.push_back(j);
+      }
     }
     // items that carry a cost (one-thread-per-lane kernels): most expensive
     // first, so the last CTAs to start are the cheapest
     if (!L.items.empty() && L.items[0].w > 0)
       std::stable_sort(L.items.begin(), L.items.end(), [](const int4& a, const int4& b) { return a.w > b.w; });
   }
+  drop_empty(P);
   return P;
 }
 
@@ -216,6 +234,34 @@ static const float* shared_op(const std::string& key, Make make) {
   g_shared_ops.emplace(std::make_pair(dev, key), p);
   return p;
 }
+// The split operator of a transform (step_split.h) on the current device,
+// shared like the mixed operators by every case of the size.
+static SplitOpDev shared_split_op(int kind, int n, int rows) {
+  static std::mutex mu;
+  static std::map<std::tuple<int, int, int, int>, SplitOpDev> cache;
+  int dev = 0;
+  cuda_check(cudaGetDevice(&dev), "cudaGetDevice");
+  std::lock_guard<std::mutex> lk(mu);
+  const auto key = std::make_tuple(dev, kind, n, rows);
+  auto it = cache.find(key);
+  if (it != cache.end()) return it->second;
+  SplitOpDev d{};
+  const SplitOp op = make_split_op(kind, n, rows, &d.wshift);
+  d.N = op.N;
+  const size_t n32 = (op.bytes.size() + 127) & ~size_t(127);
+  unsigned char* p = nullptr;
+  cuda_check(cudaMalloc(&p, n32 + op.bytes16.size()), "cudaMalloc shared operator");
+  cudaError_t e = cudaMemcpy(p, op.bytes.data(), op.bytes.size(), cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = cudaMemcpy(p + n32, op.bytes16.data(), op.bytes16.size(), cudaMemcpyHostToDevice);
+  if (e != cudaSuccess) {
+    cudaFree(p);
+    cuda_check(e, "upload shared operator");
+  }
+  d.w = p;
+  d.w16 = p + n32;
+  return cache.emplace(key, d).first->second;
+}
+
 static std::vector<float> pack_blocks(std::initializer_list<std::pair<const LMat*, long double>> blocks,
                                       int ntmax = 64) {
   int rows = 0, cols = -1;
@@ -454,7 +500,7 @@ void build_case(RbcCase* c, bool with_graph = true, char* state_region = nullptr
       size_t m = 0;
       for (const StepLaunch& L : build_step_plan(hs).launches)
         if (L.smem > m) { m = L.smem; *kernel = L.kernel; }
-      return m;
+      return m;  // (the transforms inside the passes: split is chosen below and needs less)
     };
     int kern = -1;
     for (int axis = per ? 1 : 0; axis < 2 && need_of(&kern) > smem_limit(); axis++) {
@@ -525,6 +571,42 @@ void build_case(RbcCase* c, bool with_graph = true, char* state_region = nullptr
   if (!per)
     for (int k = 0; k < 8; k++) h.s[k] = A.alloc((size_t)nx * ny * 8);
   h.mixed = p.precision == RBC_PREC_MIXED;
+  // FP64 transforms as split GEMMs; a batch's mixed case of butterfly sizes
+  // may run the FP64 plan too (the transform choice), in the same form
+  const bool fp64_plan = !h.mixed || (c->batch != nullptr && is_pow2(ny - 1) && (per || is_pow2(nx - 1)));
+  if (fp64_plan && split_step_size(h)) {
+    const int P = per ? 2 : 1;
+    int ky[2], kx[2];
+    split_terms(false, ny, ky);
+    split_terms(per, nx, kx);
+    // Chebyshev lanes of coefficients and of folded values have the same list lengths
+    auto lanes = [&](const int K[2]) { SplitLanesDev s{}; s.cE = split_chunks(K[0]); s.cO = split_chunks(K[1]); return s; };
+    h.spl_y1 = h.spl_cq = lanes(ky);
+    h.spl_x1 = h.spl_p = lanes(kx);
+    const int n_y1 = 6 * P * h.mxc, n_x1 = 8 * ny, n_p = 3 * ny, n_q = 3 * P * h.kx;
+    size_t db = 0;
+    int ml = 0;
+    for (auto& e : {std::make_pair(&h.spl_y1, n_y1), std::make_pair(&h.spl_x1, n_x1), std::make_pair(&h.spl_p, n_p),
+                    std::make_pair(&h.spl_cq, n_q)}) {
+      db = std::max(db, split_dig_bytes(e.second, e.first->cE, e.first->cO));
+      ml = std::max(ml, e.second);
+    }
+    unsigned char* dig = static_cast<unsigned char*>(A.alloc(db));
+    int* ex = static_cast<int*>(A.alloc((size_t)ml * 4));
+    for (SplitLanesDev* s : {&h.spl_y1, &h.spl_x1, &h.spl_p, &h.spl_cq}) { s->dig = dig; s->ex = ex; }
+    h.spl_yw = static_cast<double*>(A.alloc((size_t)n_y1 * ny * 8));
+    h.spl_ph = static_cast<double*>(A.alloc((size_t)n_x1 * nx * 8));
+    h.spl_q = static_cast<double*>(A.alloc((size_t)std::max(n_q, 1) * ny * 8));
+    if (!h.mixed) h.m_cv = A.alloc((size_t)3 * std::max(h.kx, 1) * h.ky * 16);
+    h.sop_yb = shared_split_op(SOP_CHEB_BWD, ny, 0);
+    h.sop_xb = shared_split_op(per ? SOP_C2R : SOP_CHEB_BWD, nx, 0);
+    for (int par = 0; par < 2; par++) {
+      h.sop_xf[par] = per ? shared_split_op(par ? SOP_R2C_IM : SOP_R2C_RE, nx, h.kx)
+                          : shared_split_op(par ? SOP_CHEB_FWD_O : SOP_CHEB_FWD_E, nx, h.kx);
+      h.sop_yf[par] = shared_split_op(par ? SOP_CHEB_FWD_O : SOP_CHEB_FWD_E, ny, h.ky);
+    }
+    h.split = 1;
+  }
   if (h.mixed) {
     for (int f = 0; f < 3; f++) h.m_y[f] = A.alloc((size_t)2 * ny * h.mx * 8);
     h.m_q = A.alloc((size_t)3 * ny * std::max(h.kx, 1) * 8);
@@ -610,9 +692,10 @@ void build_case(RbcCase* c, bool with_graph = true, char* state_region = nullptr
     for (int i = 0; i < nx; i++) { bc[2 * i] = 0.5; bc[2 * i + 1] = -0.5; }
     double* d_bc = c->phys[0];
     cuda_check(cudaMemcpyAsync(d_bc, bc.data(), bc.size() * 8, cudaMemcpyHostToDevice, st), "upload bc");
-    axis0_forward(c->sp_bc, d_bc, c->bc_vhat, 2, st);
-    space_backward(c->sp_bc, c->bc_vhat, c->bc_phys, c->tmp, st);
-    space_forward(c->sp_bc, c->bc_phys, c->bc_vhat, c->tmp, st);
+    const SpaceDev sbc = in_order_space(c->sp_bc), sfield = in_order_space(c->sp_field);
+    axis0_forward(sbc, d_bc, c->bc_vhat, 2, st);
+    space_backward(sbc, c->bc_vhat, c->bc_phys, c->tmp, st);
+    space_forward(sbc, c->bc_phys, c->bc_vhat, c->tmp, st);
     // derived constants of the step
     space_to_ortho(c->sp_bc, c->bc_vhat, bco, c->tmp, st);
     void* gxx = c->spec_tmp[0];
@@ -622,9 +705,9 @@ void build_case(RbcCase* c, bool with_graph = true, char* state_region = nullptr
     size_t nd = (size_t)h.mx * ny * (per ? 2 : 1);
     phys_combine(5, (const double*)gxx, (const double*)gyy, nullptr, p.dt, c->ka, (double*)bcd, nd, st);
     space_gradient(c->sp_bc, c->bc_vhat, gxx, 1, 0, c->scale, c->tmp, st);
-    space_backward(c->sp_field, gxx, bdx, c->tmp, st);
+    space_backward(sfield, gxx, bdx, c->tmp, st);
     space_gradient(c->sp_bc, c->bc_vhat, gxx, 0, 1, c->scale, c->tmp, st);
-    space_backward(c->sp_field, gxx, bdy, c->tmp, st);
+    space_backward(sfield, gxx, bdy, c->tmp, st);
     c->sync();
     if (h.mixed) {
       // FP32 copies of the boundary-field derivatives, transposed (ny x nx)
@@ -700,6 +783,7 @@ void capture_graph(RbcCase* c) {
   if (c->graph) cudaGraphDestroy(c->graph);
   c->gexec = nullptr;
   c->graph = nullptr;
+  drop_empty(c->plan);
   upload_plan_owned(c->plan, c->dp);
   cuda_check(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal), "begin capture");
   cudaError_t le = cudaSuccess;
@@ -746,7 +830,7 @@ namespace {
 void set_phys(RbcCase* c, int field, const std::vector<double>& v) {
   double* d = c->phys[0];
   cuda_check(cudaMemcpyAsync(d, v.data(), v.size() * 8, cudaMemcpyHostToDevice, c->stream), "upload");
-  space_forward(field_space(c, field), d, field_ptr(c, field), c->tmp, c->stream);
+  space_forward(in_order_space(field_space(c, field)), d, field_ptr(c, field), c->tmp, c->stream);
   c->sync();
 }
 
@@ -2573,7 +2657,7 @@ struct RbcServer {
 // case is built; the actual arena size replaces it afterwards).
 static size_t case_bytes_bound(const RbcParams& p) {
   const size_t n = (size_t)(p.nx + 2) * (size_t)(p.ny + 2);
-  size_t b = n * 8 * 160;                       // fields, scratch and tables
+  size_t b = n * 8 * 208;                       // fields, scratch and tables
   if (p.kind != RBC_PERIODIC) b += (size_t)p.nx * p.nx * 8 * 16;  // eigenbases and dense x operators
   if (p.precision == RBC_PREC_MIXED) b += ((size_t)p.nx * p.nx + (size_t)p.ny * p.ny) * 4 * 24;
   return b + (4u << 20);

@@ -459,6 +459,19 @@ const ChebDense& cheb_dense(int n) {
   return cache.emplace(n, std::move(t)).first->second;
 }
 
+ChebDense cheb_dense_full(int n) {
+  const std::vector<double> F = cheb_dense_forward_impl(n), B = cheb_dense_backward_impl(n);
+  ChebDense t;
+  t.fwd.resize((size_t)n * n);
+  t.bwd.resize((size_t)n * n);
+  for (int k = 0; k < n; k++)
+    for (int j = 0; j < n; j++) {
+      t.fwd[(size_t)j * n + k] = F[(size_t)k * n + j];
+      t.bwd[(size_t)j * n + k] = B[(size_t)k * n + j];
+    }
+  return t;
+}
+
 static std::vector<double> cheb_dense_forward_impl(int n) {
   int N = n - 1;
   std::vector<double> M((size_t)n * n);

@@ -72,6 +72,8 @@ struct ChebDense {
   std::vector<double> fwd, bwd;
 };
 const ChebDense& cheb_dense(int n);
+// the unsplit matrices, column-major (element of row k, column j at j n + k)
+ChebDense cheb_dense_full(int n);
 
 inline bool is_pow2(int v) { return v > 0 && (v & (v - 1)) == 0; }
 

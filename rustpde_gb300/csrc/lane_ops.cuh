@@ -638,6 +638,16 @@ static __device__ void dct1_dense(const ChebXformDev& cx, bool forward, T* in, i
                            int tid, int nth) {
   const int n = cx.n, N = n - 1, half = n >> 1, H = n - half;  // half pairs (j, N-j); H = half (+ the centre)
   const int ne = H, no = half;                                 // even and odd coefficients
+  if (cx.fwd_full != nullptr) {
+    const double* M = forward ? cx.fwd_full : cx.bwd_full;
+    const FastDiv dn(n);
+    for (int idx = tid; idx < nl * n; idx += nth) {
+      const int l = dn(idx), k = idx - l * n;
+      out[l * out_ld + k] = table_dot<T>(M + k, n, n, in + l * in_ld, 1);
+    }
+    __syncthreads();
+    return;
+  }
   if (forward) {
     const FastDiv dh(half);
     for (int idx = tid; idx < nl * half; idx += nth) {

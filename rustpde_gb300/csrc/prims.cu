@@ -234,6 +234,37 @@ void build_space(Arena& a, SpaceDev& s, int kind0, int n0, int kind1, int n1) {
                     std::to_string(smem_limit()));
 }
 
+// unsplit tables of length n on the current device, shared by every space
+static void full_tables(ChebXformDev& c) {
+  if (c.n == 0 || c.use_fft) return;
+  static std::mutex mu;
+  static std::map<std::pair<int, int>, std::pair<const double*, const double*>> cache;
+  std::lock_guard<std::mutex> lk(mu);
+  auto& e = cache[std::make_pair(current_device(), c.n)];
+  if (e.first == nullptr) {
+    const ChebDense t = cheb_dense_full(c.n);
+    const size_t b = t.fwd.size() * 8;
+    double* p = nullptr;
+    cuda_check(cudaMalloc(&p, 2 * b), "cudaMalloc transform tables");
+    cudaError_t r = cudaMemcpy(p, t.fwd.data(), b, cudaMemcpyHostToDevice);
+    if (r == cudaSuccess) r = cudaMemcpy(p + t.fwd.size(), t.bwd.data(), b, cudaMemcpyHostToDevice);
+    if (r != cudaSuccess) {
+      cudaFree(p);
+      cuda_check(r, "upload transform tables");
+    }
+    e = std::make_pair(p, p + t.fwd.size());
+  }
+  c.fwd_full = e.first;
+  c.bwd_full = e.second;
+}
+
+SpaceDev in_order_space(const SpaceDev& s) {
+  SpaceDev o = s;
+  if (!s.cplx) full_tables(o.c0);
+  full_tables(o.c1);
+  return o;
+}
+
 Band4 adi_factor(const HostBasis& b, double c) {
   // hholtz_adi.rs:44-63: Fdma::from_matrix(mat_a - mat_b * c)
   Band4 A, B;

@@ -6,6 +6,8 @@
 #pragma once
 #include <cstdint>
 
+#include "split_gemm.h"
+
 namespace rbc {
 
 // One basis along one axis (tables built by host_ops.cpp make_basis).
@@ -63,6 +65,10 @@ struct ChebXformDev {
   // coefficients), neighbouring outputs adjacent in memory:
   const double* fwd;  // [H][ne] F_{2m,j}, then [no][no] F_{2m+1,j} (j < H, j < no)
   const double* bwd;  // [ne][H] B_{j,2m}, then [no][H] B_{j,2m+1}
+  // unsplit matrices, column-major (or null): sums over all n terms in index
+  // order (prims.h in_order_space)
+  const double* fwd_full;
+  const double* bwd_full;
 };
 
 // Fourier r2c/c2r along x of physical length n (any n >= 4).  Even n runs
@@ -77,6 +83,14 @@ struct FourierXformDev {
   int rad[16];  // their radices: 4s, then 2, 3, 5, 7 and any larger prime factors
   const double2* tw;  // exp(-2 pi i t / n), t < n
   const float2* twf;  // the same table rounded to FP32 (mixed-precision form)
+};
+
+// A split operator on the device (split_gemm.h): packed digits, outputs, scale.
+struct SplitOpDev {
+  const unsigned char* w;
+  const unsigned char* w16;
+  int N;
+  int wshift;
 };
 
 enum CaseKind { KIND_BOX_ADIABATIC = 0, KIND_BOX_CONDUCTING = 1, KIND_PERIODIC = 2 };
@@ -163,6 +177,15 @@ struct CaseDev {
                   // real row padded to a multiple of 4 floats, a complex row as [re | im] parts of that length
   const float* m_bcx;  // FP32 d(fieldbc)/dx, transposed: ny x nx
   const float* m_bcy;  // FP32 d(fieldbc)/dy - m_bcg, transposed: ny x nx
+
+  // FP64 transforms as split GEMMs (step_split.cu; not with a solid mask)
+  int split;
+  int pad_s;
+  SplitLanesDev spl_y1, spl_x1, spl_p, spl_cq;  // digits of the four GEMMs' lanes (one buffer, used in turn)
+  double* spl_yw;  // G1: ny x (mxc x 6 [x 2 parts])
+  double* spl_ph;  // G2: nx x (ny x 8)
+  double* spl_q;   // G3: kx [x 2 parts] x (ny x 3); G4 writes m_cv
+  SplitOpDev sop_yb, sop_xb, sop_xf[2], sop_yf[2];
 };
 
 // Row length (floats) of the mixed form's FP32 state copy m_s32 and of the

@@ -15,6 +15,7 @@
 #include "per_device.h"
 #include "prims.h"
 #include "step_fp64.h"
+#include "step_split.h"
 
 #include <algorithm>
 
@@ -191,13 +192,18 @@ __device__ FdmaDev stage_fdma_row(const FdmaDev& f, int row, double* dst, int ti
   return r;
 }
 
-// PRE: the convection term arrives already transformed along y (m_cv, FP64,
-// from the mixed-precision form's tensor-core GEMM) instead of q.
-template <bool PRE>
+// CONV: where the convection term comes from
+//   CONV_Q      q, transformed along y here
+//   CONV_MIXED  m_cv, transformed (the mixed form's GEMM), without the linear
+//               boundary part (CaseDev::m_bclin)
+//   CONV_FULL   m_cv, transformed and complete (the split GEMMs)
+enum { CONV_Q = 0, CONV_MIXED = 1, CONV_FULL = 2 };
+template <int CONV>
 __global__ void __launch_bounds__(256) k_per_y2(const CaseDev* __restrict__ cases, const int4* __restrict__ work) {
   int4 w = work[blockIdx.x];
   const CaseDev& c = cases[w.x];
   if (c.gate != nullptr && c.gate[1] == 0) return;  // case idle this step (serving)
+  constexpr bool PRE = CONV != CONV_Q;
   const int i = w.y;
   const int ny = c.ny, myc = c.myc, kx = c.kx, ky = c.ky;
   const int ld = ny + 1;
@@ -272,7 +278,7 @@ __global__ void __launch_bounds__(256) k_per_y2(const CaseDev* __restrict__ case
   for (int k = tid; k < ny; k += nth) {
     double2 gx = mul_ik(P[k], ki) * inv_asp;
     double2 cu = CV[k], cvv = CV[ld + k], ct = CV[2 * ld + k];
-    if (PRE && c.m_bclin && i < kx && k < ky) ct = add_bclin(ct, O[ld + k], c.m_bcg, i);
+    if (CONV == CONV_MIXED && c.m_bclin && i < kx && k < ky) ct = add_bclin(ct, O[ld + k], c.m_bcg, i);
     R[k] = fnms(fnms(O[k], gx, dt), cu, dt);
     double2 that = O[2 * ld + k] + bco[(size_t)i * ny + k];
     R[ld + k] = fnms(fmas(fnms(O[ld + k], G[k], dt), that, dt), cvv, dt);
@@ -499,7 +505,7 @@ size_t smem_per_y2(const CaseDev& c) {
   size_t reg = std::max((size_t)14 * ld, (size_t)6 * wld);
   return (3 * ld + reg) * 16 + (size_t)12 * c.myc * 8 + 64;
 }
-// k_per_y2<true>: the rhs lanes reuse the convection lanes
+// with the convection term given: the rhs lanes reuse the convection lanes
 size_t smem_per_y2_pre(const CaseDev& c) {
   size_t ld = c.ny + 1;
   return (3 * ld + 11 * ld) * 16 + (size_t)12 * c.myc * 8 + 64;
@@ -611,12 +617,12 @@ size_t smem_box_x1(const CaseDev& c) {
 }
 
 // Y2: rows i < nx (ortho x).  conv (y forward, dealiased), rhs, pinv_y -> s[1..3]
-// PRE: the convection term arrives transformed (m_cv, from the tensor-core GEMMs).
-template <bool PRE>
+template <int CONV>
 __global__ void __launch_bounds__(256) k_box_y2(const CaseDev* __restrict__ cases, const int4* __restrict__ work) {
   int4 w = work[blockIdx.x];
   const CaseDev& c = cases[w.x];
   if (c.gate != nullptr && c.gate[1] == 0) return;  // case idle this step (serving)
+  constexpr bool PRE = CONV != CONV_Q;
   const int i = w.y;
   const int nx = c.nx, ny = c.ny, myc = c.myc, kx = c.kx, ky = c.ky, mxc = c.mxc;
   const int ld = ny + 1;
@@ -686,7 +692,7 @@ __global__ void __launch_bounds__(256) k_box_y2(const CaseDev* __restrict__ case
     double that = O[2 * ld + k] + bco[(size_t)i * ny + k];
     R[ld + k] = fnms(fmas(fnms(O[ld + k], G[k], dt), that, dt), CV[ld + k], dt);
     double ct = CV[2 * ld + k];
-    if (PRE && c.m_bclin && i < kx && k < ky) ct = add_bclin(ct, O[ld + k], c.m_bcg, i);
+    if (CONV == CONV_MIXED && c.m_bclin && i < kx && k < ky) ct = add_bclin(ct, O[ld + k], c.m_bcg, i);
     R[2 * ld + k] = fnms(O[2 * ld + k] + bcd[(size_t)i * ny + k], ct, dt);
   }
   __syncthreads();
@@ -993,13 +999,15 @@ cudaError_t configure_step_kernels() {
   SET_ATTR(dev::k_y1<double>);
   SET_ATTR(dev::k_y1<double2>);
   SET_ATTR(dev::k_per_x);
-  SET_ATTR(dev::k_per_y2<false>);
-  SET_ATTR(dev::k_per_y2<true>);
+  SET_ATTR(dev::k_per_y2<dev::CONV_Q>);
+  SET_ATTR(dev::k_per_y2<dev::CONV_FULL>);
+  SET_ATTR(dev::k_per_y2<dev::CONV_MIXED>);
   SET_ATTR(dev::k_per_y2a);
   SET_ATTR(dev::k_per_y2b);
   SET_ATTR(dev::k_box_x1);
-  SET_ATTR(dev::k_box_y2<false>);
-  SET_ATTR(dev::k_box_y2<true>);
+  SET_ATTR(dev::k_box_y2<dev::CONV_Q>);
+  SET_ATTR(dev::k_box_y2<dev::CONV_FULL>);
+  SET_ATTR(dev::k_box_y2<dev::CONV_MIXED>);
   SET_ATTR(dev::k_box_x2);
   SET_ATTR(dev::k_box_gpx);
   SET_ATTR(dev::k_box_y3);
@@ -1011,31 +1019,40 @@ cudaError_t configure_step_kernels() {
   SET_ATTR(dev::k_box_x4<true>);
   SET_ATTR(dev::k_box_y5);
 #undef SET_ATTR
+  e = configure_step_split_kernels();
+  if (e != cudaSuccess) return e;
   done.set();
   return cudaSuccess;
 }
 
 StepPlan build_step_plan(const CaseDev& c) {
   StepPlan p;
-  bool per = c.kind == KIND_PERIODIC;
-  auto add = [&](int kernel, int lanes, size_t smem) {
+  const bool per = c.kind == KIND_PERIODIC;
+  const bool split = c.split != 0 && c.solid_cm == nullptr;
+  auto add_if = [&](bool on, int kernel, int lanes, size_t smem) {
     StepLaunch L;
     L.kernel = kernel;
-    L.smem = clamp_smem(smem);
-    for (int i = 0; i < lanes; i++) L.items.push_back(make_int4(0, i, 1, 0));
+    L.smem = on ? clamp_smem(smem) : 0;
+    if (on)
+      for (int i = 0; i < lanes; i++) L.items.push_back(make_int4(0, i, 1, 0));
     p.launches.push_back(L);
   };
+  auto add = [&](int kernel, int lanes, size_t smem) { add_if(true, kernel, lanes, smem); };
   if (per) {
-    add(K_Y1_C, c.mxc, dev::smem_y1(c, 1, true));
-    add(K_PER_X, c.ny, dev::smem_per_x(c));
+    add_if(!split, K_Y1_C, c.mxc, dev::smem_y1(c, 1, true));
+    add_if(!split, K_PER_X, c.ny, dev::smem_per_x(c));
+    add_split_launches(c, split, p);
     // fused Y2 (one CTA per row): faster than the split Y2a/Y2b pair on this
     // GPU because each FP64 warp instruction costs its warp ~64 cycles and the
     // split leaves single-lane CTAs with long per-warp FP64 chains
-    add(K_PER_Y2, c.mx, dev::smem_per_y2(c));
+    add_if(!split, K_PER_Y2, c.mx, dev::smem_per_y2(c));
+    add_if(split, K_PER_Y2_CV, c.mx, dev::smem_per_y2_pre(c));
   } else {
-    add(K_Y1_R, c.mxc, dev::smem_y1(c, 1, false));
-    add(K_BOX_X1, c.ny, dev::smem_box_x1(c));
-    add(K_BOX_Y2, c.nx, dev::smem_box_y2(c));
+    add_if(!split, K_Y1_R, c.mxc, dev::smem_y1(c, 1, false));
+    add_if(!split, K_BOX_X1, c.ny, dev::smem_box_x1(c));
+    add_split_launches(c, split, p);
+    add_if(!split, K_BOX_Y2, c.nx, dev::smem_box_y2(c));
+    add_if(split, K_BOX_Y2_CV, c.nx, dev::smem_box_y2(c));
     add(K_BOX_X2, c.myc, dev::smem_box_x2(c));
     add(K_BOX_Y3, c.mxc, dev::smem_box_y3(c));
     add(K_BOX_X3, c.ny, dev::smem_box_x3(c));
@@ -1046,6 +1063,12 @@ StepPlan build_step_plan(const CaseDev& c) {
   return p;
 }
 
+void drop_empty(StepPlan& p) {
+  p.launches.erase(
+      std::remove_if(p.launches.begin(), p.launches.end(), [](const StepLaunch& L) { return L.empty(); }),
+      p.launches.end());
+}
+
 cudaError_t launch_step_kernel(int kernel, int nblocks, size_t smem, cudaStream_t s, const CaseDev* cases,
                                const int4* work) {
   dim3 g(nblocks), b(256);
@@ -1053,13 +1076,15 @@ cudaError_t launch_step_kernel(int kernel, int nblocks, size_t smem, cudaStream_
     case K_Y1_C: dev::k_y1<double2><<<g, b, smem, s>>>(cases, work); break;
     case K_Y1_R: dev::k_y1<double><<<g, b, smem, s>>>(cases, work); break;
     case K_PER_X: dev::k_per_x<<<g, b, smem, s>>>(cases, work); break;
-    case K_PER_Y2: dev::k_per_y2<false><<<g, b, smem, s>>>(cases, work); break;
-    case K_PER_Y2_PRE: dev::k_per_y2<true><<<g, b, smem, s>>>(cases, work); break;
+    case K_PER_Y2: dev::k_per_y2<dev::CONV_Q><<<g, b, smem, s>>>(cases, work); break;
+    case K_PER_Y2_PRE: dev::k_per_y2<dev::CONV_MIXED><<<g, b, smem, s>>>(cases, work); break;
     case K_PER_Y2A: dev::k_per_y2a<<<g, b, smem, s>>>(cases, work); break;
     case K_PER_Y2B: dev::k_per_y2b<<<g, b, smem, s>>>(cases, work); break;
     case K_BOX_X1: dev::k_box_x1<<<g, b, smem, s>>>(cases, work); break;
-    case K_BOX_Y2: dev::k_box_y2<false><<<g, b, smem, s>>>(cases, work); break;
-    case K_BOX_Y2_PRE: dev::k_box_y2<true><<<g, b, smem, s>>>(cases, work); break;
+    case K_BOX_Y2: dev::k_box_y2<dev::CONV_Q><<<g, b, smem, s>>>(cases, work); break;
+    case K_BOX_Y2_PRE: dev::k_box_y2<dev::CONV_MIXED><<<g, b, smem, s>>>(cases, work); break;
+    case K_PER_Y2_CV: dev::k_per_y2<dev::CONV_FULL><<<g, b, smem, s>>>(cases, work); break;
+    case K_BOX_Y2_CV: dev::k_box_y2<dev::CONV_FULL><<<g, b, smem, s>>>(cases, work); break;
     case K_BOX_X2: dev::k_box_x2<<<g, b, smem, s>>>(cases, work); break;
     case K_BOX_GPX: dev::k_box_gpx<<<g, b, smem, s>>>(cases, work); break;
     case K_BOX_Y3: dev::k_box_y3<<<g, b, smem, s>>>(cases, work); break;
@@ -1070,10 +1095,12 @@ cudaError_t launch_step_kernel(int kernel, int nblocks, size_t smem, cudaStream_
     case K_BOX_X4: dev::k_box_x4<false><<<g, b, smem, s>>>(cases, work); break;
     case K_BOX_X4_MIX: dev::k_box_x4<true><<<g, b, smem, s>>>(cases, work); break;
     case K_BOX_Y5: dev::k_box_y5<<<g, b, smem, s>>>(cases, work); break;
-    case K_PER_Y2_PRE_T128: dev::k_per_y2<true><<<g, dim3(128), smem, s>>>(cases, work); break;
-    case K_BOX_Y2_PRE_T128: dev::k_box_y2<true><<<g, dim3(128), smem, s>>>(cases, work); break;
+    case K_PER_Y2_PRE_T128: dev::k_per_y2<dev::CONV_MIXED><<<g, dim3(128), smem, s>>>(cases, work); break;
+    case K_BOX_Y2_PRE_T128: dev::k_box_y2<dev::CONV_MIXED><<<g, dim3(128), smem, s>>>(cases, work); break;
     case K_BOX_X3_MIX_T128: dev::k_box_x3<true><<<g, dim3(128), smem, s>>>(cases, work); break;
     case K_BOX_Y5_T128: dev::k_box_y5<<<g, dim3(128), smem, s>>>(cases, work); break;
+    case K_SPL_Y1_R: case K_SPL_Y1_C: case K_SPL_X1_BOX: case K_SPL_X1_PER: case K_SPL_PROD: case K_SPL_Q:
+      return launch_step_split_kernel(kernel, nblocks, smem, s, cases, work);
     default: return launch_mixed_kernel(kernel, nblocks, smem, s, cases, work);
   }
   return cudaGetLastError();

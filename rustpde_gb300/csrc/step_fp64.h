@@ -31,8 +31,13 @@ enum StepKernel {
   K_LP_PER_Y2F,
   // box Y4 of the mixed form (FP32 output for the eigenbasis GEMM)
   K_BOX_Y4_MIX,
+  // FP64 transforms as split GEMMs (step_split.cu)
+  K_SPL_Y1_R, K_SPL_Y1_C, K_SPL_X1_BOX, K_SPL_X1_PER, K_SPL_PROD, K_SPL_Q,
+  // Y2 with the convection term from the split GEMMs
+  K_PER_Y2_CV, K_BOX_Y2_CV,
   K_NUM_STEP_KERNELS,
-  K_GEMM = 100  // tensor-core lane GEMM (jobs instead of work items)
+  K_GEMM = 100,  // tensor-core lane GEMM (jobs instead of work items)
+  K_SPLIT_GEMM = 101  // split GEMM (sjobs instead of work items)
 };
 
 struct StepLaunch {
@@ -42,6 +47,8 @@ struct StepLaunch {
   size_t smem;
   std::vector<int4> items;       // (case index, first lane, lane count, 0)
   std::vector<GemmJobDev> jobs;  // K_GEMM only
+  std::vector<SplitJobDev> sjobs;  // K_SPLIT_GEMM only
+  bool empty() const { return items.empty() && jobs.empty() && sjobs.empty(); }
 };
 
 struct StepPlan {
@@ -49,7 +56,12 @@ struct StepPlan {
 };
 
 cudaError_t configure_step_kernels();
+// The launches of one update.  Every case of a kind gets the same sequence, so
+// that the plans of a group's cases can be merged: a launch of the form that a
+// case does not use (transforms inside the passes, or as split GEMMs) has no
+// work, and is dropped when no case of the group uses it (drop_empty).
 StepPlan build_step_plan(const CaseDev& c);
+void drop_empty(StepPlan& p);
 // largest dynamic shared memory of a launch of the mixed-precision plan (and its kernel)
 size_t mixed_plan_smem(const CaseDev& c, int* kernel);
 

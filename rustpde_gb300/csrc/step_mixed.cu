@@ -409,6 +409,12 @@ double launch_algorithmic_bytes(const StepLaunch& L, const CaseDev* cases) {
     return b;
   }
   double b = 0;
+  for (const SplitJobDev& j : L.sjobs) {
+    // lane digits, operator digits and outputs, once each
+    const double nc = j.nc[0] + j.nc[1];
+    b += j.lanes * nc * kSplitK * kSplitDigits * 2.0 + j.N * nc * kSplitDigits * 32.0 +
+         (double)j.lanes * (j.N + std::max(0, j.m_hi - j.m_lo)) * 8.0;
+  }
   for (const int4& it : L.items) {
     const CaseDev& c = cases[it.x];
     const double nx = c.nx, ny = c.ny, mx = c.mx, mxc = c.mxc, myc = c.myc, kx = c.kx, ky = c.ky;
@@ -429,10 +435,10 @@ double launch_algorithmic_bytes(const StepLaunch& L, const CaseDev* cases) {
       case K_LP_BOX_Y4: case K_BOX_Y4_MIX: kernel = K_BOX_Y4; break;
       case K_LP_BOX_Y5: kernel = K_BOX_Y5; break;
       case K_LP_PER_Y2: kernel = K_PER_Y2_PRE; break;
-      case K_PER_Y2_PRE_T128: kernel = K_PER_Y2_PRE; break;
+      case K_PER_Y2_PRE_T128: case K_PER_Y2_CV: kernel = K_PER_Y2_PRE; break;
       case K_LP_PER_Y2B: case K_LP_PER_Y2C: kernel = -1; break;  // counted with Y2A
       case K_PER_X_MIXED_T128: kernel = K_PER_X_MIXED; break;
-      case K_BOX_Y2_PRE_T128: kernel = K_BOX_Y2_PRE; break;
+      case K_BOX_Y2_PRE_T128: case K_BOX_Y2_CV: kernel = K_BOX_Y2_PRE; break;
       case K_BOX_X3_MIX_T128: kernel = K_BOX_X3_MIX; break;
       case K_BOX_Y5_T128: kernel = K_BOX_Y5; break;
       default: break;
@@ -462,6 +468,12 @@ double launch_algorithmic_bytes(const StepLaunch& L, const CaseDev* cases) {
       case K_BOX_Y5: v = 7 * myc * 8 + 3 * ny * 8; break;
       case K_BOX_PROD_MIXED: v = 13 * nx * 4; break;
       case K_BOX_GPX: v = 2 * nx * 8; break;
+      // rows or columns in, 14 bytes of digits per term out
+      case K_SPL_Y1_C: case K_SPL_Y1_R: v = 3 * myc * z + 6 * ny * (z / 8) * 14; break;
+      case K_SPL_X1_BOX: v = 6 * mxc * 8 + 2 * nx * 8 + 8 * nx * 14; break;
+      case K_SPL_X1_PER: v = 6 * mx * 16 + 8 * nx * 14; break;
+      case K_SPL_PROD: v = 8 * nx * 8 + 2 * nx * 8 + 3 * nx * 14; break;
+      case K_SPL_Q: v = 3 * ny * 8 + 3 * ny * 14; break;
       default: v = 0;
     }
     b += v * lanes;
@@ -484,8 +496,11 @@ const char* step_kernel_name(int kernel) {
                                 "lanes_box_y4", "lanes_box_y5", "lanes_periodic_y2", "periodic_y2_pre_t128",
                                 "box_y2_pre_t128", "box_x3_mix_t128", "box_y5_t128", "lanes_periodic_y2a",
                                 "lanes_periodic_y2b", "lanes_periodic_y2c", "state_f32", "periodic_x_mixed_t128",
-                                "lanes_periodic_y2_fused", "box_y4_mix"};
+                                "lanes_periodic_y2_fused", "box_y4_mix", "split_y1_real", "split_y1_complex",
+                                "split_x1_box", "split_x1_periodic", "split_products", "split_conv",
+                                "periodic_y2_cv", "box_y2_cv"};
   if (kernel == K_GEMM) return "lane_gemm";
+  if (kernel == K_SPLIT_GEMM) return "split_gemm";
   if (kernel >= 0 && kernel < K_NUM_STEP_KERNELS) return names[kernel];
   return "";
 }

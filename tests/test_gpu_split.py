@@ -1,0 +1,120 @@
+"""The FP64 step with its transforms as split GEMMs (digit products on the
+tensor cores): sizes at the edges of its tiles and of the rule that chooses it,
+against the transforms inside the passes, which the parity tests hold to the
+oracle; batches that mix the two forms; the solid mask that leaves it; its
+failure paths."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+TOL = 1e-10  # the FP64 step's bound (test_gpu_parity.py)
+
+
+@pytest.fixture(scope="module")
+def R():
+    from rustpde_gb300 import build
+    build.build()
+    import rustpde_gb300
+    return rustpde_gb300
+
+
+@pytest.fixture(scope="module")
+def O():
+    from oracle import oracle
+    oracle.build()
+    return oracle
+
+
+# (nx, ny, kind): list lengths of 47-64 terms and 16-divisible ones, last tiles
+# of 1, 16 and 17 outputs, odd and even lengths on either axis, one and several
+# lane blocks, the shortest axis with the longest, a prime Fourier length
+SIZES = [(96, 94, 0), (95, 129, 1), (98, 97, 0), (16, 600, 0), (600, 16, 1), (66, 142, 0),
+         (96, 96, 2), (101, 98, 2), (97, 95, 2), (16, 576, 2), (640, 20, 2), (128, 71, 2)]
+
+
+def _ic(c):
+    c.set_velocity(0.2, 1, 1)
+    c.set_temperature(0.2, 1, 2)
+
+
+@pytest.mark.parametrize("nx,ny,kind", SIZES)
+def test_step_matches_transforms_inside_the_passes(R, nx, ny, kind):
+    args = (nx, ny, 1e5, 0.7, 2e-3, 1.3, kind)
+    g, d = R.Navier2D(*args), R.Navier2D(*args)
+    _ic(g)
+    _ic(d)
+    d.solid = [np.zeros((nx, ny)), np.zeros((nx, ny))]  # damps nothing; its passes hold the transforms
+    g.update(3)
+    d.update(3)
+    for f in (R.TEMP, R.UX, R.UY, R.PRES, R.PSEUDO_PRES):
+        a, b = g.get(f), d.get(f)
+        err = np.linalg.norm(a - b) / np.linalg.norm(b)
+        assert err <= TOL, (f, err)
+    assert g.status() == 0 and d.status() == 0
+
+
+MIX = [(64, 64, 1e5, 1.0, 5e-3, 1.0, 0), (100, 95, 1e5, 1.0, 5e-3, 1.2, 0), (64, 33, 1e5, 0.7, 5e-3, 1.0, 2),
+       (130, 111, 1e5, 7.0, 5e-3, 1.5, 2), (129, 129, 1e5, 1.0, 5e-3, 1.0, 1)]
+
+
+def test_batch_of_both_forms_equals_single_cases(R):
+    b = R.Batch(MIX)
+    singles = [R.Navier2D(*p) for p in MIX]
+    for c, s in zip(b.cases, singles):
+        _ic(c)
+        _ic(s)
+        s.update(3)
+    b.update(3)
+    b.synchronize()
+    for c, s in zip(b.cases, singles):
+        for f in (R.TEMP, R.UX, R.UY, R.PRES, R.PSEUDO_PRES):
+            np.testing.assert_array_equal(c.get(f), s.get(f))
+
+
+@pytest.mark.parametrize("kind", [0, 2])
+def test_solid_mask_leaves_and_returns(R, O, kind):
+    args = (100, 96, 1e5, 1.0, 2e-3, 1.0, kind)
+    mask = np.zeros((100, 96))
+    mask[30:40, 20:50] = 1.0
+    g, o, plain = R.Navier2D(*args), O.Navier2D(*args), R.Navier2D(*args)
+    for c in (g, o, plain):
+        _ic(c)
+    g.solid = [mask, 0.1 * mask]
+    o.set_solid(mask, 0.1 * mask)
+    g.update(2)
+    o.update(2)
+    for f in (R.TEMP, R.UX, R.UY):
+        assert np.linalg.norm(g.get(f) - o.get(f)) <= TOL * np.linalg.norm(o.get(f)), f
+    g.solid = None
+    for f in (R.TEMP, R.UX, R.UY, R.PRES, R.PSEUDO_PRES):
+        plain.set(f, g.get(f))
+    g.update(2)
+    plain.update(2)
+    for f in (R.TEMP, R.UX, R.UY, R.PRES, R.PSEUDO_PRES):
+        np.testing.assert_array_equal(g.get(f), plain.get(f))
+
+
+@pytest.mark.parametrize("kind", [0, 2])
+def test_nonfinite_and_timeout_are_reported(R, kind):
+    args = (100, 96, 1e5, 1.0, 2e-3, 1.0, kind)
+    g = R.Navier2D(*args)
+    _ic(g)
+    t = g.get(R.TEMP)
+    t[3, 4] = np.inf
+    g.set(R.TEMP, t)
+    g.update(1)
+    assert g.status() & 1
+    h = R.Navier2D(*args)
+    _ic(h)
+    R.set_gemm_wait_limit(0)
+    try:
+        h.update(1)
+        h.synchronize()
+        assert h.status() & 2
+    finally:
+        R.set_gemm_wait_limit(-1)
+    k = R.Navier2D(*args)
+    _ic(k)
+    k.update(1)
+    assert k.status() == 0 and np.isfinite(k.get(R.TEMP)).all()
