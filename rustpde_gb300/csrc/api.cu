@@ -122,7 +122,9 @@ static void upload_plan_owned(const StepPlan& plan, DevPlan& dp) {
 
 static cudaError_t launch_entry(const StepLaunch& L, const DevPlan& dp, size_t k, cudaStream_t st,
                                 const CaseDev* cases) {
-  if (L.kernel == K_SPLIT_GEMM) return launch_split_gemm(dp.sjobs[k], dp.tiles[k], dp.ntiles[k], st);
+  if (L.kernel == K_SPLIT_GEMM)
+    return L.sjobs.empty() ? cudaSuccess
+                           : launch_split_gemm(dp.sjobs[k], dp.tiles[k], dp.ntiles[k], L.sjobs[0].digits, st);
   if (L.kernel == K_GEMM)
     return launch_lane_gemm(dp.jobs[k], dp.tiles[k], dp.ntiles[k], dp.max_nt[k], st, L.gemm_ws != 0);
   return launch_step_kernel(L.kernel, (int)L.items.size(), L.smem, st, cases, dp.work[k]);
@@ -259,6 +261,39 @@ static SplitOpDev shared_split_op(int kind, int n, int rows) {
   }
   d.w = p;
   d.w16 = p + n32;
+  return cache.emplace(key, d).first->second;
+}
+
+// The Poisson eigenbasis matrices of a basis and length in nine digits.
+static SplitMatDev shared_split_mat(int kind, int n, bool fwd) {
+  static std::mutex mu;
+  static std::map<std::tuple<int, int, int, bool>, SplitMatDev> cache;
+  int dev = 0;
+  cuda_check(cudaGetDevice(&dev), "cudaGetDevice");
+  std::lock_guard<std::mutex> lk(mu);
+  const auto key = std::make_tuple(dev, kind, n, fwd);
+  auto it = cache.find(key);
+  if (it != cache.end()) return it->second;
+  std::vector<double> F, B;
+  poisson_eigenbasis(make_basis(kind, n), F, B);
+  const SplitMat m = pack_split_mat(fwd ? F : B, n - 2);
+  const size_t nb = (m.bytes16.size() + 127) & ~size_t(127), ne = (size_t)m.N * 4;
+  unsigned char* p = nullptr;
+  cuda_check(cudaMalloc(&p, nb + 2 * ne), "cudaMalloc shared operator");
+  cudaError_t e = cudaMemcpy(p, m.bytes16.data(), m.bytes16.size(), cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = cudaMemcpy(p + nb, m.colex.data(), ne, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = cudaMemcpy(p + nb + ne, m.rowex.data(), ne, cudaMemcpyHostToDevice);
+  if (e != cudaSuccess) {
+    cudaFree(p);
+    cuda_check(e, "upload shared operator");
+  }
+  SplitMatDev d{};
+  d.w16 = p;
+  d.colex = reinterpret_cast<const int*>(p + nb);
+  d.rowex = reinterpret_cast<const int*>(p + nb + ne);
+  d.N = m.N;
+  d.K0 = m.K[0];
+  d.K1 = m.K[1];
   return cache.emplace(key, d).first->second;
 }
 
@@ -452,12 +487,17 @@ void build_case(RbcCase* c, bool with_graph = true, char* state_region = nullptr
   const int xk_t = per ? FOURIER : (p.kind == RBC_BOX_ADIABATIC ? CN : CD);
   const int xk_o = per ? FOURIER : CHEB;
   const int xk_p = per ? FOURIER : CN;
-  build_space(A, c->sp_u, xk_u, nx, CD, ny);
-  build_space(A, c->sp_t, xk_t, nx, CD, ny);
-  build_space(A, c->sp_p0, xk_o, nx, CHEB, ny);
-  build_space(A, c->sp_p1, xk_p, nx, CN, ny);
-  build_space(A, c->sp_field, xk_o, nx, CHEB, ny);
-  build_space(A, c->sp_bc, xk_o, nx, CDBC, ny);
+  // A batch's mixed case of butterfly sizes may run the FP64 plan (the transform
+  // choice) and has everything of an FP64 case; else the mixed form keeps its blocks.
+  const bool fp64_plan = p.precision != RBC_PREC_MIXED ||
+                         (c->batch != nullptr && is_pow2(ny - 1) && (per || is_pow2(nx - 1)));
+  const bool odd = fp64_plan;
+  build_space(A, c->sp_u, xk_u, nx, CD, ny, odd);
+  build_space(A, c->sp_t, xk_t, nx, CD, ny, odd);
+  build_space(A, c->sp_p0, xk_o, nx, CHEB, ny, odd);
+  build_space(A, c->sp_p1, xk_p, nx, CN, ny, odd);
+  build_space(A, c->sp_field, xk_o, nx, CHEB, ny, odd);
+  build_space(A, c->sp_bc, xk_o, nx, CDBC, ny, odd);
 
   CaseDev& h = c->hd;
   std::memset(&h, 0, sizeof h);
@@ -522,17 +562,17 @@ void build_case(RbcCase* c, bool with_graph = true, char* state_region = nullptr
   std::string err;
   if (per) {
     // Hholtz (FdmaTensor, Fourier-diagonal x) for ux, uy, temp; Poisson for pres[1]
-    h.hu_y = upload_fdma(A, hholtz_rows(c->sp_u.hb0, c->sp_u.hb1, cu[0], cu[1], 1.0, false, nullptr, nullptr, nullptr, &err));
-    h.ht_y = upload_fdma(A, hholtz_rows(c->sp_t.hb0, c->sp_t.hb1, ct[0], ct[1], 1.0, false, nullptr, nullptr, nullptr, &err));
-    h.pois_y = upload_fdma(A, hholtz_rows(c->sp_p1.hb0, c->sp_p1.hb1, cp[0], cp[1], 0.0, true, nullptr, nullptr, nullptr, &err));
+    h.hu_y = upload_fdma(A, hholtz_rows(c->sp_u.hb0, c->sp_u.hb1, cu[0], cu[1], 1.0, false, nullptr, nullptr, nullptr, &err), odd);
+    h.ht_y = upload_fdma(A, hholtz_rows(c->sp_t.hb0, c->sp_t.hb1, ct[0], ct[1], 1.0, false, nullptr, nullptr, nullptr, &err), odd);
+    h.pois_y = upload_fdma(A, hholtz_rows(c->sp_p1.hb0, c->sp_p1.hb1, cp[0], cp[1], 0.0, true, nullptr, nullptr, nullptr, &err), odd);
   } else {
     // HholtzAdi for ux, uy, temp; Poisson (eigen-decomposed x) for pres[1]
-    h.hu_y = upload_fdma(A, {adi_factor(c->sp_u.hb1, cu[1])});
-    h.hu_x = upload_fdma(A, {adi_factor(c->sp_u.hb0, cu[0])});
-    h.ht_y = upload_fdma(A, {adi_factor(c->sp_t.hb1, ct[1])});
-    h.ht_x = upload_fdma(A, {adi_factor(c->sp_t.hb0, ct[0])});
+    h.hu_y = upload_fdma(A, {adi_factor(c->sp_u.hb1, cu[1])}, odd);
+    h.hu_x = upload_fdma(A, {adi_factor(c->sp_u.hb0, cu[0])}, odd);
+    h.ht_y = upload_fdma(A, {adi_factor(c->sp_t.hb1, ct[1])}, odd);
+    h.ht_x = upload_fdma(A, {adi_factor(c->sp_t.hb0, ct[0])}, odd);
     std::vector<double> fwd, bwd;
-    h.pois_y = upload_fdma(A, hholtz_rows(c->sp_p1.hb0, c->sp_p1.hb1, cp[0], cp[1], 0.0, true, nullptr, &fwd, &bwd, &err));
+    h.pois_y = upload_fdma(A, hholtz_rows(c->sp_p1.hb0, c->sp_p1.hb1, cp[0], cp[1], 0.0, true, nullptr, &fwd, &bwd, &err), odd);
     h.pois_fwd = A.upload(transposed(fwd, nx - 2));
     h.pois_bwd = A.upload(transposed(bwd, nx - 2));
     if (p.precision == RBC_PREC_MIXED) {
@@ -571,9 +611,7 @@ void build_case(RbcCase* c, bool with_graph = true, char* state_region = nullptr
   if (!per)
     for (int k = 0; k < 8; k++) h.s[k] = A.alloc((size_t)nx * ny * 8);
   h.mixed = p.precision == RBC_PREC_MIXED;
-  // FP64 transforms as split GEMMs; a batch's mixed case of butterfly sizes
-  // may run the FP64 plan too (the transform choice), in the same form
-  const bool fp64_plan = !h.mixed || (c->batch != nullptr && is_pow2(ny - 1) && (per || is_pow2(nx - 1)));
+  h.odd = odd;
   if (fp64_plan && split_step_size(h)) {
     const int P = per ? 2 : 1;
     int ky[2], kx[2];
@@ -591,9 +629,18 @@ void build_case(RbcCase* c, bool with_graph = true, char* state_region = nullptr
       db = std::max(db, split_dig_bytes(e.second, e.first->cE, e.first->cO));
       ml = std::max(ml, e.second);
     }
+    if (split_eig_size(h)) {
+      h.split_eig = 1;
+      h.smat_f = shared_split_mat(c->sp_p1.hb0.kind, nx, true);
+      h.smat_b = shared_split_mat(c->sp_p1.hb0.kind, nx, false);
+      h.spl_z.cE = h.spl_w.cE = split_chunks(h.smat_f.K0);
+      h.spl_z.cO = h.spl_w.cO = split_chunks(h.smat_f.K1);
+      db = std::max(db, split_dig_bytes(ny, h.spl_z.cE, h.spl_z.cO, 9));
+      ml = std::max(ml, ny);
+    }
     unsigned char* dig = static_cast<unsigned char*>(A.alloc(db));
     int* ex = static_cast<int*>(A.alloc((size_t)ml * 4));
-    for (SplitLanesDev* s : {&h.spl_y1, &h.spl_x1, &h.spl_p, &h.spl_cq}) { s->dig = dig; s->ex = ex; }
+    for (SplitLanesDev* s : {&h.spl_y1, &h.spl_x1, &h.spl_p, &h.spl_cq, &h.spl_z, &h.spl_w}) { s->dig = dig; s->ex = ex; }
     h.spl_yw = static_cast<double*>(A.alloc((size_t)n_y1 * ny * 8));
     h.spl_ph = static_cast<double*>(A.alloc((size_t)n_x1 * nx * 8));
     h.spl_q = static_cast<double*>(A.alloc((size_t)std::max(n_q, 1) * ny * 8));

@@ -22,6 +22,7 @@
 // the stores, drains its MMA in flight (again bounded), frees its tensor memory
 // and returns.
 #include "lane_gemm.h"
+#include "pdl.cuh"
 #include "per_device.h"
 #include "split_gemm.h"
 #include "tc_ptx.cuh"
@@ -737,6 +738,7 @@ __device__ __forceinline__ void gemm_tile(const GemmJobDev& J, const int lane0, 
 // grouped form: tile table entries (job, first lane, output tile, 0)
 __global__ void __launch_bounds__(kGemmThreads, 2) k_lane_gemm(const GemmJobDev* __restrict__ jobs,
                                                                 const int4* __restrict__ tiles) {
+  pdl_enter();
   const int4 tl = tiles[blockIdx.x];
   gemm_tile(jobs[tl.x], tl.y, tl.z);
 }
@@ -744,6 +746,7 @@ __global__ void __launch_bounds__(kGemmThreads, 2) k_lane_gemm(const GemmJobDev*
 // the same tiles in the warp-specialised form (output tiles of at most 64 columns)
 __global__ void __launch_bounds__(kGemmThreads, 2) k_lane_gemm_ws(const GemmJobDev* __restrict__ jobs,
                                                                    const int4* __restrict__ tiles) {
+  pdl_enter();
   const int4 tl = tiles[blockIdx.x];
   const GemmJobDev& J = jobs[tl.x];
   if (J.active != nullptr && *J.active == 0) return;
@@ -753,6 +756,7 @@ __global__ void __launch_bounds__(kGemmThreads, 2) k_lane_gemm_ws(const GemmJobD
 
 // single job passed by value: block b -> lanes (b / ntiles) * 128, output tile b % ntiles
 __global__ void __launch_bounds__(kGemmThreads, 2) k_lane_gemm_one(const __grid_constant__ GemmJobDev J) {
+  pdl_enter();
   const int b = blockIdx.x;
   gemm_tile(J, (b / J.ntiles) * kGemmLanes, b % J.ntiles);
 }
@@ -928,9 +932,9 @@ cudaError_t launch_lane_gemm(const GemmJobDev* jobs, const int4* tiles, int ntil
   if (ntiles_total <= 0) return cudaSuccess;
   if (ws) {
     if (max_nt > 64) return cudaErrorInvalidValue;
-    dev::k_lane_gemm_ws<<<ntiles_total, kGemmThreads, gemm_ws_smem_bytes(max_nt), st>>>(jobs, tiles);
+    return launch_pdl(dev::k_lane_gemm_ws, ntiles_total, kGemmThreads, gemm_ws_smem_bytes(max_nt), st, jobs, tiles);
   } else {
-    dev::k_lane_gemm<<<ntiles_total, kGemmThreads, gemm_smem_bytes(max_nt), st>>>(jobs, tiles);
+    return launch_pdl(dev::k_lane_gemm, ntiles_total, kGemmThreads, gemm_smem_bytes(max_nt), st, jobs, tiles);
   }
   return cudaGetLastError();
 }

@@ -140,39 +140,42 @@ static __device__ void from_ortho(const BasisDev& b, const T* in, int in_ld, T* 
   __syncthreads();
   // forward g_i = (d_i - a_{i-2} g_{i-2}) / den_i, then x_j = g_j - w_j x_{j+2},
   // one group of threads per (lane, parity) chain
-  const double* __restrict__ off = b.fo_off;
   const double* __restrict__ dinv = b.fo_dinv;
+  const double* __restrict__ fc = b.fo_c;
   const double* __restrict__ w = b.fo_w;
+  const double* __restrict__ scan = b.fo_scan;
   auto len_of = [&](int c) { return (m - (c & 1) + 1) >> 1; };
-  chains1<16, T>(
-      2 * nl, len_of,
-      [&](int c, int t, double& a, T& v) {
-        int i = (c & 1) + 2 * t;
-        T d = out[(c >> 1) * out_ld + i];
-        double q = dinv[i];
-        a = t ? -off[i - 2] * q : 0.0;
-        v = scal(d, q);
+  chains1<T>(
+      b.odd, 2 * nl, len_of,
+      [&](int c, int t, double& a, T& v, bool first) {
+        const int i = (c & 1) + 2 * t;
+        T& d = out[(c >> 1) * out_ld + i];
+        if (first) d = scal(d, dinv[i]);  // scaled in place, by the thread that reads it back
+        v = d;
+        a = t ? fc[i] : 0.0;
       },
+      [&](int c, int gl, int r) { return __ldg(scan + r * 32 + (c & 1) * 16 + gl); },
       [&](int c, int t, T x) { out[(c >> 1) * out_ld + (c & 1) + 2 * t] = x; }, tid, nth);
   __syncthreads();
   auto top_of = [&](int c) { int par = c & 1; return ((m - 1 - par) & 1) ? m - 2 : m - 1; };
-  chains1<16, T>(
-      2 * nl, len_of,
-      [&](int c, int t, double& a, T& v) {
-        int j = top_of(c) - 2 * t;
+  chains1<T>(
+      b.odd, 2 * nl, len_of,
+      [&](int c, int t, double& a, T& v, bool) {
+        const int j = top_of(c) - 2 * t;
         v = out[(c >> 1) * out_ld + j];
         a = t ? -w[j] : 0.0;
       },
+      [&](int c, int gl, int r) { return __ldg(scan + (4 + r) * 32 + (c & 1) * 16 + gl); },
       [&](int c, int t, T x) { out[(c >> 1) * out_ld + top_of(c) - 2 * t] = x; }, tid, nth);
   __syncthreads();
 }
 
 // ------------------------------------------------------------------ derivatives
 // Chebyshev derivative of order `times` (1 or 2) of ortho lanes: out = D^times in
-// (in and out may alias only if times == 0).
+// (in and out may alias only if times == 0).  odd: the blocks of the running sums (scan_block).
 template <class T>
-static __device__ void cheb_diff(const T* in, int in_ld, T* out, int out_ld, int n, int nl, int times, T* tmp, int tmp_ld,
-                          int tid, int nth) {
+static __device__ void cheb_diff(int odd, const T* in, int in_ld, T* out, int out_ld, int n, int nl, int times, T* tmp,
+                                 int tmp_ld, int tid, int nth) {
   if (times == 0) {
     if (in != out)
       for (int idx = tid; idx < nl * n; idx += nth) {
@@ -208,12 +211,8 @@ static __device__ void cheb_diff(const T* in, int in_ld, T* out, int out_ld, int
         int par = c & 1, st = top2(c), lo = par ? 1 : 2;
         return st >= lo ? (st - lo) / 2 + 1 : 1;
       };
-      chains1<16, T>(
-          2 * nl, len_of,
-          [&](int c, int t, double& a, T& v) {
-            v = dd[(c >> 1) * dl + top2(c) - 2 * t];
-            a = t ? 1.0 : 0.0;
-          },
+      chains_sum<T>(
+          odd, 2 * nl, len_of, [&](int c, int t) { return dd[(c >> 1) * dl + top2(c) - 2 * t]; },
           [&](int c, int t, T x) { dd[(c >> 1) * dl + top2(c) - 2 * t] = x; }, tid, nth);
       __syncthreads();
       for (int l = tid; l < nl; l += nth) dd[l * dl] = fmas(dd[l * dl], dd[l * dl + 2], 0.5);
@@ -249,33 +248,45 @@ template <class T>
 __device__ void fdma_solve2(const FdmaDev& f0, const FdmaDev& f1, int split, T* x, int ld, int nl, int row0,
                             int lane_step, int tid, int nth) {
   const int m = f0.m;
-  auto fac = [&](int l) -> const FdmaDev& { return l < split ? f0 : f1; };
+  // the factor arrays of lane l (the two sets' pointers stay in registers)
   auto offs = [&](int l) -> size_t {
-    const FdmaDev& f = fac(l);
-    return (f.rows > 1) ? (size_t)(row0 + l * lane_step) * f.stride : 0;
+    const int rows = l < split ? f0.rows : f1.rows, stride = l < split ? f0.stride : f1.stride;
+    return rows > 1 ? (size_t)(row0 + l * lane_step) * stride : 0;
   };
+  auto low_of = [&](int l) { return (l < split ? f0.low : f1.low) + offs(l); };
+  auto dinv_of = [&](int l) { return (l < split ? f0.dinv : f1.dinv) + offs(l); };
+  auto up1_of = [&](int l) { return (l < split ? f0.up1 : f1.up1) + offs(l); };
+  auto up2_of = [&](int l) { return (l < split ? f0.up2 : f1.up2) + offs(l); };
   auto len_of = [&](int c) { return (m - (c & 1) + 1) >> 1; };
+  auto scan_of = [&](int l) {
+    const int rows = l < split ? f0.rows : f1.rows;
+    return (l < split ? f0.scan : f1.scan) + (rows > 1 ? (size_t)(row0 + l * lane_step) * kFdmaScan : 0);
+  };
   // forward elimination x_i -= low_{i-2} x_{i-2}
-  chains1<16, T>(
-      2 * nl, len_of,
-      [&](int c, int t, double& a, T& v) {
+  chains1<T>(
+      f0.odd, 2 * nl, len_of,
+      [&](int c, int t, double& a, T& v, bool) {
         int l = c >> 1, i = (c & 1) + 2 * t;
         v = x[l * ld + i];
-        a = t ? fac(l).low[offs(l) + i - 2] : 0.0;
+        a = t ? low_of(l)[i - 2] : 0.0;
       },
+      [&](int c, int gl, int r) { return __ldg(scan_of(c >> 1) + r * 32 + (c & 1) * 16 + gl); },
       [&](int c, int t, T v) { x[(c >> 1) * ld + (c & 1) + 2 * t] = v; }, tid, nth);
   __syncthreads();
   // back substitution x_j = (x_j - up1_j x_{j+2} - up2_j x_{j+4}) / dia_j
   auto top_of = [&](int c) { int par = c & 1; return ((m - 1 - par) & 1) ? m - 2 : m - 1; };
-  chains2<16, T>(
-      2 * nl, len_of,
-      [&](int c, int t, double& a, double& cc, T& v) {
+  chains2<T>(
+      f0.odd, 2 * nl, len_of,
+      [&](int c, int t, double& a, double& cc, T& v, bool first) {
         int l = c >> 1, j = top_of(c) - 2 * t;
-        const FdmaDev& f = fac(l);
-        size_t o = offs(l);
-        v = scal(x[l * ld + j], f.dinv[o + j]);
-        a = t ? f.up1[o + j] : 0.0;
-        cc = t >= 2 ? f.up2[o + j] : 0.0;
+        T& e = x[l * ld + j];
+        if (first) e = scal(e, dinv_of(l)[j]);  // scaled in place, by the thread that reads it back
+        v = e;
+        a = t ? up1_of(l)[j] : 0.0;
+        cc = t >= 2 ? up2_of(l)[j] : 0.0;
+      },
+      [&](int c, int gl, int r, int e) {
+        return __ldg(scan_of(c >> 1) + (4 + 4 * r + e) * 32 + (c & 1) * 16 + gl);
       },
       [&](int c, int t, T v) { x[(c >> 1) * ld + top_of(c) - 2 * t] = v; }, tid, nth);
   __syncthreads();

@@ -81,9 +81,38 @@ void cuda_check(cudaError_t e, const char* what) {
 }
 
 // ---------------------------------------------------------------- uploads
-BasisDev upload_basis(Arena& a, const HostBasis& b) {
+namespace dev {
+// composed sweep coefficients (chain_scan.cuh) of a basis's from_ortho and of
+// one row of banded factors per block: threads 0-15 even, 16-31 odd chain
+__global__ void k_scan_fo(const BasisDev b, double* out) {
+  const int q = threadIdx.x >> 4, gl = threadIdx.x & 15, m = b.m, len = (m - q + 1) >> 1;
+  const int top = ((m - 1 - q) & 1) ? m - 2 : m - 1;
+  scan_tables1(b.odd, len, gl, [&](int t) { return t ? b.fo_c[q + 2 * t] : 0.0; },
+               [&](int r, double v) { out[r * 32 + threadIdx.x] = v; });
+  scan_tables1(b.odd, len, gl, [&](int t) { return t ? -b.fo_w[top - 2 * t] : 0.0; },
+               [&](int r, double v) { out[(4 + r) * 32 + threadIdx.x] = v; });
+}
+__global__ void k_scan_fdma(const FdmaDev f, double* out_all) {
+  const int q = threadIdx.x >> 4, gl = threadIdx.x & 15, m = f.m, len = (m - q + 1) >> 1;
+  const int top = ((m - 1 - q) & 1) ? m - 2 : m - 1;
+  const size_t o = (size_t)blockIdx.x * f.stride;
+  double* out = out_all + (size_t)blockIdx.x * kFdmaScan;
+  scan_tables1(f.odd, len, gl, [&](int t) { return t ? f.low[o + q + 2 * t - 2] : 0.0; },
+               [&](int r, double v) { out[r * 32 + threadIdx.x] = v; });
+  scan_tables2(
+      f.odd, len, gl,
+      [&](int t, double& a, double& cc) {
+        a = t ? f.up1[o + top - 2 * t] : 0.0;
+        cc = t >= 2 ? f.up2[o + top - 2 * t] : 0.0;
+      },
+      [&](int r, int e, double v) { out[(4 + 4 * r + e) * 32 + threadIdx.x] = v; });
+}
+}  // namespace dev
+
+BasisDev upload_basis(Arena& a, const HostBasis& b, bool odd) {
   BasisDev d;
   std::memset(&d, 0, sizeof d);
+  d.odd = odd;
   d.kind = b.kind;
   d.n = b.n;
   d.m = b.m;
@@ -104,6 +133,11 @@ BasisDev upload_basis(Arena& a, const HostBasis& b) {
     d.fo_a = a.upload(fa);
     d.fo_b = a.upload(fb);
     d.fo_c = a.upload(fc);
+    double* sc = static_cast<double*>(a.alloc(8 * 32 * 8));
+    dev::k_scan_fo<<<1, 32>>>(d, sc);
+    cuda_check(cudaGetLastError(), "scan tables");
+    cuda_check(cudaStreamSynchronize(cudaStreamLegacy), "scan tables");
+    d.fo_scan = sc;
   }
   for (int i = 0; i < 2; i++) { d.t0[i] = b.t0[i]; d.t1[i] = b.t1[i]; }
   for (int i = 0; i < 4; i++) d.bc_inv[i] = b.bc_inv[i];
@@ -179,9 +213,10 @@ PinvDev upload_pinv(Arena& a, int n) {
   return d;
 }
 
-FdmaDev upload_fdma(Arena& a, const std::vector<Band4>& rows) {
+FdmaDev upload_fdma(Arena& a, const std::vector<Band4>& rows, bool odd) {
   FdmaDev d;
   std::memset(&d, 0, sizeof d);
+  d.odd = odd;
   int m = rows[0].n;
   int R = (int)rows.size();
   d.m = m;
@@ -202,17 +237,23 @@ FdmaDev upload_fdma(Arena& a, const std::vector<Band4>& rows) {
   d.dinv = a.upload(dinv);
   d.up1 = a.upload(up1);
   d.up2 = a.upload(up2);
+  double* sc = static_cast<double*>(a.alloc((size_t)R * kFdmaScan * 8));
+  dev::k_scan_fdma<<<R, 32>>>(d, sc);
+  cuda_check(cudaGetLastError(), "scan tables");
+  cuda_check(cudaStreamSynchronize(cudaStreamLegacy), "scan tables");
+  d.scan = sc;
   return d;
 }
 
 static size_t space_pass_smem(const SpaceDev& s);
 
-void build_space(Arena& a, SpaceDev& s, int kind0, int n0, int kind1, int n1) {
+void build_space(Arena& a, SpaceDev& s, int kind0, int n0, int kind1, int n1, bool odd) {
+  s.odd = odd;
   if (kind1 == FOURIER) throw std::runtime_error("FourierR2c is supported along axis 0 only");
   s.hb0 = make_basis(kind0, n0);
   s.hb1 = make_basis(kind1, n1);
-  s.b0 = upload_basis(a, s.hb0);
-  s.b1 = upload_basis(a, s.hb1);
+  s.b0 = upload_basis(a, s.hb0, odd);
+  s.b1 = upload_basis(a, s.hb1, odd);
   s.cplx = kind0 == FOURIER;
   if (s.cplx) s.f0 = upload_fourier(a, n0);
   else s.c0 = upload_cheb(a, n0);
@@ -374,6 +415,12 @@ std::vector<Band4> hholtz_rows(const HostBasis& bx, const HostBasis& by, double 
   return rows;
 }
 
+void poisson_eigenbasis(const HostBasis& b, std::vector<double>& fwd, std::vector<double>& bwd) {
+  std::string err;
+  // (the y basis enters the row factors only)
+  hholtz_rows(b, b, 1.0, 1.0, 0.0, true, nullptr, &fwd, &bwd, &err);
+}
+
 std::vector<double> transposed(const std::vector<double>& a, int n) {
   std::vector<double> t((size_t)n * n);
   for (int i = 0; i < n; i++)
@@ -442,6 +489,7 @@ struct PassDesc {
   int lmax, wl;
   const void* add;  // P_ADD: A[k] += add[lane*add_ls + k] (complex when in_cplx)
   long long add_ls;
+  int odd;          // blocks of the derivative's running sums (scan_block)
 };
 
 namespace dev {
@@ -495,7 +543,7 @@ __global__ void __launch_bounds__(128) k_pass(const __grid_constant__ PassDesc d
         break;
       case P_DIFF:
         if (op.arg > 0) {
-          cheb_diff<T>(A, 0, B, 0, len, 1, op.arg, Q, 0, tid, nth);
+          cheb_diff<T>(d.odd, A, 0, B, 0, len, 1, op.arg, Q, 0, tid, nth);
           T* t = A; A = B; B = t;
         }
         break;
@@ -689,6 +737,7 @@ static PassDesc base_desc(const SpaceDev& s) {
   if (!s.cplx && s.c0.use_fft) wl = std::max(wl, s.c0.L);
   if (s.cplx) wl = std::max(wl, s.f0.M);
   d.wl = wl;
+  d.odd = s.odd;
   return d;
 }
 

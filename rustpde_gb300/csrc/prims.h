@@ -59,12 +59,13 @@ struct SizeError : std::runtime_error {
 size_t smem_limit();
 
 // Device tables of one basis along one axis.
-BasisDev upload_basis(Arena& a, const HostBasis& b);
+// odd: odd scan blocks (chain_scan.cuh scan_block)
+BasisDev upload_basis(Arena& a, const HostBasis& b, bool odd = true);
 // allow_fft = false: the dense form even where n - 1 is a power of two
 ChebXformDev upload_cheb(Arena& a, int n, bool allow_fft = true);
 FourierXformDev upload_fourier(Arena& a, int n);
 PinvDev upload_pinv(Arena& a, int n);
-FdmaDev upload_fdma(Arena& a, const std::vector<Band4>& rows);  // swept factors, one per row
+FdmaDev upload_fdma(Arena& a, const std::vector<Band4>& rows, bool odd = true);  // swept factors, one per row
 
 // A 2-D space of two bases (funspace/src/space2.rs).
 struct SpaceDev {
@@ -72,10 +73,11 @@ struct SpaceDev {
   BasisDev b0, b1;
   ChebXformDev c0, c1;
   FourierXformDev f0;
+  bool odd = true;    // scan blocks of its passes (chain_scan.cuh)
   bool cplx = false;  // spectral data complex (Fourier along axis 0)
   int phys0 = 0, phys1 = 0, spec0 = 0, spec1 = 0, ortho0 = 0, ortho1 = 0;
 };
-void build_space(Arena& a, SpaceDev& s, int kind0, int n0, int kind1, int n1);
+void build_space(Arena& a, SpaceDev& s, int kind0, int n0, int kind1, int n1, bool odd = true);
 
 // The same space with dense Chebyshev transforms that sum all n terms in index
 // order.  A case's initial and boundary fields are transformed this way: the
@@ -105,6 +107,9 @@ bool build_solver(Arena& a, const SpaceDev& s, int kind, const double c[2], Solv
 std::vector<Band4> hholtz_rows(const HostBasis& bx, const HostBasis& by, double cx, double cy, double alpha,
                                bool poisson, std::vector<double>* lam_out, std::vector<double>* fwd,
                                std::vector<double>* bwd, std::string* err);
+// eigenbasis of the Poisson solve along a composite axis: forward and backward
+// matrices, (n-2) x (n-2) row-major
+void poisson_eigenbasis(const HostBasis& b, std::vector<double>& fwd, std::vector<double>& bwd);
 Band4 adi_factor(const HostBasis& b, double c);
 // n x n matrix, row-major -> column-major
 std::vector<double> transposed(const std::vector<double>& a, int n);

@@ -15,6 +15,7 @@ struct BasisDev {
   int kind;   // BaseKind
   int n;      // physical / ortho length (Fourier: physical length)
   int m;      // spectral length
+  int odd;                // scan blocks (chain_scan.cuh scan_block)
   int unit_diag;          // 1 when every diag_i is 1 (the composite bases here): the
                           // stencils skip the product, which is exact either way
   const double* diag;     // composite stencil diag (m)
@@ -27,6 +28,8 @@ struct BasisDev {
   const double* fo_a;     // diag_i / den_i (m)
   const double* fo_b;     // low2_i / den_i (m)
   const double* fo_c;     // -off_{i-2} / den_i, 0 for i < 2 (m)
+  const double* fo_scan;  // composed sweep coefficients (chain_scan.cuh): [8][32], value v of parity q, thread gl
+                          // at v 32 + 16 q + gl; 0-3 forward, 4-7 backward
   double t0[2], t1[2];    // boundary stencil
   double bc_inv[4];       // boundary least-squares inverse
 };
@@ -46,12 +49,15 @@ struct FdmaDev {
   int m;
   int rows;
   int stride;
-  int pad_;
+  int odd;             // scan blocks (chain_scan.cuh scan_block)
   const double* low;   // -low of the swept factors (m-2)
   const double* dinv;  // 1/dia (m)
   const double* up1;   // -up1/dia (m-2)
   const double* up2;   // -up2/dia (m-4)
+  const double* scan;  // composed sweep coefficients per row: [20][32] as BasisDev::fo_scan; 0-3 elimination,
+                       // 4 + 4 r + e back substitution
 };
+constexpr int kFdmaScan = 20 * 32;
 
 // Chebyshev transform along an axis of length n: FFT (n = 2^p + 1) or dense.
 struct ChebXformDev {
@@ -91,6 +97,15 @@ struct SplitOpDev {
   const unsigned char* w16;
   int N;
   int wshift;
+};
+
+// A general matrix in nine digits (SplitMat).
+struct SplitMatDev {
+  const unsigned char* w16;
+  const int* colex;
+  const int* rowex;
+  int N, K0, K1;
+  int pad_;
 };
 
 enum CaseKind { KIND_BOX_ADIABATIC = 0, KIND_BOX_CONDUCTING = 1, KIND_PERIODIC = 2 };
@@ -178,14 +193,19 @@ struct CaseDev {
   const float* m_bcx;  // FP32 d(fieldbc)/dx, transposed: ny x nx
   const float* m_bcy;  // FP32 d(fieldbc)/dy - m_bcg, transposed: ny x nx
 
+  int odd;  // scan blocks of the CTA passes (chain_scan.cuh scan_block)
   // FP64 transforms as split GEMMs (step_split.cu; not with a solid mask)
   int split;
-  int pad_s;
   SplitLanesDev spl_y1, spl_x1, spl_p, spl_cq;  // digits of the four GEMMs' lanes (one buffer, used in turn)
   double* spl_yw;  // G1: ny x (mxc x 6 [x 2 parts])
   double* spl_ph;  // G2: nx x (ny x 8)
   double* spl_q;   // G3: kx [x 2 parts] x (ny x 3); G4 writes m_cv
   SplitOpDev sop_yb, sop_xb, sop_xf[2], sop_yf[2];
+  // box: the Poisson eigenbasis products as split GEMMs too
+  int split_eig;
+  int pad_e;
+  SplitLanesDev spl_z, spl_w;  // lanes: columns of pinv_x div (ny), of the row solutions (myc)
+  SplitMatDev smat_f, smat_b;
 };
 
 // Row length (floats) of the mixed form's FP32 state copy m_s32 and of the

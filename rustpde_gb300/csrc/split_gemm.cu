@@ -41,9 +41,11 @@
 #include "split_gemm.h"
 
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 
 #include "lane_gemm.h"
+#include "pdl.cuh"
 #include "per_device.h"
 #include "tc_ptx.cuh"
 
@@ -53,10 +55,18 @@ namespace dev {
 __device__ long long g_split_wait_limit = kWaitLimit;
 
 constexpr int kSplitThreads = 320;
-constexpr int kSplitStages = 3;
-constexpr int kSplitStageBytes = kSplitChunkBytes + kSplitDigits * kSplitTile * 32;
-constexpr int kSplitCols = 8 * kSplitTile;  // tensor-memory columns of a CTA
-constexpr size_t kSplitSmem = (size_t)kSplitStages * kSplitStageBytes + 128;
+// The two precisions: 7 digits (transforms), 9 digits (eigenbasis products,
+// whose terms span more exponents than a transform's).
+template <int D>
+struct SplitForm {
+  static constexpr int kAcc = D + 1;                         // accumulators (weights i + j)
+  static constexpr int kTile = D == 7 ? kSplitTile : 16;     // widest tile
+  static constexpr int kStages = D == 7 ? 3 : 2;             // copy ring (two CTAs an SM)
+  static constexpr int kChunk = D * kSplitLanes * kSplitK * 2;
+  static constexpr int kStageBytes = kChunk + D * kTile * 32;
+  static constexpr size_t kSmem = (size_t)kStages * kStageBytes + 128;
+};
+constexpr int kSplitCols = 256;  // tensor-memory columns of a CTA
 
 __device__ __forceinline__ void mma_bf16(uint32_t tmem, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
   asm volatile(
@@ -126,18 +136,21 @@ __device__ __forceinline__ double split_double(long long v, int e) {
                               (s & (long long)0x8000000000000000ull));
 }
 
+template <int D>
 __global__ void __launch_bounds__(kSplitThreads, 2) k_split_gemm(const SplitJobDev* __restrict__ jobs,
                                                                  const int4* __restrict__ tiles) {
+  pdl_enter();
+  using F = SplitForm<D>;
   const int4 tl = tiles[blockIdx.x];
   const SplitJobDev& J = jobs[tl.x];
   if (J.active != nullptr && *J.active == 0) return;
   const int lane0 = tl.y, n0 = tl.z, NT = tl.w;
   const int tid = threadIdx.x, warp = tid >> 5, wl = tid & 31;
   extern __shared__ __align__(128) unsigned char sm[];
-  unsigned char* tail = sm + (size_t)kSplitStages * kSplitStageBytes;
-  uint64_t* full = reinterpret_cast<uint64_t*>(tail);  // [kSplitStages]
-  uint64_t* empty = full + kSplitStages;               // [kSplitStages]
-  uint64_t* accfull = empty + kSplitStages;
+  unsigned char* tail = sm + (size_t)F::kStages * F::kStageBytes;
+  uint64_t* full = reinterpret_cast<uint64_t*>(tail);  // [F::kStages]
+  uint64_t* empty = full + F::kStages;               // [F::kStages]
+  uint64_t* accfull = empty + F::kStages;
   uint64_t* accempty = accfull + 1;
   uint32_t* slot = reinterpret_cast<uint32_t*>(accempty + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(slot + 1);
@@ -150,7 +163,7 @@ __global__ void __launch_bounds__(kSplitThreads, 2) k_split_gemm(const SplitJobD
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
   if (tid == 0) {
-    for (int s = 0; s < kSplitStages; s++) {
+    for (int s = 0; s < F::kStages; s++) {
       mbar_init(&full[s], 1);
       mbar_init(&empty[s], 1);
     }
@@ -170,53 +183,53 @@ __global__ void __launch_bounds__(kSplitThreads, 2) k_split_gemm(const SplitJobD
   const int nlist = J.nc[1] > 0 ? 2 : 1;
   const int total = J.nc[0] + J.nc[1];
   // the lists of a wide tile share the columns, those of a narrow one have their own
-  const bool shared_cols = NT == kSplitTile;
+  const bool shared_cols = NT == F::kTile;
   const uint32_t list_cols = shared_cols ? 0u : (uint32_t)(8 * NT);
 
   if (warp == 8) {
     if (wl == 0) {
-      const unsigned char* a0 = J.dig + (size_t)(lane0 / kSplitLanes) * J.ctot * kSplitChunkBytes;
-      const uint32_t wbytes = (uint32_t)(kSplitDigits * NT * 32);
-      const unsigned char* w0 = (shared_cols ? J.w : J.w16) + (size_t)n0 * total * (kSplitDigits * 32);
+      const unsigned char* a0 = J.dig + (size_t)(lane0 / kSplitLanes) * J.ctot * F::kChunk;
+      const uint32_t wbytes = (uint32_t)(D * NT * 32);
+      const unsigned char* w0 = (NT == kSplitTile ? J.w : J.w16) + (size_t)n0 * total * (D * 32);
       for (int c = 0; c < total; c++) {
-        const int s = c % kSplitStages, ch = c < J.nc[0] ? J.c0[0] + c : J.c0[1] + c - J.nc[0];
-        if (c >= kSplitStages &&
-            !thread_mbar_wait(&empty[s], (uint32_t)((c / kSplitStages - 1) & 1), limit, abort_flag))
+        const int s = c % F::kStages, ch = c < J.nc[0] ? J.c0[0] + c : J.c0[1] + c - J.nc[0];
+        if (c >= F::kStages &&
+            !thread_mbar_wait(&empty[s], (uint32_t)((c / F::kStages - 1) & 1), limit, abort_flag))
           break;
-        unsigned char* st = sm + (size_t)s * kSplitStageBytes;
-        mbar_arrive_expect_tx(&full[s], kSplitChunkBytes + wbytes);
-        bulk_g2s(st, a0 + (size_t)ch * kSplitChunkBytes, kSplitChunkBytes, &full[s]);
-        bulk_g2s(st + kSplitChunkBytes, w0 + (size_t)c * wbytes, wbytes, &full[s]);
+        unsigned char* st = sm + (size_t)s * F::kStageBytes;
+        mbar_arrive_expect_tx(&full[s], F::kChunk + wbytes);
+        bulk_g2s(st, a0 + (size_t)ch * F::kChunk, F::kChunk, &full[s]);
+        bulk_g2s(st + F::kChunk, w0 + (size_t)c * wbytes, wbytes, &full[s]);
         *copied = c + 1;
       }
     }
   } else if (warp == 9) {
     if (wl == 0) {
-      const uint32_t w_lbo = (uint32_t)(kSplitDigits * NT / 8) * 128, plane = kSplitLanes * kSplitK * 2;
+      const uint32_t w_lbo = (uint32_t)(D * NT / 8) * 128, plane = kSplitLanes * kSplitK * 2;
       for (int c = 0; c < total; c++) {
-        const int s = c % kSplitStages;
-        if (!thread_mbar_wait(&full[s], (uint32_t)((c / kSplitStages) & 1), limit, abort_flag)) break;
+        const int s = c % F::kStages;
+        if (!thread_mbar_wait(&full[s], (uint32_t)((c / F::kStages) & 1), limit, abort_flag)) break;
         const bool first = c == 0 || c == J.nc[0];
         if (c == J.nc[0] && shared_cols && !thread_mbar_wait(accempty, 0, limit, abort_flag)) break;
         const uint32_t acc = tmem + (c >= J.nc[0] ? list_cols : 0u);
         tc_fence_after();
-        const uint32_t sa = smem_u32(sm + (size_t)s * kSplitStageBytes), sw = sa + kSplitChunkBytes;
+        const uint32_t sa = smem_u32(sm + (size_t)s * F::kStageBytes), sw = sa + F::kChunk;
         const uint64_t w = umma_desc(sw, w_lbo, 128);
         if (first) {
-          // digit plane 1 initialises accumulators 1..7, plane 0 accumulator 0
+          // digit plane 1 initialises accumulators 1 .. D, plane 0 accumulator 0
           const uint64_t a1 = umma_desc(sa + plane, kSplitLanes * 16, 128), a0 = umma_desc(sa, kSplitLanes * 16, 128);
-          mma_bf16(acc + NT, a1, w, split_idesc(7 * NT), 0u);
+          mma_bf16(acc + NT, a1, w, split_idesc(D * NT), 0u);
           mma_bf16(acc, a0, w, split_idesc(NT), 0u);
-          mma_bf16(acc + NT, a0, umma_desc(sw + (NT / 8) * 128, w_lbo, 128), split_idesc(6 * NT), 1u);
+          mma_bf16(acc + NT, a0, umma_desc(sw + (NT / 8) * 128, w_lbo, 128), split_idesc((D - 1) * NT), 1u);
         }
 #pragma unroll
-        for (int i = 0; i < kSplitDigits; i++) {
+        for (int i = 0; i < D; i++) {
           if (first && i < 2) continue;
-          const int nj = i == 0 ? 7 : 8 - i;
+          const int nj = i == 0 ? D : F::kAcc - i;
           mma_bf16(acc + i * NT, umma_desc(sa + i * plane, kSplitLanes * 16, 128), w, split_idesc(nj * NT), 1u);
         }
         // the last chunks' buffers are not reused: nobody waits for them
-        if (c + kSplitStages < total) mma_commit(&empty[s]);
+        if (c + F::kStages < total) mma_commit(&empty[s]);
         *issued = c + 1;
         if (c + 1 == J.nc[0] || c + 1 == total) {
           mma_commit(accfull);
@@ -236,42 +249,87 @@ __global__ void __launch_bounds__(kSplitThreads, 2) k_split_gemm(const SplitJobD
     double* mir = out + (J.mirror - n1) * es;
     out += n1 * es;
     const int ex = valid ? J.ex[lane] : 1, e = ex + J.ex_bias;
-    const bool nan = ex == 0x7ff;
-    long long v[2][8], o[8];
-    bool ok = warp_mbar_wait(accfull, 0, limit, abort_flag);
-    if (ok && (shared_cols || nlist == 1)) {
-      tc_fence_after();
-      split_sums(addr, NT, v[0]);
-      if (nb == 2) split_sums(addr + 8, NT, v[1]);
-      tc_fence_before();
-      mbar_arrive(accempty);
-    }
-    if (ok && nlist == 2) {
-      ok = warp_mbar_wait(accfull, 1, limit, abort_flag);
-      tc_fence_after();
-      if (ok && !shared_cols) split_sums(addr, NT, v[0]);
-    }
-    if (ok) {
+    const bool nan = ex == (D == 9 ? kSplitBadLane9 : 0x7ff);
+    if constexpr (D == 9) {
+      // 8 outputs: the five high and the five low weights in 64-bit integers
+      // each, both lists added, then one FP64 multiply-add
+      long long hi[8], lo[8];
 #pragma unroll
-      for (int b = 0; b < 2; b++) {
-        if (b == nb) break;
-        if (nlist == 2) split_sums(addr + list_cols + 8 * b, NT, o);
-        if (!valid) continue;
+      for (int j = 0; j < 8; j++) hi[j] = lo[j] = 0;
+      bool ok = true;
+      for (int list = 0; list < nlist && ok; list++) {
+        ok = warp_mbar_wait(accfull, (uint32_t)list, limit, abort_flag);
+        if (!ok) break;
+        tc_fence_after();
+        uint32_t r8[8];
+#pragma unroll
+        for (int d = 0; d < F::kAcc; d++) {
+          tmem_ld8(addr + d * NT, r8);
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+          const int w = 8 * (4 - d % 5);
+#pragma unroll
+          for (int j = 0; j < 8; j++) {
+            const long long x = (long long)__float2int_rn(__uint_as_float(r8[j])) << w;
+            if (d < 5) hi[j] += x;
+            else lo[j] += x;
+          }
+        }
+        tc_fence_before();
+        if (list == 0) mbar_arrive(accempty);
+      }
+      if (ok && valid) {
 #pragma unroll
         for (int j = 0; j < 8; j++) {
-          const int n = n1 + 8 * b + j;
+          const int n = n1 + j;
           if (n < N) {
-            double x = split_double(nlist == 2 ? v[b][j] + o[j] : v[b][j], e);
-            if (nan) x = __longlong_as_double(0x7FF8000000000000ll);
-            *out = x;
-          }
-          if (n >= m_lo && n < m_hi) {
-            double x = split_double(v[b][j] - o[j], e);
-            if (nan) x = __longlong_as_double(0x7FF8000000000000ll);
-            *mir = x;
+            const double x = fma((double)hi[j], 1099511627776.0, (double)lo[j]);  // hi 2^40 + lo
+            const int ee = e + J.rowex[n];
+            // scaled in two exact steps (each factor a normal power of two)
+            const int e1 = ee / 2, e2 = ee - e1;
+            const double y = x * __longlong_as_double((long long)(1023 + e1) << 52) *
+                             __longlong_as_double((long long)(1023 + e2) << 52);
+            *out = nan ? __longlong_as_double(0x7FF8000000000000ll) : y;
           }
           out += es;
-          mir -= es;
+        }
+      }
+    } else {
+      long long v[2][8], o[8];
+      bool ok = warp_mbar_wait(accfull, 0, limit, abort_flag);
+      if (ok && (shared_cols || nlist == 1)) {
+        tc_fence_after();
+        split_sums(addr, NT, v[0]);
+        if (nb == 2) split_sums(addr + 8, NT, v[1]);
+        tc_fence_before();
+        mbar_arrive(accempty);
+      }
+      if (ok && nlist == 2) {
+        ok = warp_mbar_wait(accfull, 1, limit, abort_flag);
+        tc_fence_after();
+        if (ok && !shared_cols) split_sums(addr, NT, v[0]);
+      }
+      if (ok) {
+#pragma unroll
+        for (int b = 0; b < 2; b++) {
+          if (b == nb) break;
+          if (nlist == 2) split_sums(addr + list_cols + 8 * b, NT, o);
+          if (!valid) continue;
+#pragma unroll
+          for (int j = 0; j < 8; j++) {
+            const int n = n1 + 8 * b + j;
+            if (n < N) {
+              double x = split_double(nlist == 2 ? v[b][j] + o[j] : v[b][j], e);
+              if (nan) x = __longlong_as_double(0x7FF8000000000000ll);
+              *out = x;
+            }
+            if (n >= m_lo && n < m_hi) {
+              double x = split_double(v[b][j] - o[j], e);
+              if (nan) x = __longlong_as_double(0x7FF8000000000000ll);
+              *mir = x;
+            }
+            out += es;
+            mir -= es;
+          }
         }
       }
     }
@@ -287,11 +345,11 @@ __global__ void __launch_bounds__(kSplitThreads, 2) k_split_gemm(const SplitJobD
     const int n = *issued, nw = *copied, nl = *lists;
     for (int c = n; c < nw; c++)
       for (long long i = 0; i < kWaitLimit; i++)
-        if (mbar_try(&full[c % kSplitStages], (uint32_t)((c / kSplitStages) & 1))) break;
-    for (int c = max(0, n - kSplitStages); c < n; c++)
-      if (c + kSplitStages < total)
+        if (mbar_try(&full[c % F::kStages], (uint32_t)((c / F::kStages) & 1))) break;
+    for (int c = max(0, n - F::kStages); c < n; c++)
+      if (c + F::kStages < total)
         for (long long i = 0; i < kWaitLimit; i++)
-          if (mbar_try(&empty[c % kSplitStages], (uint32_t)((c / kSplitStages) & 1))) break;
+          if (mbar_try(&empty[c % F::kStages], (uint32_t)((c / F::kStages) & 1))) break;
     if (nl > 0)
       for (long long i = 0; i < kWaitLimit; i++)
         if (mbar_try(accfull, (uint32_t)((nl - 1) & 1))) break;
@@ -303,8 +361,66 @@ __global__ void __launch_bounds__(kSplitThreads, 2) k_split_gemm(const SplitJobD
 
 }  // namespace dev
 
-size_t split_dig_bytes(int lanes, int cE, int cO) {
-  return (size_t)((lanes + kSplitLanes - 1) / kSplitLanes) * (cE + cO) * kSplitChunkBytes;
+size_t split_dig_bytes(int lanes, int cE, int cO, int digits) {
+  return (size_t)((lanes + kSplitLanes - 1) / kSplitLanes) * (cE + cO) * digits * (kSplitLanes * kSplitK * 2);
+}
+
+SplitMat pack_split_mat(const std::vector<double>& M, int n) {
+  SplitMat m;
+  m.N = n;
+  m.K[0] = std::min(n, split_chunks((n + 1) / 2) * kSplitK);
+  m.K[1] = n - m.K[0];
+  m.colex.assign(n, 0);
+  m.rowex.assign(n, 0);
+  // columns scaled by powers of two to a largest entry in [1/2, 1), then rows
+  for (int k = 0; k < n; k++) {
+    double mx = 0.0;
+    for (int r = 0; r < n; r++) mx = std::max(mx, std::fabs(M[(size_t)r * n + k]));
+    if (mx > 0.0) std::frexp(mx, &m.colex[k]);
+  }
+  for (int r = 0; r < n; r++) {
+    double mx = 0.0;
+    for (int k = 0; k < n; k++) mx = std::max(mx, std::fabs(std::ldexp(M[(size_t)r * n + k], -m.colex[k])));
+    if (mx > 0.0) std::frexp(mx, &m.rowex[r]);
+  }
+  const int nc[2] = {split_chunks(m.K[0]), split_chunks(m.K[1])}, total = nc[0] + nc[1];
+  const size_t chunk = (size_t)9 * 16 * 32;
+  m.bytes16.assign((size_t)((n + 15) / 16) * total * chunk, 0);
+  for (int r = 0; r < n; r++)
+    for (int k = 0; k < n; k++) {
+      const double w = std::ldexp(M[(size_t)r * n + k], -m.colex[k] - m.rowex[r]);  // |w| < 1
+      if (w == 0.0) continue;
+      int e;
+      const double f = std::frexp(w, &e);  // w = f 2^e, 1/2 <= |f| < 1
+      // |w| 2^70 = |f| 2^53 2^(17 + e): 53 bits shifted, as (high word, low word)
+      uint64_t a = (uint64_t)std::ldexp(std::fabs(f), 53), lo, hi;
+      const int sh = 17 + e;
+      if (sh >= 0) {
+        lo = a << sh;
+        hi = sh > 0 ? a >> (64 - sh) : 0;
+      } else {
+        hi = 0;
+        lo = -sh > 60 ? 0 : (a + (1ull << (-sh - 1))) >> -sh;
+      }
+      if (w < 0) {
+        lo = 0 - lo;
+        hi = ~hi + (lo == 0 ? 1 : 0);
+      }
+      const uint64_t b = lo + 0x8080808080808080ull;
+      const int64_t top = (int64_t)hi + (b < lo ? 1 : 0);
+      const int list = k >= m.K[0], kl = list ? k - m.K[0] : k, kk = kl % kSplitK;
+      unsigned char* c = m.bytes16.data() + ((size_t)(r / 16) * total + (list ? nc[0] : 0) + kl / kSplitK) * chunk;
+      for (int i = 0; i < 9; i++) {
+        const int d = i == 0 ? (int)top : (int)((b >> (8 * (8 - i))) & 255) - 128;
+        const float fl = (float)d;
+        uint32_t u;
+        memcpy(&u, &fl, 4);
+        const uint16_t v = (uint16_t)(u >> 16);
+        const int row = i * 16 + r % 16;
+        memcpy(c + (size_t)(kk >> 3) * (9 * 16 / 8) * 128 + (row >> 3) * 128 + (row & 7) * 16 + (kk & 7) * 2, &v, 2);
+      }
+    }
+  return m;
 }
 
 static int tile_width(int left, int most) { return left > 16 ? most : 16; }
@@ -356,7 +472,7 @@ void split_tiles(const std::vector<SplitJobDev>& jobs, std::vector<int4>& tiles)
   auto blocks = [](const SplitJobDev& j) { return (j.lanes + kSplitLanes - 1) / kSplitLanes; };
   long wide = 0;
   for (const SplitJobDev& j : jobs) wide += (long)blocks(j) * ((j.N + kSplitTile - 1) / kSplitTile);
-  const int most = wide <= kSplitNarrowTiles ? 16 : kSplitTile;
+  const int most = wide <= kSplitNarrowTiles || (!jobs.empty() && jobs[0].digits == 9) ? 16 : kSplitTile;
   for (size_t j = 0; j < jobs.size(); j++)
     for (int b = 0; b < blocks(jobs[j]); b++)
       for (int n = 0; n < jobs[j].N; n += most)
@@ -370,16 +486,19 @@ void split_tiles(const std::vector<SplitJobDev>& jobs, std::vector<int4>& tiles)
 cudaError_t configure_split_kernels() {
   static PerDeviceFlag done;
   if (done.test()) return cudaSuccess;
-  const cudaError_t e =
-      cudaFuncSetAttribute(dev::k_split_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dev::kSplitSmem);
+  cudaError_t e = cudaFuncSetAttribute(dev::k_split_gemm<7>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)dev::SplitForm<7>::kSmem);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(dev::k_split_gemm<9>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)dev::SplitForm<9>::kSmem);
   if (e == cudaSuccess) done.set();
   return e;
 }
 
-cudaError_t launch_split_gemm(const SplitJobDev* jobs, const int4* tiles, int ntiles, cudaStream_t st) {
+cudaError_t launch_split_gemm(const SplitJobDev* jobs, const int4* tiles, int ntiles, int digits, cudaStream_t st) {
   if (ntiles == 0) return cudaSuccess;
-  dev::k_split_gemm<<<ntiles, dev::kSplitThreads, dev::kSplitSmem, st>>>(jobs, tiles);
-  return cudaGetLastError();
+  if (digits == 9) return launch_pdl(dev::k_split_gemm<9>, ntiles, dev::kSplitThreads, dev::SplitForm<9>::kSmem, st, jobs, tiles);
+  return launch_pdl(dev::k_split_gemm<7>, ntiles, dev::kSplitThreads, dev::SplitForm<7>::kSmem, st, jobs, tiles);
 }
 
 cudaError_t set_split_wait_limit(long long polls) {

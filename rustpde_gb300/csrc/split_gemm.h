@@ -46,7 +46,7 @@ struct SplitLanesDev {
   int cE, cO;  // chunks of the two lists
 };
 inline int split_chunks(int k) { return (k + kSplitK - 1) / kSplitK; }
-size_t split_dig_bytes(int lanes, int cE, int cO);
+size_t split_dig_bytes(int lanes, int cE, int cO, int digits = kSplitDigits);
 
 // out[n] (lane l) of one lane set.  Two lists (nc[1] > 0): values E_n + O_n,
 // and E_n - O_n at output mirror - n for m_lo <= n < m_hi.  One list: that
@@ -67,7 +67,8 @@ struct SplitJobDev {
   int N;
   int ex_bias;             // a sum's unit is 2^(ex + ex_bias)
   int mirror, m_lo, m_hi;
-  int pad_;
+  int digits;              // 7, or 9 (one sum over both lists)
+  const int* rowex;        // 9 digits: per output, a power of two
 };
 
 // Packed operator rows: tile by tile (kSplitTile outputs, a last one of 16
@@ -80,10 +81,24 @@ struct SplitOp {
 // E and O: row-major N x K[list] integers (|.| <= 2^kSplitOpBits)
 SplitOp pack_split_op(const std::vector<int64_t>& E, int KE, const std::vector<int64_t>& O, int KO, int N);
 
+// A general n x n matrix in nine digits: entry (r, k) is w 2^(colex[k] + rowex[r]),
+// |w| < 1 and w in 70 bits.  Terms are x_k 2^colex[k] in 71 bits (split_emit9):
+// a product keeps what FP64 would at any ratio of the terms up to 2^17.  The
+// terms are two lists (an accumulator's sums stay below 2^24), added at the end.
+constexpr int kSplitShl9 = 18, kSplitOpBits9 = 70;
+constexpr int kSplitBadLane9 = 0x7fffff;  // a lane's exponent when it is not finite
+inline int split_ex_bias9() { return 56 - 1075 - kSplitShl9 - kSplitOpBits9; }
+struct SplitMat {
+  int N = 0, K[2] = {0, 0};
+  std::vector<int> colex, rowex;
+  std::vector<unsigned char> bytes16;
+};
+SplitMat pack_split_mat(const std::vector<double>& M, int n);
+
 // tiles (job, first lane, first output, tile width)
 void split_tiles(const std::vector<SplitJobDev>& jobs, std::vector<int4>& tiles);
 cudaError_t configure_split_kernels();
-cudaError_t launch_split_gemm(const SplitJobDev* jobs, const int4* tiles, int ntiles, cudaStream_t st);
+cudaError_t launch_split_gemm(const SplitJobDev* jobs, const int4* tiles, int ntiles, int digits, cudaStream_t st);
 cudaError_t set_split_wait_limit(long long polls);  // as set_gemm_wait_limit
 
 // Unit exponent of a job's sums (SplitJobDev::ex_bias): terms with shift shl,

@@ -12,6 +12,8 @@
 // Each launch takes a table of work items (case, first lane, lane count); a
 // batch of cases is the same launch with a longer table.
 #include "lane_ops.cuh"
+#include "pdl.cuh"
+#include "split_emit.cuh"
 #include "per_device.h"
 #include "prims.h"
 #include "step_fp64.h"
@@ -35,11 +37,28 @@ __device__ void load_rows3(void* const f[3], int row_len, int r0, int nr, T* dst
   __syncthreads();
 }
 
+// three lanes of n doubles, element k at base + k * stride of each array: the
+// three loads of a thread are issued together
+__device__ __forceinline__ void load_lanes3(const void* a, const void* b, const void* d, size_t base, int stride, int n,
+                                            double* dst, int ld, int tid, int nth) {
+  const double* pa = static_cast<const double*>(a) + base;
+  const double* pb = static_cast<const double*>(b) + base;
+  const double* pd = static_cast<const double*>(d) + base;
+  for (int k = tid; k < n; k += nth) {
+    const size_t o = (size_t)k * stride;
+    const double va = __ldcg(pa + o), vb = __ldcg(pb + o), vd = __ldcg(pd + o);
+    dst[k] = va;
+    dst[ld + k] = vb;
+    dst[2 * ld + k] = vd;
+  }
+}
+
 // ============================================================================
 // Y1: Y0_f = Ty^-1 Sy f,  Y1_f = Ty^-1 Dy Sy f   for f in (ux, uy, temp)
 // ============================================================================
 template <class T>
 __global__ void __launch_bounds__(256) k_y1(const CaseDev* __restrict__ cases, const int4* __restrict__ work) {
+  pdl_enter();
   int4 w = work[blockIdx.x];
   const CaseDev& c = cases[w.x];
   if (c.gate != nullptr && c.gate[1] == 0) return;  // case idle this step (serving)
@@ -58,7 +77,7 @@ __global__ void __launch_bounds__(256) k_y1(const CaseDev* __restrict__ cases, c
   void* f3[3] = {c.ux, c.uy, c.temp};
   load_rows3<T>(f3, myc, r0, nr, IN, ld, tid, nth);
   to_ortho<T>(c.ycd, IN, ld, O, ld, 3 * nr, tid, nth);
-  cheb_diff<T>(O, ld, D, ld, ny, 3 * nr, 1, TMP, ld, tid, nth);
+  cheb_diff<T>(c.odd, O, ld, D, ld, ny, 3 * nr, 1, TMP, ld, tid, nth);
   // inverse Chebyshev transform of O and D (6nr lanes, O and D contiguous)
   if (c.cy.use_fft) {
     if constexpr (sizeof(T) == 16) {
@@ -115,6 +134,7 @@ __device__ __forceinline__ double solid_damp(const CaseDev& c, int f, size_t g, 
 //  With a solid mask a ninth lane carries T = F^-1 Y0_t for the damping term.
 // ============================================================================
 __global__ void __launch_bounds__(256) k_per_x(const CaseDev* __restrict__ cases, const int4* __restrict__ work) {
+  pdl_enter();
   int4 w = work[blockIdx.x];
   const CaseDev& c = cases[w.x];
   if (c.gate != nullptr && c.gate[1] == 0) return;  // case idle this step (serving)
@@ -172,15 +192,27 @@ size_t smem_per_x(const CaseDev& c) {
 // solves (Hholtz per row), divergence, Poisson row solve, projection and the
 // pressure update (navier.rs:622-721).
 // ============================================================================
+// The ADI factors are the same for every lane.  Up to this length they are staged
+// in shared memory: a pass then has one CTA per SM, and a factor loaded inside a
+// recurrence costs its L2 latency (box 129^2: x2 25 -> 14 us, y3 28 -> 15 us).
+// Longer lanes leave several CTAs per SM to cover it, and the staging would cost
+// one of them (box 513^2).
+__host__ __device__ inline bool stage_factors(int m) { return m <= 320; }
+
 // stage the factors of row `row` of a per-row banded solver into shared memory
 __device__ FdmaDev stage_fdma_row(const FdmaDev& f, int row, double* dst, int tid, int nth) {
   const int m = f.m;
   const size_t off = (f.rows > 1) ? (size_t)row * f.stride : 0;
+  const double* __restrict__ low = f.low + off;
+  const double* __restrict__ dinv = f.dinv + off;
+  const double* __restrict__ up1 = f.up1 + off;
+  const double* __restrict__ up2 = f.up2 + off;
   for (int k = tid; k < m; k += nth) {
-    dst[k] = f.low[off + k];
-    dst[m + k] = f.dinv[off + k];
-    dst[2 * m + k] = f.up1[off + k];
-    dst[3 * m + k] = f.up2[off + k];
+    const double a = __ldg(low + k), b = __ldg(dinv + k), u = __ldg(up1 + k), v = __ldg(up2 + k);
+    dst[k] = a;
+    dst[m + k] = b;
+    dst[2 * m + k] = u;
+    dst[3 * m + k] = v;
   }
   FdmaDev r = f;
   r.rows = 1;
@@ -189,6 +221,7 @@ __device__ FdmaDev stage_fdma_row(const FdmaDev& f, int row, double* dst, int ti
   r.dinv = dst + m;
   r.up1 = dst + 2 * m;
   r.up2 = dst + 3 * m;
+  r.scan = f.scan + (f.rows > 1 ? (size_t)row * kFdmaScan : 0);
   return r;
 }
 
@@ -200,6 +233,7 @@ __device__ FdmaDev stage_fdma_row(const FdmaDev& f, int row, double* dst, int ti
 enum { CONV_Q = 0, CONV_MIXED = 1, CONV_FULL = 2 };
 template <int CONV>
 __global__ void __launch_bounds__(256) k_per_y2(const CaseDev* __restrict__ cases, const int4* __restrict__ work) {
+  pdl_enter();
   int4 w = work[blockIdx.x];
   const CaseDev& c = cases[w.x];
   if (c.gate != nullptr && c.gate[1] == 0) return;  // case idle this step (serving)
@@ -272,7 +306,7 @@ __global__ void __launch_bounds__(256) k_per_y2(const CaseDev* __restrict__ case
   for (int k = tid; k < ny; k += nth) P[k] = p0[(size_t)i * ny + k];
   __syncthreads();
   to_ortho<double2>(c.ycd, F, ld, O, ld, 3, tid, nth);
-  cheb_diff<double2>(P, ld, G, ld, ny, 1, 1, nullptr, ld, tid, nth);
+  cheb_diff<double2>(c.odd, P, ld, G, ld, ny, 1, 1, nullptr, ld, tid, nth);
   const double2* bco = static_cast<const double2*>(c.bc_ortho);
   const double2* bcd = static_cast<const double2*>(c.bc_diff);
   for (int k = tid; k < ny; k += nth) {
@@ -291,7 +325,7 @@ __global__ void __launch_bounds__(256) k_per_y2(const CaseDev* __restrict__ case
   fdma_solve2<double2>(fu, ft, 2, F, ld, 3, 0, 0, tid, nth);
   // 4. divergence = ik/s Sy ux* + Dy Sy uy*
   to_ortho<double2>(c.ycd, F, ld, O, ld, 2, tid, nth);
-  cheb_diff<double2>(O + ld, ld, G, ld, ny, 1, 1, nullptr, ld, tid, nth);
+  cheb_diff<double2>(c.odd, O + ld, ld, G, ld, ny, 1, 1, nullptr, ld, tid, nth);
   for (int k = tid; k < ny; k += nth) R[k] = mul_ik(O[k], ki) * inv_asp + G[k];  // R lane 0 = div
   __syncthreads();
   // 5. Poisson row solve -> pseudo pressure row
@@ -303,7 +337,7 @@ __global__ void __launch_bounds__(256) k_per_y2(const CaseDev* __restrict__ case
   for (int k = tid; k < myc; k += nth) p1[(size_t)i * myc + k] = X1[k];
   // 6. projection: O1 = Sy^N p1; dpdx = ik/s O1; dpdy = Dy O1
   to_ortho<double2>(c.ycn, X1, ld, O, ld, 1, tid, nth);  // O lane 0 = O1
-  cheb_diff<double2>(O, ld, G, ld, ny, 1, 1, nullptr, ld, tid, nth);  // G = dpdy
+  cheb_diff<double2>(c.odd, O, ld, G, ld, ny, 1, 1, nullptr, ld, tid, nth);  // G = dpdy
   for (int k = tid; k < ny; k += nth) {
     O[ld + k] = mul_ik(O[k], ki) * inv_asp;  // O lane 1 = dpdx
     O[2 * ld + k] = G[k];                     // O lane 2 = dpdy
@@ -340,6 +374,7 @@ __global__ void __launch_bounds__(256) k_per_y2(const CaseDev* __restrict__ case
 //  Y2b (row i): divergence, Poisson row solve, projection, pressure update.
 // ============================================================================
 __global__ void __launch_bounds__(256) k_per_y2a(const CaseDev* __restrict__ cases, const int4* __restrict__ work) {
+  pdl_enter();
   int4 w = work[blockIdx.x];
   const CaseDev& c = cases[w.x];
   if (c.gate != nullptr && c.gate[1] == 0) return;  // case idle this step (serving)
@@ -394,7 +429,7 @@ __global__ void __launch_bounds__(256) k_per_y2a(const CaseDev* __restrict__ cas
   }
   __syncthreads();
   to_ortho<double2>(c.ycd, F, ld, O, ld, f == 1 ? 2 : 1, tid, nth);  // O (and OT for uy)
-  if (f == 1) cheb_diff<double2>(P, ld, G, ld, ny, 1, 1, nullptr, ld, tid, nth);
+  if (f == 1) cheb_diff<double2>(c.odd, P, ld, G, ld, ny, 1, 1, nullptr, ld, tid, nth);
   const double2* bco = static_cast<const double2*>(c.bc_ortho) + (size_t)i * ny;
   const double2* bcd = static_cast<const double2*>(c.bc_diff) + (size_t)i * ny;
   for (int k = tid; k < ny; k += nth) {
@@ -434,6 +469,7 @@ size_t smem_per_y2a(const CaseDev& c) {
 }
 
 __global__ void __launch_bounds__(256) k_per_y2b(const CaseDev* __restrict__ cases, const int4* __restrict__ work) {
+  pdl_enter();
   int4 w = work[blockIdx.x];
   const CaseDev& c = cases[w.x];
   if (c.gate != nullptr && c.gate[1] == 0) return;  // case idle this step (serving)
@@ -458,7 +494,7 @@ __global__ void __launch_bounds__(256) k_per_y2b(const CaseDev* __restrict__ cas
   }
   __syncthreads();
   to_ortho<double2>(c.ycd, F, ld, O, ld, 2, tid, nth);
-  cheb_diff<double2>(O + ld, ld, G, ld, ny, 1, 1, nullptr, ld, tid, nth);
+  cheb_diff<double2>(c.odd, O + ld, ld, G, ld, ny, 1, 1, nullptr, ld, tid, nth);
   for (int k = tid; k < ny; k += nth) R[k] = mul_ik(O[k], ki) * inv_asp + G[k];
   __syncthreads();
   matvec_pinv<double2>(c.pinv_y, R, ld, X1, ld, 1, tid, nth);
@@ -468,7 +504,7 @@ __global__ void __launch_bounds__(256) k_per_y2b(const CaseDev* __restrict__ cas
   double2* p1 = static_cast<double2*>(c.p1) + (size_t)i * myc;
   for (int k = tid; k < myc; k += nth) p1[k] = X1[k];
   to_ortho<double2>(c.ycn, X1, ld, O, ld, 1, tid, nth);
-  cheb_diff<double2>(O, ld, G, ld, ny, 1, 1, nullptr, ld, tid, nth);
+  cheb_diff<double2>(c.odd, O, ld, G, ld, ny, 1, 1, nullptr, ld, tid, nth);
   for (int k = tid; k < ny; k += nth) {
     O[ld + k] = mul_ik(O[k], ki) * inv_asp;
     O[2 * ld + k] = G[k];
@@ -517,6 +553,7 @@ size_t smem_per_y2_pre(const CaseDev& c) {
 // X1: columns j < ny.  x-backward of the y-transformed state, products,
 // x-forward of the products (rows < kx), and d/dx p0.
 __global__ void __launch_bounds__(256) k_box_x1(const CaseDev* __restrict__ cases, const int4* __restrict__ work) {
+  pdl_enter();
   int4 w = work[blockIdx.x];
   const CaseDev& c = cases[w.x];
   if (c.gate != nullptr && c.gate[1] == 0) return;  // case idle this step (serving)
@@ -547,12 +584,10 @@ __global__ void __launch_bounds__(256) k_box_x1(const CaseDev* __restrict__ case
   to_ortho<double>(c.xu, IN, ld, OR, ld, 6, tid, nth);
   to_ortho<double>(c.xt, IN + 6 * ld, ld, OR + 6 * ld, ld, NL - 6, tid, nth);
   // d/dx for lanes 2, 4, 6 (in place through TMP)
-  for (int f = 0; f < 3; f++) {
-    double* lane = OR + (2 + 2 * f) * ld;
-    cheb_diff<double>(lane, ld, TMP, ld, nx, 1, 1, TMP + ld, ld, tid, nth);
-    for (int k = tid; k < nx; k += nth) lane[k] = TMP[k] * inv_asp;
-    __syncthreads();
-  }
+  cheb_diff<double>(c.odd, OR + 2 * ld, 2 * ld, TMP, ld, nx, 3, 1, nullptr, 0, tid, nth);
+  for (int f = 0; f < 3; f++)
+    for (int k = tid; k < nx; k += nth) OR[(2 + 2 * f) * ld + k] = TMP[f * ld + k] * inv_asp;
+  __syncthreads();
   if (c.cx.use_fft) dct1_fft_r(c.cx, false, OR, ld, PH, ld, NL, WA, WB, wld, tid, nth);
   else dct1_dense<double>(c.cx, false, OR, ld, PH, ld, NL, tid, nth);
   // products (lanes 2, 4, 6)
@@ -580,7 +615,7 @@ __global__ void __launch_bounds__(256) k_box_x1(const CaseDev* __restrict__ case
   const double* p0 = static_cast<const double*>(c.p0);
   for (int k = tid; k < nx; k += nth) IN[k] = p0[(size_t)k * ny + j];
   __syncthreads();
-  cheb_diff<double>(IN, ld, TMP, ld, nx, 1, 1, TMP + ld, ld, tid, nth);
+  cheb_diff<double>(c.odd, IN, ld, TMP, ld, nx, 1, 1, TMP + ld, ld, tid, nth);
   double* gp = static_cast<double*>(c.s[0]);
   for (int k = tid; k < nx; k += nth) gp[(size_t)k * ny + j] = TMP[k] * inv_asp;
 }
@@ -588,6 +623,7 @@ __global__ void __launch_bounds__(256) k_box_x1(const CaseDev* __restrict__ case
 // d/dx p0 / aspect for column j -> s[0] (nx x ny): the pressure-gradient part
 // of X1, run on its own in the mixed-precision step (FP64)
 __global__ void __launch_bounds__(256) k_box_gpx(const CaseDev* __restrict__ cases, const int4* __restrict__ work) {
+  pdl_enter();
   int4 w = work[blockIdx.x];
   const CaseDev& c = cases[w.x];
   if (c.gate != nullptr && c.gate[1] == 0) return;  // case idle this step (serving)
@@ -602,7 +638,7 @@ __global__ void __launch_bounds__(256) k_box_gpx(const CaseDev* __restrict__ cas
   const double* p0 = static_cast<const double*>(c.p0);
   for (int k = tid; k < nx; k += nth) IN[k] = p0[(size_t)k * ny + j];
   __syncthreads();
-  cheb_diff<double>(IN, ld, TMP, ld, nx, 1, 1, TMP + ld, ld, tid, nth);
+  cheb_diff<double>(c.odd, IN, ld, TMP, ld, nx, 1, 1, TMP + ld, ld, tid, nth);
   double* gp = static_cast<double*>(c.s[0]);
   for (int k = tid; k < nx; k += nth) gp[(size_t)k * ny + j] = TMP[k] * inv_asp;
 }
@@ -619,6 +655,7 @@ size_t smem_box_x1(const CaseDev& c) {
 // Y2: rows i < nx (ortho x).  conv (y forward, dealiased), rhs, pinv_y -> s[1..3]
 template <int CONV>
 __global__ void __launch_bounds__(256) k_box_y2(const CaseDev* __restrict__ cases, const int4* __restrict__ work) {
+  pdl_enter();
   int4 w = work[blockIdx.x];
   const CaseDev& c = cases[w.x];
   if (c.gate != nullptr && c.gate[1] == 0) return;  // case idle this step (serving)
@@ -683,7 +720,7 @@ __global__ void __launch_bounds__(256) k_box_y2(const CaseDev* __restrict__ case
   for (int k = tid; k < ny; k += nth) P[k] = p0[(size_t)i * ny + k];
   __syncthreads();
   to_ortho<double>(c.ycd, SX, ld, O, ld, 3, tid, nth);
-  cheb_diff<double>(P, ld, G, ld, ny, 1, 1, TMP, ld, tid, nth);
+  cheb_diff<double>(c.odd, P, ld, G, ld, ny, 1, 1, TMP, ld, tid, nth);
   const double* gpx = static_cast<const double*>(c.s[0]);
   const double* bco = static_cast<const double*>(c.bc_ortho);
   const double* bcd = static_cast<const double*>(c.bc_diff);
@@ -709,8 +746,12 @@ size_t smem_box_y2(const CaseDev& c) {
   return 17 * ld * 8 + 2 * 2 * wld * 16 + 64;
 }
 
+// with the convection term given: no FFT work lanes (box 513^2: three CTAs per SM instead of one)
+size_t smem_box_y2_pre(const CaseDev& c) { return 17 * (size_t)(c.ny + 1) * 8 + 64; }
+
 // X2: columns j < myc.  pinv_x then the ADI x solve.  s[1..3] -> s[4..6] (mxc x myc)
 __global__ void __launch_bounds__(256) k_box_x2(const CaseDev* __restrict__ cases, const int4* __restrict__ work) {
+  pdl_enter();
   int4 w = work[blockIdx.x];
   const CaseDev& c = cases[w.x];
   if (c.gate != nullptr && c.gate[1] == 0) return;  // case idle this step (serving)
@@ -721,24 +762,30 @@ __global__ void __launch_bounds__(256) k_box_x2(const CaseDev* __restrict__ case
   extern __shared__ double2 smem[];
   double* IN = reinterpret_cast<double*>(smem);
   double* OUT = IN + 3 * ld;
-  for (int idx = tid; idx < 3 * nx; idx += nth) {
-    int f = idx / nx, k = idx - f * nx;
-    IN[f * ld + k] = static_cast<const double*>(c.s[1 + f])[(size_t)k * myc + j];
-  }
+  double* FAC = OUT + 3 * ld;
+  const bool stage = stage_factors(mxc);
+  const FdmaDev hu = stage ? stage_fdma_row(c.hu_x, 0, FAC, tid, nth) : c.hu_x;
+  const FdmaDev ht = stage ? stage_fdma_row(c.ht_x, 0, FAC + 4 * mxc, tid, nth) : c.ht_x;
+  load_lanes3(c.s[1], c.s[2], c.s[3], (size_t)j, myc, nx, IN, ld, tid, nth);
   __syncthreads();
   matvec_pinv<double>(c.pinv_x, IN, ld, OUT, ld, 3, tid, nth);
-  fdma_solve<double>(c.hu_x, OUT, ld, 2, 0, 0, tid, nth);
-  fdma_solve<double>(c.ht_x, OUT + 2 * ld, ld, 1, 0, 0, tid, nth);
-  for (int idx = tid; idx < 3 * mxc; idx += nth) {
-    int f = idx / mxc, k = idx - f * mxc;
-    static_cast<double*>(c.s[4 + f])[(size_t)k * myc + j] = OUT[f * ld + k];
+  fdma_solve2<double>(hu, ht, 2, OUT, ld, 3, 0, 0, tid, nth);
+  double* o0 = static_cast<double*>(c.s[4]);
+  double* o1 = static_cast<double*>(c.s[5]);
+  double* o2 = static_cast<double*>(c.s[6]);
+  for (int k = tid; k < mxc; k += nth) {
+    const size_t o = (size_t)k * myc + j;
+    o0[o] = OUT[k];
+    o1[o] = OUT[ld + k];
+    o2[o] = OUT[2 * ld + k];
   }
 }
 
-size_t smem_box_x2(const CaseDev& c) { return 6 * (size_t)(c.nx + 1) * 8 + 64; }
+size_t smem_box_x2(const CaseDev& c) { return (stage_factors(c.mxc) ? 14 : 6) * (size_t)(c.nx + 1) * 8 + 64; }
 
 // Y3: rows i < mxc.  ADI y solve -> ux*, uy*, temp(new); A = Sy ux*, B = Dy Sy uy*
 __global__ void __launch_bounds__(256) k_box_y3(const CaseDev* __restrict__ cases, const int4* __restrict__ work) {
+  pdl_enter();
   int4 w = work[blockIdx.x];
   const CaseDev& c = cases[w.x];
   if (c.gate != nullptr && c.gate[1] == 0) return;  // case idle this step (serving)
@@ -751,24 +798,26 @@ __global__ void __launch_bounds__(256) k_box_y3(const CaseDev* __restrict__ case
   double* O = F + 3 * ld;
   double* B = O + 2 * ld;
   double* TMP = B + ld;
-  for (int idx = tid; idx < 3 * myc; idx += nth) {
-    int f = idx / myc, k = idx - f * myc;
-    F[f * ld + k] = static_cast<const double*>(c.s[4 + f])[(size_t)i * myc + k];
-  }
+  double* FAC = TMP + 2 * ld;
+  const bool stage = stage_factors(myc);
+  const FdmaDev hu = stage ? stage_fdma_row(c.hu_y, 0, FAC, tid, nth) : c.hu_y;
+  const FdmaDev ht = stage ? stage_fdma_row(c.ht_y, 0, FAC + 4 * myc, tid, nth) : c.ht_y;
+  load_lanes3(c.s[4], c.s[5], c.s[6], (size_t)i * myc, 1, myc, F, ld, tid, nth);
   __syncthreads();
-  fdma_solve<double>(c.hu_y, F, ld, 2, 0, 0, tid, nth);
-  fdma_solve<double>(c.ht_y, F + 2 * ld, ld, 1, 0, 0, tid, nth);
+  fdma_solve2<double>(hu, ht, 2, F, ld, 3, 0, 0, tid, nth);
   to_ortho<double>(c.ycd, F, ld, O, ld, 2, tid, nth);
-  cheb_diff<double>(O + ld, ld, B, ld, ny, 1, 1, TMP, ld, tid, nth);
+  cheb_diff<double>(c.odd, O + ld, ld, B, ld, ny, 1, 1, TMP, ld, tid, nth);
   // ux*, uy* -> s[4], s[5] (in place);  temp -> state
   bool bad = false;
-  double* tt = static_cast<double*>(c.temp);
-  for (int idx = tid; idx < 3 * myc; idx += nth) {
-    int f = idx / myc, k = idx - f * myc;
-    double v = F[f * ld + k];
-    if (f < 2) static_cast<double*>(c.s[4 + f])[(size_t)i * myc + k] = v;
-    else tt[(size_t)i * myc + k] = v;
-    bad |= !isfinite(v);
+  double* us = static_cast<double*>(c.s[4]) + (size_t)i * myc;
+  double* vs = static_cast<double*>(c.s[5]) + (size_t)i * myc;
+  double* tt = static_cast<double*>(c.temp) + (size_t)i * myc;
+  for (int k = tid; k < myc; k += nth) {
+    const double u = F[k], v = F[ld + k], t = F[2 * ld + k];
+    us[k] = u;
+    vs[k] = v;
+    tt[k] = t;
+    bad |= !(finite_v(u) && finite_v(v) && finite_v(t));
   }
   double* A = static_cast<double*>(c.s[1]);   // mxc x ny
   double* Bs = static_cast<double*>(c.s[2]);  // mxc x ny
@@ -779,13 +828,16 @@ __global__ void __launch_bounds__(256) k_box_y3(const CaseDev* __restrict__ case
   if (bad) flag_nonfinite(c.status);
 }
 
-size_t smem_box_y3(const CaseDev& c) { return 8 * (size_t)(c.ny + 1) * 8 + 64; }
+size_t smem_box_y3(const CaseDev& c) { return (stage_factors(c.myc) ? 16 : 8) * (size_t)(c.ny + 1) * 8 + 64; }
 
 // X3: columns j < ny.  div = Dx Sx A / s + Sx B  (-> s[3], nx x ny);
 // Zf = fwd * pinv_x div  (-> s[1] reused? no: s[6], mxc x ny)
-// MIX: stop after pinv_x and store it (m_z); the eigenbasis product runs as a GEMM.
-template <bool MIX>
+// The eigenbasis product: EIG_DENSE here; EIG_MIXED and EIG_SPLIT as a GEMM that
+// follows, from FP32 values (m_z) or from nine-digit lanes (spl_z).
+enum { EIG_DENSE = 0, EIG_MIXED = 1, EIG_SPLIT = 2 };
+template <int EIG>
 __global__ void __launch_bounds__(256) k_box_x3(const CaseDev* __restrict__ cases, const int4* __restrict__ work) {
+  pdl_enter();
   int4 w = work[blockIdx.x];
   const CaseDev& c = cases[w.x];
   if (c.gate != nullptr && c.gate[1] == 0) return;  // case idle this step (serving)
@@ -803,12 +855,13 @@ __global__ void __launch_bounds__(256) k_box_x3(const CaseDev* __restrict__ case
   const double* A = static_cast<const double*>(c.s[1]);
   const double* B = static_cast<const double*>(c.s[2]);
   for (int k = tid; k < mxc; k += nth) {
-    IN[k] = A[(size_t)k * ny + j];
-    IN[ld + k] = B[(size_t)k * ny + j];
+    const double a = __ldcg(A + (size_t)k * ny + j), b = __ldcg(B + (size_t)k * ny + j);
+    IN[k] = a;
+    IN[ld + k] = b;
   }
   __syncthreads();
   to_ortho<double>(c.xu, IN, ld, OR, ld, 2, tid, nth);
-  cheb_diff<double>(OR, ld, TMP, ld, nx, 1, 1, TMP + ld, ld, tid, nth);
+  cheb_diff<double>(c.odd, OR, ld, TMP, ld, nx, 1, 1, TMP + ld, ld, tid, nth);
   double* dv = static_cast<double*>(c.s[3]);
   for (int k = tid; k < nx; k += nth) {
     double v = TMP[k] * inv_asp + OR[ld + k];
@@ -817,7 +870,12 @@ __global__ void __launch_bounds__(256) k_box_x3(const CaseDev* __restrict__ case
   }
   __syncthreads();
   matvec_pinv<double>(c.pinv_x, DV, ld, Z, ld, 1, tid, nth);
-  if (MIX) {  // FP32: the input of the eigenbasis GEMM
+  if (EIG == EIG_SPLIT) {
+    split_emit9(c.spl_z, j, 1, mxc, c.smat_f.K0, c.smat_f.colex, [&](int, int k) { return Z[k]; },
+                reinterpret_cast<int*>(TMP), tid, nth);
+    return;
+  }
+  if (EIG == EIG_MIXED) {
     float* mz = static_cast<float*>(c.m_z);
     for (int r = tid; r < mxc; r += nth) mz[(size_t)r * ny + j] = (float)Z[r];
     return;
@@ -835,6 +893,7 @@ size_t smem_box_x3(const CaseDev& c) { return 8 * (size_t)(c.nx + 1) * 8 + 64; }
 // MIX: in FP32 into m_z instead, the input of the eigenbasis GEMM
 template <bool MIX>
 __global__ void __launch_bounds__(256) k_box_y4(const CaseDev* __restrict__ cases, const int4* __restrict__ work) {
+  pdl_enter();
   int4 w = work[blockIdx.x];
   const CaseDev& c = cases[w.x];
   if (c.gate != nullptr && c.gate[1] == 0) return;  // case idle this step (serving)
@@ -845,11 +904,12 @@ __global__ void __launch_bounds__(256) k_box_y4(const CaseDev* __restrict__ case
   extern __shared__ double2 smem[];
   double* IN = reinterpret_cast<double*>(smem);
   double* OUT = IN + ld;
+  const FdmaDev fp = stage_fdma_row(c.pois_y, i, OUT + ld, tid, nth);
   const double* zf = static_cast<const double*>(c.s[6]);
   for (int k = tid; k < ny; k += nth) IN[k] = zf[(size_t)i * ny + k];
   __syncthreads();
   matvec_pinv<double>(c.pinv_y, IN, ld, OUT, ld, 1, tid, nth);
-  fdma_solve<double>(c.pois_y, OUT, ld, 1, i, 0, tid, nth);
+  fdma_solve<double>(fp, OUT, ld, 1, 0, 0, tid, nth);
   if (MIX) {  // FP32 into m_z: the input of the eigenbasis GEMM
     float* wf = static_cast<float*>(c.m_z);
     for (int k = tid; k < myc; k += nth) wf[(size_t)i * myc + k] = (float)OUT[k];
@@ -859,13 +919,31 @@ __global__ void __launch_bounds__(256) k_box_y4(const CaseDev* __restrict__ case
   for (int k = tid; k < myc; k += nth) wv[(size_t)i * myc + k] = OUT[k];
 }
 
-size_t smem_box_y4(const CaseDev& c) { return 2 * (size_t)(c.ny + 1) * 8 + 64; }
+size_t smem_box_y4(const CaseDev& c) { return 6 * (size_t)(c.ny + 1) * 8 + 64; }
+
+// column j of the Poisson row solutions (s[7]) as nine-digit lanes
+__global__ void __launch_bounds__(256) k_spl_w(const CaseDev* __restrict__ cases, const int4* __restrict__ work) {
+  pdl_enter();
+  int4 w = work[blockIdx.x];
+  const CaseDev& c = cases[w.x];
+  if (c.gate != nullptr && c.gate[1] == 0) return;  // case idle this step (serving)
+  const int j = w.y, myc = c.myc, mxc = c.mxc, tid = threadIdx.x, nth = blockDim.x;
+  extern __shared__ double2 smem[];
+  double* W = reinterpret_cast<double*>(smem);
+  const double* wv = static_cast<const double*>(c.s[7]);
+  for (int k = tid; k < mxc; k += nth) W[k] = wv[(size_t)k * myc + j];
+  __syncthreads();
+  split_emit9(c.spl_w, j, 1, mxc, c.smat_b.K0, c.smat_b.colex, [&](int, int k) { return W[k]; },
+              reinterpret_cast<int*>(W + mxc), tid, nth);
+}
+static size_t smem_spl_w(const CaseDev& c) { return (size_t)c.mxc * 8 + 64; }
 
 // X4: columns j < myc.  p1 = bwd * W (p1[0][0] = 0).  E = Sx+ Dx Sx^N p1 / s,
 // Fv = Sx+ Sx^N p1 (-> s[1], s[2] as mxc x myc), Gp = Sx^N p1 (-> s[0], nx x myc)
 // MIX: p1 = bwd * W was computed by a GEMM; read it (and set p1[0][0] = 0).
 template <bool MIX>
 __global__ void __launch_bounds__(256) k_box_x4(const CaseDev* __restrict__ cases, const int4* __restrict__ work) {
+  pdl_enter();
   int4 w = work[blockIdx.x];
   const CaseDev& c = cases[w.x];
   if (c.gate != nullptr && c.gate[1] == 0) return;  // case idle this step (serving)
@@ -904,7 +982,7 @@ __global__ void __launch_bounds__(256) k_box_x4(const CaseDev* __restrict__ case
   }
   __syncthreads();
   to_ortho<double>(c.xp, PV, ld, OR, ld, 1, tid, nth);
-  cheb_diff<double>(OR, ld, TMP, ld, nx, 1, 1, TMP + ld, ld, tid, nth);
+  cheb_diff<double>(c.odd, OR, ld, TMP, ld, nx, 1, 1, TMP + ld, ld, tid, nth);
   double* gp = static_cast<double*>(c.s[0]);
   for (int k = tid; k < nx; k += nth) {
     D[k] = TMP[k] * inv_asp;
@@ -926,6 +1004,7 @@ size_t smem_box_x4(const CaseDev& c) { return 9 * (size_t)(c.nx + 1) * 8 + 64; }
 // Y5: rows i < nx.  ux = ux* - Sy+ Sy^N E ; uy = uy* - Sy+ Dy Sy^N Fv ;
 // p0 = (p0 - nu div) + Sy^N Gp / dt
 __global__ void __launch_bounds__(256) k_box_y5(const CaseDev* __restrict__ cases, const int4* __restrict__ work) {
+  pdl_enter();
   int4 w = work[blockIdx.x];
   const CaseDev& c = cases[w.x];
   if (c.gate != nullptr && c.gate[1] == 0) return;  // case idle this step (serving)
@@ -942,17 +1021,15 @@ __global__ void __launch_bounds__(256) k_box_y5(const CaseDev* __restrict__ case
   const double* e = static_cast<const double*>(c.s[1]);
   const double* fv = static_cast<const double*>(c.s[2]);
   const double* gp = static_cast<const double*>(c.s[0]);
-  for (int k = tid; k < myc; k += nth) {
-    if (i < mxc) {
-      IN[k] = e[(size_t)i * myc + k];
-      IN[ld + k] = fv[(size_t)i * myc + k];
-    }
-    IN[2 * ld + k] = gp[(size_t)i * myc + k];
+  if (i < mxc) {
+    load_lanes3(e, fv, gp, (size_t)i * myc, 1, myc, IN, ld, tid, nth);
+  } else {
+    for (int k = tid; k < myc; k += nth) IN[2 * ld + k] = gp[(size_t)i * myc + k];
   }
   __syncthreads();
   if (i < mxc) {
     to_ortho<double>(c.ycn, IN, ld, OR, ld, 2, tid, nth);
-    cheb_diff<double>(OR + ld, ld, D + ld, ld, ny, 1, 1, TMP, ld, tid, nth);
+    cheb_diff<double>(c.odd, OR + ld, ld, D + ld, ld, ny, 1, 1, TMP, ld, tid, nth);
     for (int k = tid; k < ny; k += nth) D[k] = OR[k];
     __syncthreads();
     from_ortho<double>(c.ycd, D, ld, FO, ld, 2, tid, nth);
@@ -966,7 +1043,7 @@ __global__ void __launch_bounds__(256) k_box_y5(const CaseDev* __restrict__ case
       double b = vs[(size_t)i * myc + k] - FO[ld + k];
       ux[(size_t)i * myc + k] = a;
       uy[(size_t)i * myc + k] = b;
-      bad |= !(isfinite(a) && isfinite(b));
+      bad |= !(finite_v(a) && finite_v(b));
     }
     if (bad) flag_nonfinite(c.status);
   }
@@ -1011,8 +1088,10 @@ cudaError_t configure_step_kernels() {
   SET_ATTR(dev::k_box_x2);
   SET_ATTR(dev::k_box_gpx);
   SET_ATTR(dev::k_box_y3);
-  SET_ATTR(dev::k_box_x3<false>);
-  SET_ATTR(dev::k_box_x3<true>);
+  SET_ATTR(dev::k_box_x3<dev::EIG_DENSE>);
+  SET_ATTR(dev::k_box_x3<dev::EIG_MIXED>);
+  SET_ATTR(dev::k_box_x3<dev::EIG_SPLIT>);
+  SET_ATTR(dev::k_spl_w);
   SET_ATTR(dev::k_box_y4<false>);
   SET_ATTR(dev::k_box_y4<true>);
   SET_ATTR(dev::k_box_x4<false>);
@@ -1052,12 +1131,25 @@ StepPlan build_step_plan(const CaseDev& c) {
     add_if(!split, K_BOX_X1, c.ny, dev::smem_box_x1(c));
     add_split_launches(c, split, p);
     add_if(!split, K_BOX_Y2, c.nx, dev::smem_box_y2(c));
-    add_if(split, K_BOX_Y2_CV, c.nx, dev::smem_box_y2(c));
+    add_if(split, K_BOX_Y2_CV, c.nx, dev::smem_box_y2_pre(c));
     add(K_BOX_X2, c.myc, dev::smem_box_x2(c));
     add(K_BOX_Y3, c.mxc, dev::smem_box_y3(c));
-    add(K_BOX_X3, c.ny, dev::smem_box_x3(c));
+    const bool eig = split && c.split_eig != 0;
+    auto eig_gemm = [&](const SplitLanesDev& s, const SplitMatDev& m, int lanes, void* out, long long es) {
+      StepLaunch L;
+      L.kernel = K_SPLIT_GEMM;
+      L.smem = 0;
+      if (eig) L.sjobs.push_back(split_mat_job(s, m, lanes, static_cast<double*>(out), es, c.status));
+      p.launches.push_back(L);
+    };
+    add_if(!eig, K_BOX_X3, c.ny, dev::smem_box_x3(c));
+    add_if(eig, K_SPL_X3, c.ny, dev::smem_box_x3(c));
+    eig_gemm(c.spl_z, c.smat_f, c.ny, c.s[6], c.ny);
     add(K_BOX_Y4, c.mxc, dev::smem_box_y4(c));
-    add(K_BOX_X4, c.myc, dev::smem_box_x4(c));
+    add_if(eig, K_SPL_W, c.myc, dev::smem_spl_w(c));
+    eig_gemm(c.spl_w, c.smat_b, c.myc, c.p1, c.myc);
+    add_if(!eig, K_BOX_X4, c.myc, dev::smem_box_x4(c));
+    add_if(eig, K_BOX_X4_MIX, c.myc, dev::smem_box_x4(c));
     add(K_BOX_Y5, c.nx, dev::smem_box_y5(c));
   }
   return p;
@@ -1073,32 +1165,34 @@ cudaError_t launch_step_kernel(int kernel, int nblocks, size_t smem, cudaStream_
                                const int4* work) {
   dim3 g(nblocks), b(256);
   switch (kernel) {
-    case K_Y1_C: dev::k_y1<double2><<<g, b, smem, s>>>(cases, work); break;
-    case K_Y1_R: dev::k_y1<double><<<g, b, smem, s>>>(cases, work); break;
-    case K_PER_X: dev::k_per_x<<<g, b, smem, s>>>(cases, work); break;
-    case K_PER_Y2: dev::k_per_y2<dev::CONV_Q><<<g, b, smem, s>>>(cases, work); break;
-    case K_PER_Y2_PRE: dev::k_per_y2<dev::CONV_MIXED><<<g, b, smem, s>>>(cases, work); break;
-    case K_PER_Y2A: dev::k_per_y2a<<<g, b, smem, s>>>(cases, work); break;
-    case K_PER_Y2B: dev::k_per_y2b<<<g, b, smem, s>>>(cases, work); break;
-    case K_BOX_X1: dev::k_box_x1<<<g, b, smem, s>>>(cases, work); break;
-    case K_BOX_Y2: dev::k_box_y2<dev::CONV_Q><<<g, b, smem, s>>>(cases, work); break;
-    case K_BOX_Y2_PRE: dev::k_box_y2<dev::CONV_MIXED><<<g, b, smem, s>>>(cases, work); break;
-    case K_PER_Y2_CV: dev::k_per_y2<dev::CONV_FULL><<<g, b, smem, s>>>(cases, work); break;
-    case K_BOX_Y2_CV: dev::k_box_y2<dev::CONV_FULL><<<g, b, smem, s>>>(cases, work); break;
-    case K_BOX_X2: dev::k_box_x2<<<g, b, smem, s>>>(cases, work); break;
-    case K_BOX_GPX: dev::k_box_gpx<<<g, b, smem, s>>>(cases, work); break;
-    case K_BOX_Y3: dev::k_box_y3<<<g, b, smem, s>>>(cases, work); break;
-    case K_BOX_X3: dev::k_box_x3<false><<<g, b, smem, s>>>(cases, work); break;
-    case K_BOX_X3_MIX: dev::k_box_x3<true><<<g, b, smem, s>>>(cases, work); break;
-    case K_BOX_Y4: dev::k_box_y4<false><<<g, b, smem, s>>>(cases, work); break;
-    case K_BOX_Y4_MIX: dev::k_box_y4<true><<<g, b, smem, s>>>(cases, work); break;
-    case K_BOX_X4: dev::k_box_x4<false><<<g, b, smem, s>>>(cases, work); break;
-    case K_BOX_X4_MIX: dev::k_box_x4<true><<<g, b, smem, s>>>(cases, work); break;
-    case K_BOX_Y5: dev::k_box_y5<<<g, b, smem, s>>>(cases, work); break;
-    case K_PER_Y2_PRE_T128: dev::k_per_y2<dev::CONV_MIXED><<<g, dim3(128), smem, s>>>(cases, work); break;
-    case K_BOX_Y2_PRE_T128: dev::k_box_y2<dev::CONV_MIXED><<<g, dim3(128), smem, s>>>(cases, work); break;
-    case K_BOX_X3_MIX_T128: dev::k_box_x3<true><<<g, dim3(128), smem, s>>>(cases, work); break;
-    case K_BOX_Y5_T128: dev::k_box_y5<<<g, dim3(128), smem, s>>>(cases, work); break;
+    case K_Y1_C: return launch_pdl(dev::k_y1<double2>, g, b, smem, s, cases, work);
+    case K_Y1_R: return launch_pdl(dev::k_y1<double>, g, b, smem, s, cases, work);
+    case K_PER_X: return launch_pdl(dev::k_per_x, g, b, smem, s, cases, work);
+    case K_PER_Y2: return launch_pdl(dev::k_per_y2<dev::CONV_Q>, g, b, smem, s, cases, work);
+    case K_PER_Y2_PRE: return launch_pdl(dev::k_per_y2<dev::CONV_MIXED>, g, b, smem, s, cases, work);
+    case K_PER_Y2A: return launch_pdl(dev::k_per_y2a, g, b, smem, s, cases, work);
+    case K_PER_Y2B: return launch_pdl(dev::k_per_y2b, g, b, smem, s, cases, work);
+    case K_BOX_X1: return launch_pdl(dev::k_box_x1, g, b, smem, s, cases, work);
+    case K_BOX_Y2: return launch_pdl(dev::k_box_y2<dev::CONV_Q>, g, b, smem, s, cases, work);
+    case K_BOX_Y2_PRE: return launch_pdl(dev::k_box_y2<dev::CONV_MIXED>, g, b, smem, s, cases, work);
+    case K_PER_Y2_CV: return launch_pdl(dev::k_per_y2<dev::CONV_FULL>, g, b, smem, s, cases, work);
+    case K_BOX_Y2_CV: return launch_pdl(dev::k_box_y2<dev::CONV_FULL>, g, b, smem, s, cases, work);
+    case K_SPL_X3: return launch_pdl(dev::k_box_x3<dev::EIG_SPLIT>, g, b, smem, s, cases, work);
+    case K_SPL_W: return launch_pdl(dev::k_spl_w, g, b, smem, s, cases, work);
+    case K_BOX_X2: return launch_pdl(dev::k_box_x2, g, b, smem, s, cases, work);
+    case K_BOX_GPX: return launch_pdl(dev::k_box_gpx, g, b, smem, s, cases, work);
+    case K_BOX_Y3: return launch_pdl(dev::k_box_y3, g, b, smem, s, cases, work);
+    case K_BOX_X3: return launch_pdl(dev::k_box_x3<dev::EIG_DENSE>, g, b, smem, s, cases, work);
+    case K_BOX_X3_MIX: return launch_pdl(dev::k_box_x3<dev::EIG_MIXED>, g, b, smem, s, cases, work);
+    case K_BOX_Y4: return launch_pdl(dev::k_box_y4<false>, g, b, smem, s, cases, work);
+    case K_BOX_Y4_MIX: return launch_pdl(dev::k_box_y4<true>, g, b, smem, s, cases, work);
+    case K_BOX_X4: return launch_pdl(dev::k_box_x4<false>, g, b, smem, s, cases, work);
+    case K_BOX_X4_MIX: return launch_pdl(dev::k_box_x4<true>, g, b, smem, s, cases, work);
+    case K_BOX_Y5: return launch_pdl(dev::k_box_y5, g, b, smem, s, cases, work);
+    case K_PER_Y2_PRE_T128: return launch_pdl(dev::k_per_y2<dev::CONV_MIXED>, g, dim3(128), smem, s, cases, work);
+    case K_BOX_Y2_PRE_T128: return launch_pdl(dev::k_box_y2<dev::CONV_MIXED>, g, dim3(128), smem, s, cases, work);
+    case K_BOX_X3_MIX_T128: return launch_pdl(dev::k_box_x3<dev::EIG_MIXED>, g, dim3(128), smem, s, cases, work);
+    case K_BOX_Y5_T128: return launch_pdl(dev::k_box_y5, g, dim3(128), smem, s, cases, work);
     case K_SPL_Y1_R: case K_SPL_Y1_C: case K_SPL_X1_BOX: case K_SPL_X1_PER: case K_SPL_PROD: case K_SPL_Q:
       return launch_step_split_kernel(kernel, nblocks, smem, s, cases, work);
     default: return launch_mixed_kernel(kernel, nblocks, smem, s, cases, work);

@@ -35,6 +35,8 @@ enum StepKernel {
   K_SPL_Y1_R, K_SPL_Y1_C, K_SPL_X1_BOX, K_SPL_X1_PER, K_SPL_PROD, K_SPL_Q,
   // Y2 with the convection term from the split GEMMs
   K_PER_Y2_CV, K_BOX_Y2_CV,
+  // box eigenbasis products as split GEMMs: their input lanes
+  K_SPL_X3, K_SPL_W,
   K_NUM_STEP_KERNELS,
   K_GEMM = 100,  // tensor-core lane GEMM (jobs instead of work items)
   K_SPLIT_GEMM = 101  // split GEMM (sjobs instead of work items)
@@ -115,6 +117,7 @@ size_t smem_per_x_mixed(const CaseDev& c);
 size_t smem_box_x1(const CaseDev& c);
 size_t smem_box_gpx(const CaseDev& c);
 size_t smem_box_y2(const CaseDev& c);
+size_t smem_box_y2_pre(const CaseDev& c);
 size_t smem_box_x2(const CaseDev& c);
 size_t smem_box_y3(const CaseDev& c);
 size_t smem_box_x3(const CaseDev& c);

@@ -22,6 +22,7 @@
 //
 // Work item: (case, first lane, lane count <= blockDim.x, 0).
 #include "lane_ops.cuh"
+#include "pdl.cuh"
 #include "step_fp64.h"
 
 namespace rbc {
@@ -348,6 +349,7 @@ __device__ __forceinline__ void from_ortho_par(const BasisDev& b, const T* p, lo
 
 // d/dx p0 / aspect -> s[0] (nx x ny), columns j < ny; sub = parity of the output rows
 __global__ void __launch_bounds__(128) k_lp_box_gpx(const CaseDev* __restrict__ cases, const int4* __restrict__ work) {
+  pdl_enter();
   LANE_PROLOGUE
   const int j = lane, nx = c.nx, ny = c.ny;
   const double inv_asp = 1.0 / c.aspect;
@@ -360,6 +362,7 @@ __global__ void __launch_bounds__(128) k_lp_box_gpx(const CaseDev* __restrict__ 
 // pinv_x and the ADI x solve of the three fields: s[1..3] -> s[4..6], columns
 // j < myc; sub = 2 * field + parity
 __global__ void __launch_bounds__(128) k_lp_box_x2(const CaseDev* __restrict__ cases, const int4* __restrict__ work) {
+  pdl_enter();
   LANE_PROLOGUE
   const int j = lane, myc = c.myc, f = sub >> 1, q = sub & 1;
   const double* in = static_cast<const double*>(c.s[1 + f]) + j;
@@ -373,6 +376,7 @@ __global__ void __launch_bounds__(128) k_lp_box_x2(const CaseDev* __restrict__ c
 // pinv_x div -> m_z (mxc x ny), columns j < ny; sub = parity of the rows
 // (Dx A on parity q from Sx A on parity 1 - q)
 __global__ void __launch_bounds__(128) k_lp_box_x3(const CaseDev* __restrict__ cases, const int4* __restrict__ work) {
+  pdl_enter();
   LANE_PROLOGUE
   const int j = lane, nx = c.nx, ny = c.ny, mxc = c.mxc, q = sub;
   const double inv_asp = 1.0 / c.aspect;
@@ -393,6 +397,7 @@ __global__ void __launch_bounds__(128) k_lp_box_x3(const CaseDev* __restrict__ c
 // 1 - q, from Gp of parity q formed again from p1 (the two parts share no
 // intermediate, so they run on different threads)
 __global__ void __launch_bounds__(128) k_lp_box_x4(const CaseDev* __restrict__ cases, const int4* __restrict__ work) {
+  pdl_enter();
   LANE_PROLOGUE
   const int j = lane, nx = c.nx, myc = c.myc, q = sub & 1, part = sub >> 1;
   double* p1 = static_cast<double*>(c.p1) + j;
@@ -429,6 +434,7 @@ __global__ void __launch_bounds__(128) k_lp_box_x4(const CaseDev* __restrict__ c
 // and pinv rows on the columns of parity q (dP/dy on parity q comes from p0 on
 // parity 1 - q)
 __global__ void __launch_bounds__(256) k_lp_box_y2(const CaseDev* __restrict__ cases, const int4* __restrict__ work) {
+  pdl_enter();
   ROW_PROLOGUE
   const int i = lane, ny = c.ny, myc = c.myc, mxc = c.mxc, kx = c.kx, ky = c.ky, f = sub;
   const double dt = c.dt;
@@ -516,6 +522,7 @@ __global__ void __launch_bounds__(256) k_lp_box_y2(const CaseDev* __restrict__ c
 // field + parity q: the field's chain of parity q, then A on parity q (ux) or
 // B on parity 1 - q (uy)
 __global__ void __launch_bounds__(256) k_lp_box_y3(const CaseDev* __restrict__ cases, const int4* __restrict__ work) {
+  pdl_enter();
   ROW_PROLOGUE
   const int i = lane, ny = c.ny, myc = c.myc, f = sub;
   double* F = static_cast<double*>(c.s[4 + f]) + (size_t)i * myc;
@@ -556,6 +563,7 @@ __global__ void __launch_bounds__(256) k_lp_box_y3(const CaseDev* __restrict__ c
 // rows i < mxc: pinv_y of the eigenbasis-transformed divergence and the
 // Poisson row solve: s[6] (zf, mxc x ny) -> s[7] (mxc x myc); sub = parity
 __global__ void __launch_bounds__(256) k_lp_box_y4(const CaseDev* __restrict__ cases, const int4* __restrict__ work) {
+  pdl_enter();
   ROW_PROLOGUE
   const int i = lane, ny = c.ny, myc = c.myc;
   const double* zf = static_cast<const double*>(c.s[6]) + (size_t)i * ny;
@@ -581,6 +589,7 @@ __global__ void __launch_bounds__(256) k_lp_box_y4(const CaseDev* __restrict__ c
 // p0 = (p0 - nu div) + Sy^N Gp / dt  (scratch rows: s[6], s[7]).
 // sub = 2 * part + parity q: part 0 ux, part 1 uy, part 2 p0, on parity q
 __global__ void __launch_bounds__(256) k_lp_box_y5(const CaseDev* __restrict__ cases, const int4* __restrict__ work) {
+  pdl_enter();
   ROW_PROLOGUE
   const int i = lane, ny = c.ny, myc = c.myc, mxc = c.mxc, part = sub;
   if (part == 2) {
@@ -624,6 +633,7 @@ __global__ void __launch_bounds__(256) k_lp_box_y5(const CaseDev* __restrict__ c
 // Scratch rows (ny): yw[0] div, yw[1] dp/dx, yw[2] dp/dy.
 // ============================================================================
 __global__ void __launch_bounds__(128) k_lp_per_y2(const CaseDev* __restrict__ cases, const int4* __restrict__ work) {
+  pdl_enter();
   LANE_PROLOGUE
   const int i = lane, ny = c.ny, myc = c.myc, kx = c.kx, ky = c.ky;
   const double dt = c.dt, inv_asp = 1.0 / c.aspect, ki = (double)i;
@@ -807,6 +817,7 @@ __device__ __forceinline__ void per_y2a_row(const CaseDev& c, const int i, const
   fdma_bwd_par<double2, PB>(R, out, 1, q);
 }
 __global__ void __launch_bounds__(256) k_lp_per_y2a(const CaseDev* __restrict__ cases, const int4* __restrict__ work) {
+  pdl_enter();
   ROW_PROLOGUE
   per_y2a_row(c, lane, q, sub);
 }
@@ -860,6 +871,7 @@ __device__ __forceinline__ void per_y2b_row(const CaseDev& c, const int i, const
   if (i == 0 && q == 0) p1[0] = c2(0.0, 0.0);
 }
 __global__ void __launch_bounds__(256) k_lp_per_y2b(const CaseDev* __restrict__ cases, const int4* __restrict__ work) {
+  pdl_enter();
   ROW_PROLOGUE
   per_y2b_row(c, lane, q);
 }
@@ -924,6 +936,7 @@ __device__ __forceinline__ void per_y2c_row(const CaseDev& c, const int i, const
   if (bad) atomicOr(c.status, 1u);
 }
 __global__ void __launch_bounds__(256) k_lp_per_y2c(const CaseDev* __restrict__ cases, const int4* __restrict__ work) {
+  pdl_enter();
   ROW_PROLOGUE
   per_y2c_row(c, lane, q, sub);
 }
@@ -941,6 +954,7 @@ __global__ void __launch_bounds__(256) k_lp_per_y2c(const CaseDev* __restrict__ 
 // 1.13 ms for the three launches.
 __global__ void __launch_bounds__(3 * kLaneBlock) k_lp_per_y2f(const CaseDev* __restrict__ cases,
                                                                const int4* __restrict__ work) {
+  pdl_enter();
   const int4 w = work[blockIdx.x];
   const CaseDev& c = cases[w.x];
   if (c.gate != nullptr && c.gate[1] == 0) return;  // the whole CTA: no barrier is left waiting
@@ -982,19 +996,19 @@ bool lane_kernel_rows(int kernel) {
 cudaError_t launch_lane_kernel(int kernel, int nblocks, cudaStream_t s, const CaseDev* cases, const int4* work) {
   dim3 g(nblocks, lane_kernel_subs(kernel)), b(kernel == K_LP_PER_Y2F ? 3 * kLaneBlock : kLaneBlock);
   switch (kernel) {
-    case K_LP_BOX_GPX: dev::k_lp_box_gpx<<<g, b, 0, s>>>(cases, work); break;
-    case K_LP_BOX_X2: dev::k_lp_box_x2<<<g, b, 0, s>>>(cases, work); break;
-    case K_LP_BOX_X3: dev::k_lp_box_x3<<<g, b, 0, s>>>(cases, work); break;
-    case K_LP_BOX_X4: dev::k_lp_box_x4<<<g, b, 0, s>>>(cases, work); break;
-    case K_LP_BOX_Y2: dev::k_lp_box_y2<<<g, b, 0, s>>>(cases, work); break;
-    case K_LP_BOX_Y3: dev::k_lp_box_y3<<<g, b, 0, s>>>(cases, work); break;
-    case K_LP_BOX_Y4: dev::k_lp_box_y4<<<g, b, 0, s>>>(cases, work); break;
-    case K_LP_BOX_Y5: dev::k_lp_box_y5<<<g, b, 0, s>>>(cases, work); break;
-    case K_LP_PER_Y2: dev::k_lp_per_y2<<<g, b, 0, s>>>(cases, work); break;
-    case K_LP_PER_Y2A: dev::k_lp_per_y2a<<<g, b, 0, s>>>(cases, work); break;
-    case K_LP_PER_Y2B: dev::k_lp_per_y2b<<<g, b, 0, s>>>(cases, work); break;
-    case K_LP_PER_Y2C: dev::k_lp_per_y2c<<<g, b, 0, s>>>(cases, work); break;
-    case K_LP_PER_Y2F: dev::k_lp_per_y2f<<<g, b, 0, s>>>(cases, work); break;
+    case K_LP_BOX_GPX: return launch_pdl(dev::k_lp_box_gpx, g, b, 0, s, cases, work);
+    case K_LP_BOX_X2: return launch_pdl(dev::k_lp_box_x2, g, b, 0, s, cases, work);
+    case K_LP_BOX_X3: return launch_pdl(dev::k_lp_box_x3, g, b, 0, s, cases, work);
+    case K_LP_BOX_X4: return launch_pdl(dev::k_lp_box_x4, g, b, 0, s, cases, work);
+    case K_LP_BOX_Y2: return launch_pdl(dev::k_lp_box_y2, g, b, 0, s, cases, work);
+    case K_LP_BOX_Y3: return launch_pdl(dev::k_lp_box_y3, g, b, 0, s, cases, work);
+    case K_LP_BOX_Y4: return launch_pdl(dev::k_lp_box_y4, g, b, 0, s, cases, work);
+    case K_LP_BOX_Y5: return launch_pdl(dev::k_lp_box_y5, g, b, 0, s, cases, work);
+    case K_LP_PER_Y2: return launch_pdl(dev::k_lp_per_y2, g, b, 0, s, cases, work);
+    case K_LP_PER_Y2A: return launch_pdl(dev::k_lp_per_y2a, g, b, 0, s, cases, work);
+    case K_LP_PER_Y2B: return launch_pdl(dev::k_lp_per_y2b, g, b, 0, s, cases, work);
+    case K_LP_PER_Y2C: return launch_pdl(dev::k_lp_per_y2c, g, b, 0, s, cases, work);
+    case K_LP_PER_Y2F: return launch_pdl(dev::k_lp_per_y2f, g, b, 0, s, cases, work);
     default: return cudaErrorInvalidValue;
   }
   return cudaGetLastError();

@@ -14,6 +14,7 @@
 //  periodic:  G1 (y, GEMM) -> X (FP32) -> G2 (y, GEMM) -> Y2 (FP64)
 #include "lane_ops.cuh"
 #include "lane_ops_f32.cuh"
+#include "pdl.cuh"
 #include "per_device.h"
 #include "prims.h"
 #include "step_fp64.h"
@@ -32,6 +33,7 @@ namespace dev {
 // (navier.rs:538-616, conv_term.rs:22-42)
 // ============================================================================
 __global__ void __launch_bounds__(256) k_per_x_mixed(const CaseDev* __restrict__ cases, const int4* __restrict__ work) {
+  pdl_enter();
   const int4 w = work[blockIdx.x];
   const CaseDev& c = cases[w.x];
   if (c.gate != nullptr && c.gate[1] == 0) return;  // case idle this step (serving)
@@ -85,6 +87,7 @@ __global__ void __launch_bounds__(256) k_per_x_mixed(const CaseDev* __restrict__
 // ============================================================================
 __global__ void __launch_bounds__(256) k_box_prod_mixed(const CaseDev* __restrict__ cases,
                                                         const int4* __restrict__ work) {
+  pdl_enter();
   const int4 w = work[blockIdx.x];
   const CaseDev& c = cases[w.x];
   if (c.gate != nullptr && c.gate[1] == 0) return;  // case idle this step (serving)
@@ -112,6 +115,7 @@ __global__ void __launch_bounds__(256) k_box_prod_mixed(const CaseDev* __restric
 // Serving gate: for each member case decide whether it advances in this step
 // (steps left > 0) and count the step down.
 __global__ void k_gate(const CaseDev* __restrict__ cases, const int* __restrict__ members, int n) {
+  pdl_enter();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   int* g = cases[members[i]].gate;
@@ -125,6 +129,7 @@ __global__ void k_gate(const CaseDev* __restrict__ cases, const int* __restrict_
 // instead of once per output tile inside the GEMM; the GEMM rounds FP64 input
 // to FP32 the same way)
 __global__ void __launch_bounds__(128) k_state_f32(const CaseDev* __restrict__ cases, const int4* __restrict__ work) {
+  pdl_enter();
   const int4 w = work[blockIdx.x];
   const CaseDev& c = cases[w.x];
   if (c.gate != nullptr && c.gate[1] == 0) return;
@@ -322,7 +327,7 @@ StepPlan build_mixed_plan(const CaseDev& c, const MixedOps& ops, int variant) {
   if (lane_parallel) add_lp(K_LP_BOX_GPX, ny, nx);
   else add(K_BOX_GPX, ny, dev::smem_box_gpx(c));
   if (lp) add_lp(K_LP_BOX_Y2, nx, ny);
-  else add(lane_parallel ? K_BOX_Y2_PRE_T128 : K_BOX_Y2_PRE, nx, dev::smem_box_y2(c));
+  else add(lane_parallel ? K_BOX_Y2_PRE_T128 : K_BOX_Y2_PRE, nx, dev::smem_box_y2_pre(c));
   if (lane_parallel) {
     add_lp(K_LP_BOX_X2, myc, mxc);
     add_lp(K_LP_BOX_Y3, mxc, ny);
@@ -386,10 +391,10 @@ cudaError_t configure_mixed_kernels() {
 cudaError_t launch_mixed_kernel(int kernel, int nblocks, size_t smem, cudaStream_t s, const CaseDev* cases,
                                 const int4* work) {
   switch (kernel) {
-    case K_PER_X_MIXED: dev::k_per_x_mixed<<<nblocks, 256, smem, s>>>(cases, work); break;
-    case K_STATE_F32: dev::k_state_f32<<<nblocks, 128, 0, s>>>(cases, work); break;
-    case K_PER_X_MIXED_T128: dev::k_per_x_mixed<<<nblocks, 128, smem, s>>>(cases, work); break;
-    case K_BOX_PROD_MIXED: dev::k_box_prod_mixed<<<nblocks, 256, 0, s>>>(cases, work); break;
+    case K_PER_X_MIXED: return launch_pdl(dev::k_per_x_mixed, nblocks, 256, smem, s, cases, work);
+    case K_STATE_F32: return launch_pdl(dev::k_state_f32, nblocks, 128, 0, s, cases, work);
+    case K_PER_X_MIXED_T128: return launch_pdl(dev::k_per_x_mixed, nblocks, 128, smem, s, cases, work);
+    case K_BOX_PROD_MIXED: return launch_pdl(dev::k_box_prod_mixed, nblocks, 256, 0, s, cases, work);
     default: return launch_lane_kernel(kernel, nblocks, s, cases, work);
   }
   return cudaGetLastError();
@@ -412,7 +417,7 @@ double launch_algorithmic_bytes(const StepLaunch& L, const CaseDev* cases) {
   for (const SplitJobDev& j : L.sjobs) {
     // lane digits, operator digits and outputs, once each
     const double nc = j.nc[0] + j.nc[1];
-    b += j.lanes * nc * kSplitK * kSplitDigits * 2.0 + j.N * nc * kSplitDigits * 32.0 +
+    b += j.lanes * nc * kSplitK * j.digits * 2.0 + j.N * nc * j.digits * 32.0 +
          (double)j.lanes * (j.N + std::max(0, j.m_hi - j.m_lo)) * 8.0;
   }
   for (const int4& it : L.items) {
@@ -473,6 +478,8 @@ double launch_algorithmic_bytes(const StepLaunch& L, const CaseDev* cases) {
       case K_SPL_X1_BOX: v = 6 * mxc * 8 + 2 * nx * 8 + 8 * nx * 14; break;
       case K_SPL_X1_PER: v = 6 * mx * 16 + 8 * nx * 14; break;
       case K_SPL_PROD: v = 8 * nx * 8 + 2 * nx * 8 + 3 * nx * 14; break;
+      case K_SPL_X3: v = 2 * mxc * 8 + nx * 8 + mxc * 18; break;
+      case K_SPL_W: v = mxc * (8 + 18); break;
       case K_SPL_Q: v = 3 * ny * 8 + 3 * ny * 14; break;
       default: v = 0;
     }
@@ -483,8 +490,7 @@ double launch_algorithmic_bytes(const StepLaunch& L, const CaseDev* cases) {
 
 cudaError_t launch_gate(const CaseDev* cases, const int* members, int n, cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
-  dev::k_gate<<<(n + 127) / 128, 128, 0, s>>>(cases, members, n);
-  return cudaGetLastError();
+  return launch_pdl(dev::k_gate, (n + 127) / 128, 128, 0, s, cases, members, n);
 }
 
 const char* step_kernel_name(int kernel) {
@@ -498,7 +504,7 @@ const char* step_kernel_name(int kernel) {
                                 "lanes_periodic_y2b", "lanes_periodic_y2c", "state_f32", "periodic_x_mixed_t128",
                                 "lanes_periodic_y2_fused", "box_y4_mix", "split_y1_real", "split_y1_complex",
                                 "split_x1_box", "split_x1_periodic", "split_products", "split_conv",
-                                "periodic_y2_cv", "box_y2_cv"};
+                                "periodic_y2_cv", "box_y2_cv", "split_x3", "split_poisson_rows"};
   if (kernel == K_GEMM) return "lane_gemm";
   if (kernel == K_SPLIT_GEMM) return "split_gemm";
   if (kernel >= 0 && kernel < K_NUM_STEP_KERNELS) return names[kernel];

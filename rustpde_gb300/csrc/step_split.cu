@@ -27,6 +27,7 @@
 #include <stdexcept>
 
 #include "lane_ops.cuh"
+#include "pdl.cuh"
 #include "per_device.h"
 #include "prims.h"
 #include "split_emit.cuh"
@@ -38,6 +39,7 @@ namespace dev {
 // S1: row i of ux, uy, temp.  Lanes i L + (2 f + which) P + part: L = 6 P, P parts.
 template <class T>
 __global__ void __launch_bounds__(256) k_spl_y1(const CaseDev* __restrict__ cases, const int4* __restrict__ work) {
+  pdl_enter();
   const int4 w = work[blockIdx.x];
   const CaseDev& c = cases[w.x];
   if (c.gate != nullptr && c.gate[1] == 0) return;  // case idle this step (serving)
@@ -55,7 +57,7 @@ __global__ void __launch_bounds__(256) k_spl_y1(const CaseDev* __restrict__ case
     for (int k = tid; k < myc; k += nth) IN[f * ld + k] = f3[f][(size_t)i * myc + k];
   __syncthreads();
   to_ortho<T>(c.ycd, IN, ld, O, ld, 3, tid, nth);
-  cheb_diff<T>(O, ld, D, ld, ny, 3, 1, nullptr, 0, tid, nth);
+  cheb_diff<T>(c.odd, O, ld, D, ld, ny, 3, 1, nullptr, 0, tid, nth);
   const double* base = reinterpret_cast<const double*>(O);
   auto lane = [&](int r) {  // r = (2 f + which) P + part
     const int part = P == 2 ? r & 1 : 0, l = P == 2 ? r >> 1 : r;
@@ -72,6 +74,7 @@ static size_t smem_spl_y1(const CaseDev& c) {
 
 // S2, box: column j.  Lanes 8 j + (u, v, then for ux, uy, temp: d/dx, d/dy).
 __global__ void __launch_bounds__(256) k_spl_x1_box(const CaseDev* __restrict__ cases, const int4* __restrict__ work) {
+  pdl_enter();
   const int4 w = work[blockIdx.x];
   const CaseDev& c = cases[w.x];
   if (c.gate != nullptr && c.gate[1] == 0) return;  // case idle this step (serving)
@@ -98,7 +101,7 @@ __global__ void __launch_bounds__(256) k_spl_x1_box(const CaseDev* __restrict__ 
     for (int k = tid; k < nx; k += nth) OR[l * ld + k] = stencil_at(b, IN + l * ld, k);
   }
   __syncthreads();
-  cheb_diff<double>(OR, ld, D, ld, nx, 4, 1, nullptr, 0, tid, nth);
+  cheb_diff<double>(c.odd, OR, ld, D, ld, nx, 4, 1, nullptr, 0, tid, nth);
   double* gp = static_cast<double*>(c.s[0]);  // d/dx p0 / aspect
   for (int l = 0; l < 3; l++)
     for (int k = tid; k < nx; k += nth) D[l * ld + k] *= inv_asp;
@@ -116,6 +119,7 @@ static size_t smem_spl_x1_box(const CaseDev& c) { return (size_t)18 * (c.nx + 1)
 
 // S2, periodic: the same lanes from i k / aspect and the y derivatives.
 __global__ void __launch_bounds__(256) k_spl_x1_per(const CaseDev* __restrict__ cases, const int4* __restrict__ work) {
+  pdl_enter();
   const int4 w = work[blockIdx.x];
   const CaseDev& c = cases[w.x];
   if (c.gate != nullptr && c.gate[1] == 0) return;  // case idle this step (serving)
@@ -148,6 +152,7 @@ static size_t smem_spl_x1_per(const CaseDev& c) { return (size_t)8 * c.mx * 16 +
 
 // S3: products of column j -> digits of their forward x transform, lanes 3 j + f
 __global__ void __launch_bounds__(256) k_spl_prod(const CaseDev* __restrict__ cases, const int4* __restrict__ work) {
+  pdl_enter();
   const int4 w = work[blockIdx.x];
   const CaseDev& c = cases[w.x];
   if (c.gate != nullptr && c.gate[1] == 0) return;  // case idle this step (serving)
@@ -186,6 +191,7 @@ static size_t smem_spl_prod(const CaseDev& c) { return (size_t)3 * (c.nx + 1) * 
 
 // S4: row e of the x-transformed products -> digits of the forward y transform, lanes 3 e + f
 __global__ void __launch_bounds__(256) k_spl_q(const CaseDev* __restrict__ cases, const int4* __restrict__ work) {
+  pdl_enter();
   const int4 w = work[blockIdx.x];
   const CaseDev& c = cases[w.x];
   if (c.gate != nullptr && c.gate[1] == 0) return;  // case idle this step (serving)
@@ -314,6 +320,32 @@ bool split_step_size(const CaseDev& c) {
   return c.nx * c.ny >= (fast ? 48000 : 9000);
 }
 
+SplitJobDev split_mat_job(const SplitLanesDev& s, const SplitMatDev& m, int lanes, double* out, long long es,
+                          unsigned int* status) {
+  SplitJobDev j{};
+  j.dig = s.dig;
+  j.ex = s.ex;
+  j.w = j.w16 = m.w16;
+  j.out = out;
+  j.status = status;
+  j.es = es;
+  j.lanes = lanes;
+  j.nf = 1;
+  j.parts = 1;
+  j.qs = 1;
+  j.ctot = s.cE + s.cO;
+  j.nc[0] = s.cE;
+  j.c0[1] = s.cE;
+  j.nc[1] = s.cO;
+  j.N = m.N;
+  j.ex_bias = split_ex_bias9();
+  j.digits = 9;
+  j.rowex = m.rowex;
+  return j;
+}
+
+bool split_eig_size(const CaseDev& c) { return c.kind != KIND_PERIODIC && c.nx >= 160 && c.nx <= 514; }
+
 void add_split_launches(const CaseDev& c, bool on, StepPlan& p) {
   const bool per = c.kind == KIND_PERIODIC;
   const int P = per ? 2 : 1;
@@ -352,6 +384,7 @@ void add_split_launches(const CaseDev& c, bool on, StepPlan& p) {
     j.nc[1] = s.cO;
     j.N = op.N;
     j.ex_bias = split_ex_bias(shl, op.wshift);
+    j.digits = kSplitDigits;
     return j;
   };
   // one list of a forward transform: terms E (par 0) or O (par 1)
@@ -421,12 +454,12 @@ cudaError_t launch_step_split_kernel(int kernel, int nblocks, size_t smem, cudaS
                                      const int4* work) {
   const dim3 g(nblocks), b(256);
   switch (kernel) {
-    case K_SPL_Y1_R: dev::k_spl_y1<double><<<g, b, smem, s>>>(cases, work); break;
-    case K_SPL_Y1_C: dev::k_spl_y1<double2><<<g, b, smem, s>>>(cases, work); break;
-    case K_SPL_X1_BOX: dev::k_spl_x1_box<<<g, b, smem, s>>>(cases, work); break;
-    case K_SPL_X1_PER: dev::k_spl_x1_per<<<g, b, smem, s>>>(cases, work); break;
-    case K_SPL_PROD: dev::k_spl_prod<<<g, b, smem, s>>>(cases, work); break;
-    case K_SPL_Q: dev::k_spl_q<<<g, b, smem, s>>>(cases, work); break;
+    case K_SPL_Y1_R: return launch_pdl(dev::k_spl_y1<double>, g, b, smem, s, cases, work);
+    case K_SPL_Y1_C: return launch_pdl(dev::k_spl_y1<double2>, g, b, smem, s, cases, work);
+    case K_SPL_X1_BOX: return launch_pdl(dev::k_spl_x1_box, g, b, smem, s, cases, work);
+    case K_SPL_X1_PER: return launch_pdl(dev::k_spl_x1_per, g, b, smem, s, cases, work);
+    case K_SPL_PROD: return launch_pdl(dev::k_spl_prod, g, b, smem, s, cases, work);
+    case K_SPL_Q: return launch_pdl(dev::k_spl_q, g, b, smem, s, cases, work);
     default: return cudaErrorInvalidValue;
   }
   return cudaGetLastError();

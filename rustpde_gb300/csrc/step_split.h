@@ -31,6 +31,11 @@ bool split_step_size(const CaseDev& c);
 // The launches up to the convection term m_cv (S1, GEMM, S2, GEMM, S3, GEMM, S4, GEMM)
 // (on = false: the same launches without work)
 void add_split_launches(const CaseDev& c, bool on, StepPlan& p);
+// out[r es + lane] = the matrix applied to nine-digit lanes
+SplitJobDev split_mat_job(const SplitLanesDev& s, const SplitMatDev& m, int lanes, double* out, long long es,
+                          unsigned int* status);
+// Whether a box of this size also runs its Poisson eigenbasis products so.
+bool split_eig_size(const CaseDev& c);
 cudaError_t configure_step_split_kernels();
 cudaError_t launch_step_split_kernel(int kernel, int nblocks, size_t smem, cudaStream_t s, const CaseDev* cases,
                                      const int4* work);
