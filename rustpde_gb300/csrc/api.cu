@@ -236,67 +236,6 @@ static const float* shared_op(const std::string& key, Make make) {
   g_shared_ops.emplace(std::make_pair(dev, key), p);
   return p;
 }
-// The split operator of a transform (step_split.h) on the current device,
-// shared like the mixed operators by every case of the size.
-static SplitOpDev shared_split_op(int kind, int n, int rows) {
-  static std::mutex mu;
-  static std::map<std::tuple<int, int, int, int>, SplitOpDev> cache;
-  int dev = 0;
-  cuda_check(cudaGetDevice(&dev), "cudaGetDevice");
-  std::lock_guard<std::mutex> lk(mu);
-  const auto key = std::make_tuple(dev, kind, n, rows);
-  auto it = cache.find(key);
-  if (it != cache.end()) return it->second;
-  SplitOpDev d{};
-  const SplitOp op = make_split_op(kind, n, rows, &d.wshift);
-  d.N = op.N;
-  const size_t n32 = (op.bytes.size() + 127) & ~size_t(127);
-  unsigned char* p = nullptr;
-  cuda_check(cudaMalloc(&p, n32 + op.bytes16.size()), "cudaMalloc shared operator");
-  cudaError_t e = cudaMemcpy(p, op.bytes.data(), op.bytes.size(), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(p + n32, op.bytes16.data(), op.bytes16.size(), cudaMemcpyHostToDevice);
-  if (e != cudaSuccess) {
-    cudaFree(p);
-    cuda_check(e, "upload shared operator");
-  }
-  d.w = p;
-  d.w16 = p + n32;
-  return cache.emplace(key, d).first->second;
-}
-
-// The Poisson eigenbasis matrices of a basis and length in nine digits.
-static SplitMatDev shared_split_mat(int kind, int n, bool fwd) {
-  static std::mutex mu;
-  static std::map<std::tuple<int, int, int, bool>, SplitMatDev> cache;
-  int dev = 0;
-  cuda_check(cudaGetDevice(&dev), "cudaGetDevice");
-  std::lock_guard<std::mutex> lk(mu);
-  const auto key = std::make_tuple(dev, kind, n, fwd);
-  auto it = cache.find(key);
-  if (it != cache.end()) return it->second;
-  std::vector<double> F, B;
-  poisson_eigenbasis(make_basis(kind, n), F, B);
-  const SplitMat m = pack_split_mat(fwd ? F : B, n - 2);
-  const size_t nb = (m.bytes16.size() + 127) & ~size_t(127), ne = (size_t)m.N * 4;
-  unsigned char* p = nullptr;
-  cuda_check(cudaMalloc(&p, nb + 2 * ne), "cudaMalloc shared operator");
-  cudaError_t e = cudaMemcpy(p, m.bytes16.data(), m.bytes16.size(), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(p + nb, m.colex.data(), ne, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(p + nb + ne, m.rowex.data(), ne, cudaMemcpyHostToDevice);
-  if (e != cudaSuccess) {
-    cudaFree(p);
-    cuda_check(e, "upload shared operator");
-  }
-  SplitMatDev d{};
-  d.w16 = p;
-  d.colex = reinterpret_cast<const int*>(p + nb);
-  d.rowex = reinterpret_cast<const int*>(p + nb + ne);
-  d.N = m.N;
-  d.K0 = m.K[0];
-  d.K1 = m.K[1];
-  return cache.emplace(key, d).first->second;
-}
-
 static std::vector<float> pack_blocks(std::initializer_list<std::pair<const LMat*, long double>> blocks,
                                       int ntmax = 64) {
   int rows = 0, cols = -1;
@@ -382,7 +321,22 @@ struct FsLanes {
   // mixed form: packed split operators per FS_OP_* (device)
   const float* w[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
   unsigned int* d_status = nullptr;
+  // FP64 transforms as split GEMMs (dense lengths): scratch for kSplitLanesCap
+  // lanes at a time.  It is the handle's, and calls may come from several
+  // threads and on several streams: the mutex orders them, and a call on
+  // another stream than the last one waits for that one's event.
+  std::mutex mu;
+  SplitWork work;
+  void* work_mem = nullptr;
+  cudaEvent_t done = nullptr;
+  cudaStream_t last = nullptr;
+  bool used = false;
+  ~FsLanes() {
+    if (done) cudaEventDestroy(done);
+    if (work_mem) cudaFree(work_mem);
+  }
 };
+constexpr int kSplitLanesCap = 4096;
 
 struct SvSolver {
   FsSpace* space = nullptr;
@@ -631,8 +585,8 @@ void build_case(RbcCase* c, bool with_graph = true, char* state_region = nullptr
     }
     if (split_eig_size(h)) {
       h.split_eig = 1;
-      h.smat_f = shared_split_mat(c->sp_p1.hb0.kind, nx, true);
-      h.smat_b = shared_split_mat(c->sp_p1.hb0.kind, nx, false);
+      h.smat_f = shared_split_mat(c->sp_p1.hb0.kind, nx, true, true);
+      h.smat_b = shared_split_mat(c->sp_p1.hb0.kind, nx, true, false);
       h.spl_z.cE = h.spl_w.cE = split_chunks(h.smat_f.K0);
       h.spl_z.cO = h.spl_w.cO = split_chunks(h.smat_f.K1);
       db = std::max(db, split_dig_bytes(ny, h.spl_z.cE, h.spl_z.cO, 9));
@@ -2163,6 +2117,7 @@ int fs_space_create(int base0, int n0, int base1, int n1, FsSpace** out) {
   cuda_check(configure_prim_kernels(), "configure kernels");
   std::unique_ptr<FsSpace> s(new FsSpace());
   build_space(s->arena, s->s, base0, n0, base1, n1);
+  attach_split(s->arena, s->s);
   s->tmp = s->arena.alloc(tmp_elems(s->s) * 16);
   *out = s.release();
   API_END
@@ -2282,6 +2237,18 @@ int fs_lanes_create(int base, int n, int precision, FsLanes** out) {
   p->precision = precision;
   build_lanes(p->arena, p->L, base, n);
   p->d_status = static_cast<unsigned int*>(p->arena.alloc(16));
+  if (precision == RBC_PREC_FP64 && lanes_attach_split(p->L)) {
+    const size_t db = (split_dig_bytes(kSplitLanesCap, split_chunks((n + 1) / 2), split_chunks(n / 2)) + 255) & ~size_t(255);
+    const size_t be = (size_t)kSplitLanesCap * 4, bb = (size_t)kSplitLanesCap * n * 8;
+    cuda_check(cudaMalloc(&p->work_mem, db + be + bb), "cudaMalloc lane scratch");
+    char* q = static_cast<char*>(p->work_mem);
+    p->work.dig = reinterpret_cast<unsigned char*>(q);
+    p->work.ex = reinterpret_cast<int*>(q + db);
+    p->work.buf = reinterpret_cast<double*>(q + db + be);
+    p->work.lanes = kSplitLanesCap;
+    p->work.status = p->d_status;
+    cuda_check(cudaEventCreateWithFlags(&p->done, cudaEventDisableTiming), "event");
+  }
   if (precision == RBC_PREC_MIXED) {
     const HostBasis& hb = p->L.hb;
     LMat S = lm_stencil(hb), P = lm_from_ortho(hb);
@@ -2338,7 +2305,26 @@ int fs_lanes_apply(FsLanes* p, int op, const double* d_in, double* d_out, int la
   if (op == FS_OP_HHOLTZ) require(p->L.has_solver, "fs_lanes_apply: call fs_lanes_set_hholtz first");
   cudaStream_t st = (cudaStream_t)stream;
   if (p->precision == RBC_PREC_FP64) {
-    lanes_apply(p->L, op, d_in, d_out, lanes, st);
+    // (a captured call keeps to the pass without scratch: its replays are not
+    // ordered with other calls on the handle)
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    const bool split = p->work_mem != nullptr && lanes_split_pays(p->L, op, lanes) &&
+                       cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone;
+    if (!split) {
+      (void)cudaGetLastError();
+      lanes_apply(p->L, op, d_in, d_out, lanes, st);
+    } else {
+      int il, ol;
+      lane_op_lengths(p->L, op, &il, &ol);
+      std::lock_guard<std::mutex> lk(p->mu);
+      if (p->used && p->last != st) cuda_check(cudaStreamWaitEvent(st, p->done, 0), "lane scratch");
+      for (int l = 0; l < lanes; l += kSplitLanesCap)
+        lanes_apply(p->L, op, d_in + (size_t)l * il, d_out + (size_t)l * ol, std::min(kSplitLanesCap, lanes - l), st,
+                    &p->work);
+      cuda_check(cudaEventRecord(p->done, st), "lane scratch");
+      p->last = st;
+      p->used = true;
+    }
   } else {
     int il, ol;
     lane_op_lengths(p->L, op, &il, &ol);

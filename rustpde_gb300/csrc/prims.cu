@@ -5,6 +5,8 @@
 #include <stdexcept>
 
 #include "lane_ops.cuh"
+#include "split_emit.cuh"
+#include "step_split.h"
 #include "per_device.h"
 #include "prims.h"
 
@@ -415,10 +417,10 @@ std::vector<Band4> hholtz_rows(const HostBasis& bx, const HostBasis& by, double 
   return rows;
 }
 
-void poisson_eigenbasis(const HostBasis& b, std::vector<double>& fwd, std::vector<double>& bwd) {
+void tensor_eigenbasis(const HostBasis& b, bool poisson, std::vector<double>& fwd, std::vector<double>& bwd) {
   std::string err;
   // (the y basis enters the row factors only)
-  hholtz_rows(b, b, 1.0, 1.0, 0.0, true, nullptr, &fwd, &bwd, &err);
+  hholtz_rows(b, b, 1.0, 1.0, poisson ? 0.0 : 1.0, poisson, nullptr, &fwd, &bwd, &err);
 }
 
 std::vector<double> transposed(const std::vector<double>& a, int n) {
@@ -426,6 +428,43 @@ std::vector<double> transposed(const std::vector<double>& a, int n) {
   for (int i = 0; i < n; i++)
     for (int j = 0; j < n; j++) t[(size_t)j * n + i] = a[(size_t)i * n + j];
   return t;
+}
+
+// A dense product of `lanes` lanes of n terms as a split GEMM (digits, GEMM and,
+// for a forward transform, the rest of the pass as launches of their own)
+// against inside the pass.  The split form costs about 25 us of launches and
+// latency; the product inside the pass reaches that near 4e6 multiply-adds of
+// the unfolded matrix (264 lanes of 128, or 100 of 200).
+constexpr int kSplitMatMax = 514;  // longest axis of a nine-digit matrix (two lists of 256 terms)
+static bool split_pays(int lanes, int n) { return n >= 48 && (double)lanes * n * n >= 4e6; }
+
+static bool split_fits(const ChebXformDev& c) { return c.n >= 48 && c.n <= 640 && !c.use_fft; }
+static void split_ops(ChebXformDev& c) {
+  c.sop_b = shared_split_op(SOP_CHEB_BWD, c.n, 0);
+  c.sop_f[0] = shared_split_op(SOP_CHEB_FWD_E, c.n, c.n);
+  c.sop_f[1] = shared_split_op(SOP_CHEB_FWD_O, c.n, c.n);
+}
+
+void attach_split(Arena& a, SpaceDev& s) {
+  const bool x = !s.cplx && split_fits(s.c0) && split_pays(s.phys1, s.c0.n), y = split_fits(s.c1) && split_pays(s.phys0, s.c1.n);
+  const bool mat = !s.cplx && s.hb0.composite() && !s.hb0.bc() && s.hb0.n <= kSplitMatMax && split_pays(s.phys1, s.spec0);
+  if (!x && !y && !mat) return;
+  if (x) split_ops(s.c0);
+  if (y) split_ops(s.c1);
+  size_t db = 0;
+  auto need = [&](int lanes, int n, int digits) {
+    db = std::max(db, split_dig_bytes(lanes, split_chunks((n + 1) / 2), split_chunks(n / 2), digits));
+  };
+  if (x) need(s.phys1, s.phys0, kSplitDigits);
+  if (y) need(s.phys0, s.phys1, kSplitDigits);
+  if (mat) need(s.phys1, s.phys0, 9);
+  s.work.lanes = std::max(s.phys0, s.phys1);
+  const size_t be = ((size_t)s.work.lanes * 4 + 255) & ~size_t(255), bb = (size_t)s.phys0 * s.phys1 * 8;
+  db = (db + 255) & ~size_t(255);
+  char* p = static_cast<char*>(a.alloc(db + be + bb));
+  s.work.dig = reinterpret_cast<unsigned char*>(p);
+  s.work.ex = reinterpret_cast<int*>(p + db);
+  s.work.buf = reinterpret_cast<double*>(p + db + be);
 }
 
 bool build_solver(Arena& a, const SpaceDev& s, int kind, const double c[2], SolverDev& out, std::string* err) {
@@ -453,6 +492,10 @@ bool build_solver(Arena& a, const SpaceDev& s, int kind, const double c[2], Solv
     if (out.dense) {
       out.fwd = a.upload(transposed(fwd, out.m0));
       out.bwd = a.upload(transposed(bwd, out.m0));
+      if (s.work.dig != nullptr && s.hb0.n <= kSplitMatMax && split_pays(s.ortho1, out.m0)) {
+        out.smat_f = shared_split_mat(s.hb0.kind, s.hb0.n, kind == SV_KIND_POISSON, true);
+        out.smat_b = shared_split_mat(s.hb0.kind, s.hb0.n, kind == SV_KIND_POISSON, false);
+      }
     }
     return true;
   } catch (std::exception& e) {
@@ -490,6 +533,7 @@ struct PassDesc {
   const void* add;  // P_ADD: A[k] += add[lane*add_ls + k] (complex when in_cplx)
   long long add_ls;
   int odd;          // blocks of the derivative's running sums (scan_block)
+  SplitMatDev smat;  // P_DENSE in nine digits, or null
 };
 
 namespace dev {
@@ -511,24 +555,17 @@ __device__ __forceinline__ T pass_load(const void* p, int cplx, long long off, l
   else return cplx ? static_cast<const double2*>(p)[off] : c2(static_cast<const double*>(p)[off], 0.0);
 }
 
+// load lane `lane` (and with PAIR its neighbour) and run the first nops operations on it
 template <class T, int PAIR>
-__global__ void __launch_bounds__(128) k_pass(const __grid_constant__ PassDesc d) {
-  const int lane = PAIR ? 2 * blockIdx.x : blockIdx.x;
-  const bool two = PAIR && lane + 1 < d.lanes;
-  const int tid = threadIdx.x, nth = blockDim.x;
-  extern __shared__ double2 sm[];
-  double2* WA = sm;
-  double2* WB = WA + d.wl;
-  T* A = reinterpret_cast<T*>(WB + d.wl);
-  T* B = A + d.lmax;
-  T* Q = B + d.lmax;
-  int len = d.in_len;
+__device__ __forceinline__ void pass_ops(const PassDesc& d, int lane, bool two, int nops, T*& A, T*& B, T*& Q,
+                                         double2* WA, double2* WB, int& len, int tid, int nth) {
+  len = d.in_len;
   for (int k = tid; k < len; k += nth) {
     const long long off = lane * d.in_ls + k * d.in_es;
     A[k] = pass_load<T, PAIR>(d.in, d.in_cplx, off, off + d.in_ls, two);
   }
   __syncthreads();
-  for (int o = 0; o < d.nops; o++) {
+  for (int o = 0; o < nops; o++) {
     const PassOp op = d.ops[o];
     switch (op.code) {
       case P_TO_ORTHO:
@@ -613,6 +650,21 @@ __global__ void __launch_bounds__(128) k_pass(const __grid_constant__ PassDesc d
         break;
     }
   }
+}
+
+template <class T, int PAIR>
+__global__ void __launch_bounds__(128) k_pass(const __grid_constant__ PassDesc d) {
+  const int lane = PAIR ? 2 * blockIdx.x : blockIdx.x;
+  const bool two = PAIR && lane + 1 < d.lanes;
+  const int tid = threadIdx.x, nth = blockDim.x;
+  extern __shared__ double2 sm[];
+  double2* WA = sm;
+  double2* WB = WA + d.wl;
+  T* A = reinterpret_cast<T*>(WB + d.wl);
+  T* B = A + d.lmax;
+  T* Q = B + d.lmax;
+  int len;
+  pass_ops<T, PAIR>(d, lane, two, d.nops, A, B, Q, WA, WB, len, tid, nth);
   for (int k = tid; k < len; k += nth) {
     const long long off = lane * d.out_ls + k * d.out_es;
     if constexpr (PAIR) {
@@ -627,6 +679,39 @@ __global__ void __launch_bounds__(128) k_pass(const __grid_constant__ PassDesc d
       }
       static_cast<double*>(d.out)[off] = first_part<T>(A[k]);
     }
+  }
+}
+
+// The operations before a dense product (nops of them), then the lane's digits:
+// code P_DCT_BWD: coefficients (even, odd); P_DCT_FWD: folded values; P_DENSE:
+// nine digits.  One real lane per CTA.
+__global__ void __launch_bounds__(128) k_pass_digits(const __grid_constant__ PassDesc d, const int nops, const int code,
+                                                     const SplitLanesDev S) {
+  const int lane = blockIdx.x, tid = threadIdx.x, nth = blockDim.x;
+  extern __shared__ double2 sm[];
+  double* A = reinterpret_cast<double*>(sm);
+  double* B = A + d.lmax;
+  double* Q = B + d.lmax;
+  int* em = reinterpret_cast<int*>(Q + d.lmax);
+  int len;
+  pass_ops<double, 0>(d, lane, false, nops, A, B, Q, nullptr, nullptr, len, tid, nth);
+  if (code == P_DENSE) {
+    split_emit9(S, lane, 1, len, d.smat.K0, d.smat.colex, [&](int, int k) { return A[k]; }, em, tid, nth);
+  } else if (code == P_DCT_BWD) {
+    split_emit(
+        S, lane, 1, len, (len + 1) >> 1, len >> 1, kSplitShlValue, [&](int, int k) { return A[k]; },
+        [&](int, int list, int k, auto fix) { return fix(A[2 * k + list]); }, em, tid, nth);
+  } else {
+    const int N = len - 1;
+    split_emit(
+        S, lane, 1, len, (len + 1) >> 1, len >> 1, kSplitShlSum, [&](int, int k) { return A[k]; },
+        [&](int, int list, int k, auto fix) {
+          const long long u = fix(A[k]);
+          if (2 * k == N) return u;
+          const long long v = fix(A[N - k]);
+          return list ? u - v : u + v;
+        },
+        em, tid, nth);
   }
 }
 
@@ -708,7 +793,7 @@ static size_t pass_smem_used(const PassDesc& d, size_t elem) {
 
 // Real lanes run as pairs where the pairs still give every SM two CTAs and no
 // operation has factors per lane (a pair shares them), else one by one.
-static void run_pass(PassDesc& d, cudaStream_t st) {
+static void run_pass_whole(const PassDesc& d, cudaStream_t st) {
   bool real = !d.in_cplx && !d.out_cplx, per_lane = false;
   for (int k = 0; k < d.nops; k++) {
     const int code = d.ops[k].code;
@@ -721,6 +806,72 @@ static void run_pass(PassDesc& d, cudaStream_t st) {
     dev::k_pass<double2, 1><<<(d.lanes + 1) / 2, 128, pass_smem_used(d, 16), st>>>(d);
   else dev::k_pass<double, 0><<<d.lanes, 128, pass_smem_used(d, 8), st>>>(d);
   cuda_check(cudaGetLastError(), "pass kernel launch");
+}
+
+// A pass whose dense product is worth it runs as digits, split GEMM and the rest.
+// The FP64 pipe bounds a dense product inside a pass; as a split GEMM it leaves
+// launches and copies.  264 lanes of 264, backward: 48 -> 28 us (digits 10, GEMM
+// 18); 4096 lanes of 128, backward: 68 -> 33 us (20, 13), forward with
+// from_ortho: 80 -> 58 us (17, 15, 26); the eigenbasis product of 254 lanes of
+// 255: 53 -> 29 us (11, 18).
+static void run_pass(const PassDesc& d, cudaStream_t st, const SplitWork* w = nullptr) {
+  int at = -1;
+  if (w != nullptr && w->dig != nullptr && !d.in_cplx && !d.out_cplx && d.lanes <= w->lanes)
+    for (int k = 0; k < d.nops; k++) {
+      const int code = d.ops[k].code;
+      if (code == P_FDIFF || code == P_R2C || code == P_C2R || code == P_FDMA) { at = -1; break; }
+      if (code == P_DCT_FWD && d.cx.sop_f[0].w != nullptr) at = k;
+      if (code == P_DCT_BWD && d.cx.sop_b.w != nullptr) at = k;
+      if (code == P_DENSE && d.smat.w16 != nullptr) at = k;
+    }
+  if (at >= 0 && d.cx.fwd_full != nullptr && d.ops[at].code != P_DENSE) at = -1;
+  if (at < 0) {
+    run_pass_whole(d, st);
+    return;
+  }
+  const int code = d.ops[at].code;
+  const bool dense = code == P_DENSE, last = at + 1 == d.nops;
+  const int n = dense ? d.dense_cols : d.cx.n;
+  SplitLanesDev S{};
+  S.dig = w->dig;
+  S.ex = w->ex;
+  S.cE = split_chunks(dense ? d.smat.K0 : (n + 1) / 2);
+  S.cO = split_chunks(dense ? d.smat.K1 : n / 2);
+  dev::k_pass_digits<<<d.lanes, 128, (size_t)3 * d.lmax * 8 + 64, st>>>(d, at, code, S);
+  cuda_check(cudaGetLastError(), "pass kernel launch");
+  // the product: into the output, or into buf for the rest of the pass (lanes
+  // adjacent where they are in the output)
+  const bool adj = d.out_ls == 1;
+  double* out = last ? static_cast<double*>(d.out) : w->buf;
+  const long long ls = last ? d.out_ls : adj ? 1 : n, es = last ? d.out_es : adj ? d.lanes : 1;
+  SplitJobDev j[2];
+  int nj = 1;
+  if (dense) {
+    j[0] = split_mat_job(S, d.smat, d.lanes, out, es, w->status);
+    j[0].qs = ls;
+  } else if (code == P_DCT_BWD) {
+    j[0] = split_op_job(S, d.cx.sop_b, d.lanes, kSplitShlValue, out, ls, es, w->status);
+    j[0].mirror = n - 1;
+    j[0].m_hi = n / 2;
+  } else {
+    for (int par = 0; par < 2; par++) {
+      j[par] = split_op_job(S, d.cx.sop_f[par], d.lanes, kSplitShlSum, out + par * es, ls, 2 * es, w->status);
+      j[par].c0[0] = par ? S.cE : 0;
+      j[par].nc[0] = par ? S.cO : S.cE;
+      j[par].nc[1] = 0;
+    }
+    nj = 2;
+  }
+  cuda_check(launch_split_gemm_one(j, nj, st), "split gemm launch");
+  if (last) return;
+  PassDesc e = d;
+  e.in = w->buf;
+  e.in_len = n;
+  e.in_ls = ls;
+  e.in_es = es;
+  e.nops = 0;
+  for (int k = at + 1; k < d.nops; k++) e.ops[e.nops++] = d.ops[k];
+  run_pass_whole(e, st);
 }
 
 static PassDesc base_desc(const SpaceDev& s);
@@ -767,7 +918,7 @@ void space_forward(const SpaceDev& s, const double* phys, void* spec, void* tmp,
   d.cx = s.c1; d.basis = s.b1;
   add_op(d, P_DCT_FWD);
   if (s.hb1.composite()) add_op(d, P_FROM_ORTHO);
-  run_pass(d, st);
+  run_pass(d, st, &s.work);
   PassDesc e = base_desc(s);
   set_axis0(e, tmp, 0, spec, s.cplx, s.spec1, s.phys0);
   if (s.cplx) { e.fx = s.f0; add_op(e, P_R2C); }
@@ -776,7 +927,7 @@ void space_forward(const SpaceDev& s, const double* phys, void* spec, void* tmp,
     add_op(e, P_DCT_FWD);
     if (s.hb0.composite()) add_op(e, P_FROM_ORTHO);
   }
-  run_pass(e, st);
+  run_pass(e, st, &s.work);
 }
 
 void axis0_forward(const SpaceDev& s, const double* in, void* out, int cols, cudaStream_t st) {
@@ -788,7 +939,7 @@ void axis0_forward(const SpaceDev& s, const double* in, void* out, int cols, cud
     add_op(e, P_DCT_FWD);
     if (s.hb0.composite()) add_op(e, P_FROM_ORTHO);
   }
-  run_pass(e, st);
+  run_pass(e, st, &s.work);
 }
 
 void space_backward(const SpaceDev& s, const void* spec, double* phys, void* tmp, cudaStream_t st) {
@@ -800,13 +951,13 @@ void space_backward(const SpaceDev& s, const void* spec, double* phys, void* tmp
     if (s.hb0.composite()) add_op(d, P_TO_ORTHO);
     add_op(d, P_DCT_BWD);
   }
-  run_pass(d, st);
+  run_pass(d, st, &s.work);
   PassDesc e = base_desc(s);
   set_axis1(e, tmp, 0, phys, 0, s.phys0, s.spec1, s.phys1);
   e.cx = s.c1; e.basis = s.b1;
   if (s.hb1.composite()) add_op(e, P_TO_ORTHO);
   add_op(e, P_DCT_BWD);
-  run_pass(e, st);
+  run_pass(e, st, &s.work);
 }
 
 // backward(gradient(f)) on the physical grid in two passes, the field read
@@ -827,7 +978,7 @@ void space_gradient_physical(const SpaceDev& s, const void* spec, double* phys, 
     add_op(d, P_DIFF, d0);
     add_op(d, P_DCT_BWD);
   }
-  run_pass(d, st);
+  run_pass(d, st, &s.work);
   PassDesc e = base_desc(s);
   set_axis1(e, tmp, 0, phys, 0, s.phys0, s.spec1, s.phys1);
   e.cx = s.c1; e.basis = s.b1;
@@ -841,7 +992,7 @@ void space_gradient_physical(const SpaceDev& s, const void* spec, double* phys, 
     add_op(e, P_SCALE);
   }
   add_op(e, P_DCT_BWD);
-  run_pass(e, st);
+  run_pass(e, st, &s.work);
 }
 
 void space_backward_ortho(const SpaceDev& s, const void* ortho, double* phys, void* tmp, cudaStream_t st) {
@@ -849,12 +1000,12 @@ void space_backward_ortho(const SpaceDev& s, const void* ortho, double* phys, vo
   set_axis0(d, ortho, s.cplx, tmp, 0, s.ortho1, s.ortho0);
   if (s.cplx) { d.fx = s.f0; add_op(d, P_C2R); }
   else { d.cx = s.c0; add_op(d, P_DCT_BWD); }
-  run_pass(d, st);
+  run_pass(d, st, &s.work);
   PassDesc e = base_desc(s);
   set_axis1(e, tmp, 0, phys, 0, s.phys0, s.ortho1, s.phys1);
   e.cx = s.c1;
   add_op(e, P_DCT_BWD);
-  run_pass(e, st);
+  run_pass(e, st, &s.work);
 }
 
 void space_to_ortho(const SpaceDev& s, const void* spec, void* ortho, void* tmp, cudaStream_t st) {
@@ -862,12 +1013,12 @@ void space_to_ortho(const SpaceDev& s, const void* spec, void* ortho, void* tmp,
   set_axis0(d, spec, s.cplx, tmp, s.cplx, s.spec1, s.spec0);
   d.basis = s.b0;
   add_op(d, P_TO_ORTHO);
-  run_pass(d, st);
+  run_pass(d, st, &s.work);
   PassDesc e = base_desc(s);
   set_axis1(e, tmp, s.cplx, ortho, s.cplx, s.ortho0, s.spec1, s.ortho1);
   e.basis = s.b1;
   add_op(e, P_TO_ORTHO);
-  run_pass(e, st);
+  run_pass(e, st, &s.work);
 }
 
 void space_from_ortho(const SpaceDev& s, const void* ortho, void* spec, void* tmp, cudaStream_t st) {
@@ -875,12 +1026,12 @@ void space_from_ortho(const SpaceDev& s, const void* ortho, void* spec, void* tm
   set_axis0(d, ortho, s.cplx, tmp, s.cplx, s.ortho1, s.ortho0);
   d.basis = s.b0;
   add_op(d, P_FROM_ORTHO);
-  run_pass(d, st);
+  run_pass(d, st, &s.work);
   PassDesc e = base_desc(s);
   set_axis1(e, tmp, s.cplx, spec, s.cplx, s.spec0, s.ortho1, s.spec1);
   e.basis = s.b1;
   add_op(e, P_FROM_ORTHO);
-  run_pass(e, st);
+  run_pass(e, st, &s.work);
 }
 
 void space_gradient(const SpaceDev& s, const void* spec, void* ortho, int d0, int d1, const double* scale,
@@ -890,7 +1041,7 @@ void space_gradient(const SpaceDev& s, const void* spec, void* ortho, int d0, in
   d.basis = s.b0;
   add_op(d, P_TO_ORTHO);
   add_op(d, s.cplx ? P_FDIFF : P_DIFF, d0);
-  run_pass(d, st);
+  run_pass(d, st, &s.work);
   PassDesc e = base_desc(s);
   set_axis1(e, tmp, s.cplx, ortho, s.cplx, s.ortho0, s.spec1, s.ortho1);
   e.basis = s.b1;
@@ -903,7 +1054,7 @@ void space_gradient(const SpaceDev& s, const void* spec, void* ortho, int d0, in
     e.scale = 1.0 / (s0 * s1);
     add_op(e, P_SCALE);
   }
-  run_pass(e, st);
+  run_pass(e, st, &s.work);
 }
 
 void solver_solve(const SolverDev& sv, const SpaceDev& s, const void* in_ortho, void* out_spec, void* tmp,
@@ -918,13 +1069,13 @@ void solver_solve(const SolverDev& sv, const SpaceDev& s, const void* in_ortho, 
     if (sv.has_pinv[0]) { d.pinv = sv.pinv[0]; add_op(d, P_MATVEC); }
     d.fdma = sv.adi[0];
     add_op(d, P_FDMA);
-    run_pass(d, st);
+    run_pass(d, st, &s.work);
     PassDesc e = base_desc(s);
     set_axis1(e, t0, cx, out_spec, cx, s.spec0, s.ortho1, s.spec1);
     if (sv.has_pinv[1]) { e.pinv = sv.pinv[1]; add_op(e, P_MATVEC); }
     e.fdma = sv.adi[1];
     add_op(e, P_FDMA);
-    run_pass(e, st);
+    run_pass(e, st, &s.work);
     return;
   }
   // tensor solver: pinv_x and eigenbasis forward along x, pinv_y and the
@@ -932,20 +1083,20 @@ void solver_solve(const SolverDev& sv, const SpaceDev& s, const void* in_ortho, 
   PassDesc d = base_desc(s);
   set_axis0(d, in_ortho, cx, t0, cx, s.ortho1, s.ortho0);
   if (sv.has_pinv[0]) { d.pinv = sv.pinv[0]; add_op(d, P_MATVEC); }
-  if (sv.dense) { d.dense = sv.fwd; d.dense_rows = sv.m0; d.dense_cols = sv.m0; add_op(d, P_DENSE); }
-  run_pass(d, st);
+  if (sv.dense) { d.dense = sv.fwd; d.smat = sv.smat_f; d.dense_rows = sv.m0; d.dense_cols = sv.m0; add_op(d, P_DENSE); }
+  run_pass(d, st, &s.work);
   PassDesc e = base_desc(s);
   set_axis1(e, t0, cx, sv.dense ? t1 : out_spec, cx, s.spec0, s.ortho1, s.spec1);
   if (sv.has_pinv[1]) { e.pinv = sv.pinv[1]; add_op(e, P_MATVEC); }
   e.fdma = sv.rows;
   add_op(e, P_FDMA);
-  run_pass(e, st);
+  run_pass(e, st, &s.work);
   if (sv.dense) {
     PassDesc f = base_desc(s);
     set_axis0(f, t1, cx, out_spec, cx, s.spec1, s.spec0);
-    f.dense = sv.bwd; f.dense_rows = sv.m0; f.dense_cols = sv.m0;
+    f.dense = sv.bwd; f.smat = sv.smat_b; f.dense_rows = sv.m0; f.dense_cols = sv.m0;
     add_op(f, P_DENSE);
-    run_pass(f, st);
+    run_pass(f, st, &s.work);
   }
 }
 
@@ -1053,7 +1204,17 @@ static PassDesc lanes_desc(const LanesDev& L) {
   return d;
 }
 
-void lanes_apply(const LanesDev& L, int op, const double* in, double* out, int lanes, cudaStream_t st) {
+bool lanes_attach_split(LanesDev& L) {
+  if (!split_fits(L.cx)) return false;
+  split_ops(L.cx);
+  return true;
+}
+bool lanes_split_pays(const LanesDev& L, int op, int lanes) {
+  return (op == LOP_FORWARD || op == LOP_BACKWARD) && split_pays(lanes, L.cx.n);
+}
+
+void lanes_apply(const LanesDev& L, int op, const double* in, double* out, int lanes, cudaStream_t st,
+                 const SplitWork* work) {
   int il, ol;
   lane_op_lengths(L, op, &il, &ol);
   PassDesc d = lanes_desc(L);
@@ -1070,7 +1231,7 @@ void lanes_apply(const LanesDev& L, int op, const double* in, double* out, int l
       d.fdma = L.adi; add_op(d, P_FDMA);
       break;
   }
-  run_pass(d, st);
+  run_pass(d, st, work);
 }
 
 void lanes_fdma(const LanesDev& L, double* x, int lanes, cudaStream_t st) {
@@ -1133,6 +1294,7 @@ cudaError_t configure_prim_kernels() {
   cudaError_t e = cudaFuncSetAttribute(dev::k_pass<double2, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(dev::k_pass<double2, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(dev::k_pass<double, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
+  if (e == cudaSuccess) e = configure_split_kernels();
   if (e == cudaSuccess) done.set();
   return e;
 }

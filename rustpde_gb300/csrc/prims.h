@@ -67,6 +67,16 @@ FourierXformDev upload_fourier(Arena& a, int n);
 PinvDev upload_pinv(Arena& a, int n);
 FdmaDev upload_fdma(Arena& a, const std::vector<Band4>& rows, bool odd = true);  // swept factors, one per row
 
+// Scratch of the passes whose dense products run as split GEMMs: digits and
+// exponents of the lanes, and the products a following operation reads.
+struct SplitWork {
+  unsigned char* dig = nullptr;
+  int* ex = nullptr;
+  double* buf = nullptr;
+  int lanes = 0;  // capacity
+  unsigned int* status = nullptr;
+};
+
 // A 2-D space of two bases (funspace/src/space2.rs).
 struct SpaceDev {
   HostBasis hb0, hb1;
@@ -76,7 +86,11 @@ struct SpaceDev {
   bool odd = true;    // scan blocks of its passes (chain_scan.cuh)
   bool cplx = false;  // spectral data complex (Fourier along axis 0)
   int phys0 = 0, phys1 = 0, spec0 = 0, spec1 = 0, ortho0 = 0, ortho1 = 0;
+  SplitWork work;  // empty: dense products stay inside the passes
 };
+// Operators and scratch for split GEMMs in the space's passes, where a dense
+// transform or eigenbasis product of the space is large enough to gain.
+void attach_split(Arena& a, SpaceDev& s);
 void build_space(Arena& a, SpaceDev& s, int kind0, int n0, int kind1, int n1, bool odd = true);
 
 // The same space with dense Chebyshev transforms that sum all n terms in index
@@ -97,6 +111,7 @@ struct SolverDev {
   bool dense = false;  // eigenbasis products along axis 0
   const double* fwd = nullptr;
   const double* bwd = nullptr;
+  SplitMatDev smat_f{}, smat_b{};  // the same in nine digits (spaces with split scratch)
   int m0 = 0, m1 = 0;  // spectral sizes
 };
 // c: the two coefficients of the reference constructors.  Returns false with
@@ -107,9 +122,9 @@ bool build_solver(Arena& a, const SpaceDev& s, int kind, const double c[2], Solv
 std::vector<Band4> hholtz_rows(const HostBasis& bx, const HostBasis& by, double cx, double cy, double alpha,
                                bool poisson, std::vector<double>* lam_out, std::vector<double>* fwd,
                                std::vector<double>* bwd, std::string* err);
-// eigenbasis of the Poisson solve along a composite axis: forward and backward
+// eigenbasis of a tensor solver along a composite axis 0: forward and backward
 // matrices, (n-2) x (n-2) row-major
-void poisson_eigenbasis(const HostBasis& b, std::vector<double>& fwd, std::vector<double>& bwd);
+void tensor_eigenbasis(const HostBasis& b, bool poisson, std::vector<double>& fwd, std::vector<double>& bwd);
 Band4 adi_factor(const HostBasis& b, double c);
 // n x n matrix, row-major -> column-major
 std::vector<double> transposed(const std::vector<double>& a, int n);
@@ -156,7 +171,12 @@ void build_lanes(Arena& a, LanesDev& L, int kind, int n);
 void lanes_set_hholtz(Arena& a, LanesDev& L, double c);
 // input / output lengths of an operation
 void lane_op_lengths(const LanesDev& L, int op, int* in_len, int* out_len);
-void lanes_apply(const LanesDev& L, int op, const double* in, double* out, int lanes, cudaStream_t st);
+void lanes_apply(const LanesDev& L, int op, const double* in, double* out, int lanes, cudaStream_t st,
+                 const SplitWork* work = nullptr);
+// split operators of a dense length (false: none), and whether an application
+// gains by them
+bool lanes_attach_split(LanesDev& L);
+bool lanes_split_pays(const LanesDev& L, int op, int lanes);
 // the banded part of the HholtzAdi solve alone: x (m per lane) solved in place
 void lanes_fdma(const LanesDev& L, double* x, int lanes, cudaStream_t st);
 

@@ -59,6 +59,14 @@ struct FdmaDev {
 };
 constexpr int kFdmaScan = 20 * 32;
 
+// A split operator on the device (split_gemm.h): packed digits, outputs, scale.
+struct SplitOpDev {
+  const unsigned char* w;
+  const unsigned char* w16;
+  int N;
+  int wshift;
+};
+
 // Chebyshev transform along an axis of length n: FFT (n = 2^p + 1) or dense.
 struct ChebXformDev {
   int n;
@@ -75,6 +83,7 @@ struct ChebXformDev {
   // order (prims.h in_order_space)
   const double* fwd_full;
   const double* bwd_full;
+  SplitOpDev sop_b, sop_f[2];  // split operators (prims.h attach_split), or null
 };
 
 // Fourier r2c/c2r along x of physical length n (any n >= 4).  Even n runs
@@ -89,14 +98,6 @@ struct FourierXformDev {
   int rad[16];  // their radices: 4s, then 2, 3, 5, 7 and any larger prime factors
   const double2* tw;  // exp(-2 pi i t / n), t < n
   const float2* twf;  // the same table rounded to FP32 (mixed-precision form)
-};
-
-// A split operator on the device (split_gemm.h): packed digits, outputs, scale.
-struct SplitOpDev {
-  const unsigned char* w;
-  const unsigned char* w16;
-  int N;
-  int wshift;
 };
 
 // A general matrix in nine digits (SplitMat).

@@ -137,14 +137,8 @@ __device__ __forceinline__ double split_double(long long v, int e) {
 }
 
 template <int D>
-__global__ void __launch_bounds__(kSplitThreads, 2) k_split_gemm(const SplitJobDev* __restrict__ jobs,
-                                                                 const int4* __restrict__ tiles) {
-  pdl_enter();
+__device__ __forceinline__ void split_tile(const SplitJobDev& J, const int lane0, const int n0, const int NT) {
   using F = SplitForm<D>;
-  const int4 tl = tiles[blockIdx.x];
-  const SplitJobDev& J = jobs[tl.x];
-  if (J.active != nullptr && *J.active == 0) return;
-  const int lane0 = tl.y, n0 = tl.z, NT = tl.w;
   const int tid = threadIdx.x, warp = tid >> 5, wl = tid & 31;
   extern __shared__ __align__(128) unsigned char sm[];
   unsigned char* tail = sm + (size_t)F::kStages * F::kStageBytes;
@@ -338,6 +332,16 @@ __global__ void __launch_bounds__(kSplitThreads, 2) k_split_gemm(const SplitJobD
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  if (*abort_flag != 0 && J.status == nullptr && tid < kSplitLanes && lane0 + tid < J.lanes) {
+    // no status word to report to: the outputs say it
+    const int lane = lane0 + tid, r = lane / J.nf, f = lane - r * J.nf;
+    double* out = J.out + f * J.fs + (r / J.parts) * J.qs + (r % J.parts) * J.ps;
+    for (int n = n0; n < min(n0 + NT, J.N); n++) {
+      out[n * J.es] = __longlong_as_double(0x7FF8000000000000ll);
+      if (nlist == 2 && n >= J.m_lo && n < J.m_hi)
+        out[(J.mirror - n) * J.es] = __longlong_as_double(0x7FF8000000000000ll);
+    }
+  }
   if (*abort_flag != 0 && tid == 0) {
     if (J.status != nullptr) atomicOr(J.status, kStatusGemmTimeout);
     // copies that no MMA waited for, then the MMAs in flight (commits complete
@@ -357,6 +361,31 @@ __global__ void __launch_bounds__(kSplitThreads, 2) k_split_gemm(const SplitJobD
   __syncthreads();
   if (warp == 8)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)kSplitCols));
+}
+
+// tile table entries (job, first lane, first output, tile width)
+template <int D>
+__global__ void __launch_bounds__(kSplitThreads, 2) k_split_gemm(const SplitJobDev* __restrict__ jobs,
+                                                                 const int4* __restrict__ tiles) {
+  pdl_enter();
+  const int4 tl = tiles[blockIdx.x];
+  const SplitJobDev& J = jobs[tl.x];
+  if (J.active != nullptr && *J.active == 0) return;
+  split_tile<D>(J, tl.y, tl.z, tl.w);
+}
+
+// one or two jobs passed by value: the tiles of a lane block side by side
+struct SplitJobs2 {
+  SplitJobDev j[2];
+  int first;  // tiles of job 0
+  int most;   // tile width
+};
+template <int D>
+__global__ void __launch_bounds__(kSplitThreads, 2) k_split_gemm_one(const __grid_constant__ SplitJobs2 P) {
+  const int second = (int)blockIdx.x >= P.first, b = blockIdx.x - (second ? P.first : 0);
+  const SplitJobDev& J = P.j[second];
+  const int per = (J.N + P.most - 1) / P.most, n0 = (b % per) * P.most;
+  split_tile<D>(J, (b / per) * kSplitLanes, n0, J.N - n0 > 16 ? P.most : 16);
 }
 
 }  // namespace dev
@@ -491,6 +520,12 @@ cudaError_t configure_split_kernels() {
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(dev::k_split_gemm<9>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)dev::SplitForm<9>::kSmem);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(dev::k_split_gemm_one<7>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)dev::SplitForm<7>::kSmem);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(dev::k_split_gemm_one<9>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)dev::SplitForm<9>::kSmem);
   if (e == cudaSuccess) done.set();
   return e;
 }
@@ -499,6 +534,25 @@ cudaError_t launch_split_gemm(const SplitJobDev* jobs, const int4* tiles, int nt
   if (ntiles == 0) return cudaSuccess;
   if (digits == 9) return launch_pdl(dev::k_split_gemm<9>, ntiles, dev::kSplitThreads, dev::SplitForm<9>::kSmem, st, jobs, tiles);
   return launch_pdl(dev::k_split_gemm<7>, ntiles, dev::kSplitThreads, dev::SplitForm<7>::kSmem, st, jobs, tiles);
+}
+
+cudaError_t launch_split_gemm_one(const SplitJobDev* jobs, int njobs, cudaStream_t st) {
+  dev::SplitJobs2 p{};
+  auto blocks = [](const SplitJobDev& j) { return (j.lanes + kSplitLanes - 1) / kSplitLanes; };
+  auto tiles = [&](const SplitJobDev& j, int most) { return blocks(j) * ((j.N + most - 1) / most); };
+  long wide = 0;
+  for (int k = 0; k < njobs; k++) {
+    p.j[k] = jobs[k];
+    wide += tiles(jobs[k], kSplitTile);
+  }
+  const bool nine = jobs[0].digits == 9;
+  p.most = nine || wide <= kSplitNarrowTiles ? 16 : kSplitTile;
+  p.first = tiles(p.j[0], p.most);
+  const int total = p.first + (njobs > 1 ? tiles(p.j[1], p.most) : 0);
+  if (total == 0) return cudaSuccess;
+  if (nine) dev::k_split_gemm_one<9><<<total, dev::kSplitThreads, dev::SplitForm<9>::kSmem, st>>>(p);
+  else dev::k_split_gemm_one<7><<<total, dev::kSplitThreads, dev::SplitForm<7>::kSmem, st>>>(p);
+  return cudaGetLastError();
 }
 
 cudaError_t set_split_wait_limit(long long polls) {

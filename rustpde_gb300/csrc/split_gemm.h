@@ -58,7 +58,7 @@ struct SplitJobDev {
   const unsigned char* w;    // packed operator (SplitOp), 32-wide tiles
   const unsigned char* w16;  // the same in 16-wide tiles
   double* out;
-  unsigned int* status;    // receives kStatusGemmTimeout
+  unsigned int* status;    // receives kStatusGemmTimeout (null: the tile's outputs become NaN)
   const int* active;       // when set and 0, the job's tiles do nothing (serving gate)
   long long fs, qs, ps, es;
   int lanes, nf, parts;
@@ -99,6 +99,8 @@ SplitMat pack_split_mat(const std::vector<double>& M, int n);
 void split_tiles(const std::vector<SplitJobDev>& jobs, std::vector<int4>& tiles);
 cudaError_t configure_split_kernels();
 cudaError_t launch_split_gemm(const SplitJobDev* jobs, const int4* tiles, int ntiles, int digits, cudaStream_t st);
+// at most two jobs, passed by value (no tables)
+cudaError_t launch_split_gemm_one(const SplitJobDev* jobs, int njobs, cudaStream_t st);
 cudaError_t set_split_wait_limit(long long polls);  // as set_gemm_wait_limit
 
 // Unit exponent of a job's sums (SplitJobDev::ex_bias): terms with shift shl,

@@ -24,7 +24,10 @@
 
 #include <algorithm>
 #include <cmath>
+#include <map>
+#include <mutex>
 #include <stdexcept>
+#include <tuple>
 
 #include "lane_ops.cuh"
 #include "pdl.cuh"
@@ -297,6 +300,67 @@ SplitOp make_split_op(int kind, int n, int rows, int* wshift) {
   throw std::runtime_error("make_split_op: unknown kind");
 }
 
+// The split operator of a transform (step_split.h) on the current device,
+// shared like the mixed operators by every case of the size.
+SplitOpDev shared_split_op(int kind, int n, int rows) {
+  static std::mutex mu;
+  static std::map<std::tuple<int, int, int, int>, SplitOpDev> cache;
+  int dev = 0;
+  cuda_check(cudaGetDevice(&dev), "cudaGetDevice");
+  std::lock_guard<std::mutex> lk(mu);
+  const auto key = std::make_tuple(dev, kind, n, rows);
+  auto it = cache.find(key);
+  if (it != cache.end()) return it->second;
+  SplitOpDev d{};
+  const SplitOp op = make_split_op(kind, n, rows, &d.wshift);
+  d.N = op.N;
+  const size_t n32 = (op.bytes.size() + 127) & ~size_t(127);
+  unsigned char* p = nullptr;
+  cuda_check(cudaMalloc(&p, n32 + op.bytes16.size()), "cudaMalloc shared operator");
+  cudaError_t e = cudaMemcpy(p, op.bytes.data(), op.bytes.size(), cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = cudaMemcpy(p + n32, op.bytes16.data(), op.bytes16.size(), cudaMemcpyHostToDevice);
+  if (e != cudaSuccess) {
+    cudaFree(p);
+    cuda_check(e, "upload shared operator");
+  }
+  d.w = p;
+  d.w16 = p + n32;
+  return cache.emplace(key, d).first->second;
+}
+
+// The eigenbasis matrices of a tensor solver's axis 0 in nine digits.
+SplitMatDev shared_split_mat(int kind, int n, bool poisson, bool fwd) {
+  static std::mutex mu;
+  static std::map<std::tuple<int, int, int, bool, bool>, SplitMatDev> cache;
+  int dev = 0;
+  cuda_check(cudaGetDevice(&dev), "cudaGetDevice");
+  std::lock_guard<std::mutex> lk(mu);
+  const auto key = std::make_tuple(dev, kind, n, poisson, fwd);
+  auto it = cache.find(key);
+  if (it != cache.end()) return it->second;
+  std::vector<double> F, B;
+  tensor_eigenbasis(make_basis(kind, n), poisson, F, B);
+  const SplitMat m = pack_split_mat(fwd ? F : B, n - 2);
+  const size_t nb = (m.bytes16.size() + 127) & ~size_t(127), ne = (size_t)m.N * 4;
+  unsigned char* p = nullptr;
+  cuda_check(cudaMalloc(&p, nb + 2 * ne), "cudaMalloc shared operator");
+  cudaError_t e = cudaMemcpy(p, m.bytes16.data(), m.bytes16.size(), cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = cudaMemcpy(p + nb, m.colex.data(), ne, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = cudaMemcpy(p + nb + ne, m.rowex.data(), ne, cudaMemcpyHostToDevice);
+  if (e != cudaSuccess) {
+    cudaFree(p);
+    cuda_check(e, "upload shared operator");
+  }
+  SplitMatDev d{};
+  d.w16 = p;
+  d.colex = reinterpret_cast<const int*>(p + nb);
+  d.rowex = reinterpret_cast<const int*>(p + nb + ne);
+  d.N = m.N;
+  d.K0 = m.K[0];
+  d.K1 = m.K[1];
+  return cache.emplace(key, d).first->second;
+}
+
 // ---------------------------------------------------------------------------
 // plan
 // ---------------------------------------------------------------------------
@@ -318,6 +382,31 @@ bool split_step_size(const CaseDev& c) {
   else if (c.fx.log2M < 0)
     for (int k = 0; k < c.fx.nrad; k++) fast = fast && c.fx.rad[k] <= 8;
   return c.nx * c.ny >= (fast ? 48000 : 9000);
+}
+
+SplitJobDev split_op_job(const SplitLanesDev& s, const SplitOpDev& op, int lanes, int shl, double* out, long long ls,
+                         long long es, unsigned int* status) {
+  SplitJobDev j{};
+  j.dig = s.dig;
+  j.ex = s.ex;
+  j.w = op.w;
+  j.w16 = op.w16;
+  j.out = out;
+  j.status = status;
+  j.es = es;
+  j.lanes = lanes;
+  j.nf = 1;
+  j.parts = 1;
+  j.qs = ls;
+  j.ctot = s.cE + s.cO;
+  j.c0[0] = 0;
+  j.nc[0] = s.cE;
+  j.c0[1] = s.cE;
+  j.nc[1] = s.cO;
+  j.N = op.N;
+  j.ex_bias = split_ex_bias(shl, op.wshift);
+  j.digits = kSplitDigits;
+  return j;
 }
 
 SplitJobDev split_mat_job(const SplitLanesDev& s, const SplitMatDev& m, int lanes, double* out, long long es,
@@ -344,7 +433,10 @@ SplitJobDev split_mat_job(const SplitLanesDev& s, const SplitMatDev& m, int lane
   return j;
 }
 
-bool split_eig_size(const CaseDev& c) { return c.kind != KIND_PERIODIC && c.nx >= 160 && c.nx <= 514; }
+// Dense FP64 products inside X3 and X4 | split GEMMs, us per step: box 144^2
+// 144 | 158, 160^2 156 | 160, 192^2 178 | 174, 224^2 199 | 184, 264^2 280 | 227.
+// (An accumulator's exact range ends at 256 terms a list.)
+bool split_eig_size(const CaseDev& c) { return c.kind != KIND_PERIODIC && c.nx >= 176 && c.nx <= 514; }
 
 void add_split_launches(const CaseDev& c, bool on, StepPlan& p) {
   const bool per = c.kind == KIND_PERIODIC;
@@ -365,27 +457,7 @@ void add_split_launches(const CaseDev& c, bool on, StepPlan& p) {
     p.launches.push_back(L);
   };
   auto job = [&](const SplitLanesDev& s, const SplitOpDev& op, int lanes, int shl, double* out, long long es) {
-    SplitJobDev j{};
-    j.dig = s.dig;
-    j.ex = s.ex;
-    j.w = op.w;
-    j.w16 = op.w16;
-    j.out = out;
-    j.status = c.status;
-    j.es = es;
-    j.lanes = lanes;
-    j.nf = 1;
-    j.parts = 1;
-    j.qs = 1;  // lanes adjacent
-    j.ctot = s.cE + s.cO;
-    j.c0[0] = 0;
-    j.nc[0] = s.cE;
-    j.c0[1] = s.cE;
-    j.nc[1] = s.cO;
-    j.N = op.N;
-    j.ex_bias = split_ex_bias(shl, op.wshift);
-    j.digits = kSplitDigits;
-    return j;
+    return split_op_job(s, op, lanes, shl, out, 1, es, c.status);  // lanes adjacent
   };
   // one list of a forward transform: terms E (par 0) or O (par 1)
   auto one = [&](SplitJobDev j, const SplitLanesDev& s, int par) {

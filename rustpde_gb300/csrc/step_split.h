@@ -26,11 +26,18 @@ void split_terms(bool fourier, int n, int K[2]);
 // rows: outputs to keep (one-list kinds; all for the others).  wshift: see split_ex_bias.
 SplitOp make_split_op(int kind, int n, int rows, int* wshift);
 
+// The same on the current device, shared by everything of the size.
+SplitOpDev shared_split_op(int kind, int n, int rows);
+SplitMatDev shared_split_mat(int kind, int n, bool poisson, bool fwd);
+
 // Whether a case of this size runs its FP64 transforms as split GEMMs.
 bool split_step_size(const CaseDev& c);
 // The launches up to the convection term m_cv (S1, GEMM, S2, GEMM, S3, GEMM, S4, GEMM)
 // (on = false: the same launches without work)
 void add_split_launches(const CaseDev& c, bool on, StepPlan& p);
+// out[l ls + n es] = the two lists of a transform applied to lane l
+SplitJobDev split_op_job(const SplitLanesDev& s, const SplitOpDev& op, int lanes, int shl, double* out, long long ls,
+                         long long es, unsigned int* status);
 // out[r es + lane] = the matrix applied to nine-digit lanes
 SplitJobDev split_mat_job(const SplitLanesDev& s, const SplitMatDev& m, int lanes, double* out, long long es,
                           unsigned int* status);

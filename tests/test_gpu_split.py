@@ -30,7 +30,8 @@ def O():
 # of 1, 16 and 17 outputs, odd and even lengths on either axis, one and several
 # lane blocks, the shortest axis with the longest, a prime Fourier length
 SIZES = [(96, 94, 0), (95, 129, 1), (98, 97, 0), (16, 600, 0), (600, 16, 1), (66, 142, 0),
-         (96, 96, 2), (101, 98, 2), (97, 95, 2), (16, 576, 2), (640, 20, 2), (128, 71, 2)]
+         (96, 96, 2), (101, 98, 2), (97, 95, 2), (16, 576, 2), (640, 20, 2), (128, 71, 2),
+         (176, 64, 0), (200, 150, 1), (513, 100, 0), (257, 130, 1)]
 
 
 def _ic(c):
