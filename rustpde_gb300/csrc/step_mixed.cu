@@ -400,6 +400,30 @@ cudaError_t launch_mixed_kernel(int kernel, int nblocks, size_t smem, cudaStream
   return cudaGetLastError();
 }
 
+// The kernel whose arrays a form of the same pass moves (-1: counted with another
+// launch).  Kept apart from the switch on the result: with both in one function
+// gcc 13 at -O3 sent every kernel that this one maps to itself to the default.
+__attribute__((noinline)) static int same_arrays(int kernel) {
+  switch (kernel) {
+    case K_LP_BOX_GPX: return K_BOX_GPX;
+    case K_LP_BOX_X2: return K_BOX_X2;
+    case K_LP_BOX_X3: return K_BOX_X3_MIX;
+    case K_LP_BOX_X4: return K_BOX_X4_MIX;
+    case K_LP_BOX_Y2: return K_BOX_Y2_PRE;
+    case K_LP_BOX_Y3: return K_BOX_Y3;
+    case K_LP_BOX_Y4: case K_BOX_Y4_MIX: return K_BOX_Y4;
+    case K_LP_BOX_Y5: return K_BOX_Y5;
+    case K_LP_PER_Y2: return K_PER_Y2_PRE;
+    case K_PER_Y2_PRE_T128: case K_PER_Y2_CV: return K_PER_Y2_PRE;
+    case K_LP_PER_Y2B: case K_LP_PER_Y2C: return -1;
+    case K_PER_X_MIXED_T128: return K_PER_X_MIXED;
+    case K_BOX_Y2_PRE_T128: case K_BOX_Y2_CV: return K_BOX_Y2_PRE;
+    case K_BOX_X3_MIX_T128: return K_BOX_X3_MIX;
+    case K_BOX_Y5_T128: return K_BOX_Y5;
+    default: return kernel;
+  }
+}
+
 // Algorithmic HBM bytes of one launch: every array the launch must read or
 // write, counted once (operator tables and the boundary-field constants
 // included; re-reads from L2 and shared memory are not).
@@ -430,24 +454,7 @@ double launch_algorithmic_bytes(const StepLaunch& L, const CaseDev* cases) {
     // box y4 of the mixed form also writes the solution's FP32 copy (the
     // eigenbasis GEMM's input)
     if (kernel == K_LP_BOX_Y4 || kernel == K_BOX_Y4_MIX) v += myc * 4;
-    switch (kernel) {  // the one-thread-per-lane kernels move the same arrays
-      case K_LP_BOX_GPX: kernel = K_BOX_GPX; break;
-      case K_LP_BOX_X2: kernel = K_BOX_X2; break;
-      case K_LP_BOX_X3: kernel = K_BOX_X3_MIX; break;
-      case K_LP_BOX_X4: kernel = K_BOX_X4_MIX; break;
-      case K_LP_BOX_Y2: kernel = K_BOX_Y2_PRE; break;
-      case K_LP_BOX_Y3: kernel = K_BOX_Y3; break;
-      case K_LP_BOX_Y4: case K_BOX_Y4_MIX: kernel = K_BOX_Y4; break;
-      case K_LP_BOX_Y5: kernel = K_BOX_Y5; break;
-      case K_LP_PER_Y2: kernel = K_PER_Y2_PRE; break;
-      case K_PER_Y2_PRE_T128: case K_PER_Y2_CV: kernel = K_PER_Y2_PRE; break;
-      case K_LP_PER_Y2B: case K_LP_PER_Y2C: kernel = -1; break;  // counted with Y2A
-      case K_PER_X_MIXED_T128: kernel = K_PER_X_MIXED; break;
-      case K_BOX_Y2_PRE_T128: case K_BOX_Y2_CV: kernel = K_BOX_Y2_PRE; break;
-      case K_BOX_X3_MIX_T128: kernel = K_BOX_X3_MIX; break;
-      case K_BOX_Y5_T128: kernel = K_BOX_Y5; break;
-      default: break;
-    }
+    kernel = same_arrays(kernel);
     switch (kernel) {
       case K_Y1_C: case K_Y1_R: v = 3 * myc * z + 6 * ny * z; break;
       case K_PER_X: v = 6 * mx * z + 2 * nx * 8 + 3 * kx * z; break;
