@@ -25,6 +25,7 @@
 #include "pdl.cuh"
 #include "per_device.h"
 #include "split_gemm.h"
+#include "cvt.cuh"
 #include "tc_ptx.cuh"
 
 #include <algorithm>
@@ -274,6 +275,9 @@ __device__ __forceinline__ void a_load(AChunk<T, NTHR>& a, const ATile<T, NTHR>&
   }
 }
 
+__device__ __forceinline__ float lane_f32(float v) { return v; }
+__device__ __forceinline__ float lane_f32(double v) { return to_f32(v); }
+
 template <class T, int NTHR = kGemmThreads>
 __device__ __forceinline__ void a_store(const AChunk<T, NTHR>& a, const ATile<T, NTHR>& t, unsigned char* Ahi,
                                         unsigned char* Alo) {
@@ -284,10 +288,10 @@ __device__ __forceinline__ void a_store(const AChunk<T, NTHR>& a, const ATile<T,
     float x;
     // lo is rounded to TF32 here: left to the tensor core it would be
     // truncated, a bias that accumulates along K
-    x = (float)a.v[it][0]; hi.x = tf32_rna(x); lo.x = tf32_rna(x - hi.x);
-    x = (float)a.v[it][1]; hi.y = tf32_rna(x); lo.y = tf32_rna(x - hi.y);
-    x = (float)a.v[it][2]; hi.z = tf32_rna(x); lo.z = tf32_rna(x - hi.z);
-    x = (float)a.v[it][3]; hi.w = tf32_rna(x); lo.w = tf32_rna(x - hi.w);
+    x = lane_f32(a.v[it][0]); hi.x = tf32_rna(x); lo.x = tf32_rna(x - hi.x);
+    x = lane_f32(a.v[it][1]); hi.y = tf32_rna(x); lo.y = tf32_rna(x - hi.y);
+    x = lane_f32(a.v[it][2]); hi.z = tf32_rna(x); lo.z = tf32_rna(x - hi.z);
+    x = lane_f32(a.v[it][3]); hi.w = tf32_rna(x); lo.w = tf32_rna(x - hi.w);
     const int off = t.soff0 + it * t.sstep;
     *reinterpret_cast<float4*>(Ahi + off) = hi;
     *reinterpret_cast<float4*>(Alo + off) = lo;

@@ -12,6 +12,7 @@
 // Each launch takes a table of work items (case, first lane, lane count); a
 // batch of cases is the same launch with a longer table.
 #include "lane_ops.cuh"
+#include "cvt.cuh"
 #include "pdl.cuh"
 #include "split_emit.cuh"
 #include "per_device.h"
@@ -877,7 +878,7 @@ __global__ void __launch_bounds__(256) k_box_x3(const CaseDev* __restrict__ case
   }
   if (EIG == EIG_MIXED) {
     float* mz = static_cast<float*>(c.m_z);
-    for (int r = tid; r < mxc; r += nth) mz[(size_t)r * ny + j] = (float)Z[r];
+    for (int r = tid; r < mxc; r += nth) mz[(size_t)r * ny + j] = to_f32(Z[r]);
     return;
   }
   // dense eigenbasis forward along x
@@ -912,7 +913,7 @@ __global__ void __launch_bounds__(256) k_box_y4(const CaseDev* __restrict__ case
   fdma_solve<double>(fp, OUT, ld, 1, 0, 0, tid, nth);
   if (MIX) {  // FP32 into m_z: the input of the eigenbasis GEMM
     float* wf = static_cast<float*>(c.m_z);
-    for (int k = tid; k < myc; k += nth) wf[(size_t)i * myc + k] = (float)OUT[k];
+    for (int k = tid; k < myc; k += nth) wf[(size_t)i * myc + k] = to_f32(OUT[k]);
     return;
   }
   double* wv = static_cast<double*>(c.s[7]);

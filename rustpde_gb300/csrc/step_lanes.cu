@@ -22,6 +22,7 @@
 //
 // Work item: (case, first lane, lane count <= blockDim.x, 0).
 #include "lane_ops.cuh"
+#include "cvt.cuh"
 #include "pdl.cuh"
 #include "step_fp64.h"
 
@@ -387,7 +388,7 @@ __global__ void __launch_bounds__(128) k_lp_box_x3(const CaseDev* __restrict__ c
                    [&](int i, double da) { dv[(long long)i * ny] = fma(da, inv_asp, stencil_lane<double>(c.xu, B, ny, i)); });
   float* z = static_cast<float*>(c.m_z) + j;  // FP32: the input of the eigenbasis GEMM
 #pragma unroll 4
-  for (int r = q; r < mxc; r += 2) z[(long long)r * ny] = (float)pinv_lane<double>(c.pinv_x, dv, ny, r);
+  for (int r = q; r < mxc; r += 2) z[(long long)r * ny] = to_f32(pinv_lane<double>(c.pinv_x, dv, ny, r));
 }
 
 // projection along x from p1 (computed by the eigenbasis GEMM): p1[0][0] = 0;
@@ -579,7 +580,7 @@ __global__ void __launch_bounds__(256) k_lp_box_y4(const CaseDev* __restrict__ c
     double v = wv[j] * R.dinv[j];
     if (j + 2 < R.m) v = fma(p2, R.up1[j], v);
     if (j + 4 < R.m) v = fma(p4, R.up2[j], v);
-    wf[j] = (float)v;
+    wf[j] = to_f32(v);
     p4 = p2;
     p2 = v;
   }

@@ -14,6 +14,7 @@
 //  periodic:  G1 (y, GEMM) -> X (FP32) -> G2 (y, GEMM) -> Y2 (FP64)
 #include "lane_ops.cuh"
 #include "lane_ops_f32.cuh"
+#include "cvt.cuh"
 #include "pdl.cuh"
 #include "per_device.h"
 #include "prims.h"
@@ -143,11 +144,20 @@ __global__ void __launch_bounds__(128) k_state_f32(const CaseDev* __restrict__ c
                           static_cast<const double*>(c.temp)};
   float* dst = static_cast<float*>(c.m_s32);
   // a complex row (re, im interleaved) is split into its [re | im] parts
-  for (int f = 0; f < 3; f++)
-    for (size_t k = threadIdx.x; k < rl; k += blockDim.x) {
-      const size_t o = per ? (k & 1) * mp + (k >> 1) : k;
-      dst[f * fs + i * ld + o] = (float)src[f][i * rl + k];
+  for (int f = 0; f < 3; f++) {
+    const double* __restrict__ a = src[f] + i * rl;
+    float* __restrict__ d = dst + f * fs + i * ld;
+    if (per) {
+      const double2* __restrict__ a2 = reinterpret_cast<const double2*>(a);
+      for (int k = threadIdx.x; k < myc; k += blockDim.x) {
+        const double2 v = a2[k];
+        d[k] = to_f32(v.x);
+        d[mp + k] = to_f32(v.y);
+      }
+    } else {
+      for (int k = threadIdx.x; k < myc; k += blockDim.x) d[k] = to_f32(a[k]);
     }
+  }
 }
 
 size_t smem_per_x_mixed(const CaseDev& c) {
