@@ -782,18 +782,44 @@ __global__ void k_sumsq(const double* v, size_t n, double* out) {
 }
 }  // namespace dev
 
-// shared memory of a pass: what sizes are checked against, and the part that
-// lanes of 8- or 16-byte elements use
+constexpr int kManyLanes = 8 * 152;
+
+// shared memory of a pass that sizes are checked against
 static size_t pass_smem(const PassDesc& d) {
   return (size_t)(3 * d.lmax + 2 * d.wl) * 16 + (size_t)d.lmax * 2 * 8 + 64;
 }
-static size_t pass_smem_used(const PassDesc& d, size_t elem) {
-  return (size_t)2 * d.wl * 16 + (size_t)3 * d.lmax * elem + 64;
+// what a launch of its operations on lanes of 8- or 16-byte elements needs:
+// FFT work lanes and the second and third lane buffers only where they are used
+static size_t pass_smem_used(PassDesc& d, size_t elem) {
+  bool fft = false;
+  int bufs = 1;
+  for (int k = 0; k < d.nops; k++) {
+    const int code = d.ops[k].code;
+    if (code == P_R2C || code == P_C2R || ((code == P_DCT_FWD || code == P_DCT_BWD) && d.cx.use_fft)) fft = true;
+    if (code == P_R2C || code == P_C2R || (code == P_DIFF && d.ops[k].arg > 1)) bufs = 3;
+    if (code != P_FDIFF && code != P_SCALE && code != P_FDMA && code != P_ADD) bufs = std::max(bufs, 2);
+  }
+  if (!fft) d.wl = 0;
+  return (size_t)2 * d.wl * 16 + (size_t)bufs * d.lmax * elem + 64;
+}
+
+// Threads per lane.  The recurrences of a pass keep one warp busy (two chains
+// of 16 threads); with many lanes the other warps only take up the SM's threads
+// while that one runs, so a lane gets a single warp and the SM holds 32 lanes.
+// 4096 lanes, in us: 128, from_ortho 26 -> 20, Helmholtz 38 -> 27; 512, banded
+// solve 73 -> 48.
+static int pass_threads(const PassDesc& d) {
+  bool wide = false;  // transforms and dense products use every thread
+  for (int k = 0; k < d.nops; k++) {
+    const int code = d.ops[k].code;
+    wide = wide || code == P_DCT_FWD || code == P_DCT_BWD || code == P_R2C || code == P_C2R || code == P_DENSE;
+  }
+  return !wide && d.lanes >= kManyLanes ? 32 : 128;
 }
 
 // Real lanes run as pairs where the pairs still give every SM two CTAs and no
 // operation has factors per lane (a pair shares them), else one by one.
-static void run_pass_whole(const PassDesc& d, cudaStream_t st) {
+static void run_pass_whole(PassDesc d, cudaStream_t st) {
   bool real = !d.in_cplx && !d.out_cplx, per_lane = false;
   for (int k = 0; k < d.nops; k++) {
     const int code = d.ops[k].code;
@@ -801,10 +827,12 @@ static void run_pass_whole(const PassDesc& d, cudaStream_t st) {
     if (code == P_FDMA && d.fdma.rows > 1) per_lane = true;
   }
   constexpr int kPairLanes = 2 * 2 * 152;
-  if (!real) dev::k_pass<double2, 0><<<d.lanes, 128, pass_smem_used(d, 16), st>>>(d);
-  else if (!per_lane && d.lanes >= kPairLanes)
-    dev::k_pass<double2, 1><<<(d.lanes + 1) / 2, 128, pass_smem_used(d, 16), st>>>(d);
-  else dev::k_pass<double, 0><<<d.lanes, 128, pass_smem_used(d, 8), st>>>(d);
+  const int nt = pass_threads(d);
+  const bool pair = real && !per_lane && d.lanes >= kPairLanes;
+  const size_t sm = pass_smem_used(d, real && !pair ? 8 : 16);
+  if (!real) dev::k_pass<double2, 0><<<d.lanes, nt, sm, st>>>(d);
+  else if (pair) dev::k_pass<double2, 1><<<(d.lanes + 1) / 2, nt, sm, st>>>(d);
+  else dev::k_pass<double, 0><<<d.lanes, nt, sm, st>>>(d);
   cuda_check(cudaGetLastError(), "pass kernel launch");
 }
 
@@ -837,7 +865,7 @@ static void run_pass(const PassDesc& d, cudaStream_t st, const SplitWork* w = nu
   S.ex = w->ex;
   S.cE = split_chunks(dense ? d.smat.K0 : (n + 1) / 2);
   S.cO = split_chunks(dense ? d.smat.K1 : n / 2);
-  dev::k_pass_digits<<<d.lanes, 128, (size_t)3 * d.lmax * 8 + 64, st>>>(d, at, code, S);
+  dev::k_pass_digits<<<d.lanes, d.lanes >= kManyLanes ? 32 : 128, (size_t)3 * d.lmax * 8 + 64, st>>>(d, at, code, S);
   cuda_check(cudaGetLastError(), "pass kernel launch");
   // the product: into the output, or into buf for the rest of the pass (lanes
   // adjacent where they are in the output)
