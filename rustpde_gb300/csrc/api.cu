@@ -337,6 +337,9 @@ struct FsLanes {
   }
 };
 constexpr int kSplitLanesCap = 4096;
+// The mixed form packs the lanes of a GEMM first (lane_gemm.cu) from these sizes
+// on; below, the packing launch costs what it saves.
+constexpr int kPackLanesMinN = 96, kPackLanesMin = 1024;
 
 struct SvSolver {
   FsSpace* space = nullptr;
@@ -2250,6 +2253,10 @@ int fs_lanes_create(int base, int n, int precision, FsLanes** out) {
     cuda_check(cudaEventCreateWithFlags(&p->done, cudaEventDisableTiming), "event");
   }
   if (precision == RBC_PREC_MIXED) {
+    if (n >= kPackLanesMinN) {
+      cuda_check(cudaMalloc(&p->work_mem, packed_lanes_bytes(kSplitLanesCap, n)), "cudaMalloc lane scratch");
+      cuda_check(cudaEventCreateWithFlags(&p->done, cudaEventDisableTiming), "event");
+    }
     const HostBasis& hb = p->L.hb;
     LMat S = lm_stencil(hb), P = lm_from_ortho(hb);
     p->w[FS_OP_FORWARD] = upload_split(p->arena, lm_mul(P, lm_cheb_forward(n)));
@@ -2304,37 +2311,42 @@ int fs_lanes_apply(FsLanes* p, int op, const double* d_in, double* d_out, int la
   if (lanes == 0) return RBC_OK;
   if (op == FS_OP_HHOLTZ) require(p->L.has_solver, "fs_lanes_apply: call fs_lanes_set_hholtz first");
   cudaStream_t st = (cudaStream_t)stream;
-  if (p->precision == RBC_PREC_FP64) {
-    // (a captured call keeps to the pass without scratch: its replays are not
-    // ordered with other calls on the handle)
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    const bool split = p->work_mem != nullptr && lanes_split_pays(p->L, op, lanes) &&
-                       cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone;
-    if (!split) {
-      (void)cudaGetLastError();
-      lanes_apply(p->L, op, d_in, d_out, lanes, st);
-    } else {
-      int il, ol;
-      lane_op_lengths(p->L, op, &il, &ol);
-      std::lock_guard<std::mutex> lk(p->mu);
-      if (p->used && p->last != st) cuda_check(cudaStreamWaitEvent(st, p->done, 0), "lane scratch");
-      for (int l = 0; l < lanes; l += kSplitLanesCap)
-        lanes_apply(p->L, op, d_in + (size_t)l * il, d_out + (size_t)l * ol, std::min(kSplitLanesCap, lanes - l), st,
-                    &p->work);
-      cuda_check(cudaEventRecord(p->done, st), "lane scratch");
-      p->last = st;
-      p->used = true;
-    }
-  } else {
-    int il, ol;
-    lane_op_lengths(p->L, op, &il, &ol);
-    void* ip[1] = {const_cast<double*>(d_in)};
-    void* opp[1] = {d_out};
-    GemmJobDev j = make_gemm_job(lane_rows(ip, 1, lanes, il, il, LT_F64, false),
-                                 lane_rows(opp, 1, lanes, ol, ol, LT_F64, false), p->w[op], il, ol, 1.0, p->d_status);
-    cuda_check(launch_lane_gemm_one(j, st), "lane gemm launch");
-    if (op == FS_OP_HHOLTZ) lanes_fdma(p->L, d_out, lanes, st);
+  int il, ol;
+  lane_op_lengths(p->L, op, &il, &ol);
+  const bool fp64 = p->precision == RBC_PREC_FP64;
+  // With the handle's scratch: split GEMMs (FP64) or packed GEMMs (mixed).  A
+  // captured call does without: its replays are not ordered with other calls on
+  // the handle.
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  bool scratch = p->work_mem != nullptr && (fp64 ? lanes_split_pays(p->L, op, lanes) : lanes >= kPackLanesMin);
+  if (scratch && (cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone)) {
+    (void)cudaGetLastError();
+    scratch = false;
   }
+  auto apply = [&](const double* in, double* out, int n) {
+    if (fp64) {
+      lanes_apply(p->L, op, in, out, n, st, scratch ? &p->work : nullptr);
+      return;
+    }
+    void* ip[1] = {const_cast<double*>(in)};
+    void* opp[1] = {out};
+    GemmJobDev j = make_gemm_job(lane_rows(ip, 1, n, il, il, LT_F64, false), lane_rows(opp, 1, n, ol, ol, LT_F64, false),
+                                 p->w[op], il, ol, 1.0, p->d_status);
+    if (scratch) j.apk = static_cast<const float*>(p->work_mem);
+    cuda_check(launch_lane_gemm_one(j, st), "lane gemm launch");
+  };
+  if (!scratch) {
+    apply(d_in, d_out, lanes);
+  } else {
+    std::lock_guard<std::mutex> lk(p->mu);
+    if (p->used && p->last != st) cuda_check(cudaStreamWaitEvent(st, p->done, 0), "lane scratch");
+    for (int l = 0; l < lanes; l += kSplitLanesCap)
+      apply(d_in + (size_t)l * il, d_out + (size_t)l * ol, std::min(kSplitLanesCap, lanes - l));
+    cuda_check(cudaEventRecord(p->done, st), "lane scratch");
+    p->last = st;
+    p->used = true;
+  }
+  if (!fp64 && op == FS_OP_HHOLTZ) lanes_fdma(p->L, d_out, lanes, st);
   API_END
 }
 

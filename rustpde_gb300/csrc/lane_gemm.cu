@@ -370,6 +370,7 @@ __device__ __forceinline__ void gemm_epilogue(const GemmJobDev& J, uint32_t tmem
       }
     };
     auto store_typed = [&](auto mode) {
+      if (tid >= kGemmThreads) return;  // the packed form's copy and MMA warps
       if (otype == LT_F64 && scale == 1.0)  // no FP64 product (the conversion alone runs at the FP64 rate)
         store_all([&](char* p, float f) { *reinterpret_cast<double*>(p) = (double)f; }, mode);
       else if (otype == LT_F64)
@@ -733,6 +734,173 @@ __device__ __forceinline__ void gemm_tile_ws_t(const GemmJobDev& J, const int la
   if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(ncols));
 }
 
+// ---------------------------------------------------------------------------
+// Packed form: the input lanes arrive as TF32 hi / lo tiles in the layout the
+// tensor core reads (k_pack_lanes), so that staging is one bulk copy per chunk.
+// The classic form converts a lane block once per output tile, and that
+// conversion, the loads behind it and the CTA barriers around it were most of a
+// chunk's time.  The products, partials, corrections and their order are those
+// of the other forms, so the results are the same bits.
+//   * warp 8, one thread: copies of chunk c (32 KB of lanes, the operator) into
+//     buffer c % 2 once the MMAs of chunk c-2 are done with it;
+//   * warp 9, one thread: the chunk's 12 MMAs;
+//   * warps 0-7: add the finished partial into the running total, then the
+//     epilogue.
+// Waits are bounded and an aborted tile drains as in the warp-specialised form.
+// 4096 lanes of 512 x 512: 79 -> 24 us after 9 us of packing.
+// ---------------------------------------------------------------------------
+constexpr int kPackedThreads = kGemmThreads + 64;
+constexpr int kPackedChunkBytes = 2 * kGemmLanes * kGemmKC * 4;  // hi, lo
+
+__device__ __forceinline__ void gemm_tile_packed(const GemmJobDev& J, const int lane0, const int tile_n) {
+  if (J.active != nullptr && *J.active == 0) return;
+  const int NT = J.NT;  // <= 64
+  const int tid = threadIdx.x, warp = tid >> 5, wl = tid & 31;
+  extern __shared__ __align__(128) unsigned char sm[];
+  const int wbytes = 2 * NT * kGemmKC * 4;
+  unsigned char* Ab[2] = {sm, sm + kPackedChunkBytes};
+  unsigned char* Wb[2] = {sm + 2 * kPackedChunkBytes, sm + 2 * kPackedChunkBytes + wbytes};
+  unsigned char* tail = sm + 2 * kPackedChunkBytes + 2 * wbytes;
+  uint64_t* full = reinterpret_cast<uint64_t*>(tail);  // [2]
+  uint64_t* mdone = full + 2;                          // [2]
+  uint64_t* flushed = full + 4;                        // [2]
+  uint32_t* slot = reinterpret_cast<uint32_t*>(tail + 48);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tail + 52);
+  volatile int* issued = reinterpret_cast<volatile int*>(tail + 56);   // chunks whose MMAs were committed
+  volatile int* copied = reinterpret_cast<volatile int*>(tail + 60);   // chunks whose copies were issued
+  char** ob = reinterpret_cast<char**>(tail + 64);
+  float* stage = reinterpret_cast<float*>(sm);  // epilogue staging, after the last MMA
+  if (tid < kGemmLanes) {
+    const int l = lane0 + tid;
+    ob[tid] = l < J.lanes ? const_cast<char*>(lane_addr(J.out, l)) : nullptr;
+  }
+  const uint32_t ncols = gemm_tmem_cols(NT);
+  const uint32_t corr = 2u * (uint32_t)NT, total = 3u * (uint32_t)NT;
+  if (warp == 8) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(slot)),
+                 "r"(ncols));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  if (tid == 0) {
+    for (int s = 0; s < 2; s++) {
+      mbar_init(&full[s], 1);
+      mbar_init(&mdone[s], 1);
+      mbar_init(&flushed[s], kGemmThreads);
+    }
+    *abort_flag = 0;
+    *issued = 0;
+    *copied = 0;
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *slot;
+  const long long limit = g_gemm_wait_limit;
+  const int kchunks = J.kchunks;
+  auto wait1 = [&](uint64_t* m, uint32_t parity) {  // one thread
+    for (long long i = 0; i < limit; i++) {
+      if (mbar_try(m, parity)) return true;
+      if ((i & 1023) == 1023 && *abort_flag) break;
+    }
+    *abort_flag = 1;
+    return false;
+  };
+
+  if (warp == 8) {
+    if (wl == 0) {
+      const unsigned char* a = reinterpret_cast<const unsigned char*>(J.apk) +
+                               (size_t)(lane0 / kGemmLanes) * kchunks * kPackedChunkBytes;
+      const unsigned char* w = reinterpret_cast<const unsigned char*>(J.w) + (size_t)tile_n * kchunks * wbytes;
+      for (int c = 0; c < kchunks; c++) {
+        const int s = c & 1;
+        if (c >= 2 && !wait1(&mdone[s], (uint32_t)(((c >> 1) - 1) & 1))) break;
+        mbar_arrive_expect_tx(&full[s], (uint32_t)(kPackedChunkBytes + wbytes));
+        bulk_g2s(Ab[s], a + (size_t)c * kPackedChunkBytes, kPackedChunkBytes, &full[s]);
+        bulk_g2s(Wb[s], w + (size_t)c * wbytes, (uint32_t)wbytes, &full[s]);
+        *copied = c + 1;
+      }
+    }
+  } else if (warp == 9) {
+    if (wl == 0) {
+      const uint32_t idesc = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(NT >> 3) << 17) | ((128u >> 4) << 24);
+      const uint32_t a_lbo = (kGemmLanes / 8) * 128, w_lbo = (uint32_t)(NT / 8) * 128;
+      for (int c = 0; c < kchunks; c++) {
+        const int s = c & 1;
+        if (!wait1(&full[s], (uint32_t)((c >> 1) & 1))) break;
+        if (c >= 2 && !wait1(&flushed[s], (uint32_t)(((c >> 1) - 1) & 1))) break;
+        tc_fence_after();
+        const uint32_t ah0 = smem_u32(Ab[s]), al0 = ah0 + kPackedChunkBytes / 2;
+        const uint32_t wh0 = smem_u32(Wb[s]), wl0 = wh0 + (uint32_t)NT * 128;
+        const uint32_t part = (uint32_t)(s * NT);
+#pragma unroll
+        for (int ks = 0; ks < kGemmKC / 8; ks++) {
+          const uint64_t ah = umma_desc(ah0 + ks * 2 * a_lbo, a_lbo, 128);
+          const uint64_t al = umma_desc(al0 + ks * 2 * a_lbo, a_lbo, 128);
+          const uint64_t wh = umma_desc(wh0 + ks * 2 * w_lbo, w_lbo, 128);
+          const uint64_t wlo = umma_desc(wl0 + ks * 2 * w_lbo, w_lbo, 128);
+          mma_tf32(tmem + corr, al, wh, idesc, (c > 0 || ks > 0) ? 1u : 0u);
+          mma_tf32(tmem + corr, ah, wlo, idesc, 1u);
+          mma_tf32(tmem + part, ah, wh, idesc, ks > 0 ? 1u : 0u);  // fresh partial per chunk
+        }
+        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+                         smem_u32(&mdone[s]))
+                     : "memory");
+        *issued = c + 1;
+      }
+    }
+  } else {
+    for (int c = 0; c < kchunks; c++) {
+      const int s = c & 1;
+      if (!warp_mbar_wait(&mdone[s], (uint32_t)((c >> 1) & 1), limit, abort_flag)) break;
+      tc_fence_after();
+      tmem_accumulate(tmem, (uint32_t)(s * NT), total, NT, c == 0, warp);
+      tc_fence_before();
+      mbar_arrive(&flushed[s]);
+    }
+  }
+  __syncwarp();
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  if (*abort_flag == 0) {
+    gemm_epilogue(J, tmem, total, corr, NT, tile_n, ob, stage, tid, warp, wl);
+  } else if (tid == 0) {
+    if (J.status != nullptr) atomicOr(J.status, kStatusGemmTimeout);
+    // copies not consumed by an MMA, and the last commit on each buffer, may
+    // still be in flight: wait for them (bounded) before the shared memory and
+    // the columns are given back
+    const int n = *issued, nw = *copied;
+    for (int c = n; c < nw; c++)
+      for (long long i = 0; i < kWaitLimit; i++)
+        if (mbar_try(&full[c & 1], (uint32_t)((c >> 1) & 1))) break;
+    for (int c = n - 2 < 0 ? 0 : n - 2; c < n; c++)
+      for (long long i = 0; i < kWaitLimit; i++)
+        if (mbar_try(&mdone[c & 1], (uint32_t)((c >> 1) & 1))) break;
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  if (warp == 8) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(ncols));
+}
+
+// chunk c of the lane block at lane0 as TF32 hi / lo tiles: the conversion of
+// the classic form, stored to global memory
+template <class T>
+__device__ __forceinline__ void pack_chunk(const GemmJobDev& J, int lane0, int c) {
+  __shared__ const char* ib[kGemmLanes];
+  const int tid = threadIdx.x;
+  if (tid < kGemmLanes) ib[tid] = lane0 + tid < J.lanes ? lane_addr(J.in, lane0 + tid) : nullptr;
+  __syncthreads();
+  ATile<T> at;
+  a_setup<T>(at, J, ib, tid);
+  AChunk<T> a;
+  a_load<T>(a, at, c * kGemmKC, J.K, J.in.lane_fast != 0, tid);
+  unsigned char* dst = reinterpret_cast<unsigned char*>(const_cast<float*>(J.apk)) +
+                       ((size_t)(lane0 / kGemmLanes) * J.kchunks + c) * kPackedChunkBytes;
+  a_store<T>(a, at, dst, dst + kPackedChunkBytes / 2);
+}
+
 __device__ __forceinline__ void gemm_tile(const GemmJobDev& J, const int lane0, const int tile_n) {
   if (J.active != nullptr && *J.active == 0) return;
   if (J.in.type == LT_F64) gemm_tile_t<double>(J, lane0, tile_n);
@@ -756,6 +924,33 @@ __global__ void __launch_bounds__(kGemmThreads, 2) k_lane_gemm_ws(const GemmJobD
   if (J.active != nullptr && *J.active == 0) return;
   if (J.in.type == LT_F64) gemm_tile_ws_t<double>(J, tl.y, tl.z);
   else gemm_tile_ws_t<float>(J, tl.y, tl.z);
+}
+
+// packed input (output tiles of at most 64 columns); pack table entries (job,
+// first lane, chunk, 0)
+__global__ void __launch_bounds__(kPackedThreads, 2) k_lane_gemm_packed(const GemmJobDev* __restrict__ jobs,
+                                                                        const int4* __restrict__ tiles) {
+  pdl_enter();
+  const int4 tl = tiles[blockIdx.x];
+  gemm_tile_packed(jobs[tl.x], tl.y, tl.z);
+}
+__global__ void __launch_bounds__(kGemmThreads) k_pack_lanes(const GemmJobDev* __restrict__ jobs,
+                                                             const int4* __restrict__ chunks) {
+  pdl_enter();
+  const int4 ch = chunks[blockIdx.x];
+  const GemmJobDev& J = jobs[ch.x];
+  if (J.active != nullptr && *J.active == 0) return;
+  if (J.in.type == LT_F64) pack_chunk<double>(J, ch.y, ch.z);
+  else pack_chunk<float>(J, ch.y, ch.z);
+}
+__global__ void __launch_bounds__(kPackedThreads, 2) k_lane_gemm_packed_one(const __grid_constant__ GemmJobDev J) {
+  const int b = blockIdx.x;
+  gemm_tile_packed(J, (b / J.ntiles) * kGemmLanes, b % J.ntiles);
+}
+__global__ void __launch_bounds__(kGemmThreads) k_pack_lanes_one(const __grid_constant__ GemmJobDev J) {
+  const int b = blockIdx.x;
+  if (J.in.type == LT_F64) pack_chunk<double>(J, (b / J.kchunks) * kGemmLanes, b % J.kchunks);
+  else pack_chunk<float>(J, (b / J.kchunks) * kGemmLanes, b % J.kchunks);
 }
 
 // single job passed by value: block b -> lanes (b / ntiles) * 128, output tile b % ntiles
@@ -852,6 +1047,10 @@ size_t gemm_ws_smem_bytes(int NT) {
   return std::max(dev::gemm_ws_smem_base(NT), gemm_smem_bytes(NT));
 }
 
+static size_t gemm_packed_smem_bytes(int NT) {
+  return (size_t)2 * dev::kPackedChunkBytes + (size_t)4 * NT * kGemmKC * 4 + 64 + kGemmLanes * 8;
+}
+
 cudaError_t configure_gemm_kernels() {
   static PerDeviceFlag done;
   if (done.test()) return cudaSuccess;
@@ -861,6 +1060,10 @@ cudaError_t configure_gemm_kernels() {
   e = cudaFuncSetAttribute(dev::k_lane_gemm_one, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)gemm_smem_bytes(128));
   if (e != cudaSuccess) return e;
+  for (const void* k : {(const void*)dev::k_lane_gemm_packed, (const void*)dev::k_lane_gemm_packed_one}) {
+    e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gemm_packed_smem_bytes(64));
+    if (e != cudaSuccess) return e;
+  }
   e = cudaFuncSetAttribute(dev::k_lane_gemm_ws, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)gemm_ws_smem_bytes(64));
   if (e == cudaSuccess) done.set();
@@ -873,9 +1076,21 @@ cudaError_t set_gemm_wait_limit(long long polls) {
   return e == cudaSuccess ? set_split_wait_limit(polls) : e;
 }
 
+size_t packed_lanes_bytes(int lanes, int K) {
+  return (size_t)((lanes + kGemmLanes - 1) / kGemmLanes) * ((K + kGemmKC - 1) / kGemmKC) * dev::kPackedChunkBytes;
+}
+
 cudaError_t launch_lane_gemm_one(const GemmJobDev& job, cudaStream_t st) {
-  const int blocks = ((job.lanes + kGemmLanes - 1) / kGemmLanes) * job.ntiles;
+  const int lane_blocks = (job.lanes + kGemmLanes - 1) / kGemmLanes;
+  const int blocks = lane_blocks * job.ntiles;
   if (blocks <= 0) return cudaSuccess;
+  if (job.apk != nullptr && job.NT <= 64) {
+    dev::k_pack_lanes_one<<<lane_blocks * job.kchunks, kGemmThreads, 0, st>>>(job);
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    dev::k_lane_gemm_packed_one<<<blocks, dev::kPackedThreads, gemm_packed_smem_bytes(job.NT), st>>>(job);
+    return cudaGetLastError();
+  }
   dev::k_lane_gemm_one<<<blocks, kGemmThreads, gemm_smem_bytes(job.NT), st>>>(job);
   return cudaGetLastError();
 }

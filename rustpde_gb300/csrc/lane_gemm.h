@@ -36,6 +36,7 @@ struct LaneSideDev {
 struct GemmJobDev {
   LaneSideDev in, out;
   const float* w;  // split operand packed by pack_gemm_w
+  const float* apk;  // packed form: scratch for the input lanes' hi / lo tiles (packed_lanes_bytes), else null
   unsigned int* status;  // receives kStatusGemmTimeout
   const int* active;     // when set and 0, the job's tiles do nothing (serving gate)
   double scale;
@@ -73,7 +74,10 @@ cudaError_t launch_lane_gemm(const GemmJobDev* jobs, const int4* tiles, int ntil
 // be tested; it affects every lane GEMM launched on the device afterwards.
 cudaError_t set_gemm_wait_limit(long long polls);
 
-// One job passed by value (no tables): lanes tiled in order.
+// Bytes of the packed tiles of a job's input lanes.
+size_t packed_lanes_bytes(int lanes, int K);
+// One job passed by value (no tables): lanes tiled in order.  With job.apk set
+// (and NT <= 64) the lanes are packed first and the packed form multiplies.
 cudaError_t launch_lane_gemm_one(const GemmJobDev& job, cudaStream_t st);
 // ntmax: the widest output tile (the operator w must be packed for gemm_tile_n(N, ntmax))
 GemmJobDev make_gemm_job(const LaneSideDev& in, const LaneSideDev& out, const float* w, int K, int N, double scale,
