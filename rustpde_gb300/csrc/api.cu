@@ -89,9 +89,10 @@ static void upload_plan(Arena& A, const StepPlan& plan, DevPlan& dp) {
       sj = A.upload(L.sjobs);
       t = A.upload(tiles);
       nt = (int)tiles.size();
-    } else if (L.kernel == K_GEMM) {
+    } else if (L.kernel == K_GEMM || L.kernel == K_PACK) {
       std::vector<int4> tiles;
-      gemm_tiles(L.jobs, tiles);
+      if (L.kernel == K_PACK) pack_chunks(L.jobs, tiles);
+      else gemm_tiles(L.jobs, tiles);
       j = A.upload(L.jobs);
       t = A.upload(tiles);
       nt = (int)tiles.size();
@@ -125,8 +126,9 @@ static cudaError_t launch_entry(const StepLaunch& L, const DevPlan& dp, size_t k
   if (L.kernel == K_SPLIT_GEMM)
     return L.sjobs.empty() ? cudaSuccess
                            : launch_split_gemm(dp.sjobs[k], dp.tiles[k], dp.ntiles[k], L.sjobs[0].digits, st);
+  if (L.kernel == K_PACK) return launch_pack_lanes(dp.jobs[k], dp.tiles[k], dp.ntiles[k], st);
   if (L.kernel == K_GEMM)
-    return launch_lane_gemm(dp.jobs[k], dp.tiles[k], dp.ntiles[k], dp.max_nt[k], st, L.gemm_ws != 0);
+    return launch_lane_gemm(dp.jobs[k], dp.tiles[k], dp.ntiles[k], dp.max_nt[k], st, L.gemm_form);
   return launch_step_kernel(L.kernel, (int)L.items.size(), L.smem, st, cases, dp.work[k]);
 }
 
@@ -617,6 +619,7 @@ void build_case(RbcCase* c, bool with_graph = true, char* state_region = nullptr
     h.m_cv = A.alloc((size_t)3 * std::max(h.kx, 1) * h.ky * 16);
     // FP32 state copy: rows padded to 16 bytes, complex rows as [re | im] (rbc_dev.h)
     h.m_s32 = A.alloc((size_t)3 * h.mxc * s32_row_floats(h) * 4);
+    h.m_pk = static_cast<float*>(A.alloc(mixed_pack_bytes(h)));
     h.m_bcx = static_cast<const float*>(A.alloc((size_t)nx * ny * 4));
     h.m_bcy = static_cast<const float*>(A.alloc((size_t)nx * ny * 4));
     for (MixedOps* o : mixed_sets) {
@@ -1595,7 +1598,7 @@ int rbc_batch_create(const RbcParams* params, int ncases, RbcBatch** out) {
         if (L.kernel == K_GEMM) {
           int nt = 0;
           for (const GemmJobDev& j : L.jobs) nt = std::max(nt, j.NT);
-          id = K_GEMM * 1000 + nt + (L.gemm_ws ? 500 : 0);
+          id = K_GEMM * 1000 + nt + 250 * L.gemm_form;
         }
         k.push_back(id);
       }
@@ -1650,11 +1653,16 @@ int rbc_batch_create(const RbcParams* params, int ncases, RbcBatch** out) {
         if (t < t_best_alt) {
           t_best_alt = t;
           best_alt_kernel = ks[0];
-          if (t < t_base) best = (int)a;
+          // the unpacked GEMM forms (4, 5) are timed but only RBC_BATCH_FORM
+          // takes them: alone one may lead by 10 % at a short K, in the whole
+          // step the packed form led everywhere (ms, packed | 4 | 5: 256-case
+          // ensemble 2.97 | 3.19 | 3.21, 8 cases 0.166 | 0.172 | 0.178, one
+          // 512 x 512 box 0.49 | 0.62 | 0.58)
+          if (t < t_base && a < 3) best = (int)a;
         }
       }
       if (t_base >= 0) {
-        const bool gemm = bk.plan.launches[gb[pi][0]].kernel == K_GEMM;
+        const bool gemm = bk.plan.launches[gb[pi].back()].kernel == K_GEMM;  // (packing or the state copy may come first)
         const std::vector<int>& fl = gemm ? forced_gemm : forced_fp64;
         size_t pos = 0;  // this decision's place among the batch's decisions of its kind
         for (const auto& t : b->tuning) pos += t.gemm == gemm;
@@ -1663,7 +1671,8 @@ int rbc_batch_create(const RbcParams* params, int ncases, RbcBatch** out) {
         else if (pos < fl.size()) forced = fl[pos];
         if (forced == 0) best = -1;
         else if (forced > 0 && (size_t)forced <= nalt) best = forced - 1;
-        b->tuning.push_back({bk.plan.launches[gb[pi][0]].kernel, best_alt_kernel, t_base, t_best_alt, best + 1, gemm});
+        b->tuning.push_back({gemm ? (int)K_GEMM : bk.plan.launches[gb[pi][0]].kernel, gemm ? (int)K_GEMM : best_alt_kernel,
+                             t_base, t_best_alt, best + 1, gemm});
       }
       const StepPlan& src = best >= 0 ? alts[best] : bk.plan;
       for (size_t li : (best >= 0 ? ga[best][pi] : gb[pi])) tuned.launches.push_back(src.launches[li]);

@@ -1047,7 +1047,7 @@ size_t gemm_ws_smem_bytes(int NT) {
   return std::max(dev::gemm_ws_smem_base(NT), gemm_smem_bytes(NT));
 }
 
-static size_t gemm_packed_smem_bytes(int NT) {
+size_t gemm_packed_smem_bytes(int NT) {
   return (size_t)2 * dev::kPackedChunkBytes + (size_t)4 * NT * kGemmKC * 4 + 64 + kGemmLanes * 8;
 }
 
@@ -1146,10 +1146,25 @@ LaneSideDev lane_cols(void* const* ptrs, int nf, int cols, int len, int row_len,
   return s;
 }
 
+void pack_chunks(const std::vector<GemmJobDev>& jobs, std::vector<int4>& chunks) {
+  for (size_t j = 0; j < jobs.size(); j++)
+    for (int l = 0; l < jobs[j].lanes; l += kGemmLanes)
+      for (int c = 0; c < jobs[j].kchunks; c++) chunks.push_back(make_int4((int)j, l, c, 0));
+}
+cudaError_t launch_pack_lanes(const GemmJobDev* jobs, const int4* chunks, int nchunks, cudaStream_t st) {
+  if (nchunks <= 0) return cudaSuccess;
+  return launch_pdl(dev::k_pack_lanes, nchunks, kGemmThreads, 0, st, jobs, chunks);
+}
+
 cudaError_t launch_lane_gemm(const GemmJobDev* jobs, const int4* tiles, int ntiles_total, int max_nt,
-                             cudaStream_t st, bool ws) {
+                             cudaStream_t st, int form) {
   if (ntiles_total <= 0) return cudaSuccess;
-  if (ws) {
+  if (form == 2) {
+    if (max_nt > 64) return cudaErrorInvalidValue;
+    return launch_pdl(dev::k_lane_gemm_packed, ntiles_total, dev::kPackedThreads, gemm_packed_smem_bytes(max_nt), st,
+                      jobs, tiles);
+  }
+  if (form == 1) {
     if (max_nt > 64) return cudaErrorInvalidValue;
     return launch_pdl(dev::k_lane_gemm_ws, ntiles_total, kGemmThreads, gemm_ws_smem_bytes(max_nt), st, jobs, tiles);
   } else {

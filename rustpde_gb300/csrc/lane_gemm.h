@@ -62,11 +62,17 @@ void gemm_tiles(const std::vector<GemmJobDev>& jobs, std::vector<int4>& tiles);
 size_t gemm_smem_bytes(int NT);
 // the warp-specialised form's (NT <= 64): two input and two operator chunk buffers
 size_t gemm_ws_smem_bytes(int NT);
+// the packed form's (NT <= 64): two chunk buffers of packed lanes and operator
+size_t gemm_packed_smem_bytes(int NT);
 cudaError_t configure_gemm_kernels();
-// jobs and tiles are device arrays; max_nt = largest NT among the jobs.  ws:
-// the warp-specialised form (producer, MMA and flush warps; max_nt <= 64).
+// jobs and tiles are device arrays; max_nt = largest NT among the jobs.  form 1:
+// warp-specialised (producer, MMA and flush warps; max_nt <= 64); 2: packed
+// input (max_nt <= 64, after launch_pack_lanes on the same jobs).
 cudaError_t launch_lane_gemm(const GemmJobDev* jobs, const int4* tiles, int ntiles_total, int max_nt,
-                             cudaStream_t st, bool ws = false);
+                             cudaStream_t st, int form = 0);
+// Chunks (job, first lane, chunk, 0) of a job list, and their packing.
+void pack_chunks(const std::vector<GemmJobDev>& jobs, std::vector<int4>& chunks);
+cudaError_t launch_pack_lanes(const GemmJobDev* jobs, const int4* chunks, int nchunks, cudaStream_t st);
 
 // Poll limit of the kernel's bounded completion waits on the current device
 // (negative: the default, 2^22 polls).  A small limit makes the waits run out

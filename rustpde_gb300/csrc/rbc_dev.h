@@ -191,6 +191,7 @@ struct CaseDev {
   void* m_z;      // box: FP32 pinv_x of the divergence (mxc x ny), then the FP32 Poisson row solutions (mxc x myc)
   void* m_s32;    // FP32 copy of ux, uy, temp, the y GEMM's input: 3 x mxc rows of s32_row_floats(), a
                   // real row padded to a multiple of 4 floats, a complex row as [re | im] parts of that length
+  float* m_pk;    // packed input lanes of the GEMM in hand (lane_gemm.h GemmJobDev::apk)
   const float* m_bcx;  // FP32 d(fieldbc)/dx, transposed: ny x nx
   const float* m_bcy;  // FP32 d(fieldbc)/dy - m_bcg, transposed: ny x nx
 

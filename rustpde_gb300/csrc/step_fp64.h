@@ -39,12 +39,13 @@ enum StepKernel {
   K_SPL_X3, K_SPL_W,
   K_NUM_STEP_KERNELS,
   K_GEMM = 100,  // tensor-core lane GEMM (jobs instead of work items)
+  K_PACK = 102,  // packed input lanes of the lane GEMM that follows (the same jobs)
   K_SPLIT_GEMM = 101  // split GEMM (sjobs instead of work items)
 };
 
 struct StepLaunch {
   int kernel;
-  int gemm_ws = 0;  // K_GEMM: 1 for the warp-specialised form
+  int gemm_form = 0;  // K_GEMM: 0 classic, 1 warp-specialised, 2 packed input
   int pass = -1;  // launches of one pass share the id (the autotuner swaps whole passes)
   size_t smem;
   std::vector<int4> items;       // (case index, first lane, lane count, 0)
@@ -87,6 +88,8 @@ struct MixedOps {
 // form exists, else 128-thread CTAs; 3: as 2 with the periodic Y2 launches
 // fused.  The GEMM tiles follow ops.ntmax.
 StepPlan build_mixed_plan(const CaseDev& c, const MixedOps& ops, int variant);
+// bytes of CaseDev::m_pk that build_mixed_plan's packed GEMMs use
+size_t mixed_pack_bytes(const CaseDev& c);
 int lane_kernel_subs(int kernel);
 bool lane_kernel_rows(int kernel);
 cudaError_t launch_lane_kernel(int kernel, int nblocks, cudaStream_t s, const CaseDev* cases, const int4* work);

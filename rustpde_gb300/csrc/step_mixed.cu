@@ -203,31 +203,64 @@ StepPlan build_mixed_plan(const CaseDev& c, const MixedOps& ops, int variant) {
     }
     push(L);
   };
-  auto add_gemm = [&](const GemmJobDev& j) {
+  // A GEMM launch.  With operators in tiles of 64 (and not the warp-specialised
+  // form) its input lanes are packed first, in a launch of the same pass.  The
+  // bits are the other forms', and it was the faster at every size: us of a
+  // step, classic | packed, periodic 512 x 257 148 | 121, box 129 x 129 184 |
+  // 143, box 264 x 264 281 | 198; 256-case ensemble 3.09 | 2.97 ms, its box x
+  // backward GEMMs 0.207 | 0.047 + 0.131.
+  const bool packed = ops.ntmax == 64 && !ops.ws;
+  auto add_gemms = [&](std::vector<GemmJobDev> jobs) {
+    const bool own = group < 0;
+    if (own) group = npass++;
+    if (packed) {
+      size_t off = 0;
+      for (GemmJobDev& j : jobs) {
+        j.apk = reinterpret_cast<float*>(reinterpret_cast<char*>(c.m_pk) + off);
+        off += packed_lanes_bytes(j.lanes, j.K);
+      }
+      StepLaunch P;
+      P.kernel = K_PACK;
+      P.smem = 0;
+      P.jobs = jobs;
+      push(P);
+    }
     StepLaunch L;
     L.kernel = K_GEMM;
-    L.gemm_ws = ops.ws;
-    L.smem = ops.ws ? gemm_ws_smem_bytes(j.NT) : gemm_smem_bytes(j.NT);
-    L.jobs.push_back(j);
+    L.gemm_form = packed ? 2 : ops.ws;
+    L.smem = 0;
+    for (const GemmJobDev& j : jobs)
+      L.smem = std::max(L.smem, packed ? gemm_packed_smem_bytes(j.NT) : ops.ws ? gemm_ws_smem_bytes(j.NT) : gemm_smem_bytes(j.NT));
+    L.jobs = std::move(jobs);
     push(L);
+    if (own) group = -1;
   };
+  auto add_gemm = [&](const GemmJobDev& j) { add_gemms({j}); };
   const int mx = c.mx, ny = c.ny, myc = c.myc, kx = c.kx, ky = c.ky;
   // FP32 copy of the state rows, read by G1 (rows of s32_row_floats floats)
   const int s32ld = s32_row_floats(c);
   void* s32[3];
   for (int f = 0; f < 3; f++) s32[f] = static_cast<float*>(c.m_s32) + (size_t)f * c.mxc * s32ld;
-  add(K_STATE_F32, c.mxc, 0);
+  // G1 packs its lanes straight from the FP64 state; the forms that do not pack
+  // read an FP32 copy of it, made in the same pass
+  void* st64[3] = {c.ux, c.uy, c.temp};
+  group = npass++;
+  if (!packed) add(K_STATE_F32, c.mxc, 0);
   if (c.kind == KIND_PERIODIC) {
-    // G1: rows of ux, uy, temp (complex, [re | im] parts) -> [Y0 | Y1] (FP32), stored transposed
-    LaneSideDev in = lane_rows(s32, 3, mx, myc, s32ld / 2, LT_F32, true);
-    in.elem_stride = 1;
-    in.part_stride = s32ld / 2;
+    // G1: rows of ux, uy, temp (complex; FP32 copy: [re | im] parts) -> [Y0 | Y1] (FP32), stored transposed
+    LaneSideDev in = packed ? lane_rows(st64, 3, mx, myc, myc, LT_F64, true)
+                            : lane_rows(s32, 3, mx, myc, s32ld / 2, LT_F32, true);
+    if (!packed) {
+      in.elem_stride = 1;
+      in.part_stride = s32ld / 2;
+    }
     LaneSideDev out;
     std::memset(&out, 0, sizeof out);
     for (int f = 0; f < 3; f++) out.ptr[f] = c.m_y[f];
     out.nf = 3; out.rows = mx; out.parts = 2; out.type = LT_F32;
     out.lane_stride = 2; out.part_stride = 1; out.elem_stride = 2LL * mx; out.len = 2 * ny; out.lane_fast = 1;
     add_gemm(make_gemm_job(in, out, ops.y1, myc, 2 * ny, 1.0, c.status, ops.ntmax));
+    group = -1;
     // X: FP32 convection, one CTA per column (256 threads, or 128 in the batch forms)
     add(lane_parallel ? K_PER_X_MIXED_T128 : K_PER_X_MIXED, ny, dev::smem_per_x_mixed(c));
     // G2: y transform of the x-transformed products (FP32, transposed) -> m_cv (FP64)
@@ -275,36 +308,32 @@ StepPlan build_mixed_plan(const CaseDev& c, const MixedOps& ops, int variant) {
   const int myld = pad4(mxc);
   {
     void* yo[3] = {c.m_y[0], c.m_y[1], c.m_y[2]};
-    add_gemm(make_gemm_job(lane_rows(s32, 3, mxc, myc, s32ld, LT_F32, false),
+    add_gemm(make_gemm_job(packed ? lane_rows(st64, 3, mxc, myc, myc, LT_F64, false)
+                                  : lane_rows(s32, 3, mxc, myc, s32ld, LT_F32, false),
                            side(yo, 3, mxc, 2 * ny, 1, myld, LT_F32, 1), ops.y1, myc, 2 * ny, 1.0, c.status, ops.ntmax));
+    group = -1;
   }
   // GX: x stencils, derivatives and backward transforms -> physical (transposed), one launch of 4 jobs
   {
-    StepLaunch L;
-    L.kernel = K_GEMM;
-    L.pass = npass++;
+    std::vector<GemmJobDev> jobs;
     void* a_in[2] = {c.m_y[0], c.m_y[1]};
     void* a_out[2] = {c.m_ph[0], c.m_ph[1]};
-    L.jobs.push_back(make_gemm_job(lane_rows(a_in, 2, ny, mxc, myld, LT_F32, false),
-                                   lane_rows(a_out, 2, ny, 2 * nx, 2 * nx, LT_F32, false), ops.xa, mxc, 2 * nx, 1.0,
+    jobs.push_back(make_gemm_job(lane_rows(a_in, 2, ny, mxc, myld, LT_F32, false),
+                                 lane_rows(a_out, 2, ny, 2 * nx, 2 * nx, LT_F32, false), ops.xa, mxc, 2 * nx, 1.0,
                                    c.status, ops.ntmax));
     void* b_in[2] = {fptr(c.m_y[0], (size_t)ny * myld), fptr(c.m_y[1], (size_t)ny * myld)};
     void* b_out[2] = {c.m_ph[2], c.m_ph[3]};
-    L.jobs.push_back(make_gemm_job(lane_rows(b_in, 2, ny, mxc, myld, LT_F32, false),
+    jobs.push_back(make_gemm_job(lane_rows(b_in, 2, ny, mxc, myld, LT_F32, false),
                                    lane_rows(b_out, 2, ny, nx, nx, LT_F32, false), ops.xb, mxc, nx, 1.0, c.status, ops.ntmax));
     void* c_in[1] = {c.m_y[2]};
     void* c_out[1] = {c.m_ph[4]};
-    L.jobs.push_back(make_gemm_job(lane_rows(c_in, 1, ny, mxc, myld, LT_F32, false),
+    jobs.push_back(make_gemm_job(lane_rows(c_in, 1, ny, mxc, myld, LT_F32, false),
                                    lane_rows(c_out, 1, ny, nx, nx, LT_F32, false), ops.xc, mxc, nx, 1.0, c.status, ops.ntmax));
     void* d_in[1] = {fptr(c.m_y[2], (size_t)ny * myld)};
     void* d_out[1] = {c.m_ph[5]};
-    L.jobs.push_back(make_gemm_job(lane_rows(d_in, 1, ny, mxc, myld, LT_F32, false),
+    jobs.push_back(make_gemm_job(lane_rows(d_in, 1, ny, mxc, myld, LT_F32, false),
                                    lane_rows(d_out, 1, ny, nx, nx, LT_F32, false), ops.xd, mxc, nx, 1.0, c.status, ops.ntmax));
-    size_t sm = 0;
-    for (const GemmJobDev& j : L.jobs) sm = std::max(sm, ops.ws ? gemm_ws_smem_bytes(j.NT) : gemm_smem_bytes(j.NT));
-    L.smem = sm;
-    L.gemm_ws = ops.ws;
-    p.launches.push_back(L);
+    add_gemms(std::move(jobs));
   }
   // products (FP32)
   add(K_BOX_PROD_MIXED, ny, 0);
@@ -366,6 +395,19 @@ StepPlan build_mixed_plan(const CaseDev& c, const MixedOps& ops, int variant) {
   if (lp) add_lp(K_LP_BOX_Y5, nx, ny);
   else add(lane_parallel ? K_BOX_Y5_T128 : K_BOX_Y5, nx, dev::smem_box_y5(c));
   return p;
+}
+
+// Largest packed input of the plan's GEMM launches.
+size_t mixed_pack_bytes(const CaseDev& c) {
+  MixedOps none;
+  size_t m = 0;
+  for (const StepLaunch& L : build_mixed_plan(c, none, 0).launches) {
+    if (L.kernel != K_PACK) continue;
+    size_t b = 0;
+    for (const GemmJobDev& j : L.jobs) b += packed_lanes_bytes(j.lanes, j.K);
+    m = std::max(m, b);
+  }
+  return m;
 }
 
 // Largest dynamic shared memory of the CTA passes of build_mixed_plan(c, ops,
@@ -438,10 +480,15 @@ __attribute__((noinline)) static int same_arrays(int kernel) {
 // write, counted once (operator tables and the boundary-field constants
 // included; re-reads from L2 and shared memory are not).
 double launch_algorithmic_bytes(const StepLaunch& L, const CaseDev* cases) {
+  if (L.kernel == K_PACK) {
+    double b = 0;
+    for (const GemmJobDev& j : L.jobs) b += (double)j.lanes * j.K * ((j.in.type == LT_F64 ? 8 : 4) + 8);
+    return b;
+  }
   if (L.kernel == K_GEMM) {
     double b = 0;
     for (const GemmJobDev& j : L.jobs) {
-      const double ie = j.in.type == LT_F64 ? 8 : 4, oe = j.out.type == LT_F64 ? 8 : 4;
+      const double ie = L.gemm_form == 2 || j.in.type == LT_F64 ? 8 : 4, oe = j.out.type == LT_F64 ? 8 : 4;
       b += (double)j.lanes * ((double)j.K * ie + (double)j.N * oe);
       b += (double)j.ntiles * j.kchunks * 2.0 * j.NT * kGemmKC * 4;  // split operator
     }
@@ -523,6 +570,7 @@ const char* step_kernel_name(int kernel) {
                                 "split_x1_box", "split_x1_periodic", "split_products", "split_conv",
                                 "periodic_y2_cv", "box_y2_cv", "split_x3", "split_poisson_rows"};
   if (kernel == K_GEMM) return "lane_gemm";
+  if (kernel == K_PACK) return "pack_lanes";
   if (kernel == K_SPLIT_GEMM) return "split_gemm";
   if (kernel >= 0 && kernel < K_NUM_STEP_KERNELS) return names[kernel];
   return "";

@@ -113,3 +113,33 @@ def test_space_timeout_leaves_nan(R):
     finally:
         R.set_gemm_wait_limit(-1)
     np.testing.assert_array_equal(s.forward(v), ref)
+
+
+@pytest.mark.parametrize("n", [95, 96, 97, 130, 511, 512])
+def test_mixed_lanes_in_one_call_equal_parts(R, n):
+    # from 1024 lanes and n = 96 the input is packed first (in parts of the
+    # scratch's 4096 lanes); the calls of 1000 lanes are not: the same products
+    # in the same order, so the same bits
+    L = R.Lanes(R.Base(1, n), R.PREC_MIXED, hholtz_c=5e-4)
+    rng = np.random.default_rng(n)
+    for lanes in (1024, 4097):
+        phys = rng.standard_normal((lanes, n))
+        spec = rng.standard_normal((lanes, L.m))
+        for op in (R.OP_FORWARD, R.OP_BACKWARD, R.OP_TO_ORTHO, R.OP_HHOLTZ):
+            x = spec if op in (R.OP_BACKWARD, R.OP_TO_ORTHO) else phys
+            parts = np.concatenate([L.apply(op, x[k:k + 1000]) for k in range(0, lanes, 1000)])
+            np.testing.assert_array_equal(L.apply(op, x), parts)
+    assert L.status() == 0
+
+
+def test_mixed_packed_lanes_timeout_is_reported(R):
+    L = R.Lanes(R.Base(1, 128), R.PREC_MIXED)
+    x = np.random.default_rng(6).standard_normal((1100, 128))
+    ref = L.apply(R.OP_FORWARD, x)
+    R.set_gemm_wait_limit(0)
+    try:
+        L.apply(R.OP_FORWARD, x)
+        assert L.status() & 2
+    finally:
+        R.set_gemm_wait_limit(-1)
+    np.testing.assert_array_equal(L.apply(R.OP_FORWARD, x), ref)
