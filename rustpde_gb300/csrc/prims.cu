@@ -73,6 +73,23 @@ void* Arena::alloc(size_t bytes) {
   bytes_ += bytes;
   return p;
 }
+void Arena::upload_all(std::initializer_list<std::pair<const std::vector<double>*, const double**>> tables) {
+  size_t n = 0;
+  for (const auto& t : tables) n += (t.first->size() + 31) & ~size_t(31);
+  if (n > 16384) {  // large tables: an allocation each was faster than gathering them
+    for (const auto& t : tables) *t.second = upload(*t.first);
+    return;
+  }
+  double* d = n != 0 ? static_cast<double*>(alloc(n * 8)) : nullptr;
+  std::vector<double> h(n, 0.0);
+  size_t off = 0;
+  for (const auto& t : tables) {
+    *t.second = t.first->empty() ? nullptr : d + off;
+    std::copy(t.first->begin(), t.first->end(), h.begin() + off);
+    off += (t.first->size() + 31) & ~size_t(31);
+  }
+  if (n != 0) copy_h2d(d, h.data(), n * 8);
+}
 void Arena::copy_h2d(void* d, const void* h, size_t n) {
   cudaError_t e = cudaMemcpy(d, h, n, cudaMemcpyHostToDevice);
   if (e != cudaSuccess) throw std::runtime_error(std::string("cudaMemcpy failed: ") + cudaGetErrorString(e));
@@ -118,23 +135,22 @@ BasisDev upload_basis(Arena& a, const HostBasis& b, bool odd) {
   d.kind = b.kind;
   d.n = b.n;
   d.m = b.m;
-  d.diag = a.upload(b.diag);
   d.unit_diag = !b.diag.empty() && std::all_of(b.diag.begin(), b.diag.end(), [](double v) { return v == 1.0; });
-  d.low2 = a.upload(b.low2);
-  d.fo_off = a.upload(b.fo_off);
-  d.fo_w = a.upload(b.fo_w);
-  d.fo_dinv = a.upload(b.fo_dinv);
+  std::vector<double> fa, fb, fc;
   if (!b.fo_dinv.empty()) {
     const int m = b.m;
-    std::vector<double> fa(m), fb(m), fc(m, 0.0);
+    fa.resize(m);
+    fb.resize(m);
+    fc.assign(m, 0.0);
     for (int i = 0; i < m; i++) {
       fa[i] = b.diag[i] * b.fo_dinv[i];
       fb[i] = b.low2[i] * b.fo_dinv[i];
       if (i >= 2) fc[i] = -b.fo_off[i - 2] * b.fo_dinv[i];
     }
-    d.fo_a = a.upload(fa);
-    d.fo_b = a.upload(fb);
-    d.fo_c = a.upload(fc);
+  }
+  a.upload_all({{&b.diag, &d.diag}, {&b.low2, &d.low2}, {&b.fo_off, &d.fo_off}, {&b.fo_w, &d.fo_w},
+                {&b.fo_dinv, &d.fo_dinv}, {&fa, &d.fo_a}, {&fb, &d.fo_b}, {&fc, &d.fo_c}});
+  if (!b.fo_dinv.empty()) {
     double* sc = static_cast<double*>(a.alloc(8 * 32 * 8));
     dev::k_scan_fo<<<1, 32>>>(d, sc);
     cuda_check(cudaGetLastError(), "scan tables");
@@ -162,12 +178,14 @@ ChebXformDev upload_cheb(Arena& a, int n, bool allow_fft) {
   if (d.use_fft) {
     d.L = 2 * N;
     d.log2L = ilog2(d.L);
-    d.tw = reinterpret_cast<const double2*>(a.upload(twiddles(d.L)));
+    // (six spaces of a case share these: the host's extended-precision
+    // sines and cosines of a 512 x 257 case took 4 ms six times over)
+    d.tw = reinterpret_cast<const double2*>(a.shared_table<double>(0, d.L, [&] { return twiddles(d.L); }));
   } else {
     d.L = 0;
     const ChebDense& t = cheb_dense(n);
-    d.fwd = a.upload(t.fwd);
-    d.bwd = a.upload(t.bwd);
+    d.fwd = a.shared_table<double>(1, n, [&] { return t.fwd; });
+    d.bwd = a.shared_table<double>(2, n, [&] { return t.bwd; });
   }
   return d;
 }
@@ -196,11 +214,12 @@ FourierXformDev upload_fourier(Arena& a, int n) {
       while (r % p == 0) push(p);
     if (r > 1) push(r);
   }
-  std::vector<double> tw = twiddles(n);
-  d.tw = reinterpret_cast<const double2*>(a.upload(tw));
-  std::vector<float> twf(tw.size());
-  for (size_t i = 0; i < tw.size(); i++) twf[i] = (float)tw[i];
-  d.twf = reinterpret_cast<const float2*>(a.upload(twf));
+  std::vector<double> tw;
+  d.tw = reinterpret_cast<const double2*>(a.shared_table<double>(0, n, [&] { return tw = twiddles(n); }));
+  d.twf = reinterpret_cast<const float2*>(a.shared_table<float>(3, n, [&] {
+    if (tw.empty()) tw = twiddles(n);
+    return std::vector<float>(tw.begin(), tw.end());
+  }));
   return d;
 }
 
@@ -209,9 +228,7 @@ PinvDev upload_pinv(Arena& a, int n) {
   PinvDev d;
   std::memset(&d, 0, sizeof d);
   d.n = n;
-  d.dia = a.upload(p.dia);
-  d.up1 = a.upload(p.up1);
-  d.up2 = a.upload(p.up2);
+  a.upload_all({{&p.dia, &d.dia}, {&p.up1, &d.up1}, {&p.up2, &d.up2}});
   return d;
 }
 
@@ -235,10 +252,7 @@ FdmaDev upload_fdma(Arena& a, const std::vector<Band4>& rows, bool odd) {
     for (size_t i = 0; i < f.up1.size(); i++) up1[(size_t)r * m + i] = -f.up1[i] / f.dia[i];
     for (size_t i = 0; i < f.up2.size(); i++) up2[(size_t)r * m + i] = -f.up2[i] / f.dia[i];
   }
-  d.low = a.upload(low);
-  d.dinv = a.upload(dinv);
-  d.up1 = a.upload(up1);
-  d.up2 = a.upload(up2);
+  a.upload_all({{&low, &d.low}, {&dinv, &d.dinv}, {&up1, &d.up1}, {&up2, &d.up2}});
   double* sc = static_cast<double*>(a.alloc((size_t)R * kFdmaScan * 8));
   dev::k_scan_fdma<<<R, 32>>>(d, sc);
   cuda_check(cudaGetLastError(), "scan tables");

@@ -10,6 +10,7 @@
 
 #include <stdexcept>
 #include <string>
+#include <map>
 #include <vector>
 
 #include "host_ops.h"
@@ -37,11 +38,23 @@ class Arena {
     copy_h2d(p, v.data(), v.size() * sizeof(T));
     return p;
   }
+  // several small tables in one allocation and one copy (each on a 256-byte boundary;
+  // an empty one gives a null pointer): an allocation with its zero fill and
+  // copy is 30 us of host time, and a case has some hundred small tables
+  void upload_all(std::initializer_list<std::pair<const std::vector<double>*, const double**>> tables);
+  // a read-only table of this arena's owner that several of its parts use (the
+  // transforms of one length), made once
+  template <class T, class Make> const T* shared_table(int what, int n, Make make) {
+    const void*& p = shared_[std::make_pair(what, n)];
+    if (p == nullptr) p = upload(std::vector<T>(make()));
+    return static_cast<const T*>(p);
+  }
   size_t bytes() const { return bytes_; }
 
  private:
   void copy_h2d(void* d, const void* h, size_t n);
   std::vector<void*> ptrs_;
+  std::map<std::pair<int, int>, const void*> shared_;
   size_t bytes_ = 0;
   bool ordered_ = false;
 };
