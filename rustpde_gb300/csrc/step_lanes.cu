@@ -56,10 +56,10 @@ __device__ __forceinline__ T stencil_lane(const BasisDev& b, const T* c, long lo
   if (b.kind == 0 || b.kind == 5) return c[(long long)i * s];
   const int m = b.m;
   T v = zero_v<T>();
-  if (i < m) v = b.unit_diag ? c[(long long)i * s] : scal(c[(long long)i * s], b.diag[i]);
+  if (i < m) v = b.unit_diag ? c[(long long)i * s] : scal(c[(long long)i * s], __ldg(b.diag + i));
   if (i >= 2 && i - 2 < m) {
     const T t = c[(long long)(i - 2) * s];
-    v = (i < m) ? fmas(v, t, b.low2[i - 2]) : scal(t, b.low2[i - 2]);
+    v = (i < m) ? fmas(v, t, __ldg(b.low2 + i - 2)) : scal(t, __ldg(b.low2 + i - 2));
   }
   return v;
 }
@@ -109,9 +109,9 @@ __device__ __forceinline__ void fdma_bwd_lane(const FdmaRow& f, T* x, long long 
 template <class T>
 __device__ __forceinline__ T pinv_lane(const PinvDev& p, const T* a, long long s, int r) {
   const int m = p.n - 2;
-  T v = scal(a[(long long)r * s], p.dia[r]);
-  if (r < m - 2) v = fmas(v, a[(long long)(r + 2) * s], p.up1[r]);
-  if (r < m - 4) v = fmas(v, a[(long long)(r + 4) * s], p.up2[r]);
+  T v = scal(a[(long long)r * s], __ldg(p.dia + r));
+  if (r < m - 2) v = fmas(v, a[(long long)(r + 2) * s], __ldg(p.up1 + r));
+  if (r < m - 4) v = fmas(v, a[(long long)(r + 4) * s], __ldg(p.up2 + r));
   return v;
 }
 
@@ -152,17 +152,24 @@ __device__ __forceinline__ int top_par(int n, int q) { return ((n - 1 - q) & 1) 
 // the compiler cannot reorder) left about 15 stall cycles per instruction.
 // The arithmetic and its order are those of the one-element-at-a-time form.
 constexpr int kPB = 8;
-// box y3 and y5 (row chains, 40 registers) measured best with 2 and 1 elements
-// ahead: y3 0.23 / 0.26 / 0.35 ms per ensemble step with 2 / 1 / 4, y5 0.29 /
-// 0.30 with 1 / 4
+// Row kernels: every thread streams its own row, so what is loaded ahead also
+// sits in L1 until the row's next element of the same sector is read, and more
+// elements ahead is not always better.  Box y3: recurrences 2, other loops 4;
+// y4 4; y5 1 and 8.  With every loop's loads ahead of its stores (ms per step
+// of the 256-case ensemble, before | now): y3 0.225 | 0.188, y4 0.160 | 0.129,
+// y5 0.290 | 0.238.
 constexpr int kPBY3 = 2;
 constexpr int kPBY5 = 1;
-// complex (periodic Y2) chains, elements of two doubles each: Y2A 4 (8 took
-// 196 registers, five 64-thread blocks per SM), Y2B 6, Y2C 8, each the
-// fastest measured
-constexpr int kPBC = 4;
-constexpr int kPBCB = 6;
-constexpr int kPBCC = 8;
+constexpr int kPBY3F = 4;
+constexpr int kPBY4 = 4;
+constexpr int kPBY5M = 8;
+// Periodic Y2, one part of a row per thread.  Y2A 3, Y2B 12 and Y2C 8 are the
+// fastest alone (0.40, 0.26 and 0.26 ms), 2, 8 and 2 (0.44, 0.26, 0.32 ms) in
+// the step, where the box group's passes share the L1 caches: 2.88 ms against
+// 2.95.  With whole complex rows per thread: 0.51, 0.33, 0.31 ms, step 2.99 ms.
+constexpr int kPBC = 2;
+constexpr int kPBCB = 8;
+constexpr int kPBCC = 2;
 
 // Chebyshev derivative d = D a on the indices of parity q, descending:
 // d_{n-1} = 0, d_i = 2(i+1) a_{i+1} + d_{i+2}, d_0 = a_1 + d_2 / 2; a(i)
@@ -216,9 +223,10 @@ __device__ __forceinline__ void fdma_fwd_par(const FdmaRow& f, T* x, long long s
   }
 }
 
-// Fdma back substitution on the parity-q indices of a strided lane, in place
-template <class T, int PB = kPB>
-__device__ __forceinline__ void fdma_bwd_par(const FdmaRow& f, T* x, long long s, int q) {
+// Fdma back substitution on the parity-q indices of a strided lane, its results
+// to store(j, x_j)
+template <class T, int PB = kPB, class S>
+__device__ __forceinline__ void fdma_bwd_par(const FdmaRow& f, const T* x, long long s, int q, S store) {
   T p2 = zero_v<T>(), p4 = zero_v<T>();
   for (int j0 = top_par(f.m, q); j0 >= 0; j0 -= 2 * PB) {
     T xv[PB];
@@ -239,11 +247,16 @@ __device__ __forceinline__ void fdma_bwd_par(const FdmaRow& f, T* x, long long s
       T v = scal(xv[e], dv[e]);
       if (j + 2 < f.m) v = fmas(v, p2, u1[e]);
       if (j + 4 < f.m) v = fmas(v, p4, u2[e]);
-      x[(long long)j * s] = v;
+      store(j, v);
       p4 = p2;
       p2 = v;
     }
   }
+}
+// ... in place
+template <class T, int PB = kPB>
+__device__ __forceinline__ void fdma_bwd_par(const FdmaRow& f, T* x, long long s, int q) {
+  fdma_bwd_par<T, PB>(f, x, s, q, [&](int j, T v) { x[(long long)j * s] = v; });
 }
 
 // pinv rows fused with the Fdma forward elimination on the parity-q indices:
@@ -270,6 +283,20 @@ __device__ __forceinline__ void pinv_fwd_par(const PinvDev& p, const FdmaRow& f,
       out[(long long)i * os] = v;
       xm2 = v;
     }
+  }
+}
+
+// store(k, load(k)) for k = q, q + 2, ... < n, PB loads ahead of their stores
+// (a load behind the store before it would wait out its own latency)
+template <int PB = kPB, class A, class S>
+__device__ __forceinline__ void map_par(int n, int q, A load, S store) {
+  for (int k0 = q; k0 < n; k0 += 2 * PB) {
+    double v[PB];
+#pragma unroll
+    for (int e = 0; e < PB; e++) v[e] = k0 + 2 * e < n ? load(k0 + 2 * e) : 0.0;
+#pragma unroll
+    for (int e = 0; e < PB; e++)
+      if (k0 + 2 * e < n) store(k0 + 2 * e, v[e]);
   }
 }
 
@@ -411,15 +438,17 @@ __global__ void __launch_bounds__(128) k_lp_box_x4(const CaseDev* __restrict__ c
     auto pv = [&](int r) { return (z0 && r == 0) ? 0.0 : p1[(long long)r * myc]; };
     if (b.kind == 0 || b.kind == 5) return pv(i);
     double v = 0.0;
-    if (i < b.m) v = b.unit_diag ? pv(i) : pv(i) * b.diag[i];
-    if (i >= 2 && i - 2 < b.m) v = (i < b.m) ? fma(pv(i - 2), b.low2[i - 2], v) : pv(i - 2) * b.low2[i - 2];
+    if (i < b.m) v = b.unit_diag ? pv(i) : pv(i) * __ldg(b.diag + i);
+    if (i >= 2 && i - 2 < b.m) {
+      const double low2 = __ldg(b.low2 + i - 2);
+      v = (i < b.m) ? fma(pv(i - 2), low2, v) : pv(i - 2) * low2;
+    }
     return v;
   };
   if (part == 0) {
     double* gp = static_cast<double*>(c.s[0]) + j;
     double* fv = static_cast<double*>(c.s[2]) + j;
-#pragma unroll 4
-    for (int i = q; i < nx; i += 2) gp[(long long)i * myc] = gp_at(i);
+    map_par(nx, q, gp_at, [&](int i, double v) { gp[(long long)i * myc] = v; });
     from_ortho_par<double>(c.xu, gp, myc, fv, myc, q);
   } else {
     const double inv_asp = 1.0 / c.aspect;
@@ -528,31 +557,21 @@ __global__ void __launch_bounds__(256) k_lp_box_y3(const CaseDev* __restrict__ c
   const int i = lane, ny = c.ny, myc = c.myc, f = sub;
   double* F = static_cast<double*>(c.s[4 + f]) + (size_t)i * myc;
   const FdmaRow R = fdma_row(f < 2 ? c.hu_y : c.ht_y, 0);
-  {
-    double xm2 = 0.0;
-#pragma unroll 4
-    for (int k = q; k < R.m; k += 2) {
-      double v = F[k];
-      if (k >= 2) v = fma(xm2, R.low[k - 2], v);
-      F[k] = v;
-      xm2 = v;
-    }
-  }
+  fdma_fwd_par<double, kPBY3F>(R, F, 1, q);
   fdma_bwd_par<double, kPBY3>(R, F, 1, q);
   bool bad = false;
   if (f == 2) {
     double* tt = static_cast<double*>(c.temp) + (size_t)i * myc;
-    for (int k = q; k < myc; k += 2) {
-      tt[k] = F[k];
-      bad |= !finite_v(F[k]);
-    }
+    map_par<kPBY3F>(myc, q, [&](int k) { return F[k]; }, [&](int k, double v) {
+      tt[k] = v;
+      bad |= !finite_v(v);
+    });
   } else {
     for (int k = q; k < myc; k += 2) bad |= !finite_v(F[k]);
   }
   if (f == 0) {
     double* A = static_cast<double*>(c.s[1]) + (size_t)i * ny;
-#pragma unroll 4
-    for (int k = q; k < ny; k += 2) A[k] = stencil_lane<double>(c.ycd, F, 1, k);
+    map_par<kPBY3F>(ny, q, [&](int k) { return stencil_lane<double>(c.ycd, F, 1, k); }, [&](int k, double v) { A[k] = v; });
   } else if (f == 1) {
     double* B = static_cast<double*>(c.s[2]) + (size_t)i * ny;
     diff_par<double, kPBY3>(ny, 1 - q, [&](int k) { return stencil_lane<double>(c.ycd, F, 1, k); },
@@ -574,16 +593,7 @@ __global__ void __launch_bounds__(256) k_lp_box_y4(const CaseDev* __restrict__ c
   // back substitution (FP64 in place), each result also rounded into m_z:
   // the FP32 input of the eigenbasis GEMM
   float* wf = static_cast<float*>(c.m_z) + (size_t)i * myc;
-  double p2 = 0.0, p4 = 0.0;
-#pragma unroll 4
-  for (int j = top_par(R.m, q); j >= 0; j -= 2) {
-    double v = wv[j] * R.dinv[j];
-    if (j + 2 < R.m) v = fma(p2, R.up1[j], v);
-    if (j + 4 < R.m) v = fma(p4, R.up2[j], v);
-    wf[j] = to_f32(v);
-    p4 = p2;
-    p2 = v;
-  }
+  fdma_bwd_par<double, kPBY4>(R, wv, 1, q, [&](int j, double v) { wf[j] = to_f32(v); });
 }
 
 // rows i < nx: ux = ux* - Sy+ Sy^N E ; uy = uy* - Sy+ Dy Sy^N Fv ;
@@ -597,19 +607,16 @@ __global__ void __launch_bounds__(256) k_lp_box_y5(const CaseDev* __restrict__ c
     const double* Gp = static_cast<const double*>(c.s[0]) + (size_t)i * myc;
     double* p0 = static_cast<double*>(c.p0) + (size_t)i * ny;
     const double* dv = static_cast<const double*>(c.s[3]) + (size_t)i * ny;
-#pragma unroll 4
-    for (int k = q; k < ny; k += 2) {
-      const double v = fnms(p0[k], dv[k], c.nu);
-      p0[k] = fmas(v, stencil_lane<double>(c.ycn, Gp, 1, k), c.inv_dt);
-    }
+    map_par<kPBY5M>(ny, q, [&](int k) {
+      return fmas(fnms(p0[k], dv[k], c.nu), stencil_lane<double>(c.ycn, Gp, 1, k), c.inv_dt);
+    }, [&](int k, double v) { p0[k] = v; });
     return;
   }
   if (i >= mxc) return;
   double* d = static_cast<double*>(c.s[6 + part]) + (size_t)i * ny;
   if (part == 0) {  // Sy^N E on parity q
     const double* E = static_cast<const double*>(c.s[1]) + (size_t)i * myc;
-#pragma unroll 4
-    for (int k = q; k < ny; k += 2) d[k] = stencil_lane<double>(c.ycn, E, 1, k);
+    map_par<kPBY5M>(ny, q, [&](int k) { return stencil_lane<double>(c.ycn, E, 1, k); }, [&](int k, double v) { d[k] = v; });
   } else {  // Dy Sy^N Fv on parity q (from Sy^N Fv on parity 1 - q)
     const double* Fv = static_cast<const double*>(c.s[2]) + (size_t)i * myc;
     diff_par<double, kPBY5>(ny, q, [&](int k) { return stencil_lane<double>(c.ycn, Fv, 1, k); },
@@ -619,11 +626,10 @@ __global__ void __launch_bounds__(256) k_lp_box_y5(const CaseDev* __restrict__ c
   double* u = static_cast<double*>(part == 0 ? c.ux : c.uy) + (size_t)i * myc;
   const double* us = static_cast<const double*>(c.s[4 + part]) + (size_t)i * myc;
   bool bad = false;
-  for (int k = q; k < myc; k += 2) {
-    const double a = us[k] - d[k];
+  map_par<kPBY5M>(myc, q, [&](int k) { return us[k] - d[k]; }, [&](int k, double a) {
     u[k] = a;
     bad |= !finite_v(a);
-  }
+  });
   if (bad) atomicOr(c.status, 1u);
 }
 
@@ -743,59 +749,99 @@ __global__ void __launch_bounds__(128) k_lp_per_y2(const CaseDev* __restrict__ c
 }
 
 // ============================================================================
-// Periodic Y2 as three launches of one thread per sub-lane (rows i < mx,
-// complex).  Y2A writes the Helmholtz solutions to scratch (yw[3..5]) because
-// the uy right-hand side reads the old temperature; Y2C moves them into the
-// state.  Same operations as k_lp_per_y2 (navier.rs:622-721).
+// Periodic Y2 as three launches of one thread per sub-lane (rows i < mx).  The
+// real and imaginary parts of a row are sub-lanes of their own: every operator
+// is real, and the factor ik of the x derivative only hands one part's value
+// to the other's chain.  Y2A writes the Helmholtz solutions to scratch
+// (yw[3..5]) because the uy right-hand side reads the old temperature; Y2C
+// moves them into the state.  Same operations as k_lp_per_y2 (navier.rs:622-721).
+// The four threads of a row (part, parity) are neighbours in a warp: elements k
+// and k + 1 of a row are one sector.
 // ============================================================================
-// Y2A, field f, parity q: right-hand side, pinv rows and the row's banded
+// threads (row, parity, part): part h = 0 real, 1 imaginary
+#define ROW_PROLOGUE_CPLX                                                    \
+  const int4 w = work[blockIdx.x];                                           \
+  if ((int)(threadIdx.x >> 2) >= w.z) return;                                \
+  const CaseDev& c = cases[w.x];                                             \
+  if (c.gate != nullptr && c.gate[1] == 0) return;                           \
+  const int lane = w.y + (int)(threadIdx.x >> 2);                            \
+  const int q = (int)(threadIdx.x >> 1) & 1, h = (int)threadIdx.x & 1;       \
+  const int sub = (int)blockIdx.y;                                           \
+  (void)sub;
+
+// part h of row i of a complex array with rows of ld elements (stride 2)
+__device__ __forceinline__ const double* part_row(const void* a, size_t i, int ld, int h) {
+  return static_cast<const double*>(a) + 2 * i * ld + h;
+}
+__device__ __forceinline__ double* part_row(void* a, size_t i, int ld, int h) {
+  return static_cast<double*>(a) + 2 * i * ld + h;
+}
+
+// the pinv factors of row k, loaded with a batch's elements: behind the stores
+// of the elements before it, each would wait out its own latency
+struct PinvCoef {
+  double dia, up1, up2;
+};
+__device__ __forceinline__ PinvCoef pinv_coef(const PinvDev& p, int k, int m) {
+  PinvCoef r{0.0, 0.0, 0.0};
+  if (k >= 0 && k < m) r.dia = __ldg(p.dia + k);
+  if (k >= 0 && k < m - 2) r.up1 = __ldg(p.up1 + k);
+  if (k >= 0 && k < m - 4) r.up2 = __ldg(p.up2 + k);
+  return r;
+}
+
+// Y2A, field f, parity q, part h: right-hand side, pinv rows and the row's banded
 // Helmholtz solve of one field on the columns of parity q
 template <int PB = kPBC>
-__device__ __forceinline__ void per_y2a_row(const CaseDev& c, const int i, const int q, const int f) {
+__device__ __forceinline__ void per_y2a_row(const CaseDev& c, const int i, const int q, const int h, const int f) {
   const int ny = c.ny, myc = c.myc, kx = c.kx, ky = c.ky;
   const double dt = c.dt, inv_asp = 1.0 / c.aspect, kis = (double)i * inv_asp;  // ik/s
   const void* st3[3] = {c.ux, c.uy, c.temp};
-  const double2* Fo = static_cast<const double2*>(st3[f]) + (size_t)i * myc;
-  const double2* To = static_cast<const double2*>(c.temp) + (size_t)i * myc;
-  const double2* Uo = static_cast<const double2*>(c.uy) + (size_t)i * myc;
-  const double2* P = static_cast<const double2*>(c.p0) + (size_t)i * ny;
-  const double2* cv = static_cast<const double2*>(c.m_cv);
-  const double2* bco = static_cast<const double2*>(c.bc_ortho) + (size_t)i * ny;
-  const double2* bcd = static_cast<const double2*>(c.bc_diff) + (size_t)i * ny;
-  double2* out = static_cast<double2*>(c.yw[3 + f]) + (size_t)i * ny;
+  const double* Fo = part_row(st3[f], i, myc, h);
+  const double* To = part_row(static_cast<const void*>(c.temp), i, myc, h);
+  const double* Uo = part_row(static_cast<const void*>(c.uy), i, myc, h);
+  // f = 0 takes ik/s p0: the other part of p0
+  const double* P = part_row(static_cast<const void*>(c.p0), i, ny, f == 0 ? 1 - h : h);
+  const double* cv = static_cast<const double*>(c.m_cv) + h;
+  const double* bco = part_row(static_cast<const void*>(c.bc_ortho), i, ny, h);
+  const double* bcd = part_row(static_cast<const void*>(c.bc_diff), i, ny, h);
+  double* out = part_row(c.yw[3 + f], i, ny, h);
+  const bool bclin = c.m_bclin && !(i == 0 && h == 1);  // (add_bclin: row 0 takes the real part only)
   const PinvDev& pv = c.pinv_y;
-  double2 r2 = c2(0.0, 0.0), r4 = c2(0.0, 0.0), g2 = c2(0.0, 0.0);
+  double r2 = 0.0, r4 = 0.0, g2 = 0.0;
   for (int k0 = top_par(ny, q); k0 >= 0; k0 -= 2 * PB) {
     // the batch's loads first (stencil, convection, pressure, boundary terms)
-    double2 ov[PB], cvv[PB], pk[PB], xv[PB];
+    double ov[PB], cvv[PB], pk[PB], xv[PB];
+    PinvCoef pc[PB];
 #pragma unroll
     for (int e = 0; e < PB; e++) {
       const int k = k0 - 2 * e;
-      ov[e] = cvv[e] = pk[e] = xv[e] = c2(0.0, 0.0);
+      ov[e] = cvv[e] = pk[e] = xv[e] = 0.0;
+      pc[e] = pinv_coef(pv, k, myc);
       if (k < 0) continue;
-      ov[e] = stencil_lane<double2>(c.ycd, Fo, 1, k);
-      if (i < kx && k < ky) cvv[e] = cv[((size_t)f * kx + i) * ky + k];
-      if (f == 0) pk[e] = P[k];
+      ov[e] = stencil_lane<double>(c.ycd, Fo, 2, k);
+      if (i < kx && k < ky) cvv[e] = cv[2 * (((size_t)f * kx + i) * ky + k)];
+      if (f == 0) pk[e] = P[2 * k];
       else if (f == 1) {
-        if (k < ny - 1) pk[e] = P[k + 1];
-        xv[e] = stencil_lane<double2>(c.ycd, To, 1, k) + bco[k];
+        if (k < ny - 1) pk[e] = P[2 * (k + 1)];
+        xv[e] = stencil_lane<double>(c.ycd, To, 2, k) + bco[2 * k];
       } else {
-        xv[e] = bcd[k];
-        if (c.m_bclin && i < kx && k < ky) cvv[e] = add_bclin(cvv[e], stencil_lane<double2>(c.ycd, Uo, 1, k), c.m_bcg, i);
+        xv[e] = bcd[2 * k];
+        if (bclin && i < kx && k < ky) cvv[e] = fma(stencil_lane<double>(c.ycd, Uo, 2, k), c.m_bcg, cvv[e]);
       }
     }
 #pragma unroll
     for (int e = 0; e < PB; e++) {
       const int k = k0 - 2 * e;
       if (k < 0) break;
-      const double2 o = ov[e], cvk = cvv[e];
-      double2 r;
+      const double o = ov[e], cvk = cvv[e];
+      double r;
       if (f == 0) {
-        const double2 gx = mul_ik(pk[e], kis);
+        const double gx = (h == 0 ? -pk[e] : pk[e]) * kis;
         r = fnms(fnms(o, gx, dt), cvk, dt);
       } else if (f == 1) {  // dP/dy at k (descending derivative recurrence), buoyancy
-        double2 g;
-        if (k == ny - 1) g = c2(0.0, 0.0);
+        double g;
+        if (k == ny - 1) g = 0.0;
         else if (k >= 1) g = fmas(g2, pk[e], exact_double(2 * k + 2));
         else g = fmas(pk[e], g2, 0.5);
         g2 = g;
@@ -804,145 +850,152 @@ __device__ __forceinline__ void per_y2a_row(const CaseDev& c, const int i, const
         r = fnms(o + xv[e], cvk, dt);
       }
       if (k < myc) {
-        double2 v = scal(r, pv.dia[k]);
-        if (k < myc - 2) v = fmas(v, r2, pv.up1[k]);
-        if (k < myc - 4) v = fmas(v, r4, pv.up2[k]);
-        out[k] = v;
+        double v = r * pc[e].dia;
+        if (k < myc - 2) v = fmas(v, r2, pc[e].up1);
+        if (k < myc - 4) v = fmas(v, r4, pc[e].up2);
+        out[2 * k] = v;
       }
       r4 = r2;
       r2 = r;
     }
   }
   const FdmaRow R = fdma_row(f < 2 ? c.hu_y : c.ht_y, i);
-  fdma_fwd_par<double2, PB>(R, out, 1, q);
-  fdma_bwd_par<double2, PB>(R, out, 1, q);
+  fdma_fwd_par<double, PB>(R, out, 2, q);
+  fdma_bwd_par<double, PB>(R, out, 2, q);
 }
-__global__ void __launch_bounds__(256) k_lp_per_y2a(const CaseDev* __restrict__ cases, const int4* __restrict__ work) {
+__global__ void __launch_bounds__(2 * kLaneBlock) k_lp_per_y2a(const CaseDev* __restrict__ cases,
+                                                               const int4* __restrict__ work) {
   pdl_enter();
-  ROW_PROLOGUE
-  per_y2a_row(c, lane, q, sub);
+  ROW_PROLOGUE_CPLX
+  per_y2a_row(c, lane, q, h, sub);
 }
 
-// Y2B, parity q: divergence ik/s Sy ux* + Dy Sy uy* on parity q (from uy* on
-// parity 1 - q), pinv rows and the Poisson row solve -> p1 (p1[0,0] = 0)
+// Y2B, parity q, part h: divergence ik/s Sy ux* + Dy Sy uy* on parity q (from
+// uy* on parity 1 - q and the other part of ux*), pinv rows and the Poisson row
+// solve -> p1 (p1[0,0] = 0)
 template <int PB = kPBCB>
-__device__ __forceinline__ void per_y2b_row(const CaseDev& c, const int i, const int q) {
+__device__ __forceinline__ void per_y2b_row(const CaseDev& c, const int i, const int q, const int h) {
   const int ny = c.ny, myc = c.myc;
   const double inv_asp = 1.0 / c.aspect, kis = (double)i * inv_asp;  // ik/s
-  const double2* U = static_cast<const double2*>(c.yw[3]) + (size_t)i * ny;
-  const double2* V = static_cast<const double2*>(c.yw[4]) + (size_t)i * ny;
-  double2* dvr = static_cast<double2*>(c.yw[0]) + (size_t)i * ny;
-  double2* p1 = static_cast<double2*>(c.p1) + (size_t)i * myc;
+  const double* U = part_row(static_cast<const void*>(c.yw[3]), i, ny, 1 - h);
+  const double* V = part_row(static_cast<const void*>(c.yw[4]), i, ny, h);
+  double* dvr = part_row(c.yw[0], i, ny, h);
+  double* p1 = part_row(c.p1, i, myc, h);
   const PinvDev& pv = c.pinv_y;
-  double2 g2 = c2(0.0, 0.0), w2 = c2(0.0, 0.0), w4 = c2(0.0, 0.0);
+  double g2 = 0.0, w2 = 0.0, w4 = 0.0;
   for (int k0 = top_par(ny, q); k0 >= 0; k0 -= 2 * PB) {
-    double2 ov[PB], vv[PB];  // Sy ux* at k, Sy uy* at k + 1
+    double ov[PB], vv[PB];  // Sy ux* at k (the other part), Sy uy* at k + 1
+    PinvCoef pc[PB];
 #pragma unroll
     for (int e = 0; e < PB; e++) {
       const int k = k0 - 2 * e;
-      ov[e] = vv[e] = c2(0.0, 0.0);
+      ov[e] = vv[e] = 0.0;
+      pc[e] = pinv_coef(pv, k, myc);
       if (k < 0) continue;
-      ov[e] = stencil_lane<double2>(c.ycd, U, 1, k);
-      if (k < ny - 1) vv[e] = stencil_lane<double2>(c.ycd, V, 1, k + 1);
+      ov[e] = stencil_lane<double>(c.ycd, U, 2, k);
+      if (k < ny - 1) vv[e] = stencil_lane<double>(c.ycd, V, 2, k + 1);
     }
 #pragma unroll
     for (int e = 0; e < PB; e++) {
       const int k = k0 - 2 * e;
       if (k < 0) break;
-      double2 g;
-      if (k == ny - 1) g = c2(0.0, 0.0);
+      double g;
+      if (k == ny - 1) g = 0.0;
       else if (k >= 1) g = fmas(g2, vv[e], exact_double(2 * k + 2));
       else g = fmas(vv[e], g2, 0.5);
       g2 = g;
-      const double2 d = c2(fma(-ov[e].y, kis, g.x), fma(ov[e].x, kis, g.y));  // ik/s Sy ux* + g
-      dvr[k] = d;
+      const double d = fma(h == 0 ? -ov[e] : ov[e], kis, g);  // ik/s Sy ux* + g
+      dvr[2 * k] = d;
       if (k < myc) {
-        double2 v = scal(d, pv.dia[k]);
-        if (k < myc - 2) v = fmas(v, w2, pv.up1[k]);
-        if (k < myc - 4) v = fmas(v, w4, pv.up2[k]);
-        p1[k] = v;
+        double v = d * pc[e].dia;
+        if (k < myc - 2) v = fmas(v, w2, pc[e].up1);
+        if (k < myc - 4) v = fmas(v, w4, pc[e].up2);
+        p1[2 * k] = v;
       }
       w4 = w2;
       w2 = d;
     }
   }
   const FdmaRow R = fdma_row(c.pois_y, i);
-  fdma_fwd_par<double2, PB>(R, p1, 1, q);
-  fdma_bwd_par<double2, PB>(R, p1, 1, q);
-  if (i == 0 && q == 0) p1[0] = c2(0.0, 0.0);
+  fdma_fwd_par<double, PB>(R, p1, 2, q);
+  fdma_bwd_par<double, PB>(R, p1, 2, q);
+  if (i == 0 && q == 0) p1[0] = 0.0;
 }
-__global__ void __launch_bounds__(256) k_lp_per_y2b(const CaseDev* __restrict__ cases, const int4* __restrict__ work) {
+__global__ void __launch_bounds__(2 * kLaneBlock) k_lp_per_y2b(const CaseDev* __restrict__ cases,
+                                                               const int4* __restrict__ work) {
   pdl_enter();
-  ROW_PROLOGUE
-  per_y2b_row(c, lane, q);
+  ROW_PROLOGUE_CPLX
+  per_y2b_row(c, lane, q, h);
 }
 
-// Y2C, parity q and part: part 0: O1 = Sy^N p1, dp/dx, pres[0] and ux,
-// temperature on parity q; part 1: dp/dy on parity 1 - q and uy there
+// Y2C, parity q, part h of p1.  pass 0: O1 = Sy^N p1 and pres[0] in part h, dp/dx
+// = ik/s O1 and ux in the other part, the temperature, on parity q; pass 1:
+// dp/dy on parity 1 - q and uy there, in part h
 template <int PB = kPBCC>
-__device__ __forceinline__ void per_y2c_row(const CaseDev& c, const int i, const int q, const int part) {
+__device__ __forceinline__ void per_y2c_row(const CaseDev& c, const int i, const int q, const int h, const int pass) {
   const int ny = c.ny, myc = c.myc;
   const double inv_asp = 1.0 / c.aspect, kis = (double)i * inv_asp;  // ik/s
-  const double2* p1 = static_cast<const double2*>(c.p1) + (size_t)i * myc;
+  const double* p1 = part_row(static_cast<const void*>(c.p1), i, myc, h);
   bool bad = false;
-  if (part == 0) {
-    double2* dpx = static_cast<double2*>(c.yw[1]) + (size_t)i * ny;
-    double2* P = static_cast<double2*>(c.p0) + (size_t)i * ny;
-    const double2* dvr = static_cast<const double2*>(c.yw[0]) + (size_t)i * ny;
+  if (pass == 0) {
+    double* dpx = part_row(c.yw[1], i, ny, 1 - h);
+    double* P = part_row(c.p0, i, ny, h);
+    const double* dvr = part_row(static_cast<const void*>(c.yw[0]), i, ny, h);
     for (int k0 = q; k0 < ny; k0 += 2 * PB) {
-      double2 ov[PB], pv0[PB], dv[PB];
+      double ov[PB], pv0[PB], dv[PB];
 #pragma unroll
       for (int e = 0; e < PB; e++) {
         const int k = k0 + 2 * e;
-        ov[e] = pv0[e] = dv[e] = c2(0.0, 0.0);
+        ov[e] = pv0[e] = dv[e] = 0.0;
         if (k >= ny) continue;
-        ov[e] = stencil_lane<double2>(c.ycn, p1, 1, k);
-        pv0[e] = P[k];
-        dv[e] = dvr[k];
+        ov[e] = stencil_lane<double>(c.ycn, p1, 2, k);
+        pv0[e] = P[2 * k];
+        dv[e] = dvr[2 * k];
       }
 #pragma unroll
       for (int e = 0; e < PB; e++) {
         const int k = k0 + 2 * e;
         if (k >= ny) break;
-        dpx[k] = mul_ik(ov[e], kis);
-        const double2 v = fnms(pv0[e], dv[e], c.nu);
-        P[k] = fmas(v, ov[e], c.inv_dt);
+        dpx[2 * k] = (h == 0 ? ov[e] : -ov[e]) * kis;
+        const double v = fnms(pv0[e], dv[e], c.nu);
+        P[2 * k] = fmas(v, ov[e], c.inv_dt);
       }
     }
-    from_ortho_par<double2, PB>(c.ycd, dpx, 1, dpx, 1, q);
-    const double2* U = static_cast<const double2*>(c.yw[3]) + (size_t)i * ny;
-    const double2* T = static_cast<const double2*>(c.yw[5]) + (size_t)i * ny;
-    double2* ux = static_cast<double2*>(c.ux) + (size_t)i * myc;
-    double2* tt = static_cast<double2*>(c.temp) + (size_t)i * myc;
-    for (int k = q; k < myc; k += 2) {
-      const double2 a = U[k] - dpx[k];
-      const double2 t = T[k];
-      ux[k] = a;
-      tt[k] = t;
-      bad |= !(finite_v(a) && finite_v(t));
-    }
+    from_ortho_par<double, PB>(c.ycd, dpx, 2, dpx, 2, q);
+    const double* U = part_row(static_cast<const void*>(c.yw[3]), i, ny, 1 - h);
+    const double* T = part_row(static_cast<const void*>(c.yw[5]), i, ny, 1 - h);
+    double* ux = part_row(c.ux, i, myc, 1 - h);
+    double* tt = part_row(c.temp, i, myc, 1 - h);
+    map_par<PB>(myc, q, [&](int k) { return U[2 * k] - dpx[2 * k]; }, [&](int k, double a) {
+      ux[2 * k] = a;
+      bad |= !finite_v(a);
+    });
+    map_par<PB>(myc, q, [&](int k) { return T[2 * k]; }, [&](int k, double t) {
+      tt[2 * k] = t;
+      bad |= !finite_v(t);
+    });
   } else {
-    double2* dpy = static_cast<double2*>(c.yw[2]) + (size_t)i * ny;
-    diff_par<double2, PB>(ny, 1 - q, [&](int k) { return stencil_lane<double2>(c.ycn, p1, 1, k); },
-                      [&](int k, double2 d) { dpy[k] = d; });
-    from_ortho_par<double2, PB>(c.ycd, dpy, 1, dpy, 1, 1 - q);
-    const double2* V = static_cast<const double2*>(c.yw[4]) + (size_t)i * ny;
-    double2* uy = static_cast<double2*>(c.uy) + (size_t)i * myc;
-    for (int k = 1 - q; k < myc; k += 2) {
-      const double2 b = V[k] - dpy[k];
-      uy[k] = b;
+    double* dpy = part_row(c.yw[2], i, ny, h);
+    diff_par<double, PB>(ny, 1 - q, [&](int k) { return stencil_lane<double>(c.ycn, p1, 2, k); },
+                         [&](int k, double d) { dpy[2 * k] = d; });
+    from_ortho_par<double, PB>(c.ycd, dpy, 2, dpy, 2, 1 - q);
+    const double* V = part_row(static_cast<const void*>(c.yw[4]), i, ny, h);
+    double* uy = part_row(c.uy, i, myc, h);
+    map_par<PB>(myc, 1 - q, [&](int k) { return V[2 * k] - dpy[2 * k]; }, [&](int k, double b) {
+      uy[2 * k] = b;
       bad |= !finite_v(b);
-    }
+    });
   }
   if (bad) atomicOr(c.status, 1u);
 }
-__global__ void __launch_bounds__(256) k_lp_per_y2c(const CaseDev* __restrict__ cases, const int4* __restrict__ work) {
+__global__ void __launch_bounds__(2 * kLaneBlock) k_lp_per_y2c(const CaseDev* __restrict__ cases,
+                                                               const int4* __restrict__ work) {
   pdl_enter();
-  ROW_PROLOGUE
-  per_y2c_row(c, lane, q, sub);
+  ROW_PROLOGUE_CPLX
+  per_y2c_row(c, lane, q, h, sub);
 }
 
-// The three phases in one launch: a CTA of three 64-thread groups per work
+// The three phases in one launch: a CTA of three 128-thread groups per work
 // item of up to 32 rows runs Y2A (group = field), then Y2B (group 0), then
 // Y2C (groups 0 and 1 = part), with a CTA barrier between the phases.  Every
 // array a phase reads is a row of this item's, written by the CTA's own
@@ -950,23 +1003,22 @@ __global__ void __launch_bounds__(256) k_lp_per_y2c(const CaseDev* __restrict__ 
 // thread does the arithmetic of the three launches (the elements loaded ahead
 // change only the order of the loads), so the results are the same.  The
 // rows' intermediates are re-read while they are still in L1/L2, and two
-// launch tails go.  Four elements ahead in every phase (128 registers) was
-// the fastest of (2..4, 2..6, 2..8) on the 256-case ensemble: 1.07 ms against
-// 1.13 ms for the three launches.
-__global__ void __launch_bounds__(3 * kLaneBlock) k_lp_per_y2f(const CaseDev* __restrict__ cases,
+// launch tails go.  Whole step, three launches | this: 20 periodic cases 0.75 |
+// 0.70 ms, 67 cases 1.05 | 0.93, 129 cases 1.37 | 1.56.
+__global__ void __launch_bounds__(6 * kLaneBlock) k_lp_per_y2f(const CaseDev* __restrict__ cases,
                                                                const int4* __restrict__ work) {
   pdl_enter();
   const int4 w = work[blockIdx.x];
   const CaseDev& c = cases[w.x];
   if (c.gate != nullptr && c.gate[1] == 0) return;  // the whole CTA: no barrier is left waiting
-  const int t = (int)(threadIdx.x % kLaneBlock), grp = (int)(threadIdx.x / kLaneBlock);
-  const bool active = (t >> 1) < w.z;
-  const int lane = w.y + (t >> 1), q = t & 1;
-  if (active) per_y2a_row<4>(c, lane, q, grp);
+  const int t = (int)(threadIdx.x % (2 * kLaneBlock)), grp = (int)(threadIdx.x / (2 * kLaneBlock));
+  const bool active = (t >> 2) < w.z;
+  const int lane = w.y + (t >> 2), q = (t >> 1) & 1, h = t & 1;
+  if (active) per_y2a_row<4>(c, lane, q, h, grp);
   __syncthreads();
-  if (active && grp == 0) per_y2b_row<4>(c, lane, q);
+  if (active && grp == 0) per_y2b_row<4>(c, lane, q, h);
   __syncthreads();
-  if (active && grp < 2) per_y2c_row<4>(c, lane, q, grp);
+  if (active && grp < 2) per_y2c_row<4>(c, lane, q, h, grp);
 }
 
 #undef LANE_PROLOGUE
@@ -995,7 +1047,9 @@ bool lane_kernel_rows(int kernel) {
 }
 
 cudaError_t launch_lane_kernel(int kernel, int nblocks, cudaStream_t s, const CaseDev* cases, const int4* work) {
-  dim3 g(nblocks, lane_kernel_subs(kernel)), b(kernel == K_LP_PER_Y2F ? 3 * kLaneBlock : kLaneBlock);
+  dim3 g(nblocks, lane_kernel_subs(kernel)), b(kLaneBlock);
+  if (kernel == K_LP_PER_Y2F) b.x = 6 * kLaneBlock;
+  else if (kernel == K_LP_PER_Y2A || kernel == K_LP_PER_Y2B || kernel == K_LP_PER_Y2C) b.x = 2 * kLaneBlock;
   switch (kernel) {
     case K_LP_BOX_GPX: return launch_pdl(dev::k_lp_box_gpx, g, b, 0, s, cases, work);
     case K_LP_BOX_X2: return launch_pdl(dev::k_lp_box_x2, g, b, 0, s, cases, work);
