@@ -231,9 +231,12 @@ __device__ FdmaDev stage_fdma_row(const FdmaDev& f, int row, double* dst, int ti
 //   CONV_MIXED  m_cv, transformed (the mixed form's GEMM), without the linear
 //               boundary part (CaseDev::m_bclin)
 //   CONV_FULL   m_cv, transformed and complete (the split GEMMs)
+// Registers: CONV_Q is held to 64 (four CTAs per SM): at 80 the 457 to 608 rows of
+// a small batch took a second wave (8 cases of 128 x 65: 76 us against 54).  The
+// other two serve larger rows, where the spills cost more (512 x 257: 2 us).
 enum { CONV_Q = 0, CONV_MIXED = 1, CONV_FULL = 2 };
 template <int CONV>
-__global__ void __launch_bounds__(256) k_per_y2(const CaseDev* __restrict__ cases, const int4* __restrict__ work) {
+__global__ void __launch_bounds__(256, CONV == CONV_Q ? 4 : 1) k_per_y2(const CaseDev* __restrict__ cases, const int4* __restrict__ work) {
   pdl_enter();
   int4 w = work[blockIdx.x];
   const CaseDev& c = cases[w.x];
@@ -751,7 +754,9 @@ size_t smem_box_y2(const CaseDev& c) {
 size_t smem_box_y2_pre(const CaseDev& c) { return 17 * (size_t)(c.ny + 1) * 8 + 64; }
 
 // X2: columns j < myc.  pinv_x then the ADI x solve.  s[1..3] -> s[4..6] (mxc x myc)
-__global__ void __launch_bounds__(256) k_box_x2(const CaseDev* __restrict__ cases, const int4* __restrict__ work) {
+// (four CTAs per SM here and in k_box_y3: with 80 registers three fitted; box
+// 513 x 513 step 502 -> 475 us, 8 cases of 65 x 65 149 -> 139)
+__global__ void __launch_bounds__(256, 4) k_box_x2(const CaseDev* __restrict__ cases, const int4* __restrict__ work) {
   pdl_enter();
   int4 w = work[blockIdx.x];
   const CaseDev& c = cases[w.x];
@@ -785,7 +790,7 @@ __global__ void __launch_bounds__(256) k_box_x2(const CaseDev* __restrict__ case
 size_t smem_box_x2(const CaseDev& c) { return (stage_factors(c.mxc) ? 14 : 6) * (size_t)(c.nx + 1) * 8 + 64; }
 
 // Y3: rows i < mxc.  ADI y solve -> ux*, uy*, temp(new); A = Sy ux*, B = Dy Sy uy*
-__global__ void __launch_bounds__(256) k_box_y3(const CaseDev* __restrict__ cases, const int4* __restrict__ work) {
+__global__ void __launch_bounds__(256, 4) k_box_y3(const CaseDev* __restrict__ cases, const int4* __restrict__ work) {
   pdl_enter();
   int4 w = work[blockIdx.x];
   const CaseDev& c = cases[w.x];
