@@ -343,6 +343,18 @@ constexpr int kSplitLanesCap = 4096;
 // on; below, the packing launch costs what it saves.
 constexpr int kPackLanesMinN = 96, kPackLanesMin = 1024;
 
+// The handle's scratch; without the memory for it the calls take the forms that
+// need none.
+static bool lane_scratch(FsLanes* p, size_t bytes) {
+  if (cudaMalloc(&p->work_mem, bytes) != cudaSuccess) {
+    (void)cudaGetLastError();
+    p->work_mem = nullptr;
+    return false;
+  }
+  cuda_check(cudaEventCreateWithFlags(&p->done, cudaEventDisableTiming), "event");
+  return true;
+}
+
 struct SvSolver {
   FsSpace* space = nullptr;
   Arena arena;
@@ -2329,20 +2341,17 @@ int fs_lanes_create(int base, int n, int precision, FsLanes** out) {
   if (precision == RBC_PREC_FP64 && lanes_attach_split(p->L)) {
     const size_t db = (split_dig_bytes(kSplitLanesCap, split_chunks((n + 1) / 2), split_chunks(n / 2)) + 255) & ~size_t(255);
     const size_t be = (size_t)kSplitLanesCap * 4, bb = (size_t)kSplitLanesCap * n * 8;
-    cuda_check(cudaMalloc(&p->work_mem, db + be + bb), "cudaMalloc lane scratch");
-    char* q = static_cast<char*>(p->work_mem);
-    p->work.dig = reinterpret_cast<unsigned char*>(q);
-    p->work.ex = reinterpret_cast<int*>(q + db);
-    p->work.buf = reinterpret_cast<double*>(q + db + be);
-    p->work.lanes = kSplitLanesCap;
-    p->work.status = p->d_status;
-    cuda_check(cudaEventCreateWithFlags(&p->done, cudaEventDisableTiming), "event");
+    if (lane_scratch(p.get(), db + be + bb)) {
+      char* q = static_cast<char*>(p->work_mem);
+      p->work.dig = reinterpret_cast<unsigned char*>(q);
+      p->work.ex = reinterpret_cast<int*>(q + db);
+      p->work.buf = reinterpret_cast<double*>(q + db + be);
+      p->work.lanes = kSplitLanesCap;
+      p->work.status = p->d_status;
+    }
   }
   if (precision == RBC_PREC_MIXED) {
-    if (n >= kPackLanesMinN) {
-      cuda_check(cudaMalloc(&p->work_mem, packed_lanes_bytes(kSplitLanesCap, n)), "cudaMalloc lane scratch");
-      cuda_check(cudaEventCreateWithFlags(&p->done, cudaEventDisableTiming), "event");
-    }
+    if (n >= kPackLanesMinN) lane_scratch(p.get(), packed_lanes_bytes(kSplitLanesCap, n));
     const HostBasis& hb = p->L.hb;
     LMat S = lm_stencil(hb), P = lm_from_ortho(hb);
     p->w[FS_OP_FORWARD] = upload_split(p->arena, lm_mul(P, lm_cheb_forward(n)));
@@ -2788,7 +2797,7 @@ struct RbcServer {
 // case is built; the actual arena size replaces it afterwards).
 static size_t case_bytes_bound(const RbcParams& p) {
   const size_t n = (size_t)(p.nx + 2) * (size_t)(p.ny + 2);
-  size_t b = n * 8 * 208;                       // fields, scratch and tables
+  size_t b = n * 8 * 160;                       // fields, scratch and tables
   if (p.kind != RBC_PERIODIC) b += (size_t)p.nx * p.nx * 8 * 16;  // eigenbases and dense x operators
   if (p.precision == RBC_PREC_MIXED) b += ((size_t)p.nx * p.nx + (size_t)p.ny * p.ny) * 4 * 24;
   return b + (4u << 20);
