@@ -371,16 +371,21 @@ SplitMatDev shared_split_mat(int kind, int n, bool poisson, bool fwd) {
 //                   128^2 187 | 172; periodic 96x80 92 | 92, 128^2 117 | 111, 64x256 261 | 139
 //   FFT (2^p + 1)   box 129^2 171 | 174, 257^2 371 | 301; periodic 128x65 82 | 92,
 //                   256x129 115 | 120, 512x257 250 | 195
+//   Fourier length with a prime factor above 8 (a direct sum in the passes):
+//                   22x17 144 | 72, 26x33 178 | 74, 66x48 154 | 82, 110x33 162 | 80,
+//                   47x33 1648 | 76, 106x33 2088 | 80
 // so the lines lie at 9000 grid points where an axis has no fast butterfly in
-// the passes (a Fourier length with a prime factor above 8 counts as dense),
-// and at 48000 where every axis has one.  A list holds at most 320 terms
+// the passes, at 48000 where every axis has one, and nowhere for a Fourier
+// length with a prime factor above 8.  A list holds at most 320 terms
 // (split_gemm.cu), hence lengths up to 640.
 bool split_step_size(const CaseDev& c) {
   if (c.nx < 16 || c.ny < 16 || c.nx > 640 || c.ny > 640) return false;
   bool fast = c.cy.use_fft != 0;
+  int radix = 2;
   if (c.kind != KIND_PERIODIC) fast = fast && c.cx.use_fft != 0;
   else if (c.fx.log2M < 0)
-    for (int k = 0; k < c.fx.nrad; k++) fast = fast && c.fx.rad[k] <= 8;
+    for (int k = 0; k < c.fx.nrad; k++) radix = std::max(radix, c.fx.rad[k]);
+  if (radix > 8) return true;
   return c.nx * c.ny >= (fast ? 48000 : 9000);
 }
 

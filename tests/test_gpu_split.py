@@ -119,3 +119,10 @@ def test_nonfinite_and_timeout_are_reported(R, kind):
     _ic(k)
     k.update(1)
     assert k.status() == 0 and np.isfinite(k.get(R.TEMP)).all()
+
+
+@pytest.mark.parametrize("nx,ny", [(17, 16), (22, 17), (23, 16), (26, 33), (47, 17), (106, 33), (599, 16)])
+def test_small_prime_fourier_lengths(R, nx, ny):
+    # a Fourier length with a prime factor above 8 takes the digit GEMMs at any
+    # size from 16 x 16 on: few rows, short lists, one lane block
+    test_step_matches_transforms_inside_the_passes(R, nx, ny, 2)
