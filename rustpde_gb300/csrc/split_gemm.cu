@@ -144,8 +144,8 @@ __device__ __forceinline__ void split_tile(const SplitJobDev& J, const int lane0
   unsigned char* tail = sm + (size_t)F::kStages * F::kStageBytes;
   uint64_t* full = reinterpret_cast<uint64_t*>(tail);  // [F::kStages]
   uint64_t* empty = full + F::kStages;               // [F::kStages]
-  uint64_t* accfull = empty + F::kStages;
-  uint64_t* accempty = accfull + 1;
+  uint64_t* accfull = empty + F::kStages;            // [2], see split_acc_wait
+  uint64_t* accempty = accfull + 2;
   uint32_t* slot = reinterpret_cast<uint32_t*>(accempty + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(slot + 1);
   volatile int* issued = abort_flag + 1;   // chunks whose MMAs were issued
@@ -161,7 +161,7 @@ __device__ __forceinline__ void split_tile(const SplitJobDev& J, const int lane0
       mbar_init(&full[s], 1);
       mbar_init(&empty[s], 1);
     }
-    mbar_init(accfull, 1);
+    for (int l = 0; l < 2; l++) mbar_init(&accfull[l], 1);
     mbar_init(accempty, 256);
     *abort_flag = 0;
     *issued = 0;
@@ -226,7 +226,7 @@ __device__ __forceinline__ void split_tile(const SplitJobDev& J, const int lane0
         if (c + F::kStages < total) mma_commit(&empty[s]);
         *issued = c + 1;
         if (c + 1 == J.nc[0] || c + 1 == total) {
-          mma_commit(accfull);
+          mma_commit(&accfull[split_acc_wait(c < J.nc[0] ? 0 : 1).barrier]);
           *lists = *lists + 1;
         }
       }
@@ -243,6 +243,10 @@ __device__ __forceinline__ void split_tile(const SplitJobDev& J, const int lane0
     double* mir = out + (J.mirror - n1) * es;
     out += n1 * es;
     const int ex = valid ? J.ex[lane] : 1, e = ex + J.ex_bias;
+    auto list_wait = [&](int list) {  // that list's accumulators are complete
+      const SplitAccWait w = split_acc_wait(list);
+      return warp_mbar_wait(&accfull[w.barrier], w.parity, limit, abort_flag);
+    };
     const bool nan = ex == (D == 9 ? kSplitBadLane9 : 0x7ff);
     if constexpr (D == 9) {
       // 8 outputs: the five high and the five low weights in 64-bit integers
@@ -252,7 +256,7 @@ __device__ __forceinline__ void split_tile(const SplitJobDev& J, const int lane0
       for (int j = 0; j < 8; j++) hi[j] = lo[j] = 0;
       bool ok = true;
       for (int list = 0; list < nlist && ok; list++) {
-        ok = warp_mbar_wait(accfull, (uint32_t)list, limit, abort_flag);
+        ok = list_wait(list);
         if (!ok) break;
         tc_fence_after();
         uint32_t r8[8];
@@ -289,7 +293,7 @@ __device__ __forceinline__ void split_tile(const SplitJobDev& J, const int lane0
       }
     } else {
       long long v[2][8], o[8];
-      bool ok = warp_mbar_wait(accfull, 0, limit, abort_flag);
+      bool ok = list_wait(0);
       if (ok && (shared_cols || nlist == 1)) {
         tc_fence_after();
         split_sums(addr, NT, v[0]);
@@ -298,7 +302,7 @@ __device__ __forceinline__ void split_tile(const SplitJobDev& J, const int lane0
         mbar_arrive(accempty);
       }
       if (ok && nlist == 2) {
-        ok = warp_mbar_wait(accfull, 1, limit, abort_flag);
+        ok = list_wait(1);
         tc_fence_after();
         if (ok && !shared_cols) split_sums(addr, NT, v[0]);
       }
@@ -354,9 +358,11 @@ __device__ __forceinline__ void split_tile(const SplitJobDev& J, const int lane0
       if (c + F::kStages < total)
         for (long long i = 0; i < kWaitLimit; i++)
           if (mbar_try(&empty[c % F::kStages], (uint32_t)((c / F::kStages) & 1))) break;
-    if (nl > 0)
+    for (int l = 0; l < nl; l++) {
+      const SplitAccWait w = split_acc_wait(l);
       for (long long i = 0; i < kWaitLimit; i++)
-        if (mbar_try(accfull, (uint32_t)((nl - 1) & 1))) break;
+        if (mbar_try(&accfull[w.barrier], w.parity)) break;
+    }
   }
   __syncthreads();
   if (warp == 8)

@@ -95,6 +95,18 @@ struct SplitMat {
 };
 SplitMat pack_split_mat(const std::vector<double>& M, int n);
 
+// The barrier (of two) and the phase parity that say a list's accumulators are
+// complete.  A barrier per list, because nothing holds the MMA thread back
+// between the lists where each has columns of its own: on one barrier it could
+// complete both lists' phases before a warp has looked once, and a wait for the
+// first phase's parity then never ends (a try_wait sees only whether the
+// barrier is past the phase in hand).
+struct SplitAccWait {
+  int barrier;
+  uint32_t parity;
+};
+__host__ __device__ constexpr SplitAccWait split_acc_wait(int list) { return {list, 0}; }
+
 // tiles (job, first lane, first output, tile width)
 void split_tiles(const std::vector<SplitJobDev>& jobs, std::vector<int4>& tiles);
 cudaError_t configure_split_kernels();
