@@ -146,7 +146,8 @@ __device__ __forceinline__ void split_tile(const SplitJobDev& J, const int lane0
   uint64_t* empty = full + F::kStages;               // [F::kStages]
   uint64_t* accfull = empty + F::kStages;            // [2], see split_acc_wait
   uint64_t* accempty = accfull + 2;
-  uint32_t* slot = reinterpret_cast<uint32_t*>(accempty + 1);
+  uint64_t* drain = accempty + 1;                    // MMAs in flight when the tile gave up
+  uint32_t* slot = reinterpret_cast<uint32_t*>(drain + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(slot + 1);
   volatile int* issued = abort_flag + 1;   // chunks whose MMAs were issued
   volatile int* copied = abort_flag + 2;   // chunks whose copies were issued
@@ -163,6 +164,7 @@ __device__ __forceinline__ void split_tile(const SplitJobDev& J, const int lane0
     }
     for (int l = 0; l < 2; l++) mbar_init(&accfull[l], 1);
     mbar_init(accempty, 256);
+    mbar_init(drain, 1);
     *abort_flag = 0;
     *issued = 0;
     *copied = 0;
@@ -230,6 +232,7 @@ __device__ __forceinline__ void split_tile(const SplitJobDev& J, const int lane0
           *lists = *lists + 1;
         }
       }
+      if (split_drain_commit(*issued, total)) mma_commit(drain);
     }
   } else {
     // warp w: lanes 32 (w % 4) .., outputs (NT / 2) (w / 4) .. of the tile, 8 at a time
@@ -348,8 +351,8 @@ __device__ __forceinline__ void split_tile(const SplitJobDev& J, const int lane0
   }
   if (*abort_flag != 0 && tid == 0) {
     if (J.status != nullptr) atomicOr(J.status, kStatusGemmTimeout);
-    // copies that no MMA waited for, then the MMAs in flight (commits complete
-    // in order: the last one of each kind), before the memory is given back
+    // copies that no MMA waited for, then every commit, the last of which covers
+    // all MMAs issued, before the memory is given back
     const int n = *issued, nw = *copied, nl = *lists;
     for (int c = n; c < nw; c++)
       for (long long i = 0; i < kWaitLimit; i++)
@@ -363,6 +366,9 @@ __device__ __forceinline__ void split_tile(const SplitJobDev& J, const int lane0
       for (long long i = 0; i < kWaitLimit; i++)
         if (mbar_try(&accfull[w.barrier], w.parity)) break;
     }
+    if (split_drain_commit(n, total))
+      for (long long i = 0; i < kWaitLimit; i++)
+        if (mbar_try(drain, 0)) break;
   }
   __syncthreads();
   if (warp == 8)

@@ -107,6 +107,11 @@ struct SplitAccWait {
 };
 __host__ __device__ constexpr SplitAccWait split_acc_wait(int list) { return {list, 0}; }
 
+// Whether an MMA thread that gave up after `issued` of `total` chunks commits
+// once more, so that the tile can wait for what it issued: the last chunks free
+// no buffer and so commit nothing before their list's end.
+__host__ __device__ constexpr bool split_drain_commit(int issued, int total) { return issued > 0 && issued < total; }
+
 // tiles (job, first lane, first output, tile width)
 void split_tiles(const std::vector<SplitJobDev>& jobs, std::vector<int4>& tiles);
 cudaError_t configure_split_kernels();

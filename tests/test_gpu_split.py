@@ -126,3 +126,20 @@ def test_small_prime_fourier_lengths(R, nx, ny):
     # a Fourier length with a prime factor above 8 takes the digit GEMMs at any
     # size from 16 x 16 on: few rows, short lists, one lane block
     test_step_matches_transforms_inside_the_passes(R, nx, ny, 2)
+
+
+@pytest.mark.parametrize("limit", [0, 1, 2, 4, 16])
+def test_space_that_gives_up_midway(R, limit):
+    # waits that run out somewhere along a tile's chunks: an output is the
+    # product or NaN, and the next call is as if nothing had happened
+    s = R.Space2(R.Base(1, 264), R.Base(1, 265))
+    v = np.random.default_rng(8).standard_normal((264, 265))
+    spec = s.forward(v)
+    ref = s.backward(spec)
+    R.set_gemm_wait_limit(limit)
+    try:
+        got = s.backward(spec)
+    finally:
+        R.set_gemm_wait_limit(-1)
+    assert (np.isnan(got) | (got == ref)).all()
+    np.testing.assert_array_equal(s.backward(spec), ref)
