@@ -325,13 +325,14 @@ struct FsLanes {
   unsigned int* d_status = nullptr;
   // FP64 transforms as split GEMMs (dense lengths): scratch for kSplitLanesCap
   // lanes at a time.  It is the handle's, and calls may come from several
-  // threads and on several streams: the mutex orders them, and a call on
-  // another stream than the last one waits for that one's event.
+  // threads and on several streams: the mutex orders the host side, and every
+  // call's stream waits for the event of the call before (equal stream handles
+  // would not tell: cudaStreamPerThread is one handle for a stream per thread,
+  // and a destroyed stream's handle can come back while its work still runs).
   std::mutex mu;
   SplitWork work;
   void* work_mem = nullptr;
   cudaEvent_t done = nullptr;
-  cudaStream_t last = nullptr;
   bool used = false;
   ~FsLanes() {
     if (done) cudaEventDestroy(done);
@@ -2434,11 +2435,10 @@ int fs_lanes_apply(FsLanes* p, int op, const double* d_in, double* d_out, int la
     apply(d_in, d_out, lanes);
   } else {
     std::lock_guard<std::mutex> lk(p->mu);
-    if (p->used && p->last != st) cuda_check(cudaStreamWaitEvent(st, p->done, 0), "lane scratch");
+    if (p->used) cuda_check(cudaStreamWaitEvent(st, p->done, 0), "lane scratch");
     for (int l = 0; l < lanes; l += kSplitLanesCap)
       apply(d_in + (size_t)l * il, d_out + (size_t)l * ol, std::min(kSplitLanesCap, lanes - l));
     cuda_check(cudaEventRecord(p->done, st), "lane scratch");
-    p->last = st;
     p->used = true;
   }
   if (!fp64 && op == FS_OP_HHOLTZ) lanes_fdma(p->L, d_out, lanes, st);

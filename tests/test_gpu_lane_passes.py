@@ -143,3 +143,37 @@ def test_mixed_packed_lanes_timeout_is_reported(R):
     finally:
         R.set_gemm_wait_limit(-1)
     np.testing.assert_array_equal(L.apply(R.OP_FORWARD, x), ref)
+
+
+def test_lanes_on_the_streams_of_two_threads_share_the_scratch_in_order(R):
+    # cudaStreamPerThread: one handle value, a stream of its own in each thread
+    import threading
+    import ctypes
+    n, lanes, per_thread = 130, 4096, ctypes.c_void_p(2)
+    L = R.Lanes(R.Base(1, n))
+    rng = np.random.default_rng(9)
+    a, b = rng.standard_normal((2, lanes, n))
+    ref = [L.apply(R.OP_FORWARD, x) for x in (a, b)]
+    ins = [R.DeviceArray.from_host(x) for x in (a, b)]
+    outs = [[R.DeviceArray((lanes, L.m)) for _ in range(8)] for _ in range(2)]
+    R._check(R.lib().rbc_device_synchronize())
+    gate, errors = threading.Barrier(2), []
+
+    def work(k):
+        try:
+            gate.wait(60)
+            for o in outs[k]:
+                L.apply_dev(R.OP_FORWARD, ins[k], o, lanes, per_thread)
+        except Exception as e:  # noqa: BLE001
+            errors.append(e)
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors
+    R._check(R.lib().rbc_device_synchronize())
+    for k in range(2):
+        for o in outs[k]:
+            np.testing.assert_array_equal(o.to_host(), ref[k])
