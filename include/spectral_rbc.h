@@ -419,11 +419,13 @@ int fs_gradient(FsSpace* s, const double* d_spec, double* d_ortho, int deriv0, i
  * reference (Field2::forward, src/field.rs:103-107, allocates freely).
  *
  * The call allocates nothing, on the device or the host: the intermediate
- * array between the two axis passes (phys0 x spec1 doubles) lives in a fixed
- * device buffer of FS_NOALLOC_SCRATCH_BYTES that the library owns, one per
- * device.  A space whose intermediate needs more returns RBC_ERR_INVALID
- * before anything is enqueued.  Nothing in the buffer has to start at zero:
- * the first pass writes every element the second pass reads.
+ * array between the two axis passes (phys0 x spec1 doubles) lives in
+ * FS_NOALLOC_SCRATCH_BYTES of a fixed device buffer that the library owns, one
+ * per device, and what else the kernels need as scratch in another 13 MiB of
+ * it; nothing of the space's own that other calls write is used.  A space whose
+ * intermediate needs more returns RBC_ERR_INVALID before anything is enqueued.
+ * Nothing in the buffer has to start at zero: the first pass writes every
+ * element the second pass reads.
  *
  * The first call on a device looks the buffer's address up (this can load
  * the library's device code); make it before any stream capture, with the

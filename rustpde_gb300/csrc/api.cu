@@ -2278,9 +2278,13 @@ int fs_gradient(FsSpace* s, const double* d_spec, double* d_ortho, int deriv0, i
 // ---- fs_forward_noalloc: fixed device scratch instead of the space's own.
 // The buffer is a file-scope device array, so it exists as soon as the
 // library's device code is loaded on a device; its address is looked up once
-// per device and cached.
+// per device and cached.  Behind the intermediate's part lies split scratch, so
+// that the call takes the kernels of fs_forward without the space's own, which
+// other calls on the space may be using: every space whose intermediate fits
+// 4 MiB needs at most 12.6 MiB of it (3276 x 162).
 namespace {
-static __device__ __align__(256) double g_noalloc_scratch[FS_NOALLOC_SCRATCH_BYTES / sizeof(double)];
+constexpr size_t kNoallocSplitBytes = 13u << 20;
+static __device__ __align__(256) double g_noalloc_scratch[(FS_NOALLOC_SCRATCH_BYTES + kNoallocSplitBytes) / sizeof(double)];
 constexpr int kNoallocMaxDevices = 64;
 std::atomic<void*> g_noalloc_addr[kNoallocMaxDevices];
 
@@ -2314,8 +2318,9 @@ int fs_forward_noalloc(FsSpace* s, const double* d_phys, double* d_spec, void* s
     throw ApiError(RBC_ERR_INVALID, "fs_forward_noalloc: the space needs " + std::to_string(need) +
                                         " bytes of scratch, more than the fixed " +
                                         std::to_string((size_t)FS_NOALLOC_SCRATCH_BYTES));
-  void* scratch = noalloc_scratch_for_current_device();
-  space_forward(s->s, d_phys, d_spec, scratch, (cudaStream_t)stream);
+  char* scratch = static_cast<char*>(noalloc_scratch_for_current_device());
+  const SplitWork work = split_forward_work(s->s, scratch + FS_NOALLOC_SCRATCH_BYTES, kNoallocSplitBytes);
+  space_forward(s->s, d_phys, d_spec, scratch, (cudaStream_t)stream, &work);
   API_END
 }
 

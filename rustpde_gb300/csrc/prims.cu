@@ -459,6 +459,32 @@ static void split_ops(ChebXformDev& c) {
   c.sop_f[1] = shared_split_op(SOP_CHEB_FWD_O, c.n, c.n);
 }
 
+// Layout of split scratch: digits (db bytes), exponents, products.  Returns its size.
+static size_t split_work_at(const SpaceDev& s, size_t db, char* p, SplitWork& w) {
+  w.lanes = std::max(s.phys0, s.phys1);
+  const size_t be = ((size_t)w.lanes * 4 + 255) & ~size_t(255), bb = (size_t)s.phys0 * s.phys1 * 8;
+  db = (db + 255) & ~size_t(255);
+  if (p != nullptr) {
+    w.dig = reinterpret_cast<unsigned char*>(p);
+    w.ex = reinterpret_cast<int*>(p + db);
+    w.buf = reinterpret_cast<double*>(p + db + be);
+  }
+  return db + be + bb;
+}
+static size_t split_digits_of(int lanes, int n, int digits) {
+  return split_dig_bytes(lanes, split_chunks((n + 1) / 2), split_chunks(n / 2), digits);
+}
+
+SplitWork split_forward_work(const SpaceDev& s, void* mem, size_t bytes) {
+  SplitWork w;
+  if (s.work.dig == nullptr) return w;
+  size_t db = 0;
+  if (s.c0.sop_b.w != nullptr) db = std::max(db, split_digits_of(s.phys1, s.phys0, kSplitDigits));
+  if (s.c1.sop_b.w != nullptr) db = std::max(db, split_digits_of(s.phys0, s.phys1, kSplitDigits));
+  if (db != 0 && split_work_at(s, db, nullptr, w) <= bytes) split_work_at(s, db, static_cast<char*>(mem), w);
+  return w;
+}
+
 void attach_split(Arena& a, SpaceDev& s) {
   const bool x = !s.cplx && split_fits(s.c0) && split_pays(s.phys1, s.c0.n), y = split_fits(s.c1) && split_pays(s.phys0, s.c1.n);
   const bool mat = !s.cplx && s.hb0.composite() && !s.hb0.bc() && s.hb0.n <= kSplitMatMax && split_pays(s.phys1, s.spec0);
@@ -466,19 +492,10 @@ void attach_split(Arena& a, SpaceDev& s) {
   if (x) split_ops(s.c0);
   if (y) split_ops(s.c1);
   size_t db = 0;
-  auto need = [&](int lanes, int n, int digits) {
-    db = std::max(db, split_dig_bytes(lanes, split_chunks((n + 1) / 2), split_chunks(n / 2), digits));
-  };
-  if (x) need(s.phys1, s.phys0, kSplitDigits);
-  if (y) need(s.phys0, s.phys1, kSplitDigits);
-  if (mat) need(s.phys1, s.phys0, 9);
-  s.work.lanes = std::max(s.phys0, s.phys1);
-  const size_t be = ((size_t)s.work.lanes * 4 + 255) & ~size_t(255), bb = (size_t)s.phys0 * s.phys1 * 8;
-  db = (db + 255) & ~size_t(255);
-  char* p = static_cast<char*>(a.alloc(db + be + bb));
-  s.work.dig = reinterpret_cast<unsigned char*>(p);
-  s.work.ex = reinterpret_cast<int*>(p + db);
-  s.work.buf = reinterpret_cast<double*>(p + db + be);
+  if (x) db = std::max(db, split_digits_of(s.phys1, s.phys0, kSplitDigits));
+  if (y) db = std::max(db, split_digits_of(s.phys0, s.phys1, kSplitDigits));
+  if (mat) db = std::max(db, split_digits_of(s.phys1, s.phys0, 9));
+  split_work_at(s, db, static_cast<char*>(a.alloc(split_work_at(s, db, nullptr, s.work))), s.work);
 }
 
 bool build_solver(Arena& a, const SpaceDev& s, int kind, const double c[2], SolverDev& out, std::string* err) {
@@ -954,13 +971,15 @@ static void set_axis1(PassDesc& d, const void* in, int in_cplx, void* out, int o
 }
 static void add_op(PassDesc& d, int code, int arg = 0) { d.ops[d.nops++] = PassOp{code, arg}; }
 
-void space_forward(const SpaceDev& s, const double* phys, void* spec, void* tmp, cudaStream_t st) {
+void space_forward(const SpaceDev& s, const double* phys, void* spec, void* tmp, cudaStream_t st,
+                   const SplitWork* work) {
+  if (work == nullptr) work = &s.work;
   PassDesc d = base_desc(s);
   set_axis1(d, phys, 0, tmp, 0, s.phys0, s.phys1, s.spec1);
   d.cx = s.c1; d.basis = s.b1;
   add_op(d, P_DCT_FWD);
   if (s.hb1.composite()) add_op(d, P_FROM_ORTHO);
-  run_pass(d, st, &s.work);
+  run_pass(d, st, work);
   PassDesc e = base_desc(s);
   set_axis0(e, tmp, 0, spec, s.cplx, s.spec1, s.phys0);
   if (s.cplx) { e.fx = s.f0; add_op(e, P_R2C); }
@@ -969,7 +988,7 @@ void space_forward(const SpaceDev& s, const double* phys, void* spec, void* tmp,
     add_op(e, P_DCT_FWD);
     if (s.hb0.composite()) add_op(e, P_FROM_ORTHO);
   }
-  run_pass(e, st, &s.work);
+  run_pass(e, st, work);
 }
 
 void axis0_forward(const SpaceDev& s, const double* in, void* out, int cols, cudaStream_t st) {

@@ -104,6 +104,9 @@ struct SpaceDev {
 // Operators and scratch for split GEMMs in the space's passes, where a dense
 // transform or eigenbasis product of the space is large enough to gain.
 void attach_split(Arena& a, SpaceDev& s);
+// Scratch for the space's forward transform alone in `bytes` of other memory (256-byte aligned):
+// empty when the space has no split form or it does not fit.
+SplitWork split_forward_work(const SpaceDev& s, void* mem, size_t bytes);
 void build_space(Arena& a, SpaceDev& s, int kind0, int n0, int kind1, int n1, bool odd = true);
 
 // The same space with dense Chebyshev transforms that sum all n terms in index
@@ -144,7 +147,9 @@ std::vector<double> transposed(const std::vector<double>& a, int n);
 
 // 2-D operations (enqueued on `st`; `tmp` must hold max(phys0,spec0,ortho0) x
 // max(phys1,spec1,ortho1) complex values).
-void space_forward(const SpaceDev& s, const double* phys, void* spec, void* tmp, cudaStream_t st);
+// work: split scratch in place of the space's own
+void space_forward(const SpaceDev& s, const double* phys, void* spec, void* tmp, cudaStream_t st,
+                   const SplitWork* work = nullptr);
 void space_backward(const SpaceDev& s, const void* spec, double* phys, void* tmp, cudaStream_t st);
 // forward transform along axis 0 only of a (phys0 x cols) real array (Transform::forward_inplace, axis 0)
 void axis0_forward(const SpaceDev& s, const double* in, void* out, int cols, cudaStream_t st);

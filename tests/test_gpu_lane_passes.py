@@ -177,3 +177,27 @@ def test_lanes_on_the_streams_of_two_threads_share_the_scratch_in_order(R):
     for k in range(2):
         for o in outs[k]:
             np.testing.assert_array_equal(o.to_host(), ref[k])
+
+
+@pytest.mark.parametrize("k0,n0,k1,n1", [(0, 512, 0, 257), (5, 1000, 1, 300), (1, 264, 2, 265)])
+def test_noalloc_forward_beside_other_calls_of_the_space(R, k0, n0, k1, n1):
+    # the documented shared state of fs_forward_noalloc is the library's buffer
+    # alone: calls of the same space on another stream may overlap it
+    torch = pytest.importorskip("torch")
+    s = R.Space2(R.Base(k0, n0), R.Base(k1, n1))
+    rng = np.random.default_rng(n0)
+    v = rng.standard_normal((n0, n1))
+    spec = s.forward(rng.standard_normal((n0, n1)))
+    want, back = s.forward(v), s.backward(spec)
+    d_v, d_spec = R.DeviceArray.from_host(v), R.DeviceArray.from_host(spec)
+    outs = [R.DeviceArray(s.spectral, s.is_complex) for _ in range(10)]
+    backs = [R.DeviceArray(s.physical, False) for _ in range(10)]
+    a, b = torch.cuda.Stream(), torch.cuda.Stream()
+    R._check(R.lib().rbc_device_synchronize())
+    for o, p in zip(outs, backs):
+        s.forward_noalloc_dev(d_v, o, a.cuda_stream)
+        s.backward_dev(d_spec, p, b.cuda_stream)
+    torch.cuda.synchronize()
+    for o, p in zip(outs, backs):
+        np.testing.assert_array_equal(o.to_host(), want)
+        np.testing.assert_array_equal(p.to_host(), back)
