@@ -571,8 +571,11 @@ namespace dev {
 // One lane per CTA, or a pair of real lanes.  T and PAIR:
 //   double2, 0  complex lanes (either side may be real: imaginary part 0 / dropped)
 //   double,  0  real lanes
-//   double2, 1  two real lanes as the parts of one complex lane: every operation
-//               here but the Fourier ones is linear with real coefficients
+//   double2, 1  two real lanes as the parts of one complex lane: stencils, scans
+//               and dense products are linear with real coefficients and keep
+//               the parts apart.  The FFT transforms do not (each part's rounding
+//               is relative to both, and a NaN in one reaches the other): a pass
+//               with one of them never takes pairs.
 // FP64 issue bounds the pass, so a real lane run as a complex one with a zero
 // imaginary part cost twice its products.
 template <class T> __device__ __forceinline__ double first_part(T v);
@@ -848,18 +851,20 @@ static int pass_threads(const PassDesc& d) {
   return !wide && d.lanes >= kManyLanes ? 32 : 128;
 }
 
-// Real lanes run as pairs where the pairs still give every SM two CTAs and no
-// operation has factors per lane (a pair shares them), else one by one.
+// Real lanes run as pairs where the pairs still give every SM two CTAs, no
+// operation mixes a pair's parts (an FFT) and none has factors per lane (a pair
+// shares them), else one by one.
 static void run_pass_whole(PassDesc d, cudaStream_t st) {
-  bool real = !d.in_cplx && !d.out_cplx, per_lane = false;
+  bool real = !d.in_cplx && !d.out_cplx, per_lane = false, fft = false;
   for (int k = 0; k < d.nops; k++) {
     const int code = d.ops[k].code;
     if (code == P_FDIFF || code == P_R2C || code == P_C2R) real = false;
     if (code == P_FDMA && d.fdma.rows > 1) per_lane = true;
+    if ((code == P_DCT_FWD || code == P_DCT_BWD) && d.cx.use_fft) fft = true;
   }
   constexpr int kPairLanes = 2 * 2 * 152;
   const int nt = pass_threads(d);
-  const bool pair = real && !per_lane && d.lanes >= kPairLanes;
+  const bool pair = real && !per_lane && !fft && d.lanes >= kPairLanes;
   const size_t sm = pass_smem_used(d, real && !pair ? 8 : 16);
   if (!real) dev::k_pass<double2, 0><<<d.lanes, nt, sm, st>>>(d);
   else if (pair) dev::k_pass<double2, 1><<<(d.lanes + 1) / 2, nt, sm, st>>>(d);

@@ -201,3 +201,24 @@ def test_noalloc_forward_beside_other_calls_of_the_space(R, k0, n0, k1, n1):
     for o, p in zip(outs, backs):
         np.testing.assert_array_equal(o.to_host(), want)
         np.testing.assert_array_equal(p.to_host(), back)
+
+
+@pytest.mark.parametrize("n", [17, 129, 257, 46, 130])
+def test_lanes_do_not_see_their_neighbours(R, n):
+    # a lane's result is the same bits whatever the lane beside it holds: lanes
+    # eight decades apart, a lane of zeros, a NaN, an infinity
+    lanes = 700
+    L = R.Lanes(R.Base(1, n), R.PREC_FP64, hholtz_c=5e-4)
+    rng = np.random.default_rng(n)
+    for op in (R.OP_FORWARD, R.OP_BACKWARD, R.OP_TO_ORTHO, R.OP_FROM_ORTHO, R.OP_HHOLTZ):
+        x = rng.standard_normal((lanes, L.m if op in (R.OP_BACKWARD, R.OP_TO_ORTHO) else n))
+        ref = L.apply(op, x)
+        for first in (0, 1):
+            y = x.copy()
+            y[first::2] *= 1e8
+            y[first + 10] = 0.0
+            y[first + 20, 3] = np.nan
+            y[first + 30, 2] = np.inf
+            got = L.apply(op, y)
+            np.testing.assert_array_equal(got[1 - first::2], ref[1 - first::2])
+            assert (got[first + 10] == 0).all()
