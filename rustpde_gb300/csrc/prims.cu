@@ -901,7 +901,11 @@ static void run_pass(const PassDesc& d, cudaStream_t st, const SplitWork* w = nu
   S.ex = w->ex;
   S.cE = split_chunks(dense ? d.smat.K0 : (n + 1) / 2);
   S.cO = split_chunks(dense ? d.smat.K1 : n / 2);
-  dev::k_pass_digits<<<d.lanes, d.lanes >= kManyLanes ? 32 : 128, (size_t)3 * d.lmax * 8 + 64, st>>>(d, at, code, S);
+  // three buffers of this axis's lanes (at most 640 values: below the 48 KB that
+  // need no attribute), not of the space's longer axis, which may have 3628
+  PassDesc g = d;
+  g.lmax = std::max(d.in_len, n) + 2;
+  dev::k_pass_digits<<<d.lanes, d.lanes >= kManyLanes ? 32 : 128, (size_t)3 * g.lmax * 8 + 64, st>>>(g, at, code, S);
   cuda_check(cudaGetLastError(), "pass kernel launch");
   // the product: into the output, or into buf for the rest of the pass (lanes
   // adjacent where they are in the output)

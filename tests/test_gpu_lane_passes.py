@@ -222,3 +222,14 @@ def test_lanes_do_not_see_their_neighbours(R, n):
             got = L.apply(op, y)
             np.testing.assert_array_equal(got[1 - first::2], ref[1 - first::2])
             assert (got[first + 10] == 0).all()
+
+
+@pytest.mark.parametrize("k0,n0,k1,n1", [(5, 2048, 1, 200), (1, 264, 2, 2200), (1, 2049, 1, 100), (0, 3626, 2, 640)])
+def test_space_with_one_long_axis(R, O, k0, n0, k1, n1):
+    # a dense length beside an axis of more than 2044 points
+    test_space_transforms_match_oracle(R, O, k0, n0, k1, n1)
+
+
+def test_poisson_with_one_long_axis(R, O):
+    # 198 modes as digit products over 2100 lanes
+    test_poisson_with_split_eigenbasis_matches_oracle(R, O, 200, 2100)
