@@ -142,9 +142,10 @@ int rbc_get_dt(const RbcCase* c, double* dt);    /* Integrate::get_dt lib.rs:141
 /* Status word of the case (bits stay set until the case is destroyed; a
  * batch clears its cases' words when it is created):
  *   bit 0 (1): a non-finite value was written to the state;
- *   bit 1 (2): RBC_PREC_MIXED only -- a tensor-core completion wait of a lane
- *              GEMM timed out, so that step's results are incomplete (the
- *              kernel skipped its stores and returned instead of hanging). */
+ *   bit 1 (2): a tensor-core completion wait timed out, so that step's results
+ *              are incomplete (RBC_PREC_MIXED: the kernel skipped its stores
+ *              and returned instead of hanging; RBC_PREC_FP64: NaN in their
+ *              place, so that bit 0 follows and rbc_exit stops a loop). */
 int rbc_status(RbcCase* c, int* status);
 /* Integrate::exit (navier.rs:855-862): *stop = 1 if ||div|| is NaN */
 int rbc_exit(RbcCase* c, int* stop);
@@ -461,16 +462,19 @@ int fs_lanes_shape(const FsLanes* p, int* n, int* m);
 int fs_lanes_set_hholtz(FsLanes* p, double c);
 int fs_lanes_apply(FsLanes* p, int op, const double* d_in, double* d_out, int lanes, void* stream);
 /* Waits for `stream`, then returns and clears the status word of the applies
- * enqueued so far: bit 1 (2) when a tensor-core completion wait of an
- * RBC_PREC_MIXED apply timed out (its output is incomplete); 0 otherwise. */
+ * enqueued so far: bit 1 (2) when a tensor-core completion wait timed out, 0
+ * otherwise.  An RBC_PREC_MIXED apply's output is then incomplete; an
+ * RBC_PREC_FP64 apply (transforms of a dense length, many lanes) has left NaN
+ * in what it lost. */
 int fs_lanes_status(FsLanes* p, void* stream, unsigned int* status);
 
-/* Test hook (no counterpart in the reference): the poll limit of the lane
- * GEMM's bounded completion waits on the current device; a negative value
+/* Test hook (no counterpart in the reference): the poll limit of the tensor-core
+ * kernels' bounded completion waits on the current device; a negative value
  * restores the default (2^22 polls).  A limit of 0 makes every wait run out at
- * once, so that the time-out path -- status bit 1 set, stores skipped, the
- * MMAs in flight drained, tensor memory freed -- can be exercised without a
- * hung GPU.  It applies to every RBC_PREC_MIXED handle on the device. */
+ * once, so that the time-out path -- status bit 1 set, stores skipped or NaN,
+ * the MMAs in flight drained, tensor memory freed -- can be exercised without a
+ * hung GPU.  It applies to every handle on the device that uses the tensor
+ * cores: RBC_PREC_MIXED, and RBC_PREC_FP64 where its transforms run there. */
 int rbc_set_gemm_wait_limit(long long polls);
 
 /* ---- solvers ----------------------------------------------------------------

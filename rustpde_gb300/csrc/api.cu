@@ -3058,7 +3058,7 @@ static void server_finish(RbcServer* S) {
     res.t_admit = sl.t_admit;
     unsigned int st = 0;
     cuda_check(cudaMemcpy(&st, sl.c->hd.status, sizeof st, cudaMemcpyDeviceToHost), "status");
-    res.status = st == 0 ? RBC_OK : ((st & 1u) ? RBC_ERR_NUMERIC : RBC_ERR_CUDA);
+    res.status = st == 0 ? RBC_OK : ((st & kStatusGemmTimeout) ? RBC_ERR_CUDA : RBC_ERR_NUMERIC);
     if (sl.cancelled) res.status = RBC_ERR_CANCELLED;
     res.nu = eval_case(sl.c, RBC_NU);
     res.ke = eval_case(sl.c, RBC_KE);

@@ -35,9 +35,9 @@
 // x forward 18.1 -> 11.8, y forward 20.7 -> 12.4 (the same transforms inside
 // the FP64 passes: about 100, 150, 60 and 70 us).
 //
-// Every wait is bounded: on time-out the tile sets kStatusGemmTimeout, stores
-// nothing, waits (bounded) for its copies and MMAs in flight, frees its tensor
-// memory and returns.
+// Every wait is bounded: on time-out the tile sets kStatusGemmTimeout, makes its
+// outputs NaN, waits (bounded) for its copies and MMAs in flight, frees its
+// tensor memory and returns.
 #include "split_gemm.h"
 
 #include <algorithm>
@@ -339,8 +339,8 @@ __device__ __forceinline__ void split_tile(const SplitJobDev& J, const int lane0
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  if (*abort_flag != 0 && J.status == nullptr && tid < kSplitLanes && lane0 + tid < J.lanes) {
-    // no status word to report to: the outputs say it
+  if (*abort_flag != 0 && tid < kSplitLanes && lane0 + tid < J.lanes) {
+    // FP64 callers need not ask for a status: the outputs say that they are lost
     const int lane = lane0 + tid, r = lane / J.nf, f = lane - r * J.nf;
     double* out = J.out + f * J.fs + (r / J.parts) * J.qs + (r % J.parts) * J.ps;
     for (int n = n0; n < min(n0 + NT, J.N); n++) {

@@ -58,7 +58,7 @@ struct SplitJobDev {
   const unsigned char* w;    // packed operator (SplitOp), 32-wide tiles
   const unsigned char* w16;  // the same in 16-wide tiles
   double* out;
-  unsigned int* status;    // receives kStatusGemmTimeout (null: the tile's outputs become NaN)
+  unsigned int* status;    // receives kStatusGemmTimeout, or null (a lost tile's outputs become NaN either way)
   const int* active;       // when set and 0, the job's tiles do nothing (serving gate)
   long long fs, qs, ps, es;
   int lanes, nf, parts;

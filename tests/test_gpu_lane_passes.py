@@ -233,3 +233,23 @@ def test_space_with_one_long_axis(R, O, k0, n0, k1, n1):
 def test_poisson_with_one_long_axis(R, O):
     # 198 modes as digit products over 2100 lanes
     test_poisson_with_split_eigenbasis_matches_oracle(R, O, 200, 2100)
+
+
+@pytest.mark.parametrize("op", ["OP_FORWARD", "OP_BACKWARD"])
+def test_fp64_lanes_timeout_leaves_nan_and_is_reported(R, op):
+    n, lanes = 130, 700
+    op = getattr(R, op)
+    L = R.Lanes(R.Base(1, n))
+    x = np.random.default_rng(7).standard_normal((lanes, n if op == R.OP_FORWARD else L.m))
+    ref = L.apply(op, x)
+    assert L.status() == 0
+    d_in, d_out = R.DeviceArray.from_host(x), R.DeviceArray.from_host(ref)
+    R.set_gemm_wait_limit(0)
+    try:
+        L.apply_dev(op, d_in, d_out, lanes)
+        assert L.status() & 2
+    finally:
+        R.set_gemm_wait_limit(-1)
+    assert np.isnan(d_out.to_host()).all()
+    np.testing.assert_array_equal(L.apply(op, x), ref)
+    assert L.status() == 0

@@ -143,3 +143,20 @@ def test_space_that_gives_up_midway(R, limit):
         R.set_gemm_wait_limit(-1)
     assert (np.isnan(got) | (got == ref)).all()
     np.testing.assert_array_equal(s.backward(spec), ref)
+
+
+@pytest.mark.parametrize("kind", [0, 2])
+def test_fp64_step_that_gives_up_does_not_look_well(R, kind):
+    # a caller that steps in FP64 and asks for no status sees it in the fields
+    c = R.Navier2D(100, 96, 1e5, 1.0, 2e-3, 1.0, kind)
+    _ic(c)
+    R.set_gemm_wait_limit(0)
+    try:
+        c.update(1)
+        c.synchronize()
+    finally:
+        R.set_gemm_wait_limit(-1)
+    assert c.status() & 2
+    for f in (R.TEMP, R.UX, R.UY):
+        assert np.isnan(c.get(f)).any()
+    assert c.exit()
