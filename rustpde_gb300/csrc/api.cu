@@ -603,8 +603,8 @@ void build_case(RbcCase* c, bool with_graph = true, char* state_region = nullptr
     }
     if (split_eig_size(h)) {
       h.split_eig = 1;
-      h.smat_f = shared_split_mat(c->sp_p1.hb0.kind, nx, true, true);
-      h.smat_b = shared_split_mat(c->sp_p1.hb0.kind, nx, true, false);
+      h.smat_f = shared_split_mat(A, c->sp_p1.hb0.kind, nx, true, true);
+      h.smat_b = shared_split_mat(A, c->sp_p1.hb0.kind, nx, true, false);
       h.spl_z.cE = h.spl_w.cE = split_chunks(h.smat_f.K0);
       h.spl_z.cO = h.spl_w.cO = split_chunks(h.smat_f.K1);
       db = std::max(db, split_dig_bytes(ny, h.spl_z.cE, h.spl_z.cO, 9));
@@ -617,12 +617,12 @@ void build_case(RbcCase* c, bool with_graph = true, char* state_region = nullptr
     h.spl_ph = static_cast<double*>(A.alloc((size_t)n_x1 * nx * 8));
     h.spl_q = static_cast<double*>(A.alloc((size_t)std::max(n_q, 1) * ny * 8));
     if (!h.mixed) h.m_cv = A.alloc((size_t)3 * std::max(h.kx, 1) * h.ky * 16);
-    h.sop_yb = shared_split_op(SOP_CHEB_BWD, ny, 0);
-    h.sop_xb = shared_split_op(per ? SOP_C2R : SOP_CHEB_BWD, nx, 0);
+    h.sop_yb = shared_split_op(A, SOP_CHEB_BWD, ny, 0);
+    h.sop_xb = shared_split_op(A, per ? SOP_C2R : SOP_CHEB_BWD, nx, 0);
     for (int par = 0; par < 2; par++) {
-      h.sop_xf[par] = per ? shared_split_op(par ? SOP_R2C_IM : SOP_R2C_RE, nx, h.kx)
-                          : shared_split_op(par ? SOP_CHEB_FWD_O : SOP_CHEB_FWD_E, nx, h.kx);
-      h.sop_yf[par] = shared_split_op(par ? SOP_CHEB_FWD_O : SOP_CHEB_FWD_E, ny, h.ky);
+      h.sop_xf[par] = per ? shared_split_op(A, par ? SOP_R2C_IM : SOP_R2C_RE, nx, h.kx)
+                          : shared_split_op(A, par ? SOP_CHEB_FWD_O : SOP_CHEB_FWD_E, nx, h.kx);
+      h.sop_yf[par] = shared_split_op(A, par ? SOP_CHEB_FWD_O : SOP_CHEB_FWD_E, ny, h.ky);
     }
     h.split = 1;
   }
@@ -712,7 +712,7 @@ void build_case(RbcCase* c, bool with_graph = true, char* state_region = nullptr
     for (int i = 0; i < nx; i++) { bc[2 * i] = 0.5; bc[2 * i + 1] = -0.5; }
     double* d_bc = c->phys[0];
     cuda_check(cudaMemcpyAsync(d_bc, bc.data(), bc.size() * 8, cudaMemcpyHostToDevice, st), "upload bc");
-    const SpaceDev sbc = in_order_space(c->sp_bc), sfield = in_order_space(c->sp_field);
+    const SpaceDev sbc = in_order_space(c->sp_bc, A), sfield = in_order_space(c->sp_field, A);
     axis0_forward(sbc, d_bc, c->bc_vhat, 2, st);
     space_backward(sbc, c->bc_vhat, c->bc_phys, c->tmp, st);
     space_forward(sbc, c->bc_phys, c->bc_vhat, c->tmp, st);
@@ -850,7 +850,7 @@ namespace {
 void set_phys(RbcCase* c, int field, const std::vector<double>& v) {
   double* d = c->phys[0];
   cuda_check(cudaMemcpyAsync(d, v.data(), v.size() * 8, cudaMemcpyHostToDevice, c->stream), "upload");
-  space_forward(in_order_space(field_space(c, field)), d, field_ptr(c, field), c->tmp, c->stream);
+  space_forward(in_order_space(field_space(c, field), c->arena), d, field_ptr(c, field), c->tmp, c->stream);
   c->sync();
 }
 
@@ -2344,7 +2344,7 @@ int fs_lanes_create(int base, int n, int precision, FsLanes** out) {
   p->precision = precision;
   build_lanes(p->arena, p->L, base, n);
   p->d_status = static_cast<unsigned int*>(p->arena.alloc(16));
-  if (precision == RBC_PREC_FP64 && lanes_attach_split(p->L)) {
+  if (precision == RBC_PREC_FP64 && lanes_attach_split(p->arena, p->L)) {
     const size_t db = (split_dig_bytes(kSplitLanesCap, split_chunks((n + 1) / 2), split_chunks(n / 2)) + 255) & ~size_t(255);
     const size_t be = (size_t)kSplitLanesCap * 4, bb = (size_t)kSplitLanesCap * n * 8;
     if (lane_scratch(p.get(), db + be + bb)) {

@@ -9,7 +9,9 @@
 #include "step_split.h"
 #include "per_device.h"
 #include "prims.h"
+#include "shared_dev.h"
 
+#include <list>
 #include <map>
 #include <mutex>
 #include <tuple>
@@ -47,12 +49,20 @@ Arena::~Arena() {
     for (void* p : ptrs_) cudaFree(p);
   }
 }
+// Out of memory: clear the error (a launch check would report it as its own) and
+// give up idle shared tables; true when there were any.
+static bool alloc_again(cudaError_t e) {
+  if (e != cudaErrorMemoryAllocation) return false;
+  (void)cudaGetLastError();
+  return shared_recent_drop();
+}
 void* Arena::alloc(size_t bytes) {
   if (bytes == 0) bytes = 16;
   void* p = nullptr;
   if (ordered_) {
     cudaStream_t s = pool_stream();
     cudaError_t e = cudaMallocAsync(&p, bytes, s);
+    if (alloc_again(e)) e = cudaMallocAsync(&p, bytes, s);
     if (e != cudaSuccess) throw std::runtime_error(std::string("cudaMalloc failed: ") + cudaGetErrorString(e));
     e = cudaMemsetAsync(p, 0, bytes, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);  // usable from any stream once this returns
@@ -62,6 +72,7 @@ void* Arena::alloc(size_t bytes) {
     }
   } else {
     cudaError_t e = cudaMalloc(&p, bytes);
+    if (alloc_again(e)) e = cudaMalloc(&p, bytes);
     if (e != cudaSuccess) throw std::runtime_error(std::string("cudaMalloc failed: ") + cudaGetErrorString(e));
     e = cudaMemset(p, 0, bytes);
     if (e != cudaSuccess) {
@@ -73,6 +84,61 @@ void* Arena::alloc(size_t bytes) {
   bytes_ += bytes;
   return p;
 }
+void Arena::keep(const std::shared_ptr<const DevBlock>& b) {
+  if (std::find(kept_.begin(), kept_.end(), b) == kept_.end()) kept_.push_back(b);
+}
+
+// ---------------------------------------------------------------- shared tables
+DevBlock::~DevBlock() {
+  if (p != nullptr) cudaFree(p);
+}
+std::shared_ptr<DevBlock> make_dev_block(size_t bytes) {
+  auto b = std::make_shared<DevBlock>();
+  cudaError_t e = cudaMalloc(&b->p, bytes);
+  if (alloc_again(e)) e = cudaMalloc(&b->p, bytes);
+  cuda_check(e, "cudaMalloc shared table");
+  b->bytes = bytes;
+  return b;
+}
+namespace {
+struct Recent {
+  std::mutex mu;
+  std::list<std::shared_ptr<const DevBlock>> blocks;  // most recent first
+  size_t bytes = 0;
+};
+Recent& recent() {
+  static Recent* r = new Recent;  // (not destroyed: the runtime may be gone by then)
+  return *r;
+}
+}  // namespace
+// Blocks given up are freed outside the lock: cudaFree waits for the device.
+void shared_recent_touch(const std::shared_ptr<const DevBlock>& b) {
+  std::list<std::shared_ptr<const DevBlock>> gone;
+  Recent& r = recent();
+  std::lock_guard<std::mutex> lk(r.mu);
+  auto it = std::find(r.blocks.begin(), r.blocks.end(), b);
+  if (it != r.blocks.end()) {
+    r.blocks.splice(r.blocks.begin(), r.blocks, it);
+    return;
+  }
+  r.blocks.push_front(b);
+  r.bytes += b->bytes;
+  while (r.bytes > kSharedRecentBytes) {
+    r.bytes -= r.blocks.back()->bytes;
+    gone.splice(gone.end(), r.blocks, std::prev(r.blocks.end()));
+  }
+}
+bool shared_recent_drop() {
+  std::list<std::shared_ptr<const DevBlock>> gone;
+  {
+    Recent& r = recent();
+    std::lock_guard<std::mutex> lk(r.mu);
+    gone.swap(r.blocks);
+    r.bytes = 0;
+  }
+  return !gone.empty();
+}
+
 void Arena::upload_all(std::initializer_list<std::pair<const std::vector<double>*, const double**>> tables) {
   size_t n = 0;
   for (const auto& t : tables) n += (t.first->size() + 31) & ~size_t(31);
@@ -292,33 +358,27 @@ void build_space(Arena& a, SpaceDev& s, int kind0, int n0, int kind1, int n1, bo
 }
 
 // unsplit tables of length n on the current device, shared by every space
-static void full_tables(ChebXformDev& c) {
+static void full_tables(Arena& owner, ChebXformDev& c) {
   if (c.n == 0 || c.use_fft) return;
-  static std::mutex mu;
-  static std::map<std::pair<int, int>, std::pair<const double*, const double*>> cache;
-  std::lock_guard<std::mutex> lk(mu);
-  auto& e = cache[std::make_pair(current_device(), c.n)];
-  if (e.first == nullptr) {
+  static SharedDev<std::pair<int, int>, std::pair<const double*, const double*>> cache;
+  const auto t = cache.get({current_device(), c.n}, owner, [&](std::pair<const double*, const double*>& out) {
     const ChebDense t = cheb_dense_full(c.n);
     const size_t b = t.fwd.size() * 8;
-    double* p = nullptr;
-    cuda_check(cudaMalloc(&p, 2 * b), "cudaMalloc transform tables");
-    cudaError_t r = cudaMemcpy(p, t.fwd.data(), b, cudaMemcpyHostToDevice);
-    if (r == cudaSuccess) r = cudaMemcpy(p + t.fwd.size(), t.bwd.data(), b, cudaMemcpyHostToDevice);
-    if (r != cudaSuccess) {
-      cudaFree(p);
-      cuda_check(r, "upload transform tables");
-    }
-    e = std::make_pair(p, p + t.fwd.size());
-  }
-  c.fwd_full = e.first;
-  c.bwd_full = e.second;
+    auto mem = make_dev_block(2 * b);
+    double* p = static_cast<double*>(mem->p);
+    cuda_check(cudaMemcpy(p, t.fwd.data(), b, cudaMemcpyHostToDevice), "upload transform tables");
+    cuda_check(cudaMemcpy(p + t.fwd.size(), t.bwd.data(), b, cudaMemcpyHostToDevice), "upload transform tables");
+    out = {p, p + t.fwd.size()};
+    return mem;
+  });
+  c.fwd_full = t.first;
+  c.bwd_full = t.second;
 }
 
-SpaceDev in_order_space(const SpaceDev& s) {
+SpaceDev in_order_space(const SpaceDev& s, Arena& owner) {
   SpaceDev o = s;
-  if (!s.cplx) full_tables(o.c0);
-  full_tables(o.c1);
+  if (!s.cplx) full_tables(owner, o.c0);
+  full_tables(owner, o.c1);
   return o;
 }
 
@@ -453,10 +513,10 @@ constexpr int kSplitMatMax = 514;  // longest axis of a nine-digit matrix (two l
 static bool split_pays(int lanes, int n) { return n >= 48 && (double)lanes * n * n >= 4e6; }
 
 static bool split_fits(const ChebXformDev& c) { return c.n >= 48 && c.n <= 640 && !c.use_fft; }
-static void split_ops(ChebXformDev& c) {
-  c.sop_b = shared_split_op(SOP_CHEB_BWD, c.n, 0);
-  c.sop_f[0] = shared_split_op(SOP_CHEB_FWD_E, c.n, c.n);
-  c.sop_f[1] = shared_split_op(SOP_CHEB_FWD_O, c.n, c.n);
+static void split_ops(Arena& a, ChebXformDev& c) {
+  c.sop_b = shared_split_op(a, SOP_CHEB_BWD, c.n, 0);
+  c.sop_f[0] = shared_split_op(a, SOP_CHEB_FWD_E, c.n, c.n);
+  c.sop_f[1] = shared_split_op(a, SOP_CHEB_FWD_O, c.n, c.n);
 }
 
 // Layout of split scratch: digits (db bytes), exponents, products.  Returns its size.
@@ -489,8 +549,8 @@ void attach_split(Arena& a, SpaceDev& s) {
   const bool x = !s.cplx && split_fits(s.c0) && split_pays(s.phys1, s.c0.n), y = split_fits(s.c1) && split_pays(s.phys0, s.c1.n);
   const bool mat = !s.cplx && s.hb0.composite() && !s.hb0.bc() && s.hb0.n <= kSplitMatMax && split_pays(s.phys1, s.spec0);
   if (!x && !y && !mat) return;
-  if (x) split_ops(s.c0);
-  if (y) split_ops(s.c1);
+  if (x) split_ops(a, s.c0);
+  if (y) split_ops(a, s.c1);
   size_t db = 0;
   if (x) db = std::max(db, split_digits_of(s.phys1, s.phys0, kSplitDigits));
   if (y) db = std::max(db, split_digits_of(s.phys0, s.phys1, kSplitDigits));
@@ -524,8 +584,8 @@ bool build_solver(Arena& a, const SpaceDev& s, int kind, const double c[2], Solv
       out.fwd = a.upload(transposed(fwd, out.m0));
       out.bwd = a.upload(transposed(bwd, out.m0));
       if (s.work.dig != nullptr && s.hb0.n <= kSplitMatMax && split_pays(s.ortho1, out.m0)) {
-        out.smat_f = shared_split_mat(s.hb0.kind, s.hb0.n, kind == SV_KIND_POISSON, true);
-        out.smat_b = shared_split_mat(s.hb0.kind, s.hb0.n, kind == SV_KIND_POISSON, false);
+        out.smat_f = shared_split_mat(a, s.hb0.kind, s.hb0.n, kind == SV_KIND_POISSON, true);
+        out.smat_b = shared_split_mat(a, s.hb0.kind, s.hb0.n, kind == SV_KIND_POISSON, false);
       }
     }
     return true;
@@ -1274,9 +1334,9 @@ static PassDesc lanes_desc(const LanesDev& L) {
   return d;
 }
 
-bool lanes_attach_split(LanesDev& L) {
+bool lanes_attach_split(Arena& a, LanesDev& L) {
   if (!split_fits(L.cx)) return false;
-  split_ops(L.cx);
+  split_ops(a, L.cx);
   return true;
 }
 bool lanes_split_pays(const LanesDev& L, int op, int lanes) {

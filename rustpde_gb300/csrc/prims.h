@@ -8,15 +8,20 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <map>
+#include <memory>
 #include <stdexcept>
 #include <string>
-#include <map>
 #include <vector>
 
 #include "host_ops.h"
 #include "rbc_dev.h"
 
 namespace rbc {
+
+struct DevBlock;  // shared_dev.h
+// Give up the shared tables that no object holds; whether there were any.
+bool shared_recent_drop();
 
 // Owner of device allocations (freed on destruction).  By default blocks come
 // from cudaMalloc (whose free waits for the device).  A stream-ordered arena
@@ -49,11 +54,14 @@ class Arena {
     if (p == nullptr) p = upload(std::vector<T>(make()));
     return static_cast<const T*>(p);
   }
+  // hold a shared table (shared_dev.h) until the arena goes; not counted in bytes()
+  void keep(const std::shared_ptr<const DevBlock>& b);
   size_t bytes() const { return bytes_; }
 
  private:
   void copy_h2d(void* d, const void* h, size_t n);
   std::vector<void*> ptrs_;
+  std::vector<std::shared_ptr<const DevBlock>> kept_;
   std::map<std::pair<int, int>, const void*> shared_;
   size_t bytes_ = 0;
   bool ordered_ = false;
@@ -114,7 +122,7 @@ void build_space(Arena& a, SpaceDev& s, int kind0, int n0, int kind1, int n1, bo
 // mixed form rounds its state to FP32, and a last-bit change of the initial
 // state moves its results by 2e-9 after a few steps, so the summation order of
 // the set-up is part of what makes a run reproducible.
-SpaceDev in_order_space(const SpaceDev& s);
+SpaceDev in_order_space(const SpaceDev& s, Arena& owner);  // owner: of its tables
 
 // Solvers (src/solver/{hholtz,hholtz_adi,poisson}.rs) on a space.
 enum SolverKindDev { SV_KIND_HHOLTZ = 0, SV_KIND_HHOLTZ_ADI = 1, SV_KIND_POISSON = 2 };
@@ -193,7 +201,7 @@ void lanes_apply(const LanesDev& L, int op, const double* in, double* out, int l
                  const SplitWork* work = nullptr);
 // split operators of a dense length (false: none), and whether an application
 // gains by them
-bool lanes_attach_split(LanesDev& L);
+bool lanes_attach_split(Arena& a, LanesDev& L);
 bool lanes_split_pays(const LanesDev& L, int op, int lanes);
 // the banded part of the HholtzAdi solve alone: x (m per lane) solved in place
 void lanes_fdma(const LanesDev& L, double* x, int lanes, cudaStream_t st);

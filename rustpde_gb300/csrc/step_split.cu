@@ -24,8 +24,6 @@
 
 #include <algorithm>
 #include <cmath>
-#include <map>
-#include <mutex>
 #include <stdexcept>
 #include <tuple>
 
@@ -33,6 +31,7 @@
 #include "pdl.cuh"
 #include "per_device.h"
 #include "prims.h"
+#include "shared_dev.h"
 #include "split_emit.cuh"
 #include "step_fp64.h"
 
@@ -300,65 +299,48 @@ SplitOp make_split_op(int kind, int n, int rows, int* wshift) {
   throw std::runtime_error("make_split_op: unknown kind");
 }
 
-// The split operator of a transform (step_split.h) on the current device,
-// shared like the mixed operators by every case of the size.
-SplitOpDev shared_split_op(int kind, int n, int rows) {
-  static std::mutex mu;
-  static std::map<std::tuple<int, int, int, int>, SplitOpDev> cache;
+SplitOpDev shared_split_op(Arena& owner, int kind, int n, int rows) {
+  static SharedDev<std::tuple<int, int, int, int>, SplitOpDev> cache;
   int dev = 0;
   cuda_check(cudaGetDevice(&dev), "cudaGetDevice");
-  std::lock_guard<std::mutex> lk(mu);
-  const auto key = std::make_tuple(dev, kind, n, rows);
-  auto it = cache.find(key);
-  if (it != cache.end()) return it->second;
-  SplitOpDev d{};
-  const SplitOp op = make_split_op(kind, n, rows, &d.wshift);
-  d.N = op.N;
-  const size_t n32 = (op.bytes.size() + 127) & ~size_t(127);
-  unsigned char* p = nullptr;
-  cuda_check(cudaMalloc(&p, n32 + op.bytes16.size()), "cudaMalloc shared operator");
-  cudaError_t e = cudaMemcpy(p, op.bytes.data(), op.bytes.size(), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(p + n32, op.bytes16.data(), op.bytes16.size(), cudaMemcpyHostToDevice);
-  if (e != cudaSuccess) {
-    cudaFree(p);
-    cuda_check(e, "upload shared operator");
-  }
-  d.w = p;
-  d.w16 = p + n32;
-  return cache.emplace(key, d).first->second;
+  return cache.get(std::make_tuple(dev, kind, n, rows), owner, [&](SplitOpDev& d) {
+    const SplitOp op = make_split_op(kind, n, rows, &d.wshift);
+    d.N = op.N;
+    const size_t n32 = (op.bytes.size() + 127) & ~size_t(127);
+    auto mem = make_dev_block(n32 + op.bytes16.size());
+    unsigned char* p = static_cast<unsigned char*>(mem->p);
+    cuda_check(cudaMemcpy(p, op.bytes.data(), op.bytes.size(), cudaMemcpyHostToDevice), "upload shared operator");
+    cuda_check(cudaMemcpy(p + n32, op.bytes16.data(), op.bytes16.size(), cudaMemcpyHostToDevice),
+               "upload shared operator");
+    d.w = p;
+    d.w16 = p + n32;
+    return mem;
+  });
 }
 
 // The eigenbasis matrices of a tensor solver's axis 0 in nine digits.
-SplitMatDev shared_split_mat(int kind, int n, bool poisson, bool fwd) {
-  static std::mutex mu;
-  static std::map<std::tuple<int, int, int, bool, bool>, SplitMatDev> cache;
+SplitMatDev shared_split_mat(Arena& owner, int kind, int n, bool poisson, bool fwd) {
+  static SharedDev<std::tuple<int, int, int, bool, bool>, SplitMatDev> cache;
   int dev = 0;
   cuda_check(cudaGetDevice(&dev), "cudaGetDevice");
-  std::lock_guard<std::mutex> lk(mu);
-  const auto key = std::make_tuple(dev, kind, n, poisson, fwd);
-  auto it = cache.find(key);
-  if (it != cache.end()) return it->second;
-  std::vector<double> F, B;
-  tensor_eigenbasis(make_basis(kind, n), poisson, F, B);
-  const SplitMat m = pack_split_mat(fwd ? F : B, n - 2);
-  const size_t nb = (m.bytes16.size() + 127) & ~size_t(127), ne = (size_t)m.N * 4;
-  unsigned char* p = nullptr;
-  cuda_check(cudaMalloc(&p, nb + 2 * ne), "cudaMalloc shared operator");
-  cudaError_t e = cudaMemcpy(p, m.bytes16.data(), m.bytes16.size(), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(p + nb, m.colex.data(), ne, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(p + nb + ne, m.rowex.data(), ne, cudaMemcpyHostToDevice);
-  if (e != cudaSuccess) {
-    cudaFree(p);
-    cuda_check(e, "upload shared operator");
-  }
-  SplitMatDev d{};
-  d.w16 = p;
-  d.colex = reinterpret_cast<const int*>(p + nb);
-  d.rowex = reinterpret_cast<const int*>(p + nb + ne);
-  d.N = m.N;
-  d.K0 = m.K[0];
-  d.K1 = m.K[1];
-  return cache.emplace(key, d).first->second;
+  return cache.get(std::make_tuple(dev, kind, n, poisson, fwd), owner, [&](SplitMatDev& d) {
+    std::vector<double> F, B;
+    tensor_eigenbasis(make_basis(kind, n), poisson, F, B);
+    const SplitMat m = pack_split_mat(fwd ? F : B, n - 2);
+    const size_t nb = (m.bytes16.size() + 127) & ~size_t(127), ne = (size_t)m.N * 4;
+    auto mem = make_dev_block(nb + 2 * ne);
+    unsigned char* p = static_cast<unsigned char*>(mem->p);
+    cuda_check(cudaMemcpy(p, m.bytes16.data(), m.bytes16.size(), cudaMemcpyHostToDevice), "upload shared operator");
+    cuda_check(cudaMemcpy(p + nb, m.colex.data(), ne, cudaMemcpyHostToDevice), "upload shared operator");
+    cuda_check(cudaMemcpy(p + nb + ne, m.rowex.data(), ne, cudaMemcpyHostToDevice), "upload shared operator");
+    d.w16 = p;
+    d.colex = reinterpret_cast<const int*>(p + nb);
+    d.rowex = reinterpret_cast<const int*>(p + nb + ne);
+    d.N = m.N;
+    d.K0 = m.K[0];
+    d.K1 = m.K[1];
+    return mem;
+  });
 }
 
 // ---------------------------------------------------------------------------

@@ -11,6 +11,7 @@
 namespace rbc {
 
 struct StepPlan;
+class Arena;
 
 // Split operators (host form) of the Chebyshev and Fourier transforms.
 enum SplitOpKind {
@@ -26,9 +27,10 @@ void split_terms(bool fourier, int n, int K[2]);
 // rows: outputs to keep (one-list kinds; all for the others).  wshift: see split_ex_bias.
 SplitOp make_split_op(int kind, int n, int rows, int* wshift);
 
-// The same on the current device, shared by everything of the size.
-SplitOpDev shared_split_op(int kind, int n, int rows);
-SplitMatDev shared_split_mat(int kind, int n, bool poisson, bool fwd);
+// The same on the current device, shared by everything of the size (shared_dev.h); owner: the
+// user's arena.
+SplitOpDev shared_split_op(Arena& owner, int kind, int n, int rows);
+SplitMatDev shared_split_mat(Arena& owner, int kind, int n, bool poisson, bool fwd);
 
 // Whether a case of this size runs its FP64 transforms as split GEMMs.
 bool split_step_size(const CaseDev& c);

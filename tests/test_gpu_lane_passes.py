@@ -253,3 +253,26 @@ def test_fp64_lanes_timeout_leaves_nan_and_is_reported(R, op):
     assert np.isnan(d_out.to_host()).all()
     np.testing.assert_array_equal(L.apply(op, x), ref)
     assert L.status() == 0
+
+
+def test_tables_of_sizes_no_longer_in_use_are_given_back(R):
+    # digit operators and transform tables are shared by size and go with their
+    # last user, up to 64 MB of the most recent ones
+    torch = pytest.importorskip("torch")
+
+    def free():
+        R._check(R.lib().rbc_device_synchronize())
+        return torch.cuda.mem_get_info()[0]
+
+    def use(n):
+        L = R.Lanes(R.Base(1, n))
+        s = R.Space2(R.Base(1, n), R.Base(2, n + 1))
+        c = R.Navier2D(16, n, 1e5, 1.0, 1e-3, 1.0, 0)
+        c.set_temperature(0.2, 1, 1)
+        del L, s, c
+
+    use(480)
+    before = free()
+    for n in range(482, 522, 2):  # 20 sizes; 15 MB of tables each
+        use(n)
+    assert before - free() <= 80 * 2**20
