@@ -84,8 +84,10 @@ void* Arena::alloc(size_t bytes) {
   bytes_ += bytes;
   return p;
 }
-void Arena::keep(const std::shared_ptr<const DevBlock>& b) {
-  if (std::find(kept_.begin(), kept_.end(), b) == kept_.end()) kept_.push_back(b);
+bool Arena::keep(const std::shared_ptr<const DevBlock>& b) {
+  if (std::find(kept_.begin(), kept_.end(), b) != kept_.end()) return false;
+  kept_.push_back(b);
+  return true;
 }
 
 // ---------------------------------------------------------------- shared tables

@@ -54,8 +54,9 @@ class Arena {
     if (p == nullptr) p = upload(std::vector<T>(make()));
     return static_cast<const T*>(p);
   }
-  // hold a shared table (shared_dev.h) until the arena goes; not counted in bytes()
-  void keep(const std::shared_ptr<const DevBlock>& b);
+  // hold a shared table (shared_dev.h) until the arena goes; not counted in
+  // bytes().  False when it was held already.
+  bool keep(const std::shared_ptr<const DevBlock>& b);
   size_t bytes() const { return bytes_; }
 
  private:

@@ -48,8 +48,9 @@ class SharedDev {
       }
       t = e.second;
     }
-    owner.keep(b);
-    shared_recent_touch(b);
+    // (a table that its owner has had before is not new use: set-up calls of a
+    // case that exists allocate and free nothing)
+    if (owner.keep(b)) shared_recent_touch(b);
     return t;
   }
 
