@@ -257,6 +257,23 @@ static std::string op_key(const std::string& k, int ntmax) {
   return ntmax == 64 ? k : k + ":nt" + std::to_string(ntmax);
 }
 
+static bool out_of_memory(const std::exception& e) {
+  return std::string(e.what()).find("cudaMalloc") != std::string::npos;
+}
+// An object with the scratch of its faster forms (digit GEMMs, packed GEMM
+// input), or without where the device has not the memory for that: they made
+// a case up to twice as large, and what fitted without them still has to.
+template <class F>
+static auto make_or_spare(F make) {
+  try {
+    return make(false);
+  } catch (std::exception& e) {
+    if (!out_of_memory(e)) throw;
+  }
+  (void)cudaGetLastError();
+  return make(true);
+}
+
 struct RbcCase {
   RbcParams p{};
   bool periodic = false;
@@ -284,6 +301,7 @@ struct RbcCase {
   double time = 0.0;
   bool own_stream = true;
   bool in_batch = false;
+  bool spare = false;  // made without the scratch of its faster forms (make_or_spare)
   int* gate_mem = nullptr;  // device int[2] used by the serving loop (CaseDev::gate)
   // Statistics (statistics.rs): averages in the `field` space, allocated on first use
   void* st_field[4] = {nullptr, nullptr, nullptr, nullptr};  // temp, ux, uy, nusselt (spectral)
@@ -584,7 +602,7 @@ void build_case(RbcCase* c, bool with_graph = true, char* state_region = nullptr
     for (int k = 0; k < 8; k++) h.s[k] = A.alloc((size_t)nx * ny * 8);
   h.mixed = p.precision == RBC_PREC_MIXED;
   h.odd = odd;
-  if (fp64_plan && split_step_size(h)) {
+  if (fp64_plan && !c->spare && split_step_size(h)) {
     const int P = per ? 2 : 1;
     int ky[2], kx[2];
     split_terms(false, ny, ky);
@@ -632,7 +650,7 @@ void build_case(RbcCase* c, bool with_graph = true, char* state_region = nullptr
     h.m_cv = A.alloc((size_t)3 * std::max(h.kx, 1) * h.ky * 16);
     // FP32 state copy: rows padded to 16 bytes, complex rows as [re | im] (rbc_dev.h)
     h.m_s32 = A.alloc((size_t)3 * h.mxc * s32_row_floats(h) * 4);
-    h.m_pk = static_cast<float*>(A.alloc(mixed_pack_bytes(h)));
+    if (!c->spare) h.m_pk = static_cast<float*>(A.alloc(mixed_pack_bytes(h)));
     h.m_bcx = static_cast<const float*>(A.alloc((size_t)nx * ny * 4));
     h.m_bcy = static_cast<const float*>(A.alloc((size_t)nx * ny * 4));
     for (MixedOps* o : mixed_sets) {
@@ -985,12 +1003,15 @@ int rbc_create(const RbcParams* params, RbcCase** out) {
   const RbcParams& p = *params;
   validate_params(p);
   cuda_check(configure_prim_kernels(), "configure kernels");
-  std::unique_ptr<RbcCase> c(new RbcCase());
-  c->p = p;
-  c->periodic = p.kind == RBC_PERIODIC;
-  cuda_check(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking), "stream create");
-  build_case(c.get());
-  *out = c.release();
+  *out = make_or_spare([&](bool spare) {
+    std::unique_ptr<RbcCase> c(new RbcCase());
+    c->p = p;
+    c->periodic = p.kind == RBC_PERIODIC;
+    c->spare = spare;
+    cuda_check(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking), "stream create");
+    build_case(c.get());
+    return c.release();
+  });
   API_END
 }
 
@@ -1551,15 +1572,7 @@ static void batch_solid_changed(RbcCase* c) {
   batch_capture_graphs(b);
 }
 
-extern "C" {
-
-int rbc_batch_create(const RbcParams* params, int ncases, RbcBatch** out) {
-  API_BEGIN
-  TraceRange tr("rbc_batch_create");
-  require(params != nullptr && out != nullptr && ncases > 0, "rbc_batch_create: invalid argument");
-  *out = nullptr;
-  for (int i = 0; i < ncases; i++) validate_params(params[i]);
-  cuda_check(configure_prim_kernels(), "configure kernels");
+static RbcBatch* make_batch(const RbcParams* params, int ncases, bool spare) {
   std::unique_ptr<RbcBatch> b(new RbcBatch());
   cuda_check(cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking), "stream create");
   // groups of equal kind (box / periodic) and precision, any size: one launch
@@ -1608,6 +1621,7 @@ int rbc_batch_create(const RbcParams* params, int ncases, RbcBatch** out) {
     c->in_batch = true;
     c->batch = b.get();
     c->batch_index = i;
+    c->spare = spare;
     build_case(c.get(), false, b->d_state + b->state_offset[i]);
     b->cases.push_back(c.release());
   }
@@ -1866,7 +1880,19 @@ int rbc_batch_create(const RbcParams* params, int ncases, RbcBatch** out) {
                    [&](size_t x, size_t y) { return bucket_ms[x] < bucket_ms[y]; });
   b->io_events.resize(nb);
   for (auto& e : b->io_events) cuda_check(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "event");
-  *out = b.release();
+  return b.release();
+}
+
+extern "C" {
+
+int rbc_batch_create(const RbcParams* params, int ncases, RbcBatch** out) {
+  API_BEGIN
+  TraceRange tr("rbc_batch_create");
+  require(params != nullptr && out != nullptr && ncases > 0, "rbc_batch_create: invalid argument");
+  *out = nullptr;
+  for (int i = 0; i < ncases; i++) validate_params(params[i]);
+  cuda_check(configure_prim_kernels(), "configure kernels");
+  *out = make_or_spare([&](bool spare) { return make_batch(params, ncases, spare); });
   API_END
 }
 
@@ -2217,11 +2243,13 @@ int fs_space_create(int base0, int n0, int base1, int n1, FsSpace** out) {
   require(base0 >= 0 && base0 <= 5 && base1 >= 0 && base1 <= 4, "fs_space_create: unknown base (Fourier along axis 0 only)");
   require(n0 >= 4 && n1 >= 4 && n0 <= 8192 && n1 <= 8192, "fs_space_create: sizes must be in [4, 8192]");
   cuda_check(configure_prim_kernels(), "configure kernels");
-  std::unique_ptr<FsSpace> s(new FsSpace());
-  build_space(s->arena, s->s, base0, n0, base1, n1);
-  attach_split(s->arena, s->s);
-  s->tmp = s->arena.alloc(tmp_elems(s->s) * 16);
-  *out = s.release();
+  *out = make_or_spare([&](bool spare) {
+    std::unique_ptr<FsSpace> s(new FsSpace());
+    build_space(s->arena, s->s, base0, n0, base1, n1);
+    if (!spare) attach_split(s->arena, s->s);
+    s->tmp = s->arena.alloc(tmp_elems(s->s) * 16);
+    return s.release();
+  });
   API_END
 }
 int fs_space_destroy(FsSpace* s) {
@@ -2847,30 +2875,37 @@ static void server_worker(RbcServer* S) {
         S->building++;
         S->building_ids.insert(r.id);
       }
-      std::unique_ptr<RbcCase> c(new RbcCase());
-      c->p = r.p;
-      c->periodic = r.p.kind == RBC_PERIODIC;
-      c->stream = st;
-      c->own_stream = false;
-      c->in_batch = true;  // stepped by the server only
-      c->arena.set_stream_ordered(true);
-      bool fits = true;
-      try {
+      std::unique_ptr<RbcCase> c;
+      auto make = [&](bool spare) {  // whether the case fits the budget
+        c.reset(new RbcCase());
+        c->p = r.p;
+        c->periodic = r.p.kind == RBC_PERIODIC;
+        c->stream = st;
+        c->own_stream = false;
+        c->in_batch = true;  // stepped by the server only
+        c->spare = spare;
+        c->arena.set_stream_ordered(true);
         build_case(c.get(), false);
-        fits = c->arena.bytes() <= S->cfg.hbm_budget_bytes;
-        if (fits) {
-          // initial fields: set_velocity(0.2, 1, 1) and seeded temperature noise 1e-3
-          apply_mode(c.get(), RBC_UX, 0.2, 1.0, 1.0, true);
-          apply_mode(c.get(), RBC_UY, -0.2, 1.0, 1.0, false);
-          set_temperature_noise(c.get(), 1e-3, r.seed);
-          const int g[2] = {(int)r.steps, 0};
-          cuda_check(cudaMemcpyAsync(c->gate_mem, g, sizeof g, cudaMemcpyHostToDevice, st), "gate");
-          cuda_check(cudaStreamSynchronize(st), "setup synchronize");
+        if (c->arena.bytes() > S->cfg.hbm_budget_bytes) return false;
+        // initial fields: set_velocity(0.2, 1, 1) and seeded temperature noise 1e-3
+        apply_mode(c.get(), RBC_UX, 0.2, 1.0, 1.0, true);
+        apply_mode(c.get(), RBC_UY, -0.2, 1.0, 1.0, false);
+        set_temperature_noise(c.get(), 1e-3, r.seed);
+        const int g[2] = {(int)r.steps, 0};
+        cuda_check(cudaMemcpyAsync(c->gate_mem, g, sizeof g, cudaMemcpyHostToDevice, st), "gate");
+        cuda_check(cudaStreamSynchronize(st), "setup synchronize");
+        return true;
+      };
+      bool fits = false;
+      for (int spare = 0; spare < 2 && !fits; spare++) {  // (as make_or_spare, and within the budget)
+        try {
+          fits = make(spare != 0);
+          if (!fits && !c->hd.split && c->hd.m_pk == nullptr) break;  // nothing to leave out
+        } catch (std::exception& e) {
+          // an allocation that fails is an answer for this request, not for the loop
+          if (!out_of_memory(e)) throw;
+          (void)cudaGetLastError();
         }
-      } catch (std::exception& e) {
-        // an allocation that fails is an answer for this request, not for the loop
-        if (std::string(e.what()).find("cudaMalloc") == std::string::npos) throw;
-        fits = false;
       }
       const size_t bytes = c->arena.bytes();
       std::lock_guard<std::mutex> lk(S->mu);
@@ -2955,7 +2990,10 @@ static void server_rebuild(RbcServer* S) {
     int found = -1;
     for (size_t k = 0; k < S->buckets.size(); k++) {
       const RbcParams& q = S->active[S->buckets[k].members[0]].r.p;
-      if ((q.kind == RBC_PERIODIC) == (p.kind == RBC_PERIODIC) && q.precision == p.precision) found = (int)k;
+      // (a mixed case without packed input has other launches)
+      const bool form = p.precision != RBC_PREC_MIXED ||
+                        S->active[S->buckets[k].members[0]].c->spare == S->active[i].c->spare;
+      if ((q.kind == RBC_PERIODIC) == (p.kind == RBC_PERIODIC) && q.precision == p.precision && form) found = (int)k;
     }
     if (found < 0) {
       S->buckets.emplace_back();

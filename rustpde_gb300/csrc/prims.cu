@@ -586,8 +586,14 @@ bool build_solver(Arena& a, const SpaceDev& s, int kind, const double c[2], Solv
       out.fwd = a.upload(transposed(fwd, out.m0));
       out.bwd = a.upload(transposed(bwd, out.m0));
       if (s.work.dig != nullptr && s.hb0.n <= kSplitMatMax && split_pays(s.ortho1, out.m0)) {
-        out.smat_f = shared_split_mat(a, s.hb0.kind, s.hb0.n, kind == SV_KIND_POISSON, true);
-        out.smat_b = shared_split_mat(a, s.hb0.kind, s.hb0.n, kind == SV_KIND_POISSON, false);
+        try {
+          out.smat_f = shared_split_mat(a, s.hb0.kind, s.hb0.n, kind == SV_KIND_POISSON, true);
+          out.smat_b = shared_split_mat(a, s.hb0.kind, s.hb0.n, kind == SV_KIND_POISSON, false);
+        } catch (std::exception& e) {  // no memory for them: the products stay inside the passes
+          if (std::string(e.what()).find("cudaMalloc") == std::string::npos) throw;
+          (void)cudaGetLastError();
+          out.smat_f = out.smat_b = SplitMatDev{};
+        }
       }
     }
     return true;
@@ -1338,7 +1344,14 @@ static PassDesc lanes_desc(const LanesDev& L) {
 
 bool lanes_attach_split(Arena& a, LanesDev& L) {
   if (!split_fits(L.cx)) return false;
-  split_ops(a, L.cx);
+  try {
+    split_ops(a, L.cx);
+  } catch (std::exception& e) {  // no memory for them: the transforms stay inside the passes
+    if (std::string(e.what()).find("cudaMalloc") == std::string::npos) throw;
+    (void)cudaGetLastError();
+    L.cx.sop_b = L.cx.sop_f[0] = L.cx.sop_f[1] = SplitOpDev{};
+    return false;
+  }
   return true;
 }
 bool lanes_split_pays(const LanesDev& L, int op, int lanes) {

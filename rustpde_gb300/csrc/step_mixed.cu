@@ -209,7 +209,8 @@ StepPlan build_mixed_plan(const CaseDev& c, const MixedOps& ops, int variant) {
   // step, classic | packed, periodic 512 x 257 148 | 121, box 129 x 129 184 |
   // 143, box 264 x 264 281 | 198; 256-case ensemble 3.09 | 2.97 ms, its box x
   // backward GEMMs 0.207 | 0.047 + 0.131.
-  const bool packed = ops.ntmax == 64 && !ops.ws;
+  // A case made without the memory for it (m_pk null) takes the classic form.
+  const bool packed = ops.ntmax == 64 && !ops.ws && c.m_pk != nullptr;
   auto add_gemms = [&](std::vector<GemmJobDev> jobs) {
     const bool own = group < 0;
     if (own) group = npass++;
@@ -400,8 +401,10 @@ StepPlan build_mixed_plan(const CaseDev& c, const MixedOps& ops, int variant) {
 // Largest packed input of the plan's GEMM launches.
 size_t mixed_pack_bytes(const CaseDev& c) {
   MixedOps none;
+  CaseDev t = c;
+  t.m_pk = reinterpret_cast<float*>(16);  // (sizes only: a form that packs)
   size_t m = 0;
-  for (const StepLaunch& L : build_mixed_plan(c, none, 0).launches) {
+  for (const StepLaunch& L : build_mixed_plan(t, none, 0).launches) {
     if (L.kernel != K_PACK) continue;
     size_t b = 0;
     for (const GemmJobDev& j : L.jobs) b += packed_lanes_bytes(j.lanes, j.K);
