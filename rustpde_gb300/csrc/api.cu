@@ -341,8 +341,10 @@ struct FsLanes {
   // mixed form: packed split operators per FS_OP_* (device)
   const float* w[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
   unsigned int* d_status = nullptr;
-  // FP64 transforms as split GEMMs (dense lengths): scratch for kSplitLanesCap
-  // lanes at a time.  It is the handle's, and calls may come from several
+  // Scratch of the split GEMMs (FP64) or of the packed input (mixed) for
+  // work_lanes lanes at a time, made by the first call that uses it and grown up
+  // to kSplitLanesCap lanes (at 512 points 46 and 17 MB): a handle whose calls
+  // take other forms has none.  It is the handle's, and calls may come from several
   // threads and on several streams: the mutex orders the host side, and every
   // call's stream waits for the event of the call before (equal stream handles
   // would not tell: cudaStreamPerThread is one handle for a stream per thread,
@@ -350,6 +352,8 @@ struct FsLanes {
   std::mutex mu;
   SplitWork work;
   void* work_mem = nullptr;
+  int work_lanes = 0;
+  size_t refused = ~size_t(0);  // bytes for which there was no memory
   cudaEvent_t done = nullptr;
   bool used = false;
   ~FsLanes() {
@@ -362,15 +366,39 @@ constexpr int kSplitLanesCap = 4096;
 // on; below, the packing launch costs what it saves.
 constexpr int kPackLanesMinN = 96, kPackLanesMin = 1024;
 
-// The handle's scratch; without the memory for it the calls take the forms that
-// need none.
-static bool lane_scratch(FsLanes* p, size_t bytes) {
-  if (cudaMalloc(&p->work_mem, bytes) != cudaSuccess) {
+// Scratch for up to `lanes` lanes at a time (the handle's mutex held); false
+// where there is no memory for any: the call then takes the form that needs none.
+static bool lane_scratch(FsLanes* p, int lanes) {
+  const int n = p->L.hb.n, want = std::min(kSplitLanesCap, (lanes + kSplitLanes - 1) / kSplitLanes * kSplitLanes);
+  if (want <= p->work_lanes) return true;
+  const bool fp64 = p->precision == RBC_PREC_FP64;
+  const size_t db = (split_dig_bytes(want, split_chunks((n + 1) / 2), split_chunks(n / 2)) + 255) & ~size_t(255);
+  const size_t be = ((size_t)want * 4 + 255) & ~size_t(255), bb = (size_t)want * n * 8;
+  const size_t bytes = fp64 ? db + be + bb : packed_lanes_bytes(want, n);
+  if (bytes >= p->refused) return p->work_lanes > 0;
+  if (p->done == nullptr) cuda_check(cudaEventCreateWithFlags(&p->done, cudaEventDisableTiming), "event");
+  // another thread's capture does not mind: nothing here touches its stream
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  cuda_check(cudaThreadExchangeStreamCaptureMode(&mode), "capture mode");
+  void* mem = nullptr;
+  const cudaError_t e = cudaMalloc(&mem, bytes);
+  if (e == cudaSuccess && p->work_mem != nullptr) cudaFree(p->work_mem);  // waits for the calls that use it
+  cuda_check(cudaThreadExchangeStreamCaptureMode(&mode), "capture mode");
+  if (e != cudaSuccess) {
     (void)cudaGetLastError();
-    p->work_mem = nullptr;
-    return false;
+    p->refused = bytes;
+    return p->work_lanes > 0;
   }
-  cuda_check(cudaEventCreateWithFlags(&p->done, cudaEventDisableTiming), "event");
+  p->work_mem = mem;
+  p->work_lanes = want;
+  if (fp64) {
+    char* q = static_cast<char*>(mem);
+    p->work.dig = reinterpret_cast<unsigned char*>(q);
+    p->work.ex = reinterpret_cast<int*>(q + db);
+    p->work.buf = reinterpret_cast<double*>(q + db + be);
+    p->work.lanes = want;
+    p->work.status = p->d_status;
+  }
   return true;
 }
 
@@ -2372,20 +2400,8 @@ int fs_lanes_create(int base, int n, int precision, FsLanes** out) {
   p->precision = precision;
   build_lanes(p->arena, p->L, base, n);
   p->d_status = static_cast<unsigned int*>(p->arena.alloc(16));
-  if (precision == RBC_PREC_FP64 && lanes_attach_split(p->arena, p->L)) {
-    const size_t db = (split_dig_bytes(kSplitLanesCap, split_chunks((n + 1) / 2), split_chunks(n / 2)) + 255) & ~size_t(255);
-    const size_t be = (size_t)kSplitLanesCap * 4, bb = (size_t)kSplitLanesCap * n * 8;
-    if (lane_scratch(p.get(), db + be + bb)) {
-      char* q = static_cast<char*>(p->work_mem);
-      p->work.dig = reinterpret_cast<unsigned char*>(q);
-      p->work.ex = reinterpret_cast<int*>(q + db);
-      p->work.buf = reinterpret_cast<double*>(q + db + be);
-      p->work.lanes = kSplitLanesCap;
-      p->work.status = p->d_status;
-    }
-  }
+  if (precision == RBC_PREC_FP64) lanes_attach_split(p->arena, p->L);
   if (precision == RBC_PREC_MIXED) {
-    if (n >= kPackLanesMinN) lane_scratch(p.get(), packed_lanes_bytes(kSplitLanesCap, n));
     const HostBasis& hb = p->L.hb;
     LMat S = lm_stencil(hb), P = lm_from_ortho(hb);
     p->w[FS_OP_FORWARD] = upload_split(p->arena, lm_mul(P, lm_cheb_forward(n)));
@@ -2447,7 +2463,7 @@ int fs_lanes_apply(FsLanes* p, int op, const double* d_in, double* d_out, int la
   // captured call does without: its replays are not ordered with other calls on
   // the handle.
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  bool scratch = p->work_mem != nullptr && (fp64 ? lanes_split_pays(p->L, op, lanes) : lanes >= kPackLanesMin);
+  bool scratch = fp64 ? lanes_split_pays(p->L, op, lanes) : p->L.hb.n >= kPackLanesMinN && lanes >= kPackLanesMin;
   if (scratch && (cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone)) {
     (void)cudaGetLastError();
     scratch = false;
@@ -2464,15 +2480,21 @@ int fs_lanes_apply(FsLanes* p, int op, const double* d_in, double* d_out, int la
     if (scratch) j.apk = static_cast<const float*>(p->work_mem);
     cuda_check(launch_lane_gemm_one(j, st), "lane gemm launch");
   };
+  std::unique_lock<std::mutex> lk(p->mu, std::defer_lock);
+  if (scratch) {
+    lk.lock();
+    scratch = lane_scratch(p, lanes);
+    if (!scratch) lk.unlock();
+  }
   if (!scratch) {
     apply(d_in, d_out, lanes);
   } else {
-    std::lock_guard<std::mutex> lk(p->mu);
     if (p->used) cuda_check(cudaStreamWaitEvent(st, p->done, 0), "lane scratch");
-    for (int l = 0; l < lanes; l += kSplitLanesCap)
-      apply(d_in + (size_t)l * il, d_out + (size_t)l * ol, std::min(kSplitLanesCap, lanes - l));
+    for (int l = 0; l < lanes; l += p->work_lanes)
+      apply(d_in + (size_t)l * il, d_out + (size_t)l * ol, std::min(p->work_lanes, lanes - l));
     cuda_check(cudaEventRecord(p->done, st), "lane scratch");
     p->used = true;
+    lk.unlock();
   }
   if (!fp64 && op == FS_OP_HHOLTZ) lanes_fdma(p->L, d_out, lanes, st);
   API_END

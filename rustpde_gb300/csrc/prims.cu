@@ -1342,20 +1342,18 @@ static PassDesc lanes_desc(const LanesDev& L) {
   return d;
 }
 
-bool lanes_attach_split(Arena& a, LanesDev& L) {
-  if (!split_fits(L.cx)) return false;
+void lanes_attach_split(Arena& a, LanesDev& L) {
+  if (!split_fits(L.cx)) return;
   try {
     split_ops(a, L.cx);
   } catch (std::exception& e) {  // no memory for them: the transforms stay inside the passes
     if (std::string(e.what()).find("cudaMalloc") == std::string::npos) throw;
     (void)cudaGetLastError();
     L.cx.sop_b = L.cx.sop_f[0] = L.cx.sop_f[1] = SplitOpDev{};
-    return false;
   }
-  return true;
 }
 bool lanes_split_pays(const LanesDev& L, int op, int lanes) {
-  return (op == LOP_FORWARD || op == LOP_BACKWARD) && split_pays(lanes, L.cx.n);
+  return L.cx.sop_b.w != nullptr && (op == LOP_FORWARD || op == LOP_BACKWARD) && split_pays(lanes, L.cx.n);
 }
 
 void lanes_apply(const LanesDev& L, int op, const double* in, double* out, int lanes, cudaStream_t st,

@@ -200,9 +200,9 @@ void lanes_set_hholtz(Arena& a, LanesDev& L, double c);
 void lane_op_lengths(const LanesDev& L, int op, int* in_len, int* out_len);
 void lanes_apply(const LanesDev& L, int op, const double* in, double* out, int lanes, cudaStream_t st,
                  const SplitWork* work = nullptr);
-// split operators of a dense length (false: none), and whether an application
-// gains by them
-bool lanes_attach_split(Arena& a, LanesDev& L);
+// split operators of a dense length, and whether there are any and an
+// application gains by them
+void lanes_attach_split(Arena& a, LanesDev& L);
 bool lanes_split_pays(const LanesDev& L, int op, int lanes);
 // the banded part of the HholtzAdi solve alone: x (m per lane) solved in place
 void lanes_fdma(const LanesDev& L, double* x, int lanes, cudaStream_t st);

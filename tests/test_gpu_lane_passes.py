@@ -276,3 +276,31 @@ def test_tables_of_sizes_no_longer_in_use_are_given_back(R):
     for n in range(482, 522, 2):  # 20 sizes; 15 MB of tables each
         use(n)
     assert before - free() <= 80 * 2**20
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_lane_scratch_is_made_by_the_calls_that_use_it(R, precision):
+    torch = pytest.importorskip("torch")
+
+    def free():
+        R._check(R.lib().rbc_device_synchronize())
+        return torch.cuda.mem_get_info()[0]
+
+    n, ops = 500, (R.OP_FORWARD, R.OP_BACKWARD)
+    first = R.Lanes(R.Base(1, n), precision)  # operators that handles share, and kernels
+    rng = np.random.default_rng(12)
+    x = {op: rng.standard_normal((5000, n if op == R.OP_FORWARD else first.m)) for op in ops}
+    ref = {op: first.apply(op, x[op]) for op in ops}
+    before = free()
+    handles = [R.Lanes(R.Base(1, n), precision) for _ in range(8)]
+    for L in handles:  # too few lanes for it
+        L.apply(R.OP_FORWARD, x[R.OP_FORWARD][:8])
+    # tables of a handle: the dense transforms (2 MB), mixed the five operators of 4 n^2 bytes in two parts
+    assert before - free() <= 8 * (16 if precision else 6) * 2**20
+    for L, lanes in zip(handles, (1100, 1025, 4096, 4097, 5000, 3000, 128, 2000)):
+        for k in (lanes, 5000, lanes):  # grown, then used for fewer lanes
+            for op in ops:
+                got = L.apply(op, x[op][:k])
+                if k >= 1024:  # (fewer lanes may take the pass: another rounding)
+                    np.testing.assert_array_equal(got, ref[op][:k])
+        assert L.status() == 0
