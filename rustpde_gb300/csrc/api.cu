@@ -506,10 +506,11 @@ void build_case(RbcCase* c, bool with_graph = true, char* state_region = nullptr
   const int xk_o = per ? FOURIER : CHEB;
   const int xk_p = per ? FOURIER : CN;
   // A batch's mixed case of butterfly sizes may run the FP64 plan (the transform
-  // choice) and has everything of an FP64 case; else the mixed form keeps its blocks.
+  // choice), with split GEMMs where they pay.  Its scan blocks are the mixed form's
+  // all the same: they are part of the tables that the mixed plan reads too.
   const bool fp64_plan = p.precision != RBC_PREC_MIXED ||
                          (c->batch != nullptr && is_pow2(ny - 1) && (per || is_pow2(nx - 1)));
-  const bool odd = fp64_plan;
+  const bool odd = p.precision != RBC_PREC_MIXED;
   build_space(A, c->sp_u, xk_u, nx, CD, ny, odd);
   build_space(A, c->sp_t, xk_t, nx, CD, ny, odd);
   build_space(A, c->sp_p0, xk_o, nx, CHEB, ny, odd);

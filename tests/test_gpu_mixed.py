@@ -252,3 +252,21 @@ def test_mixed_batch_one_call_equals_single_steps(R, monkeypatch):
         assert bs[0].cases[i].get_time() == bs[1].cases[i].get_time()
         for f in FIELDS:
             assert np.array_equal(bs[0].cases[i].get(f), bs[1].cases[i].get(f)), (i, f)
+
+
+@pytest.mark.parametrize("nx,ny,kind", [(64, 257, 2), (257, 129, 0), (257, 257, 1)])
+def test_batch_in_the_single_cases_forms_has_its_bits(R, monkeypatch, nx, ny, kind):
+    # lengths 2^p + 1 with scans of 128 elements a chain: a batch may run them in
+    # FP64, and the mixed form of such a case is still the single case's
+    p = (nx, ny, 1e6, 1.0, 2e-3, 1.0, kind)
+    monkeypatch.setenv("RBC_BATCH_FORM", "0;0;0")
+    b = R.Batch([p], precision=R.PREC_MIXED)
+    s = R.Navier2D(*p, precision=R.PREC_MIXED)
+    for c in (b.cases[0], s):
+        c.set_velocity(0.2, 1, 1)
+        c.set_temperature(0.2, 1, 2)
+    b.update(4)
+    b.synchronize()
+    s.update(4)
+    for f in (R.TEMP, R.UX, R.UY, R.PRES, R.PSEUDO_PRES):
+        np.testing.assert_array_equal(b.cases[0].get(f), s.get(f))
