@@ -76,12 +76,14 @@ def test_case_without_room_for_its_digits(R, batch):
         assert one.status() == 0
         return [one.get(f) for f in (R.TEMP, R.UX, R.UY)]
 
+    run(*make())  # kernels and graphs loaded
+    gc.collect()
+    before = _free(torch, R)
     c, one = make()
     want = run(c, one)
-    before = _free(torch, R)
+    full = before - _free(torch, R)
     del c, one
     gc.collect()
-    full = _free(torch, R) - before
     # the digits, the y- and the x-transformed fields: 6 and 8 values per point and more
     scratch = 8 * 14 * 400 * 400
     with _leave(torch, R, full - scratch // 2):
