@@ -363,7 +363,11 @@ struct FsLanes {
 };
 constexpr int kSplitLanesCap = 4096;
 // The mixed form packs the lanes of a GEMM first (lane_gemm.cu) from these sizes
-// on; below, the packing launch costs what it saves.
+// on.  One forward transform, us, packed | not, at 1024 lanes: 64 points 16.4 |
+// 12.3, 96 16.4 | 16.4, 128 16.4 | 20.5, 192 18.5 | 26.7, 256 20.5 | 32.8, 512
+// 24.6 | 57.3; from 128 to 4096 lanes the two hardly change but at 512 points
+// (4096 lanes: 34.9 | 79.0).  The length decides; the lanes' line keeps calls
+// of few lanes free of scratch.
 constexpr int kPackLanesMinN = 96, kPackLanesMin = 1024;
 
 // Scratch for up to `lanes` lanes at a time (the handle's mutex held); false

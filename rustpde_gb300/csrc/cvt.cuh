@@ -1,8 +1,8 @@
-// cvt.cuh -- FP64 <-> FP32 conversions in integer operations.
+// cvt.cuh -- FP64 -> FP32 conversion in integer operations.
 //
 // This GPU converts between FP64 and FP32 at its FP64 rate, two per clock and
 // SM; ten integer operations run at a hundred per clock.  Results are those of
-// the conversions (round to nearest even); what falls outside FP32's normal
+// the conversion (round to nearest even); what falls outside FP32's normal
 // range, other than zeros, goes through the instruction.
 #pragma once
 #include <cuda_runtime.h>
@@ -20,13 +20,6 @@ __device__ __forceinline__ float to_f32(double d) {
   }
   if (e <= 872u) return __uint_as_float(s);  // below half of the smallest subnormal
   return (float)d;
-}
-
-__device__ __forceinline__ double to_f64(float f) {
-  const unsigned b = __float_as_uint(f), e = (b >> 23) & 0xffu, s = b & 0x80000000u;
-  if (e - 1u < 254u) return __hiloint2double((int)(s | ((e + 896u) << 20) | ((b >> 3) & 0xfffffu)), (int)(b << 29));
-  if ((b << 1) == 0) return __hiloint2double((int)s, 0);
-  return (double)f;
 }
 
 }  // namespace dev

@@ -1167,10 +1167,8 @@ cudaError_t launch_lane_gemm(const GemmJobDev* jobs, const int4* tiles, int ntil
   if (form == 1) {
     if (max_nt > 64) return cudaErrorInvalidValue;
     return launch_pdl(dev::k_lane_gemm_ws, ntiles_total, kGemmThreads, gemm_ws_smem_bytes(max_nt), st, jobs, tiles);
-  } else {
-    return launch_pdl(dev::k_lane_gemm, ntiles_total, kGemmThreads, gemm_smem_bytes(max_nt), st, jobs, tiles);
   }
-  return cudaGetLastError();
+  return launch_pdl(dev::k_lane_gemm, ntiles_total, kGemmThreads, gemm_smem_bytes(max_nt), st, jobs, tiles);
 }
 
 }  // namespace rbc

@@ -197,7 +197,10 @@ size_t smem_per_x(const CaseDev& c) {
 // in shared memory: a pass then has one CTA per SM, and a factor loaded inside a
 // recurrence costs its L2 latency (box 129^2: x2 25 -> 14 us, y3 28 -> 15 us).
 // Longer lanes leave several CTAs per SM to cover it, and the staging would cost
-// one of them (box 513^2).
+// one of them.  Box step, us, staged | not: 129^2 138.4 | 139.3, 200^2 184.7 |
+// 186.6, 264^2 228.1 | 229.7, 300^2 242.4 | 245.4, 320^2 258.2 | 259.2, 360^2
+// 296.9 | 298.8, 450^2 369.1 | 371.2, 513^2 497.0 | 474.7.  The line lies where
+// the gain has become half a percent.
 __host__ __device__ inline bool stage_factors(int m) { return m <= 320; }
 
 // stage the factors of row `row` of a per-row banded solver into shared memory
@@ -1203,7 +1206,6 @@ cudaError_t launch_step_kernel(int kernel, int nblocks, size_t smem, cudaStream_
       return launch_step_split_kernel(kernel, nblocks, smem, s, cases, work);
     default: return launch_mixed_kernel(kernel, nblocks, smem, s, cases, work);
   }
-  return cudaGetLastError();
 }
 
 }  // namespace rbc

@@ -1066,7 +1066,6 @@ cudaError_t launch_lane_kernel(int kernel, int nblocks, cudaStream_t s, const Ca
     case K_LP_PER_Y2F: return launch_pdl(dev::k_lp_per_y2f, g, b, 0, s, cases, work);
     default: return cudaErrorInvalidValue;
   }
-  return cudaGetLastError();
 }
 
 }  // namespace rbc

@@ -452,7 +452,6 @@ cudaError_t launch_mixed_kernel(int kernel, int nblocks, size_t smem, cudaStream
     case K_BOX_PROD_MIXED: return launch_pdl(dev::k_box_prod_mixed, nblocks, 256, 0, s, cases, work);
     default: return launch_lane_kernel(kernel, nblocks, s, cases, work);
   }
-  return cudaGetLastError();
 }
 
 // The kernel whose arrays a form of the same pass moves (-1: counted with another

@@ -521,7 +521,6 @@ cudaError_t launch_step_split_kernel(int kernel, int nblocks, size_t smem, cudaS
     case K_SPL_Q: return launch_pdl(dev::k_spl_q, g, b, smem, s, cases, work);
     default: return cudaErrorInvalidValue;
   }
-  return cudaGetLastError();
 }
 
 }  // namespace rbc

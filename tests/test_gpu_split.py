@@ -160,3 +160,45 @@ def test_fp64_step_that_gives_up_does_not_look_well(R, kind):
     for f in (R.TEMP, R.UX, R.UY):
         assert np.isnan(c.get(f)).any()
     assert c.exit()
+
+
+def _values(n):
+    """Chebyshev coefficients -> values, and back, in extended precision."""
+    N = n - 1
+    j = np.arange(n)
+    pi = np.longdouble("3.14159265358979323846264338327950288")
+    cos = np.cos(pi * (np.outer(j, j) % (2 * N)).astype(np.longdouble) / N)
+    sign = np.where(j % 2, -1, 1).astype(np.longdouble)
+    end = np.where((j == 0) | (j == N), 0.5, 1.0).astype(np.longdouble)
+    return cos * sign[None, :], cos * (2 / np.longdouble(N) * sign * end)[:, None] * end[None, :]
+
+
+@pytest.mark.parametrize("n", [49, 130, 263, 640])
+def test_digit_products_of_uneven_lanes(R, n):
+    # lanes over 300 decades, near both ends of the exponent range, subnormal,
+    # with values that differ in their last bit, with the largest digits.  The
+    # bound is a dot product's in FP64, n 2^-53 sum |w x|, plus the fixed point of
+    # a lane and of the operator against their largest values, n 2^-54 |w| |x|
+    lanes = -(-4_000_000 // (n * n))
+    rng = np.random.default_rng(n)
+    k = np.arange(n)
+    x = rng.standard_normal((lanes, n))
+    x[1::9] *= 10.0 ** (-300.0 * k / n)
+    x[2::9] *= 1e300
+    x[3::9] *= 1e-310
+    x[4::9] = 1.0 + k * 2.0**-52
+    x[5::9] = np.where(k % 2, -1, 1) * (2.0 - 2.0**-52)
+    x[6::9] = np.where(k == n // 3, np.pi, 0.0)
+    x[7::9] = np.where(rng.integers(0, 2, n), 1, -1) * np.ldexp(float(0x10808080808080), -52)
+    x[8::9] *= np.where(k % 2, 1e10, 1e-6)
+    L = R.Lanes(R.Base(0, n))
+    B, F = _values(n)
+    X = x.astype(np.longdouble)
+    for op, M in ((R.OP_BACKWARD, B), (R.OP_FORWARD, F)):
+        got = L.apply(op, x)
+        want = X @ M.T
+        bound = n * 2.0**-53 * (np.abs(X) @ np.abs(M).T) + n * 2.0**-54 * np.abs(M).max() * np.abs(X).max(axis=1)[:, None]
+        worst = (np.abs(got - want) / (bound + 2.0**-1073)).max(axis=1)
+        assert worst.max() <= 1, (op, worst.argmax() % 9, float(worst.max()))
+        print(n, op, [float(worst[r::9].max()) for r in range(9)])
+    assert L.status() == 0
