@@ -285,13 +285,20 @@ __device__ __forceinline__ void a_store(const AChunk<T, NTHR>& a, const ATile<T,
 #pragma unroll
   for (int it = 0; it < kItems; it++) {
     float4 hi, lo;
-    float x;
-    // lo is rounded to TF32 here: left to the tensor core it would be
-    // truncated, a bias that accumulates along K
-    x = lane_f32(a.v[it][0]); hi.x = tf32_rna(x); lo.x = tf32_rna(x - hi.x);
-    x = lane_f32(a.v[it][1]); hi.y = tf32_rna(x); lo.y = tf32_rna(x - hi.y);
-    x = lane_f32(a.v[it][2]); hi.z = tf32_rna(x); lo.z = tf32_rna(x - hi.z);
-    x = lane_f32(a.v[it][3]); hi.w = tf32_rna(x); lo.w = tf32_rna(x - hi.w);
+    if (t.src[it] == nullptr) {
+      // a lane past the last: zeros, without the conversions (in integer
+      // operations a zero takes longer than a value: one lane of 127, 16.4 us with
+      // FP64 conversions, 18.4 with integer ones, 14.4 with this)
+      hi = lo = make_float4(0.f, 0.f, 0.f, 0.f);
+    } else {
+      float x;
+      // lo is rounded to TF32 here: left to the tensor core it would be
+      // truncated, a bias that accumulates along K
+      x = lane_f32(a.v[it][0]); hi.x = tf32_rna(x); lo.x = tf32_rna(x - hi.x);
+      x = lane_f32(a.v[it][1]); hi.y = tf32_rna(x); lo.y = tf32_rna(x - hi.y);
+      x = lane_f32(a.v[it][2]); hi.z = tf32_rna(x); lo.z = tf32_rna(x - hi.z);
+      x = lane_f32(a.v[it][3]); hi.w = tf32_rna(x); lo.w = tf32_rna(x - hi.w);
+    }
     const int off = t.soff0 + it * t.sstep;
     *reinterpret_cast<float4*>(Ahi + off) = hi;
     *reinterpret_cast<float4*>(Alo + off) = lo;

@@ -304,3 +304,14 @@ def test_lane_scratch_is_made_by_the_calls_that_use_it(R, precision):
                 if k >= 1024:  # (fewer lanes may take the pass: another rounding)
                     np.testing.assert_array_equal(got, ref[op][:k])
         assert L.status() == 0
+
+
+@pytest.mark.parametrize("n", [20, 127, 200])
+def test_mixed_lanes_in_any_number_have_the_same_bits(R, n):
+    # lane blocks of 128 with rows past the last lane, unpacked and packed
+    L = R.Lanes(R.Base(1, n), R.PREC_MIXED)
+    x = np.random.default_rng(n).standard_normal((1200, n))
+    ref = L.apply(R.OP_FORWARD, x)
+    for lanes in (1, 2, 31, 127, 128, 129, 1023, 1025):
+        np.testing.assert_array_equal(L.apply(R.OP_FORWARD, x[:lanes]), ref[:lanes])
+    assert L.status() == 0
