@@ -343,8 +343,7 @@ struct FsLanes {
   unsigned int* d_status = nullptr;
   // Scratch of the split GEMMs (FP64) or of the packed input (mixed) for
   // work_lanes lanes at a time, made by the first call that uses it and grown up
-  // to kSplitLanesCap lanes (at 512 points 46 and 17 MB): a handle whose calls
-  // take other forms has none.  It is the handle's, and calls may come from several
+  // to lane_cap lanes: a handle whose calls take other forms has none.  It is the handle's, and calls may come from several
   // threads and on several streams: the mutex orders the host side, and every
   // call's stream waits for the event of the call before (equal stream handles
   // would not tell: cudaStreamPerThread is one handle for a stream per thread,
@@ -361,7 +360,18 @@ struct FsLanes {
     if (work_mem) cudaFree(work_mem);
   }
 };
+// Lanes at a time.  FP64 lanes have 36 bytes of scratch a value, 4.5 times their
+// input: 4096 lanes (46 MB at 512 points) fill the SMs.  Packed lanes have 8, as
+// much as their input, and their two launches are short, so that parts of 4096
+// took longer than the whole in the form without: 20000 lanes, us, without |
+// parts of 4096 | at once: 96 points 34.8 | 82.0 | 28.8, 128 49.3 | 82.0 | 30.8,
+// 256 133 | 113 | 59.5, 512 386 | 178 | 133; 100000 lanes of 128 154 | 410 | 103.
 constexpr int kSplitLanesCap = 4096;
+constexpr size_t kPackLanesCapBytes = 128u << 20;
+static int lane_cap(const FsLanes& p) {
+  if (p.precision == RBC_PREC_FP64) return kSplitLanesCap;
+  return std::max<int>(kSplitLanesCap, (int)(kPackLanesCapBytes / packed_lanes_bytes(kGemmLanes, p.L.hb.n)) * kGemmLanes);
+}
 // The mixed form packs the lanes of a GEMM first (lane_gemm.cu) from these sizes
 // on.  One forward transform, us, packed | not, at 1024 lanes: 64 points 16.4 |
 // 12.3, 96 16.4 | 16.4, 128 16.4 | 20.5, 192 18.5 | 26.7, 256 20.5 | 32.8, 512
@@ -373,7 +383,8 @@ constexpr int kPackLanesMinN = 96, kPackLanesMin = 1024;
 // Scratch for up to `lanes` lanes at a time (the handle's mutex held); false
 // where there is no memory for any: the call then takes the form that needs none.
 static bool lane_scratch(FsLanes* p, int lanes) {
-  const int n = p->L.hb.n, want = std::min(kSplitLanesCap, (lanes + kSplitLanes - 1) / kSplitLanes * kSplitLanes);
+  const int n = p->L.hb.n, cap = lane_cap(*p);
+  const int want = lanes >= cap ? cap : (lanes + kSplitLanes - 1) / kSplitLanes * kSplitLanes;
   if (want <= p->work_lanes) return true;
   const bool fp64 = p->precision == RBC_PREC_FP64;
   const size_t db = (split_dig_bytes(want, split_chunks((n + 1) / 2), split_chunks(n / 2)) + 255) & ~size_t(255);
