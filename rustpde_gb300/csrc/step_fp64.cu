@@ -234,12 +234,18 @@ __device__ FdmaDev stage_fdma_row(const FdmaDev& f, int row, double* dst, int ti
 //   CONV_MIXED  m_cv, transformed (the mixed form's GEMM), without the linear
 //               boundary part (CaseDev::m_bclin)
 //   CONV_FULL   m_cv, transformed and complete (the split GEMMs)
-// Registers: CONV_Q is held to 64 (four CTAs per SM): at 80 the 457 to 608 rows of
-// a small batch took a second wave (8 cases of 128 x 65: 76 us against 54).  The
-// other two serve larger rows, where the spills cost more (512 x 257: 2 us).
+// Registers (BOUND: CTAs per SM they have to allow): left to itself the compiler
+// takes 118, two CTAs of 256 threads per SM.  That is the faster for one case,
+// whose rows are about two per SM, and for rows whose shared memory allows no
+// more (y2_many).  Many shorter rows want four CTAs (64 registers, some spills),
+// or seven of 128 threads (72).  us per step, 118 | 64 registers: one case of 512 x
+// 257 171.9 | 173.6, 600 x 300 213 | 218, four of 512 x 257 385 | 396; batches of
+// 16 x (200 x 150) 506 | 420, 32 x (128 x 128) 602 | 509; mixed, CTAs of 256 threads:
+// 64 x (128 x 65) 568 | 391; of 128 threads, 118 | 72: 32 x (128 x 65) 203 | 169.
+// CONV_Q is always held to 64 (8 cases of 128 x 65: 76 us at 80 registers, 54).
 enum { CONV_Q = 0, CONV_MIXED = 1, CONV_FULL = 2 };
-template <int CONV>
-__global__ void __launch_bounds__(256, CONV == CONV_Q ? 4 : 1) k_per_y2(const CaseDev* __restrict__ cases, const int4* __restrict__ work) {
+template <int CONV, int NT = 256, int BOUND = 1>
+__global__ void __launch_bounds__(NT, BOUND) k_per_y2(const CaseDev* __restrict__ cases, const int4* __restrict__ work) {
   pdl_enter();
   int4 w = work[blockIdx.x];
   const CaseDev& c = cases[w.x];
@@ -1085,9 +1091,12 @@ cudaError_t configure_step_kernels() {
   SET_ATTR(dev::k_y1<double>);
   SET_ATTR(dev::k_y1<double2>);
   SET_ATTR(dev::k_per_x);
-  SET_ATTR(dev::k_per_y2<dev::CONV_Q>);
-  SET_ATTR(dev::k_per_y2<dev::CONV_FULL>);
-  SET_ATTR(dev::k_per_y2<dev::CONV_MIXED>);
+  SET_ATTR((dev::k_per_y2<dev::CONV_Q, 256, 4>));
+  SET_ATTR((dev::k_per_y2<dev::CONV_FULL, 256, 1>));
+  SET_ATTR((dev::k_per_y2<dev::CONV_FULL, 256, 4>));
+  SET_ATTR((dev::k_per_y2<dev::CONV_MIXED, 256, 1>));
+  SET_ATTR((dev::k_per_y2<dev::CONV_MIXED, 256, 4>));
+  SET_ATTR((dev::k_per_y2<dev::CONV_MIXED, 128, 7>));
   SET_ATTR(dev::k_per_y2a);
   SET_ATTR(dev::k_per_y2b);
   SET_ATTR(dev::k_box_x1);
@@ -1170,6 +1179,10 @@ void drop_empty(StepPlan& p) {
       p.launches.end());
 }
 
+// Whether k_per_y2 takes few registers: more rows than two per SM, and shared
+// memory for a third CTA there.
+static bool y2_many(int nblocks, size_t smem) { return nblocks > 2 * 152 && 3 * (smem + 1024) <= smem_limit() + 1024; }
+
 cudaError_t launch_step_kernel(int kernel, int nblocks, size_t smem, cudaStream_t s, const CaseDev* cases,
                                const int4* work) {
   dim3 g(nblocks), b(256);
@@ -1177,14 +1190,18 @@ cudaError_t launch_step_kernel(int kernel, int nblocks, size_t smem, cudaStream_
     case K_Y1_C: return launch_pdl(dev::k_y1<double2>, g, b, smem, s, cases, work);
     case K_Y1_R: return launch_pdl(dev::k_y1<double>, g, b, smem, s, cases, work);
     case K_PER_X: return launch_pdl(dev::k_per_x, g, b, smem, s, cases, work);
-    case K_PER_Y2: return launch_pdl(dev::k_per_y2<dev::CONV_Q>, g, b, smem, s, cases, work);
-    case K_PER_Y2_PRE: return launch_pdl(dev::k_per_y2<dev::CONV_MIXED>, g, b, smem, s, cases, work);
+    case K_PER_Y2: return launch_pdl(dev::k_per_y2<dev::CONV_Q, 256, 4>, g, b, smem, s, cases, work);
+    case K_PER_Y2_PRE:
+      if (y2_many(nblocks, smem)) return launch_pdl(dev::k_per_y2<dev::CONV_MIXED, 256, 4>, g, b, smem, s, cases, work);
+      return launch_pdl(dev::k_per_y2<dev::CONV_MIXED, 256, 1>, g, b, smem, s, cases, work);
     case K_PER_Y2A: return launch_pdl(dev::k_per_y2a, g, b, smem, s, cases, work);
     case K_PER_Y2B: return launch_pdl(dev::k_per_y2b, g, b, smem, s, cases, work);
     case K_BOX_X1: return launch_pdl(dev::k_box_x1, g, b, smem, s, cases, work);
     case K_BOX_Y2: return launch_pdl(dev::k_box_y2<dev::CONV_Q>, g, b, smem, s, cases, work);
     case K_BOX_Y2_PRE: return launch_pdl(dev::k_box_y2<dev::CONV_MIXED>, g, b, smem, s, cases, work);
-    case K_PER_Y2_CV: return launch_pdl(dev::k_per_y2<dev::CONV_FULL>, g, b, smem, s, cases, work);
+    case K_PER_Y2_CV:
+      if (y2_many(nblocks, smem)) return launch_pdl(dev::k_per_y2<dev::CONV_FULL, 256, 4>, g, b, smem, s, cases, work);
+      return launch_pdl(dev::k_per_y2<dev::CONV_FULL, 256, 1>, g, b, smem, s, cases, work);
     case K_BOX_Y2_CV: return launch_pdl(dev::k_box_y2<dev::CONV_FULL>, g, b, smem, s, cases, work);
     case K_SPL_X3: return launch_pdl(dev::k_box_x3<dev::EIG_SPLIT>, g, b, smem, s, cases, work);
     case K_SPL_W: return launch_pdl(dev::k_spl_w, g, b, smem, s, cases, work);
@@ -1198,7 +1215,7 @@ cudaError_t launch_step_kernel(int kernel, int nblocks, size_t smem, cudaStream_
     case K_BOX_X4: return launch_pdl(dev::k_box_x4<false>, g, b, smem, s, cases, work);
     case K_BOX_X4_MIX: return launch_pdl(dev::k_box_x4<true>, g, b, smem, s, cases, work);
     case K_BOX_Y5: return launch_pdl(dev::k_box_y5, g, b, smem, s, cases, work);
-    case K_PER_Y2_PRE_T128: return launch_pdl(dev::k_per_y2<dev::CONV_MIXED>, g, dim3(128), smem, s, cases, work);
+    case K_PER_Y2_PRE_T128: return launch_pdl(dev::k_per_y2<dev::CONV_MIXED, 128, 7>, g, dim3(128), smem, s, cases, work);
     case K_BOX_Y2_PRE_T128: return launch_pdl(dev::k_box_y2<dev::CONV_MIXED>, g, dim3(128), smem, s, cases, work);
     case K_BOX_X3_MIX_T128: return launch_pdl(dev::k_box_x3<dev::EIG_MIXED>, g, dim3(128), smem, s, cases, work);
     case K_BOX_Y5_T128: return launch_pdl(dev::k_box_y5, g, dim3(128), smem, s, cases, work);

@@ -111,3 +111,23 @@ def test_step_io_equals_set_step_get(R, precision):
     bs[0].update(1)
     bs[0].get_state_all(ref.array)
     assert np.array_equal(ref.array, out.array)
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_many_rows_have_the_single_cases_bits(R, monkeypatch, precision):
+    # 408 rows in the periodic y pass: more than two per SM, which take another
+    # compilation of the pass than one case's 51
+    p = (100, 96, 1e5, 1.0, 2e-3, 1.0, 2)
+    if precision:
+        monkeypatch.setenv("RBC_BATCH_FORM", "0;0;0")
+    b = R.Batch([p] * 8, precision=precision)
+    s = R.Navier2D(*p, precision=precision)
+    for c in list(b.cases) + [s]:
+        c.set_velocity(0.2, 1, 1)
+        c.set_temperature(0.2, 1, 2)
+    b.update(3)
+    b.synchronize()
+    s.update(3)
+    for c in b.cases:
+        for f in (R.TEMP, R.UX, R.UY, R.PRES, R.PSEUDO_PRES):
+            np.testing.assert_array_equal(c.get(f), s.get(f))
