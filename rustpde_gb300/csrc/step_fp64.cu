@@ -235,14 +235,17 @@ __device__ FdmaDev stage_fdma_row(const FdmaDev& f, int row, double* dst, int ti
 //               boundary part (CaseDev::m_bclin)
 //   CONV_FULL   m_cv, transformed and complete (the split GEMMs)
 // Registers (BOUND: CTAs per SM they have to allow): left to itself the compiler
-// takes 118, two CTAs of 256 threads per SM.  That is the faster for one case,
-// whose rows are about two per SM, and for rows whose shared memory allows no
-// more (y2_many).  Many shorter rows want four CTAs (64 registers, some spills),
-// or seven of 128 threads (72).  us per step, 118 | 64 registers: one case of 512 x
-// 257 171.9 | 173.6, 600 x 300 213 | 218, four of 512 x 257 385 | 396; batches of
-// 16 x (200 x 150) 506 | 420, 32 x (128 x 128) 602 | 509; mixed, CTAs of 256 threads:
-// 64 x (128 x 65) 568 | 391; of 128 threads, 118 | 72: 32 x (128 x 65) 203 | 169.
-// CONV_Q is always held to 64 (8 cases of 128 x 65: 76 us at 80 registers, 54).
+// takes 118, so that two CTAs of 256 threads fill an SM.  One case, with about two
+// rows per SM, is fastest so.  The rows of a batch want four CTAs (64 registers,
+// some spills), or three (80, none) where their shared memory allows only two;
+// and the other group's passes, on their own branch of the graph, need registers
+// beside them: at 118 a batch of both kinds took longer than its groups one after
+// the other.  us per step, 118 | held: one case of 512 x 257 171.9 | 172.6 (80), 600 x
+// 300 213 | 217 (80); four of 512 x 257, mixed 385 | 393 (80); 16 x (200 x 150)
+// 506 | 420 (64), 32 x (128 x 128) 602 | 509 (64); mixed 64 x (128 x 65) 568 | 391 (64);
+// mixed ensembles of 48, 64 and 128 cases 1248 | 985, 1505 | 1210, 2189 | 1929 (80).  The
+// CTAs of 128 threads: 32 x (128 x 65) 203 | 169 (72).  CONV_Q is always held to 64 (8
+// cases of 128 x 65: 76 us at 80 registers, 54).
 enum { CONV_Q = 0, CONV_MIXED = 1, CONV_FULL = 2 };
 template <int CONV, int NT = 256, int BOUND = 1>
 __global__ void __launch_bounds__(NT, BOUND) k_per_y2(const CaseDev* __restrict__ cases, const int4* __restrict__ work) {
@@ -1093,8 +1096,10 @@ cudaError_t configure_step_kernels() {
   SET_ATTR(dev::k_per_x);
   SET_ATTR((dev::k_per_y2<dev::CONV_Q, 256, 4>));
   SET_ATTR((dev::k_per_y2<dev::CONV_FULL, 256, 1>));
+  SET_ATTR((dev::k_per_y2<dev::CONV_FULL, 256, 3>));
   SET_ATTR((dev::k_per_y2<dev::CONV_FULL, 256, 4>));
   SET_ATTR((dev::k_per_y2<dev::CONV_MIXED, 256, 1>));
+  SET_ATTR((dev::k_per_y2<dev::CONV_MIXED, 256, 3>));
   SET_ATTR((dev::k_per_y2<dev::CONV_MIXED, 256, 4>));
   SET_ATTR((dev::k_per_y2<dev::CONV_MIXED, 128, 7>));
   SET_ATTR(dev::k_per_y2a);
@@ -1179,9 +1184,19 @@ void drop_empty(StepPlan& p) {
       p.launches.end());
 }
 
-// Whether k_per_y2 takes few registers: more rows than two per SM, and shared
-// memory for a third CTA there.
-static bool y2_many(int nblocks, size_t smem) { return nblocks > 2 * 152 && 3 * (smem + 1024) <= smem_limit() + 1024; }
+// CTAs per SM that k_per_y2's registers have to allow in a launch of so many rows
+static int y2_bound(int rows, size_t smem) {
+  if (rows <= 2 * 152) return 1;
+  return 3 * (smem + 1024) <= smem_limit() + 1024 ? 4 : 3;  // (1 KB of a CTA's shared memory is the system's)
+}
+template <int CONV>
+static cudaError_t launch_per_y2(int rows, size_t smem, cudaStream_t s, const CaseDev* cases, const int4* work) {
+  switch (y2_bound(rows, smem)) {
+    case 4: return launch_pdl(dev::k_per_y2<CONV, 256, 4>, rows, 256, smem, s, cases, work);
+    case 3: return launch_pdl(dev::k_per_y2<CONV, 256, 3>, rows, 256, smem, s, cases, work);
+    default: return launch_pdl(dev::k_per_y2<CONV, 256, 1>, rows, 256, smem, s, cases, work);
+  }
+}
 
 cudaError_t launch_step_kernel(int kernel, int nblocks, size_t smem, cudaStream_t s, const CaseDev* cases,
                                const int4* work) {
@@ -1191,17 +1206,13 @@ cudaError_t launch_step_kernel(int kernel, int nblocks, size_t smem, cudaStream_
     case K_Y1_R: return launch_pdl(dev::k_y1<double>, g, b, smem, s, cases, work);
     case K_PER_X: return launch_pdl(dev::k_per_x, g, b, smem, s, cases, work);
     case K_PER_Y2: return launch_pdl(dev::k_per_y2<dev::CONV_Q, 256, 4>, g, b, smem, s, cases, work);
-    case K_PER_Y2_PRE:
-      if (y2_many(nblocks, smem)) return launch_pdl(dev::k_per_y2<dev::CONV_MIXED, 256, 4>, g, b, smem, s, cases, work);
-      return launch_pdl(dev::k_per_y2<dev::CONV_MIXED, 256, 1>, g, b, smem, s, cases, work);
+    case K_PER_Y2_PRE: return launch_per_y2<dev::CONV_MIXED>(nblocks, smem, s, cases, work);
     case K_PER_Y2A: return launch_pdl(dev::k_per_y2a, g, b, smem, s, cases, work);
     case K_PER_Y2B: return launch_pdl(dev::k_per_y2b, g, b, smem, s, cases, work);
     case K_BOX_X1: return launch_pdl(dev::k_box_x1, g, b, smem, s, cases, work);
     case K_BOX_Y2: return launch_pdl(dev::k_box_y2<dev::CONV_Q>, g, b, smem, s, cases, work);
     case K_BOX_Y2_PRE: return launch_pdl(dev::k_box_y2<dev::CONV_MIXED>, g, b, smem, s, cases, work);
-    case K_PER_Y2_CV:
-      if (y2_many(nblocks, smem)) return launch_pdl(dev::k_per_y2<dev::CONV_FULL, 256, 4>, g, b, smem, s, cases, work);
-      return launch_pdl(dev::k_per_y2<dev::CONV_FULL, 256, 1>, g, b, smem, s, cases, work);
+    case K_PER_Y2_CV: return launch_per_y2<dev::CONV_FULL>(nblocks, smem, s, cases, work);
     case K_BOX_Y2_CV: return launch_pdl(dev::k_box_y2<dev::CONV_FULL>, g, b, smem, s, cases, work);
     case K_SPL_X3: return launch_pdl(dev::k_box_x3<dev::EIG_SPLIT>, g, b, smem, s, cases, work);
     case K_SPL_W: return launch_pdl(dev::k_spl_w, g, b, smem, s, cases, work);
