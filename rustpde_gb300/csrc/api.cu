@@ -1797,12 +1797,16 @@ static RbcBatch* make_batch(const RbcParams* params, int ncases, bool spare) {
         if (t < t_best_alt) {
           t_best_alt = t;
           best_alt_kernel = ks[0];
-          // the unpacked GEMM forms (4, 5) are timed but only RBC_BATCH_FORM
-          // takes them: alone one may lead by 10 % at a short K, in the whole
-          // step the packed form led everywhere (ms, packed | 4 | 5: 256-case
-          // ensemble 2.97 | 3.19 | 3.21, 8 cases 0.166 | 0.172 | 0.178, one
-          // 512 x 512 box 0.49 | 0.62 | 0.58)
-          if (t < t_base && a < 3) best = (int)a;
+          // GEMMs without packed input: 128-output tiles (4) where they lead by a
+          // tenth, which is groups of many small cases, whose short lanes leave a
+          // packing launch nothing to save.  (Alone a form leads by more than in the
+          // step, where launches overlap.)  us per step, packed | 4: 256 boxes of 24^2
+          // 235 | 199, 200 of 32^2 262 | 225, 64 of 64^2 313 | 304, 16 of 128^2 375 | 377,
+          // 64 periodic of 64^2 156 | 158, 256-case ensemble 2.97 | 3.19 ms.  The
+          // warp-specialised form (5) led nowhere (207, 232, 315, 377, 166 us, 3.21 ms):
+          // only RBC_BATCH_FORM takes it.
+          const float line = a < 3 ? t_base : a == 3 ? 0.9f * t_base : 0.f;
+          if (t < line) best = (int)a;
         }
       }
       if (t_base >= 0) {
