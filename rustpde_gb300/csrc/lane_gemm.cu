@@ -173,6 +173,7 @@ __device__ __forceinline__ bool mma_wait(uint64_t* mbar, uint32_t parity, long l
 template <class T, int NTHR = kGemmThreads>
 struct AChunk {
   T v[1024 / NTHR][4];
+  unsigned none;  // bit it: item it has no element (a lane past the last, or four k past K)
 };
 
 // A thread's items are the same in every chunk of a tile: item it of thread
@@ -233,6 +234,10 @@ __device__ __forceinline__ void a_load(AChunk<T, NTHR>& a, const ATile<T, NTHR>&
                                        int tid) {
   constexpr int kItems = 1024 / NTHR;
   const int o = k0 * t.es;
+  a.none = 0;
+#pragma unroll
+  for (int it = 0; it < kItems; it++)
+    if (t.src[it] == nullptr) a.none |= 1u << it;
   if (k0 + kGemmKC <= K) {
     if (t.vec) {
 #pragma unroll
@@ -266,6 +271,7 @@ __device__ __forceinline__ void a_load(AChunk<T, NTHR>& a, const ATile<T, NTHR>&
       int l, kq;
       item_lane_quad(tid + NTHR * it, lane_fast, l, kq);
       const T* p = t.src[it];
+      if (k0 + kq * 4 >= K) a.none |= 1u << it;
 #pragma unroll
       for (int e = 0; e < 4; e++) {
         const int k = k0 + kq * 4 + e;
@@ -285,10 +291,10 @@ __device__ __forceinline__ void a_store(const AChunk<T, NTHR>& a, const ATile<T,
 #pragma unroll
   for (int it = 0; it < kItems; it++) {
     float4 hi, lo;
-    if (t.src[it] == nullptr) {
-      // a lane past the last: zeros, without the conversions (in integer
-      // operations a zero takes longer than a value: one lane of 127, 16.4 us with
-      // FP64 conversions, 18.4 with integer ones, 14.4 with this)
+    if ((a.none >> it) & 1u) {
+      // zeros, without the conversions (in integer operations a zero takes longer
+      // than a value: one lane of 127, 16.4 us with FP64 conversions, 18.4 with
+      // integer ones, 14.4 with this)
       hi = lo = make_float4(0.f, 0.f, 0.f, 0.f);
     } else {
       float x;
