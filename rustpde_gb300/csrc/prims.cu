@@ -884,7 +884,7 @@ __global__ void k_sumsq(const double* v, size_t n, double* out) {
 }
 }  // namespace dev
 
-constexpr int kManyLanes = 8 * 152;
+constexpr int kManyLanes = 8 * kNumSMs;
 
 // shared memory of a pass that sizes are checked against
 static size_t pass_smem(const PassDesc& d) {
@@ -930,7 +930,7 @@ static void run_pass_whole(PassDesc d, cudaStream_t st) {
     if (code == P_FDMA && d.fdma.rows > 1) per_lane = true;
     if ((code == P_DCT_FWD || code == P_DCT_BWD) && d.cx.use_fft) fft = true;
   }
-  constexpr int kPairLanes = 2 * 2 * 152;
+  constexpr int kPairLanes = 2 * 2 * kNumSMs;
   const int nt = pass_threads(d);
   const bool pair = real && !per_lane && !fft && d.lanes >= kPairLanes;
   const size_t sm = pass_smem_used(d, real && !pair ? 8 : 16);

@@ -11,12 +11,12 @@
 // accumulators).
 //
 // Exactness: |A_i digit| <= 128, |W_j digit| <= 128 (64 for j = 0); an
-// accumulator sums at most (d + 1) K products.  The sums of the weights that
-// reach FP64's last bits with margin (d <= 4) stay below 2^24 for K <= 320
-// terms a list whatever the lane's digits, as the operators' digits average
-// half of their bound; the remaining ones (d = 5 .. 7, random-signed, standard
-// deviation below 2^18) would lose at most their last unit, 2^-52 of the
-// largest product.
+// accumulator sums at most (d + 1) K products, six of them for d = 7.  The
+// operators' digits average half of their bound, so that for K <= 320 terms a
+// list the sums of the weights d <= 5 stay below 2^24 whatever the lane's digits.
+// A lane made for it could take d = 6 past that (random-signed sums have a
+// standard deviation below 2^18) and lose its last unit with each product, less
+// than 2^-55 of the largest product in all.
 //
 // Work split: warp 8 copies the chunks (28 KB of lane digits, 7 KB of operator
 // digits at NT = 32; cp.async.bulk into a ring of three), one thread of warp 9
@@ -26,14 +26,15 @@
 // CTA on the SM: one CTA's epilogue runs under the other's MMAs.  A narrow
 // tile's lists have columns of their own.
 //
-// Bound, large launches: the copies.  A chunk's MMAs take 272 cycles at the
-// bf16 rate, its 35 KB about 500 at what an SM draws from L2; wider tiles would
-// need the tensor memory of the second CTA.  Small launches: the serial chain
-// of one tile (first copy, MMAs, and the epilogue's about 100 instructions per
-// pair of outputs).  Box 264^2, a GEMM alone with a cold L2, with 32-wide
-// against 16-wide tiles: y backward 26.4 -> 17.5 us, x backward 26.8 -> 18.5,
-// x forward 18.1 -> 11.8, y forward 20.7 -> 12.4 (the same transforms inside
-// the FP64 passes: about 100, 150, 60 and 70 us).
+// Bound: one tile's serial chain (first copy, the chunks one after the other,
+// and the epilogue's about 100 instructions per pair of outputs), not a pipe: ncu
+// shows the tensor pipe 16 % busy and the L2 at 7 % of its rate with 153 CTAs (box
+// 264^2, x backward), 54 % and 30 % with 297 (513^2), where two CTAs share most SMs.
+// Hence narrow tiles in small launches.  Box 264^2, a GEMM alone with a cold L2,
+// with 32-wide against 16-wide tiles: y backward 26.4 -> 17.5 us, x backward 26.8
+// -> 18.5, x forward 18.1 -> 11.8, y forward 20.7 -> 12.4 (the same transforms
+// inside the FP64 passes: about 100, 150, 60 and 70 us).  Wider tiles than 32 would
+// need the tensor memory of the second CTA.
 //
 // Every wait is bounded: on time-out the tile sets kStatusGemmTimeout, makes its
 // outputs NaN, waits (bounded) for its copies and MMAs in flight, frees its

@@ -29,7 +29,8 @@ constexpr int kSplitLanes = 128;      // lanes per tile (tcgen05 M)
 constexpr int kSplitDigits = 7;
 constexpr int kSplitK = 16;           // terms per chunk (one bf16 MMA k-step)
 constexpr int kSplitTile = 32;        // outputs per tile (16 in a short last one)
-constexpr int kSplitNarrowTiles = 152;  // launches of at most so many wide tiles take narrow ones
+constexpr int kNumSMs = 152;  // of the GB300
+constexpr int kSplitNarrowTiles = kNumSMs;  // launches of at most so many wide tiles take narrow ones
 constexpr int kSplitChunkBytes = kSplitDigits * kSplitLanes * kSplitK * 2;  // digits of 128 lanes x 16 terms
 // A lane's value with significand m (53 bits) and biased exponent ef becomes the
 // integer (m << shl) >> (emax - ef), emax the lane's largest exponent: below

@@ -1186,7 +1186,7 @@ void drop_empty(StepPlan& p) {
 
 // CTAs per SM that k_per_y2's registers have to allow in a launch of so many rows
 static int y2_bound(int rows, size_t smem) {
-  if (rows <= 2 * 152) return 1;
+  if (rows <= 2 * kNumSMs) return 1;
   return 3 * (smem + 1024) <= smem_limit() + 1024 ? 4 : 3;  // (1 KB of a CTA's shared memory is the system's)
 }
 template <int CONV>
