@@ -203,8 +203,9 @@ const char* rbc_kernel_name(int kernel);
  * entry; an empty part is left to the autotuner.  FP64 passes: 0 a CTA per
  * lane, 1 128-thread CTAs, 2 one thread per sub-lane, 3 the same with the
  * periodic Y2 launches fused into one.  GEMM passes: 0 output tiles of up to
- * 64 columns, 4 up to 128, 5 64 in the warp-specialised form (producer, MMA
- * and flush warps; all 0 when the part is missing).  Groups: mixed-
+ * 64 columns from packed input, 4 up to 128 without packing, 5 64 in the
+ * warp-specialised form (producer, MMA and flush warps; all 0 when the part is
+ * missing).  The results do not depend on the GEMM forms.  Groups: mixed-
  * precision cases whose Chebyshev lengths are all 2^p + 1 are grouped apart,
  * and each such group runs its transforms as tensor-core GEMMs (0) or as the
  * FP64 plan's FFT butterflies (1; at least as accurate), whichever its step
